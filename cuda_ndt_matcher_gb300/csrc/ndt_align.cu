@@ -678,7 +678,7 @@ __device__ __forceinline__ int search_point(const MapView& m, const uint32_t* of
             inb[k] = (lz >> m.bits[2]) == 0u;
             key[k] = kxy | (lz << bxy);
             home[k] = mix32(key[k]) & m.mask;
-            sv[k] = inb[k] ? __ldg(m.slots + home[k]) : make_uint4(EMPTY_KEY, 0u, 0u, 0u);
+            sv[k] = inb[k] ? __ldg(m.slots + home[k]) : make_uint4(0u, 0u, 0u, EMPTY_KEY);
         }
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
@@ -686,14 +686,14 @@ __device__ __forceinline__ int search_point(const MapView& m, const uint32_t* of
             if (!inb[k]) continue;
             uint4 v = sv[k];
             int32_t s = (int32_t)home[k];
-            if (v.x != key[k]) {
-                if (v.x == EMPTY_KEY) continue;
+            if (v.w != key[k]) {
+                if (v.w == EMPTY_KEY) continue;
                 s = probe_next(m, key[k], home[k], &v);
                 if (s < 0) continue;
             }
-            const float e0 = (qh[0] - __uint_as_float(v.y)) + ql[0];
-            const float e1 = (qh[1] - __uint_as_float(v.z)) + ql[1];
-            const float e2 = (qh[2] - __uint_as_float(v.w)) + ql[2];
+            const float e0 = (qh[0] - __uint_as_float(v.x)) + ql[0];
+            const float e1 = (qh[1] - __uint_as_float(v.y)) + ql[1];
+            const float e2 = (qh[2] - __uint_as_float(v.z)) + ql[2];
             if (fmaf(e0, e0, fmaf(e1, e1, e2 * e2)) > m.r2) continue;
             nbl[cnt * nbl_stride] = (uint32_t)s;
             cnt++;
@@ -707,24 +707,34 @@ __device__ __forceinline__ int search_point(const MapView& m, const uint32_t* of
 // (J^T M J blocks A_HTR.., A_HRR..) in the thread's shared-memory column sacc[k * nbl_stride]
 // (they change once per point; keeping them out of registers leaves the search and pair
 // work room without spilling to local memory)
+// What one point's listed voxels add up to
+struct PointSums {
+    float S, G0, G1, G2, M0, M1, M2, M3, M4, M5;
+};
+
 template <bool CPU_SEM>
-__device__ __forceinline__ void point_pairs(const MapView& m, const float* pv, const float* qh,
-                                            const float* ql, int cnt, const float* fr,
-                                            float d1f, float d2f, float* acc, float* sacc,
-                                            int& ncorr, const uint32_t* nbl, int nbl_stride);
+__device__ __forceinline__ void pair_terms(const MapView& m, const float* qh, const float* ql,
+                                           int cnt, float d1f, float d2f, const uint32_t* list,
+                                           int stride, PointSums& p);
+__device__ __forceinline__ void point_contract(const float* pv, const float* fr,
+                                               const PointSums& p, float* acc, float* sacc,
+                                               int stride);
 
 template <bool CPU_SEM>
 __device__ __forceinline__ void point_terms(const MapView& m, const uint32_t* off27,
                                             float px, float py, float pz,
                                             const float* fr, int max_nb, float d1f, float d2f,
-                                            float* acc, float* sacc, int& ncorr, uint32_t* nbl,
-                                            int nbl_stride) {
+                                            float* acc, float* sacc, int& ncorr, uint32_t* list,
+                                            int stride) {
     const float pv[3] = {px, py, pz};
     float qh[3], ql[3];
     transform_point(fr, pv, qh, ql);
-    const int cnt = search_point(m, off27, qh, ql, max_nb, nbl, nbl_stride);
+    const int cnt = search_point(m, off27, qh, ql, max_nb, list, stride);
     if (cnt == 0) return;
-    point_pairs<CPU_SEM>(m, pv, qh, ql, cnt, fr, d1f, d2f, acc, sacc, ncorr, nbl, nbl_stride);
+    PointSums p{};
+    pair_terms<CPU_SEM>(m, qh, ql, cnt, d1f, d2f, list, stride, p);
+    ncorr += cnt;
+    point_contract(pv, fr, p, acc, sacc, stride);
 }
 
 // Neighbour search of the points of a group of NPW lanes, the lanes sharing each point's
@@ -737,8 +747,8 @@ __device__ __forceinline__ void point_terms(const MapView& m, const uint32_t* of
 template <int NPW>
 __device__ __forceinline__ int search_group(const MapView& m, const uint32_t* off27,
                                             const float* qh, const float* ql, uint32_t bits,
-                                            uint32_t corner, int max_nb, uint32_t* nbl,
-                                            int nbl_stride, int lane) {
+                                            uint32_t corner, int max_nb, uint32_t* list,
+                                            int stride, int lane) {
     const int g0 = lane & ~(NPW - 1), j = lane & (NPW - 1);
     int my_cnt = 0;
 #pragma unroll 1
@@ -772,12 +782,12 @@ __device__ __forceinline__ int search_group(const MapView& m, const uint32_t* of
 #pragma unroll
         for (int o = 1; o < NPW; o <<= 1) accm |= __shfl_xor_sync(0xffffffffu, accm, o);
         if (lane == src) {
-            // the point's lane lists its accepted voxels in order (slots re-read: L1 hits)
+            // the point's lane lists its accepted voxels in order (entries re-read: L1 hits)
             int c = 0;
             uint32_t mm = accm;
             while (mm != 0u && c < max_nb) {
                 const uint32_t b = (uint32_t)(__ffs(mm) - 1);
-                nbl[c * nbl_stride] = (uint32_t)__float_as_int(
+                list[c * stride] = (uint32_t)__float_as_int(
                     __ldg(reinterpret_cast<const float*>(m.grid + (cq + off27[b])) + 3));
                 mm &= mm - 1u;
                 ++c;
@@ -788,35 +798,25 @@ __device__ __forceinline__ int search_group(const MapView& m, const uint32_t* of
     return my_cnt;
 }
 
+// The voxels of a list: S, G, M of the point. e = exp(-d2 sq / 2) is 2^(k2 sq) with
+// k2 = -d2 log2(e) / 2 carried as two floats (the constant -log2(e) / 2 split into two floats,
+// then an exact product split: k2h + k2l), so the argument is as accurate as the product d2 sq
+// itself: two operations and the base-2 exponential per pair.
 template <bool CPU_SEM>
-__device__ __forceinline__ void point_pairs(const MapView& m, const float* pv, const float* qh,
-                                            const float* ql, int cnt, const float* fr,
-                                            float d1f, float d2f, float* acc, float* sacc,
-                                            int& ncorr, const uint32_t* nbl, int nbl_stride) {
-    // ---- pairs: S, G, M aggregated over the listed voxels
-    float S = 0.f, G0 = 0.f, G1 = 0.f, G2 = 0.f;
-    float M0 = 0.f, M1 = 0.f, M2 = 0.f, M3 = 0.f, M4 = 0.f, M5 = 0.f;
+__device__ __forceinline__ void pair_terms(const MapView& m, const float* qh, const float* ql,
+                                           int cnt, float d1f, float d2f, const uint32_t* list,
+                                           int stride, PointSums& p) {
     const float d1d2 = d1f * d2f;
-    // e = exp(-d2 sq / 2) as 2^(k2 sq) with k2 = -d2 log2(e) / 2 carried as two floats (the
-    // constant -log2(e) / 2 split into two floats, then an exact product split: k2h + k2l), so the
-    // argument is as accurate as the product d2 sq itself: two operations and the base-2
-    // exponential per pair
     const float k2h = d2f * -0.72134751081466674805f;
     const float k2l = fmaf(d2f, -0.72134751081466674805f, -k2h) + d2f * -9.6298151675000554e-09f;
 #pragma unroll 1
     for (int j = 0; j < cnt; ++j) {
-        const uint32_t s = nbl[j * nbl_stride];
-        const uint4 v = __ldg(m.slots + s);
-        const float4 ca = __ldg(m.slot_icov + 2 * (size_t)s);
-        const float4 cb = __ldg(m.slot_icov + 2 * (size_t)s + 1);
-        const float x0 = (qh[0] - __uint_as_float(v.y)) + ql[0];
-        const float x1 = (qh[1] - __uint_as_float(v.z)) + ql[1];
-        const float x2 = (qh[2] - __uint_as_float(v.w)) + ql[2];
-        // C = [[ca.x ca.y ca.z] [ca.y ca.w cb.x] [ca.z cb.x cb.y]]
-        const float c0 = fmaf(ca.x, x0, fmaf(ca.y, x1, ca.z * x2));
-        const float c1 = fmaf(ca.y, x0, fmaf(ca.w, x1, cb.x * x2));
-        const float c2 = fmaf(ca.z, x0, fmaf(cb.x, x1, cb.y * x2));
-        const float sq = fmaf(x0, c0, fmaf(x1, c1, x2 * c2));
+        float x[3], C[6];
+        load_voxel(m, list[j * stride], qh, ql, x, C);
+        const float c0 = fmaf(C[0], x[0], fmaf(C[1], x[1], C[2] * x[2]));
+        const float c1 = fmaf(C[1], x[0], fmaf(C[3], x[1], C[4] * x[2]));
+        const float c2 = fmaf(C[2], x[0], fmaf(C[4], x[1], C[5] * x[2]));
+        const float sq = fmaf(x[0], c0, fmaf(x[1], c1, x[2] * c2));
         const float e = exp2f(fmaf(k2h, sq, k2l * sq));
         if (CPU_SEM) {
             const float wn = d2f * e;  // compute_derivative_single: zero unless d2*e in [0,1]
@@ -824,24 +824,28 @@ __device__ __forceinline__ void point_pairs(const MapView& m, const float* pv, c
         }
         const float w = d1d2 * e;
         const float wd = w * d2f;
-        S = fmaf(-d1f, e, S);
-        G0 = fmaf(w, c0, G0);
-        G1 = fmaf(w, c1, G1);
-        G2 = fmaf(w, c2, G2);
+        p.S = fmaf(-d1f, e, p.S);
+        p.G0 = fmaf(w, c0, p.G0);
+        p.G1 = fmaf(w, c1, p.G1);
+        p.G2 = fmaf(w, c2, p.G2);
         // M += w C - wd c c^T, as two multiply-adds per entry
         const float u0 = wd * c0, u1 = wd * c1, u2 = wd * c2;
-        M0 = fmaf(-u0, c0, fmaf(w, ca.x, M0));
-        M1 = fmaf(-u0, c1, fmaf(w, ca.y, M1));
-        M2 = fmaf(-u0, c2, fmaf(w, ca.z, M2));
-        M3 = fmaf(-u1, c1, fmaf(w, ca.w, M3));
-        M4 = fmaf(-u1, c2, fmaf(w, cb.x, M4));
-        M5 = fmaf(-u2, c2, fmaf(w, cb.y, M5));
+        p.M0 = fmaf(-u0, c0, fmaf(w, C[0], p.M0));
+        p.M1 = fmaf(-u0, c1, fmaf(w, C[1], p.M1));
+        p.M2 = fmaf(-u0, c2, fmaf(w, C[2], p.M2));
+        p.M3 = fmaf(-u1, c1, fmaf(w, C[3], p.M3));
+        p.M4 = fmaf(-u1, c2, fmaf(w, C[4], p.M4));
+        p.M5 = fmaf(-u2, c2, fmaf(w, C[5], p.M5));
     }
-    if (cnt == 0) return;
-    ncorr += cnt;
-    const float G[3] = {G0, G1, G2};
-    const float Ms[3][3] = {{M0, M1, M2}, {M1, M3, M4}, {M2, M4, M5}};
-    acc[A_SC] += S;
+}
+
+// A point's sums contracted with its Jacobian into the accumulators
+__device__ __forceinline__ void point_contract(const float* pv, const float* fr,
+                                               const PointSums& p, float* acc, float* sacc,
+                                               int stride) {
+    const float G[3] = {p.G0, p.G1, p.G2};
+    const float Ms[3][3] = {{p.M0, p.M1, p.M2}, {p.M1, p.M3, p.M4}, {p.M2, p.M4, p.M5}};
+    acc[A_SC] += p.S;
     // J_k = A_k p, MJ_k = M J_k
     float J[3][3], MJ[3][3];
 #pragma unroll
@@ -861,20 +865,20 @@ __device__ __forceinline__ void point_pairs(const MapView& m, const float* pv, c
 #pragma unroll
         for (int b = 0; b < 3; ++b) acc[A_GP + 3 * a + b] = fmaf(G[a], pv[b], acc[A_GP + 3 * a + b]);
 #pragma unroll
-        for (int k = 0; k < 3; ++k) sacc[(3 * a + k) * nbl_stride] += MJ[k][a];
+        for (int k = 0; k < 3; ++k) sacc[(3 * a + k) * stride] += MJ[k][a];
     }
-    acc[A_M + 0] += M0;
-    acc[A_M + 1] += M1;
-    acc[A_M + 2] += M2;
-    acc[A_M + 3] += M3;
-    acc[A_M + 4] += M4;
-    acc[A_M + 5] += M5;
+    acc[A_M + 0] += p.M0;
+    acc[A_M + 1] += p.M1;
+    acc[A_M + 2] += p.M2;
+    acc[A_M + 3] += p.M3;
+    acc[A_M + 4] += p.M4;
+    acc[A_M + 5] += p.M5;
     int kl = 0;
 #pragma unroll
     for (int k = 0; k < 3; ++k)
 #pragma unroll
         for (int l = k; l < 3; ++l, ++kl) {
-            float& h = sacc[(A_HRR - A_HTR + kl) * nbl_stride];
+            float& h = sacc[(A_HRR - A_HTR + kl) * stride];
             h = fmaf(J[k][0], MJ[l][0], fmaf(J[k][1], MJ[l][1], fmaf(J[k][2], MJ[l][2], h)));
         }
 }
@@ -888,28 +892,22 @@ template <bool CPU_SEM>
 __device__ __forceinline__ void point_terms_ls(const MapView& m, const uint32_t* off27,
                                                float px, float py, float pz,
                                                const float* fr, int max_nb, float d1f, float d2f,
-                                               float* a, int& ncorr, uint32_t* nbl,
-                                               int nbl_stride) {
+                                               float* a, int& ncorr, uint32_t* list, int stride) {
     const float pv[3] = {px, py, pz};
     float qh[3], ql[3];
     transform_point(fr, pv, qh, ql);
-    const int cnt = search_point(m, off27, qh, ql, max_nb, nbl, nbl_stride);
+    const int cnt = search_point(m, off27, qh, ql, max_nb, list, stride);
     if (cnt == 0) return;
     float S = 0.f, G[3] = {0.f, 0.f, 0.f};
     const float d1d2 = d1f * d2f;
 #pragma unroll 1
     for (int j = 0; j < cnt; ++j) {
-        const uint32_t s = nbl[j * nbl_stride];
-        const uint4 v = __ldg(m.slots + s);
-        const float4 ca = __ldg(m.slot_icov + 2 * (size_t)s);
-        const float4 cb = __ldg(m.slot_icov + 2 * (size_t)s + 1);
-        const float x0 = (qh[0] - __uint_as_float(v.y)) + ql[0];
-        const float x1 = (qh[1] - __uint_as_float(v.z)) + ql[1];
-        const float x2 = (qh[2] - __uint_as_float(v.w)) + ql[2];
-        const float c0 = fmaf(ca.x, x0, fmaf(ca.y, x1, ca.z * x2));
-        const float c1 = fmaf(ca.y, x0, fmaf(ca.w, x1, cb.x * x2));
-        const float c2 = fmaf(ca.z, x0, fmaf(cb.x, x1, cb.y * x2));
-        const float sq = fmaf(x0, c0, fmaf(x1, c1, x2 * c2));
+        float x[3], C[6];
+        load_voxel(m, list[j * stride], qh, ql, x, C);
+        const float c0 = fmaf(C[0], x[0], fmaf(C[1], x[1], C[2] * x[2]));
+        const float c1 = fmaf(C[1], x[0], fmaf(C[3], x[1], C[4] * x[2]));
+        const float c2 = fmaf(C[2], x[0], fmaf(C[4], x[1], C[5] * x[2]));
+        const float sq = fmaf(x[0], c0, fmaf(x[1], c1, x[2] * c2));
         const float e = expf(-0.5f * d2f * sq);
         if (CPU_SEM) {
             const float wn = d2f * e;  // compute_derivative_single: zero unless d2*e in [0,1]
@@ -1448,11 +1446,11 @@ __global__ void __launch_bounds__(THREADS, 65536 / (THREADS * REGCAP))
     constexpr int NW = THREADS / 32;
     __shared__ AlignShared sh;
     __shared__ uint32_t s_off27[32];  // neighbour offsets of the dense index
-    // dynamic shared memory: [max_nb][THREADS] accepted slots per thread, then the trailing
+    // dynamic shared memory: [max_nb][THREADS] listed records per thread, then the trailing
     // NACC - A_HTR accumulators [NACC - A_HTR][THREADS], then the line search's warp sums
-    extern __shared__ uint32_t nbl_smem[];
+    extern __shared__ uint32_t list_smem[];
     float* const sacc =
-        reinterpret_cast<float*>(nbl_smem + (size_t)P.max_nb * THREADS) + threadIdx.x;
+        reinterpret_cast<float*>(list_smem + (size_t)P.max_nb * THREADS) + threadIdx.x;
     cg::cluster_group cluster = cg::this_cluster();
     const int K = P.cluster;
     const int rank = (int)cluster.block_rank();
@@ -1507,7 +1505,7 @@ __global__ void __launch_bounds__(THREADS, 65536 / (THREADS * REGCAP))
                   pz = __ldg(pts + 3 * (size_t)i + 2);
             if (!(isfinite(px) && isfinite(py) && isfinite(pz))) continue;
             point_terms<CPU_SEM>(m, s_off27, px, py, pz, fr, P.max_nb, P.d1f, P.d2f, acc, sacc, nc,
-                                 nbl_smem + tid, THREADS);
+                                 list_smem + tid, THREADS);
         }
 #pragma unroll
         for (int k = 0; k < NACC - A_HTR; ++k) acc[A_HTR + k] = sacc[k * THREADS];
@@ -1636,7 +1634,7 @@ __global__ void __launch_bounds__(THREADS, 65536 / (THREADS * REGCAP))
             // rank's points, one candidate after another; FP64 warp sums of each candidate
             // kept in shared memory, summed over the CTA, then over the cluster by rank 0
             double* lsw = reinterpret_cast<double*>(
-                nbl_smem + (size_t)(P.max_nb + NACC - A_HTR) * THREADS);
+                list_smem + (size_t)(P.max_nb + NACC - A_HTR) * THREADS);
             for (int c = c_lo; c < c_hi; ++c) {
                 float a[LS_VALS];
 #pragma unroll
@@ -1648,7 +1646,7 @@ __global__ void __launch_bounds__(THREADS, 65536 / (THREADS * REGCAP))
                           pz = __ldg(pts + 3 * (size_t)i + 2);
                     if (!(isfinite(px) && isfinite(py) && isfinite(pz))) continue;
                     point_terms_ls<CPU_SEM>(m, s_off27, px, py, pz, sh.ls_fr[c], P.max_nb, P.d1f,
-                                            P.d2f, a, lc, nbl_smem + tid, THREADS);
+                                            P.d2f, a, lc, list_smem + tid, THREADS);
                 }
                 double* wout = lsw + ((size_t)warp * LS_MAX + c) * LS_VALS;
                 warp_sum16(a, lane, LS_USED - 1, wout);
@@ -2082,9 +2080,9 @@ __global__ void __launch_bounds__(THREADS, 65536 / (THREADS * REGCAP))
     __shared__ int s_job, s_lw, s_flag;
     __shared__ uint32_t s_chunk, s_gen, s_nch;
     // dynamic shared memory as in k_ndt_align: neighbour lists, then the trailing accumulators
-    extern __shared__ uint32_t nbl_smem[];
+    extern __shared__ uint32_t list_smem[];
     float* const sacc =
-        reinterpret_cast<float*>(nbl_smem + (size_t)P.max_nb * THREADS) + threadIdx.x;
+        reinterpret_cast<float*>(list_smem + (size_t)P.max_nb * THREADS) + threadIdx.x;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const MapView& m = P.map;
     const uint32_t B = P.num_jobs;
@@ -2095,7 +2093,7 @@ __global__ void __launch_bounds__(THREADS, 65536 / (THREADS * REGCAP))
     // boundary, up to 3 points early)
     __shared__ __align__(8) uint64_t s_stage_bar;
     float* const stage =
-        reinterpret_cast<float*>(nbl_smem + (size_t)(P.max_nb + NACC - A_HTR) * THREADS);
+        reinterpret_cast<float*>(list_smem + (size_t)(P.max_nb + NACC - A_HTR) * THREADS);
     uint32_t stage_phase = 0;
     if (tid == 0) {
         s_lw = 0;
@@ -2316,11 +2314,14 @@ __global__ void __launch_bounds__(THREADS, 65536 / (THREADS * REGCAP))
                     }
                 }
                 const int cnt = search_group<NPW>(m, s_off27, qh, ql, bits, corner, P.max_nb,
-                                                  nbl_smem + tid, THREADS, lane);
+                                                  list_smem + tid, THREADS, lane);
                 __syncwarp();  // the group's list entries are visible to the point's lane
-                if (cnt > 0)
-                    point_pairs<CPU_SEM>(m, pv, qh, ql, cnt, sh.fr, P.d1f, P.d2f, acc, sacc, nc,
-                                         nbl_smem + tid, THREADS);
+                if (cnt > 0) {
+                    PointSums ps{};
+                    pair_terms<CPU_SEM>(m, qh, ql, cnt, P.d1f, P.d2f, list_smem + tid, THREADS, ps);
+                    nc += cnt;
+                    point_contract(pv, sh.fr, ps, acc, sacc, THREADS);
+                }
                 __syncwarp();  // lists are read before the next round rewrites them
             }
         } else {
@@ -2329,7 +2330,7 @@ __global__ void __launch_bounds__(THREADS, 65536 / (THREADS * REGCAP))
                 load_point(i, pv);
                 if (!(isfinite(pv[0]) && isfinite(pv[1]) && isfinite(pv[2]))) continue;
                 point_terms<CPU_SEM>(m, s_off27, pv[0], pv[1], pv[2], sh.fr, P.max_nb, P.d1f,
-                                     P.d2f, acc, sacc, nc, nbl_smem + tid, THREADS);
+                                     P.d2f, acc, sacc, nc, list_smem + tid, THREADS);
             }
         }
 #pragma unroll
@@ -2449,7 +2450,7 @@ static int launch_t(const AlignParams& p, int K, cudaStream_t s) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(p.num_jobs * K, 1, 1);
     cfg.blockDim = dim3(T, 1, 1);
-    // [max_nb][T] neighbour lists, [NACC - A_HTR][T] accumulators, then (line search)
+    // [max_nb][T] voxel lists, [NACC - A_HTR][T] accumulators, then (line search)
     // [T/32][LS_MAX][LS_VALS] FP64 warp sums; the first two are multiples of 8 bytes (T is)
     cfg.dynamicSmemBytes = (size_t)T * (p.max_nb + NACC - A_HTR) * sizeof(uint32_t) +
                            (p.ls_cands > 0 ? (size_t)(T / 32) * LS_MAX * LS_VALS * sizeof(double)

@@ -205,7 +205,7 @@ struct ndt_ctx {
     cudaEvent_t ev_in0 = nullptr, ev_in1 = nullptr;  // counter reset / last chunk copied
     Map map;
     BuildScratch bs;
-    DevBuf d_in, d_jobs, d_aout, d_sjobs, d_sout, d_part, d_status, d_q, d_qidx, d_qcnt;
+    DevBuf d_in, d_jobs, d_aout, d_sjobs, d_sout, d_part, d_sdone, d_status, d_q, d_qidx, d_qcnt;
     PinBuf h_pts, h_jobs, h_aout, h_sjobs, h_sout, h_misc, h_arrive;
     double d1 = 0, d2 = 0;
     ndt_stats stats{};
@@ -258,6 +258,16 @@ struct ndt_ctx {
 static void async_drain(ndt_ctx* c) {
     for (auto& s : c->slots)
         if (s.ticket && s.ctx) cudaStreamSynchronize(s.ctx->stream);
+}
+
+// Scoring workspace of nj jobs of at most max_n points: partials, and one finished-block
+// counter per job, zero at allocation and left at zero by every launch.
+static int score_reserve(ndt_ctx* c, uint32_t nj, uint32_t max_n) {
+    int rc = dev_reserve(c->d_part, score_part_bytes(nj, max_n));
+    if (rc || (size_t)nj * 4 <= c->d_sdone.bytes) return rc;
+    if ((rc = dev_reserve(c->d_sdone, (size_t)nj * 4))) return rc;
+    return cuda_fail(cudaMemsetAsync(c->d_sdone.p, 0, c->d_sdone.bytes, c->stream),
+                     "score counters");
 }
 
 // Finishes a background rebuild: joins its thread and, when it succeeded, makes the standby
@@ -504,7 +514,7 @@ int ndt_ctx_destroy(ndt_ctx* c) {
                       &c->bs_tile.seg_starts, &c->bs_tile.seg_valid, &c->bs_tile.seg_rank,
                       &c->bs_tile.seg_rec, &c->bs_tile.small, &c->d_tile_refs})
         dev_free(*b);
-    for (DevBuf* b : {&c->map_b.slots, &c->map_b.slot_icov, &c->map_b.slot_vidx, &c->map_b.grid,
+    for (DevBuf* b : {&c->map_b.slots, &c->map_b.icov8, &c->map_b.slot_vidx, &c->map_b.grid,
                       &c->map_b.nmask,
                       &c->map_b.vox_coord, &c->map_b.vox_mean, &c->map_b.vox_cov,
                       &c->map_b.vox_icov, &c->map_b.vox_count, &c->bs_b.keys_a, &c->bs_b.keys_b,
@@ -514,14 +524,14 @@ int ndt_ctx_destroy(ndt_ctx* c) {
         dev_free(*b);
     if (c->bstream) cudaStreamDestroy(c->bstream);
     drop_graphs(c);
-    for (DevBuf* b : {&c->map.slots, &c->map.slot_icov, &c->map.slot_vidx, &c->map.grid,
+    for (DevBuf* b : {&c->map.slots, &c->map.icov8, &c->map.slot_vidx, &c->map.grid,
                       &c->map.nmask,
                       &c->map.vox_coord,
                       &c->map.vox_mean, &c->map.vox_cov, &c->map.vox_icov, &c->map.vox_count,
                       &c->bs.keys_a, &c->bs.keys_b, &c->bs.vals_a, &c->bs.vals_b, &c->bs.tmp,
                       &c->bs.seg_ids, &c->bs.seg_starts, &c->bs.seg_valid, &c->bs.seg_rank,
                       &c->bs.seg_rec, &c->bs.small, &c->d_in, &c->d_jobs, &c->d_aout,
-                      &c->d_sjobs, &c->d_sout, &c->d_part, &c->d_status, &c->d_q, &c->d_qidx,
+                      &c->d_sjobs, &c->d_sout, &c->d_part, &c->d_sdone, &c->d_status, &c->d_q, &c->d_qidx,
                       &c->d_qcnt, &c->d_trace, &c->d_qjobs, &c->d_qctl, &c->d_qframe,
                       &c->d_qpart, &c->d_qoff})
         dev_free(*b);
@@ -914,8 +924,7 @@ static int run_align_enqueue(ndt_ctx* c, const float* d_pts, std::vector<AlignJo
            sob = nj * sizeof(ScoreOut);
     if ((rc = dev_reserve(c->d_jobs, jb)) || (rc = dev_reserve(c->d_aout, ob)) ||
         (rc = dev_reserve(c->d_sjobs, sjb)) || (rc = dev_reserve(c->d_sout, sob)) ||
-        (rc = dev_reserve(c->d_part, score_part_bytes(nj, max_n))) ||
-        (rc = pin_reserve(c->h_jobs, jb + sjb)) || (rc = pin_reserve(c->h_aout, ob + sob + 16)))
+        (rc = score_reserve(c, nj, max_n)) || (rc = pin_reserve(c->h_jobs, jb + sjb)) || (rc = pin_reserve(c->h_aout, ob + sob + 16)))
         return rc;
     AlignJob* hj = (AlignJob*)c->h_jobs.p;
     ScoreJob* hs = (ScoreJob*)((char*)c->h_jobs.p + jb);
@@ -1061,8 +1070,8 @@ static int run_align_enqueue(ndt_ctx* c, const float* d_pts, std::vector<AlignJo
             cudaEventRecordWithFlags(c->ev1, st, evf);
         }
         r = launch_score(c->map.view, d_pts, (const ScoreJob*)c->d_sjobs.p, nj, max_n,
-                         (const AlignOut*)c->d_aout.p, c->d_part.p, (ScoreOut*)c->d_sout.p,
-                         (float)c->d1, (float)c->d2, st);
+                         (const AlignOut*)c->d_aout.p, c->d_part.p, (uint32_t*)c->d_sdone.p,
+                         (ScoreOut*)c->d_sout.p, (float)c->d1, (float)c->d2, st);
         if (r) return r;
         cudaEventRecordWithFlags(c->ev2, st, evf);
         cudaMemcpyAsync(ho, c->d_aout.p, ob, cudaMemcpyDeviceToHost, st);
@@ -1080,6 +1089,7 @@ static int run_align_enqueue(ndt_ctx* c, const float* d_pts, std::vector<AlignJo
             c->map_gen, c->cfg_gen, (uint64_t)(uintptr_t)d_pts, (uint64_t)(uintptr_t)c->d_jobs.p,
             (uint64_t)(uintptr_t)c->d_aout.p, (uint64_t)(uintptr_t)c->d_sjobs.p,
             (uint64_t)(uintptr_t)c->d_sout.p, (uint64_t)(uintptr_t)c->d_part.p,
+            (uint64_t)(uintptr_t)c->d_sdone.p,
             (uint64_t)(uintptr_t)c->h_jobs.p, (uint64_t)(uintptr_t)c->h_aout.p};
         size_t gi = c->graphs.size();
         for (size_t i = 0; i < c->graphs.size(); ++i)
@@ -1929,7 +1939,7 @@ int ndt_eval_batch(ndt_ctx* c, const float* xyz, uint64_t n, const double* T34, 
     size_t sjb = m * sizeof(ScoreJob), sob = m * sizeof(ScoreOut);
     if ((rc = pin_reserve(c->h_pts, n * 12 + 16)) || (rc = dev_reserve(c->d_in, n * 12 + 16)) ||
         (rc = dev_reserve(c->d_sjobs, sjb)) || (rc = dev_reserve(c->d_sout, sob)) ||
-        (rc = dev_reserve(c->d_part, score_part_bytes((uint32_t)m, (uint32_t)n))) ||
+        (rc = score_reserve(c, (uint32_t)m, (uint32_t)n)) ||
         (rc = pin_reserve(c->h_sjobs, sjb)) || (rc = pin_reserve(c->h_sout, sob)))
         return rc;
     if (n) std::memcpy(c->h_pts.p, xyz, n * 12);
@@ -1948,8 +1958,9 @@ int ndt_eval_batch(ndt_ctx* c, const float* xyz, uint64_t n, const double* T34, 
     cudaMemcpyAsync(c->d_sjobs.p, hs, sjb, cudaMemcpyHostToDevice, st);
     cudaEventRecord(c->ev0, st);
     if ((rc = launch_score(c->map.view, (const float*)c->d_in.p, (const ScoreJob*)c->d_sjobs.p,
-                           (uint32_t)m, (uint32_t)n, nullptr, c->d_part.p, (ScoreOut*)c->d_sout.p,
-                           (float)c->d1, (float)c->d2, st)))
+                           (uint32_t)m, (uint32_t)n, nullptr, c->d_part.p,
+                           (uint32_t*)c->d_sdone.p, (ScoreOut*)c->d_sout.p, (float)c->d1,
+                           (float)c->d2, st)))
         return rc;
     cudaEventRecord(c->ev1, st);
     cudaMemcpyAsync(c->h_sout.p, c->d_sout.p, sob, cudaMemcpyDeviceToHost, st);

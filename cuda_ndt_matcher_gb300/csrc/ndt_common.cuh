@@ -1,16 +1,19 @@
 // ndt_common.cuh — device-side definitions shared by the NDT kernels (sm_103a).
 //
 // Voxel map layout in HBM (built by voxel_build.cu, read by ndt_align.cu / ndt_score.cu):
-//   slots[cap]      uint4 {key32, mean.x, mean.y, mean.z}: open-addressing hash, 16 B per
-//                   slot, key32 = EMPTY_KEY when free. The stored key is the cell relative
-//                   to the map's minimum cell (key_bits per axis, <= 31 bits in total); the
-//                   home slot is mix32(key32) masked by the power-of-two capacity (the
-//                   reference uses the MurmurHash3 64-bit finaliser of a 63-bit packed key,
-//                   src/cuda_ffi/csrc/voxel_hash.cu:33-58). One 16-byte load both tests the
-//                   key and yields the centroid for the radius check.
-//   slot_icov[cap]  2 x float4 {c00, c01, c02, c11}, {c12, c22, 0, 0}: inverse covariance of
-//                   the voxel in that slot (one 32-byte sector per accepted neighbour).
-//   slot_vidx[cap]  int32 voxel index (ascending coordinate-Morton order), for the query API.
+//   rmean[r]        float4 {mean.x, mean.y, mean.z, -} of voxel record r
+//   icov8[8 r]      its inverse covariance {c00, c01, c02, c11, c12, c22, 0, 0}: one 32-byte
+//                   sector, read by one 256-bit load. With the dense cell index a record is a
+//                   voxel (ascending coordinate-Morton order: neighbouring voxels share cache
+//                   lines, and nothing is padding); with the hash it is a hash slot.
+//   slots[cap]      hash maps only (rmean is this array): uint4 {mean.x, mean.y, mean.z, key32},
+//                   open addressing, 16 B per slot, key32 = EMPTY_KEY when free. The stored
+//                   key is the cell relative to the map's minimum cell (key_bits per axis, <= 31
+//                   bits in total); the home slot is mix32(key32) masked by the power-of-two
+//                   capacity (the reference uses the MurmurHash3 64-bit finaliser of a 63-bit
+//                   packed key, src/cuda_ffi/csrc/voxel_hash.cu:33-58). One 16-byte load both
+//                   tests the key and yields the centroid for the radius check.
+//   slot_vidx[cap]  hash maps only: int32 voxel index of a slot, for the query API.
 #pragma once
 
 #include <cstdint>
@@ -30,9 +33,10 @@ constexpr uint32_t ST_QUEUE_STALL = 1u << 3;  // work-queue kernel found no prog
 constexpr uint32_t ST_STAGE_TIMEOUT = 1u << 4;  // a point-staging bulk copy did not land in 1 s
 
 struct MapView {
-    const uint4* slots;
-    const float4* slot_icov;
-    const int32_t* slot_vidx;
+    const uint4* slots;      // null when the dense index serves
+    const float4* rmean;
+    const float* icov8;
+    const int32_t* slot_vidx;  // null when the dense index serves
     uint32_t mask;        // capacity - 1
     uint32_t max_probe;   // longest insert displacement; queries scan max_probe + 1 slots
     int32_t min_cell[3];
@@ -43,8 +47,8 @@ struct MapView {
     uint32_t num_voxels;
     int32_t exact_inv;    // inv_res is a power of two (q * inv_res is exact in f32)
     // dense cell index (null when the hash serves): grid[(lx * ext[1] + ly) * ext[2] + lz]
-    // = {centroid x, y, z, slot as int bits} of the voxel in local cell (lx, ly, lz), or
-    // slot -1 for an empty cell
+    // = {centroid x, y, z, voxel as int bits} of the voxel in local cell (lx, ly, lz), or
+    // -1 for an empty cell
     const float4* grid;
     uint32_t ext[3];
     // neighbourhood masks over the dense index's box grown by one cell on every side, 2^msh
@@ -140,11 +144,11 @@ __device__ __forceinline__ int32_t probe(const MapView& m, uint32_t key, uint32_
     uint32_t s = home;
     for (uint32_t j = 0; j <= m.max_probe; ++j) {
         uint4 v = __ldg(m.slots + s);
-        if (v.x == key) {
+        if (v.w == key) {
             *out = v;
             return (int32_t)s;
         }
-        if (v.x == EMPTY_KEY) return -1;
+        if (v.w == EMPTY_KEY) return -1;
         s = (s + 1) & m.mask;
     }
     return -1;
@@ -156,16 +160,35 @@ __device__ __forceinline__ int32_t probe_next(const MapView& m, uint32_t key, ui
     for (uint32_t j = 1; j <= m.max_probe; ++j) {
         uint32_t s = (home + j) & m.mask;
         uint4 v = __ldg(m.slots + s);
-        if (v.x == key) {
+        if (v.w == key) {
             *out = v;
             return (int32_t)s;
         }
-        if (v.x == EMPTY_KEY) return -1;
+        if (v.w == EMPTY_KEY) return -1;
     }
     return -1;
 }
 
-// Voxel of cell (gx, gy, gz): its slot (or -1) and centroid, through the dense index when
+// Inverse covariance of record r: c00, c01, c02, c11, c12, c22 in c[0..5].
+__device__ __forceinline__ void load_icov(const MapView& m, uint32_t r, float* c) {
+    float p0, p1;  // the record's padding
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3]), "=f"(c[4]), "=f"(c[5]), "=f"(p0),
+          "=f"(p1)
+        : "l"(m.icov8 + 8 * (size_t)r));
+}
+
+// x = (qh + ql) - centroid and the inverse covariance of record r
+__device__ __forceinline__ void load_voxel(const MapView& m, uint32_t r, const float* qh,
+                                           const float* ql, float* x, float* c) {
+    const float4 mu = __ldg(m.rmean + r);
+    load_icov(m, r, c);
+    x[0] = (qh[0] - mu.x) + ql[0];
+    x[1] = (qh[1] - mu.y) + ql[1];
+    x[2] = (qh[2] - mu.z) + ql[2];
+}
+
+// Record (or -1) and centroid of the voxel of cell (gx, gy, gz), through the dense index when
 // the map has one, else through the hash.
 __device__ __forceinline__ int32_t find_cell(const MapView& m, int32_t gx, int32_t gy,
                                              int32_t gz, float* cx, float* cy, float* cz) {
@@ -184,9 +207,9 @@ __device__ __forceinline__ int32_t find_cell(const MapView& m, int32_t gx, int32
     if (!cell_slot(m, gx, gy, gz, key, home)) return -1;
     uint4 sv;
     const int32_t s = probe(m, key, home, &sv);
-    *cx = __uint_as_float(sv.y);
-    *cy = __uint_as_float(sv.z);
-    *cz = __uint_as_float(sv.w);
+    *cx = __uint_as_float(sv.x);
+    *cy = __uint_as_float(sv.y);
+    *cz = __uint_as_float(sv.z);
     return s;
 }
 
@@ -220,6 +243,106 @@ __device__ __forceinline__ uint32_t cell_oct_of_sum(const MapView& m, const floa
         oct = (oct << 1) | (f - fl >= 0.5f ? 1u : 0u);
     }
     return oct;
+}
+
+// Neighbour search of the point q = qh + ql, in rounds. A round tests the cells' voxels in the
+// reference's order (dx outer, dy, dz inner) from where the last round stopped, and lists those
+// within one resolution, at most `room` (and LIST_CAP), in the thread's column of shared
+// memory: list[k * stride] = {q - centroid, record as int bits}. The list carries the
+// difference, so scoring a listed voxel takes one 256-bit load of its inverse covariance
+// instead of three loads on two cache lines: the kernels that search are bound by the lines
+// their loads touch in L1. `state` is what remains to be tested: with the dense index the
+// neighbourhood mask's bits (search_begin), with the hash the next of the 27 cells. Returns the
+// number listed; another round can only find more while search_more(state).
+constexpr int LIST_CAP = 8;
+
+__device__ __forceinline__ uint32_t search_begin(const MapView& m, const int32_t* gc,
+                                                 uint32_t oct, uint32_t& corner) {
+    corner = 0u;
+    return m.grid ? nbhd_mask(m, gc, oct, corner) : 0u;
+}
+
+__device__ __forceinline__ bool search_more(const MapView& m, uint32_t state) {
+    return m.grid ? state != 0u : state < 27u;
+}
+
+__device__ __forceinline__ int search_round(const MapView& m, const uint32_t* off27,
+                                            const int32_t* gc, const float* qh, const float* ql,
+                                            uint32_t& state, uint32_t corner, int room,
+                                            float4* list, int stride) {
+    int cnt = 0;
+    const int cap = min(room, LIST_CAP);
+    auto test = [&](float mx, float my, float mz, int32_t r) {
+        const float e0 = (qh[0] - mx) + ql[0];
+        const float e1 = (qh[1] - my) + ql[1];
+        const float e2 = (qh[2] - mz) + ql[2];
+        if (fmaf(e0, e0, fmaf(e1, e1, e2 * e2)) > m.r2) return;
+        list[cnt * stride] = make_float4(e0, e1, e2, __int_as_float(r));
+        cnt++;
+    };
+    if (m.grid) {
+        // {centroid, record} entries of the mask's cells, NB_BATCH independent loads at a time
+        constexpr int NB_BATCH = 4;
+#pragma unroll 1
+        while (state != 0u && cnt < cap) {
+            float4 e[NB_BATCH];
+            uint32_t rem = state;
+#pragma unroll
+            for (int k = 0; k < NB_BATCH; ++k) {
+                const uint32_t b = (uint32_t)(__ffs(rem) - 1) & 31u;  // 31 when empty
+                e[k] = rem != 0u ? __ldg(m.grid + (corner + off27[b]))
+                                 : make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
+                rem &= rem - 1u;
+            }
+#pragma unroll
+            for (int k = 0; k < NB_BATCH; ++k) {
+                const int32_t r = __float_as_int(e[k].w);
+                if (r < 0 || cnt >= cap) break;
+                state &= state - 1u;
+                test(e[k].x, e[k].y, e[k].z, r);
+            }
+        }
+        return cnt;
+    }
+    const uint32_t bxy = m.bits[0] + m.bits[1];
+    const uint32_t lz0 = (uint32_t)(gc[2] - m.min_cell[2]);
+#pragma unroll 1
+    for (int c9 = (int)state / 3; c9 < 9 && cnt < cap; ++c9) {
+        const int k0 = (int)state - 3 * c9;  // first cell of the column still to test
+        const int dx = c9 / 3 - 1, dy = c9 % 3 - 1;
+        const uint32_t lx = (uint32_t)(gc[0] + dx - m.min_cell[0]);
+        const uint32_t ly = (uint32_t)(gc[1] + dy - m.min_cell[1]);
+        if (!((lx >> m.bits[0]) | (ly >> m.bits[1]))) {
+            const uint32_t kxy = lx | (ly << m.bits[0]);
+            uint4 sv[3];
+            uint32_t key[3], home[3];
+            bool inb[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {  // the column's three home slots, loaded together
+                const uint32_t lz = lz0 + (uint32_t)(k - 1);
+                inb[k] = k >= k0 && (lz >> m.bits[2]) == 0u;
+                key[k] = kxy | (lz << bxy);
+                home[k] = mix32(key[k]) & m.mask;
+                sv[k] = inb[k] ? __ldg(m.slots + home[k]) : make_uint4(0u, 0u, 0u, EMPTY_KEY);
+            }
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                if (cnt >= cap) return cnt;  // state names this cell
+                state = 3u * c9 + k + 1u;
+                if (!inb[k]) continue;
+                uint4 v = sv[k];
+                int32_t r = (int32_t)home[k];
+                if (v.w != key[k]) {
+                    if (v.w == EMPTY_KEY) continue;
+                    r = probe_next(m, key[k], home[k], &v);
+                    if (r < 0) continue;
+                }
+                test(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), r);
+            }
+        }
+        state = 3u * c9 + 3u;
+    }
+    return cnt;
 }
 
 // Offsets in the reference's fixed order (ndt_graph_kernels.cu:29-39): dx outer, dz inner.

@@ -52,7 +52,7 @@ int cuda_fail(cudaError_t e, const char* what);
 
 // Device-resident voxel map.
 struct Map {
-    DevBuf slots, slot_icov, slot_vidx, grid, nmask;
+    DevBuf slots, icov8, slot_vidx, grid, nmask;
     DevBuf vox_coord, vox_mean, vox_cov, vox_icov, vox_count;
     MapView view{};
     ndt_map_info info{};
@@ -292,9 +292,10 @@ struct ScoreOut {
     uint64_t ncorr;
 };
 size_t score_part_bytes(uint32_t num_jobs, uint32_t max_n);
+// part: score_part_bytes; done: one word per job, zero before the launch and after it
 int launch_score(const MapView& map, const float* pts, const ScoreJob* jobs, uint32_t num_jobs,
-                 uint32_t max_n, const AlignOut* align_out, void* part, ScoreOut* out, float d1,
-                 float d2, cudaStream_t s);
+                 uint32_t max_n, const AlignOut* align_out, void* part, uint32_t* done,
+                 ScoreOut* out, float d1, float d2, cudaStream_t s);
 int launch_query(const MapView& map, const float* q, size_t n, int max_nb, int32_t* idx,
                  int32_t* cnt, cudaStream_t s);
 

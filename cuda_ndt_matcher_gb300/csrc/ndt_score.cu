@@ -12,13 +12,15 @@
 // The transform is either given (evaluate_*), or built from an alignment's final pose vector
 // with nalgebra's from_euler_angles (Rz*Ry*Rx), the isometry the reference evaluates NVTL on
 // after an alignment (src/ndt_cuda/src/optimization/types.rs:156-161, solver.rs:386,424).
-// Block partials are reduced in a fixed order by a second kernel: results are deterministic.
+// Block partials are added in a fixed order: results are deterministic.
+#include <algorithm>
+
 #include "ndt_internal.h"
 
 namespace ndtgb {
 
-constexpr int ST = 256;          // threads per block
-constexpr int SCHUNK = ST * 8;   // points per block
+constexpr int ST = 128;  // threads per block
+constexpr uint32_t SCORE_MAX_PPT = 8;
 
 struct ScorePartial {
     double nvtl_sum;
@@ -27,24 +29,63 @@ struct ScorePartial {
     uint64_t ncorr;
 };
 
-// nalgebra from_euler_angles (Rz*Ry*Rx) transform in FP64
-__device__ void zyx_T(const double* pose, double* T) {
-    double sr, cr, sp, cp, sy, cy;
-    sincos(pose[3], &sr, &cr);
-    sincos(pose[4], &sp, &cp);
-    sincos(pose[5], &sy, &cy);
-    T[0] = cy * cp;
-    T[1] = cy * sp * sr - sy * cr;
-    T[2] = cy * sp * cr + sy * sr;
-    T[3] = pose[0];
-    T[4] = sy * cp;
-    T[5] = sy * sp * sr + cy * cr;
-    T[6] = sy * sp * cr - cy * sr;
-    T[7] = pose[1];
-    T[8] = -sp;
-    T[9] = cp * sr;
-    T[10] = cp * cr;
-    T[11] = pose[2];
+// Points per thread of a launch over `jobs` jobs of at most max_n points: one while the grid
+// is small, so a single scan's points spread over every SM (a 20k-point scan: 157 blocks
+// instead of 10; scoring it is one dependent chain of loads per point, 54 -> 16 us), then
+// doubled, up to 8, while about four blocks per resident slot (152 SMs x 8) remain: the
+// block's set-up and reduction are then paid once per 8 points (filling the slots once, four
+// and sixteen times measured 70, 64 and 72 us on 64 scans of 2k-40k points).
+static uint32_t score_ppt(uint32_t jobs, uint32_t max_n) {
+    uint32_t ppt = 1;
+    while (ppt < SCORE_MAX_PPT &&
+           (uint64_t)jobs * (((uint64_t)max_n + ST * 2 * ppt - 1) / (ST * 2 * ppt)) >=
+               4ull * 152 * 8)
+        ppt *= 2;
+    return ppt;
+}
+
+static uint32_t score_blocks(uint32_t jobs, uint32_t max_n) {
+    const uint32_t per = ST * score_ppt(jobs, max_n);
+    return std::max<uint32_t>(1u, (uint32_t)(((uint64_t)max_n + per - 1) / per));
+}
+
+// Transform of one job (row-major 3x4, FP64) by the lanes of one warp, as hi/lo f32 pairs: the
+// given matrix, or nalgebra's from_euler_angles (Rz*Ry*Rx) of an alignment's final pose: three
+// lanes take a sine and cosine each (about 1,700 cycles of dependent FP64 apiece), twelve an
+// entry each.
+__device__ __forceinline__ void job_transform(const ScoreJob& job, const AlignOut* aout,
+                                              double* trig, float* Th, float* Tl, int lane) {
+    double v = 0.0;
+    if (job.pose_src == 1) {
+        const double* pose = aout[job.out_index].pose;
+        if (lane < 3) {
+            double s, c;
+            sincos(pose[3 + lane], &s, &c);
+            trig[2 * lane] = s;
+            trig[2 * lane + 1] = c;
+        }
+        __syncwarp();
+        if (lane < 12) {
+            const double sr = trig[0], cr = trig[1], sp = trig[2], cp = trig[3], sy = trig[4],
+                         cy = trig[5];
+            const int i = lane >> 2, j = lane & 3;
+            if (j == 3) {
+                v = pose[i];
+            } else if (i == 2) {
+                v = j == 0 ? -sp : cp * (j == 1 ? sr : cr);
+            } else {
+                const double a = i == 0 ? cy : sy;  // the factor of the sin p terms
+                const double b = i == 0 ? -sy : cy;
+                v = j == 0 ? a * cp : (j == 1 ? a * sp * sr + b * cr : a * sp * cr - b * sr);
+            }
+        }
+    } else if (lane < 12) {
+        v = job.T[lane];
+    }
+    if (lane < 12) {
+        Th[lane] = (float)v;
+        Tl[lane] = (float)(v - (double)Th[lane]);
+    }
 }
 
 // q = T p as an unevaluated sum qh + ql: T given as hi/lo f32 pairs, TwoProd/TwoSum
@@ -71,150 +112,175 @@ __device__ __forceinline__ void transform_comp(const float* Th, const float* Tl,
     }
 }
 
-__global__ void __launch_bounds__(ST) k_score(MapView m, const float* __restrict__ pts,
-                                              const ScoreJob* __restrict__ jobs,
-                                              const AlignOut* __restrict__ aout, float d1,
-                                              float d2, ScorePartial* __restrict__ part) {
+// s + e == a + b exactly
+__device__ __forceinline__ void two_sum_f(float a, float b, float& s, float& e) {
+    s = a + b;
+    const float bp = s - a;
+    e = (a - (s - bp)) + (b - bp);
+}
+
+// hi + lo += (oh + ol), both unevaluated f32 pairs
+__device__ __forceinline__ void pair_add(float& hi, float& lo, float oh, float ol) {
+    float e;
+    two_sum_f(hi, oh, hi, e);
+    lo += ol + e;
+}
+
+// One block per `chunk` points of a job (bx blocks per job in the grid; those past the job's
+// end leave at once). A point's voxels are first listed (the radius test, candidates loaded
+// four at a time), then scored: the lanes of a warp stay on one instruction stream. The FP64
+// unit takes 16 cycles per SM for a warp instruction, so a thread's and a block's sums are
+// kept as f32 pairs (TwoSum: 48 bits, against the terms' own 24) and become FP64 once per
+// block. The block that finishes a job last adds its partials in a fixed order: no second
+// launch. `done` counts a job's finished blocks and is back at zero when the launch ends.
+// Bound: dependent loads (mask, candidates, records) and instruction issue. One 20k-point scan
+// 54 -> 16 us, 20k points at 100 poses 132 -> 112 us, 64 scans of 2k-40k 92 -> 62 us, 256 x
+// 20k points 266 -> 261 us.
+__global__ void __launch_bounds__(ST, 8) k_score(MapView m, const float* __restrict__ pts,
+                                                 const ScoreJob* __restrict__ jobs,
+                                                 const AlignOut* __restrict__ aout, float d1,
+                                                 float d2, uint32_t bx, uint32_t chunk,
+                                                 ScorePartial* __restrict__ part,
+                                                 uint32_t* __restrict__ done,
+                                                 ScoreOut* __restrict__ out) {
     __shared__ float Th[12], Tl[12];
-    __shared__ double red[ST / 32][2];
-    __shared__ unsigned long long redc[ST / 32][2];
-    __shared__ uint32_t s_off[32];  // neighbour offsets of the dense index
-    nbhd_offsets(m, s_off);         // read after the barrier below
-    const ScoreJob job = jobs[blockIdx.y];
-    const size_t pidx = (size_t)blockIdx.y * gridDim.x + blockIdx.x;
-    const uint32_t first = blockIdx.x * SCHUNK;
-    if (threadIdx.x == 0) {
-        double T[12];
-        if (job.pose_src == 1) {
-            zyx_T(aout[job.out_index].pose, T);
-        } else {
-            for (int i = 0; i < 12; ++i) T[i] = job.T[i];
-        }
-        for (int i = 0; i < 12; ++i) {
-            Th[i] = (float)T[i];
-            Tl[i] = (float)(T[i] - (double)Th[i]);
-        }
-    }
+    __shared__ double trig[6];
+    __shared__ float red[ST / 32][4];
+    __shared__ uint32_t redc[ST / 32][2];
+    __shared__ uint32_t s_off[32];            // neighbour offsets of the dense index
+    __shared__ float4 s_list[LIST_CAP][ST];   // listed voxels per thread
+    __shared__ bool s_last;
+    const uint32_t j = blockIdx.x / bx, blk = blockIdx.x % bx;
+    const ScoreJob& job = jobs[j];
+    const uint32_t n = job.n, nblk = max(1u, (n + chunk - 1u) / chunk);
+    if (blk >= nblk) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    nbhd_offsets(m, s_off);
+    if (warp == 0) job_transform(job, aout, trig, Th, Tl, lane);
     __syncthreads();
-    double nv = 0.0, sc = 0.0;
-    unsigned long long nvc = 0, nc = 0;
+    float nvh = 0.f, nvl = 0.f, sch = 0.f, scl = 0.f;
+    uint32_t nvc = 0, nc = 0;
     const float* P = pts + 3 * job.offset;
-    uint32_t last = min(job.n, first + SCHUNK);
+    const uint32_t first = blk * chunk, last = min(n, first + chunk);
+    float4* const list = &s_list[0][threadIdx.x];
     for (uint32_t i = first + threadIdx.x; i < last; i += ST) {
         float px = __ldg(P + 3 * (size_t)i), py = __ldg(P + 3 * (size_t)i + 1),
               pz = __ldg(P + 3 * (size_t)i + 2);
         if (!(isfinite(px) && isfinite(py) && isfinite(pz))) continue;
         float qh[3], ql[3];
         transform_comp(Th, Tl, px, py, pz, qh, ql);
-        const float qx = qh[0], qy = qh[1], qz = qh[2];
         int32_t gc[3];
         const uint32_t oct = cell_oct_of_sum(m, qh, ql, gc);
-        const int32_t gx = gc[0], gy = gc[1], gz = gc[2];
+        uint32_t corner;
+        uint32_t state = search_begin(m, gc, oct, corner);
+        int total = 0;
         float best = -INFINITY, sum = 0.f;
-        int cnt = 0;
-        // one voxel with centroid (mx, my, mz) in slot s: radius test, then its score term
-        auto visit = [&](int32_t s, float mx, float my, float mz) {
-            const float x0 = (qx - mx) + ql[0], x1 = (qy - my) + ql[1], x2 = (qz - mz) + ql[2];
-            if (fmaf(x0, x0, fmaf(x1, x1, x2 * x2)) > m.r2) return;
-            const float4 ca = __ldg(m.slot_icov + 2 * (size_t)s);
-            const float4 cb = __ldg(m.slot_icov + 2 * (size_t)s + 1);
-            const float c0 = fmaf(ca.x, x0, fmaf(ca.y, x1, ca.z * x2));
-            const float c1 = fmaf(ca.y, x0, fmaf(ca.w, x1, cb.x * x2));
-            const float c2 = fmaf(ca.z, x0, fmaf(cb.x, x1, cb.y * x2));
-            const float md = fmaf(x0, c0, fmaf(x1, c1, x2 * c2));
-            const float s0 = -d1 * expf(-d2 * md * 0.5f);
-            best = fmaxf(best, s0);
-            sum += s0;
-            cnt++;
-        };
-        if (m.grid) {  // occupied neighbours only, in the same order, from the mask
-            uint32_t corner;
-            uint32_t bits = nbhd_mask(m, gc, oct, corner);
+        do {
+            const int cnt = search_round(m, s_off, gc, qh, ql, state, corner, MAX_NB_ALL, list, ST);
+            total += cnt;
 #pragma unroll 1
-            while (bits != 0u) {
-                const uint32_t b = (uint32_t)(__ffs(bits) - 1);
-                bits &= bits - 1u;
-                const float4 e = __ldg(m.grid + (corner + s_off[b]));
-                visit(__float_as_int(e.w), e.x, e.y, e.z);
+            for (int k = 0; k < cnt; ++k) {
+                const float4 x = list[k * ST];
+                float C[6];
+                load_icov(m, __float_as_uint(x.w), C);
+                const float c0 = fmaf(C[0], x.x, fmaf(C[1], x.y, C[2] * x.z));
+                const float c1 = fmaf(C[1], x.x, fmaf(C[3], x.y, C[4] * x.z));
+                const float c2 = fmaf(C[2], x.x, fmaf(C[4], x.y, C[5] * x.z));
+                const float md = fmaf(x.x, c0, fmaf(x.y, c1, x.z * c2));
+                const float s0 = -d1 * expf(-d2 * md * 0.5f);
+                best = fmaxf(best, s0);
+                sum += s0;
             }
-        } else {
-#pragma unroll 1
-            for (int c = 0; c < 27; ++c) {
-                int dx, dy, dz;
-                offset27(c, dx, dy, dz);
-                float mx, my, mz;
-                const int32_t s = find_cell(m, (int32_t)((uint32_t)gx + (uint32_t)dx),
-                                            (int32_t)((uint32_t)gy + (uint32_t)dy),
-                                            (int32_t)((uint32_t)gz + (uint32_t)dz), &mx, &my,
-                                            &mz);
-                if (s >= 0) visit(s, mx, my, mz);
-            }
-        }
-        if (cnt) {
-            nv += (double)best;
-            nvc++;
-            sc += (double)sum;
-            nc += (unsigned long long)cnt;
-        }
+        } while (search_more(m, state));
+        if (total == 0) continue;
+        float e;
+        two_sum_f(nvh, best, nvh, e);
+        nvl += e;
+        two_sum_f(sch, sum, sch, e);
+        scl += e;
+        nvc++;
+        nc += (uint32_t)total;
     }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-        nv += __shfl_xor_sync(0xffffffffu, nv, o);
-        sc += __shfl_xor_sync(0xffffffffu, sc, o);
-        nvc += __shfl_xor_sync(0xffffffffu, nvc, o);
-        nc += __shfl_xor_sync(0xffffffffu, nc, o);
+        pair_add(nvh, nvl, __shfl_xor_sync(0xffffffffu, nvh, o),
+                 __shfl_xor_sync(0xffffffffu, nvl, o));
+        pair_add(sch, scl, __shfl_xor_sync(0xffffffffu, sch, o),
+                 __shfl_xor_sync(0xffffffffu, scl, o));
     }
+    nvc = __reduce_add_sync(0xffffffffu, nvc);
+    nc = __reduce_add_sync(0xffffffffu, nc);
     if (lane == 0) {
-        red[warp][0] = nv;
-        red[warp][1] = sc;
+        red[warp][0] = nvh;
+        red[warp][1] = nvl;
+        red[warp][2] = sch;
+        red[warp][3] = scl;
         redc[warp][0] = nvc;
         redc[warp][1] = nc;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        ScorePartial p{0.0, 0.0, 0, 0};
-        for (int w = 0; w < ST / 32; ++w) {
-            p.nvtl_sum += red[w][0];
-            p.score_sum += red[w][1];
-            p.nvtl_count += redc[w][0];
-            p.ncorr += redc[w][1];
+        for (int w = 1; w < ST / 32; ++w) {
+            pair_add(nvh, nvl, red[w][0], red[w][1]);
+            pair_add(sch, scl, red[w][2], red[w][3]);
+            nvc += redc[w][0];
+            nc += redc[w][1];
         }
-        part[pidx] = p;
+        // an infinite sum has no low part
+        const ScorePartial p{(double)nvh + (isfinite(nvh) ? (double)nvl : 0.0),
+                             (double)sch + (isfinite(sch) ? (double)scl : 0.0), nvc, nc};
+        if (nblk == 1u) {
+            out[j] = ScoreOut{p.nvtl_sum, p.score_sum, p.nvtl_count, p.ncorr};
+            s_last = false;
+        } else {
+            part[(size_t)j * bx + blk] = p;
+            __threadfence();
+            s_last = atomicAdd(done + j, 1u) == nblk - 1u;
+        }
     }
-}
-
-__global__ void k_score_reduce(const ScorePartial* __restrict__ part, uint32_t bx,
-                               uint32_t njobs, ScoreOut* __restrict__ out) {
-    uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= njobs) return;
-    ScoreOut o{0.0, 0.0, 0, 0};
-    for (uint32_t b = 0; b < bx; ++b) {
-        const ScorePartial& p = part[(size_t)j * bx + b];
-        o.nvtl_sum += p.nvtl_sum;
-        o.score_sum += p.score_sum;
-        o.nvtl_count += p.nvtl_count;
-        o.ncorr += p.ncorr;
+    __syncthreads();
+    if (!s_last || warp != 0) return;
+    __threadfence();  // acquire: every block's partial is visible
+    // lane l adds the partials l, l + 32, ..., then the lanes in a tree
+    ScorePartial t{0.0, 0.0, 0, 0};
+    for (uint32_t b = lane; b < nblk; b += 32) {
+        const ScorePartial* q = part + (size_t)j * bx + b;
+        t.nvtl_sum += __ldcg(&q->nvtl_sum);
+        t.score_sum += __ldcg(&q->score_sum);
+        t.nvtl_count += __ldcg((const unsigned long long*)&q->nvtl_count);
+        t.ncorr += __ldcg((const unsigned long long*)&q->ncorr);
     }
-    out[j] = o;
-}
-
-int launch_score(const MapView& map, const float* pts, const ScoreJob* jobs, uint32_t num_jobs,
-                  uint32_t max_n, const AlignOut* align_out, void* part, ScoreOut* out, float d1,
-                  float d2, cudaStream_t s) {
-    if (num_jobs == 0) return 0;
-    uint32_t bx = (max_n + SCHUNK - 1) / SCHUNK;
-    if (bx == 0) bx = 1;
-    k_score<<<dim3(bx, num_jobs), ST, 0, s>>>(map, pts, jobs, align_out, d1, d2,
-                                              (ScorePartial*)part);
-    k_score_reduce<<<(num_jobs + 127) / 128, 128, 0, s>>>((ScorePartial*)part, bx, num_jobs, out);
-    return cuda_fail(cudaGetLastError(), "score launch");
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        t.nvtl_sum += __shfl_xor_sync(0xffffffffu, t.nvtl_sum, o);
+        t.score_sum += __shfl_xor_sync(0xffffffffu, t.score_sum, o);
+        t.nvtl_count += __shfl_xor_sync(0xffffffffu, (unsigned long long)t.nvtl_count, o);
+        t.ncorr += __shfl_xor_sync(0xffffffffu, (unsigned long long)t.ncorr, o);
+    }
+    if (lane == 0) {
+        out[j] = ScoreOut{t.nvtl_sum, t.score_sum, t.nvtl_count, t.ncorr};
+        done[j] = 0u;
+    }
 }
 
 size_t score_part_bytes(uint32_t num_jobs, uint32_t max_n) {
-    uint32_t bx = (max_n + SCHUNK - 1) / SCHUNK;
-    if (bx == 0) bx = 1;
-    return (size_t)bx * num_jobs * sizeof(ScorePartial);
+    return (size_t)score_blocks(num_jobs, max_n) * num_jobs * sizeof(ScorePartial);
+}
+
+int launch_score(const MapView& map, const float* pts, const ScoreJob* jobs, uint32_t num_jobs,
+                 uint32_t max_n, const AlignOut* align_out, void* part, uint32_t* done,
+                 ScoreOut* out, float d1, float d2, cudaStream_t s) {
+    if (num_jobs == 0) return 0;
+    const uint32_t bx = score_blocks(num_jobs, max_n);
+    const uint64_t grid = (uint64_t)bx * num_jobs;
+    if (grid > 0x7FFFFFFFull) {
+        set_error("score launch: too many points times poses");
+        return NDT_ERR_CAPACITY;
+    }
+    k_score<<<(unsigned)grid, ST, 0, s>>>(map, pts, jobs, align_out, d1, d2, bx,
+                                          ST * score_ppt(num_jobs, max_n), (ScorePartial*)part,
+                                          done, out);
+    return cuda_fail(cudaGetLastError(), "score launch");
 }
 
 // Standalone neighbour query with the graph kernel's semantics, f32 arithmetic unfused.
@@ -236,7 +302,7 @@ __global__ void k_query(MapView m, const float* __restrict__ q, size_t n, int ma
                                     (int32_t)((uint32_t)gz + (uint32_t)dz), &mx, &my, &mz);
         if (s < 0) continue;
         if (dist2_rn(qx, qy, qz, mx, my, mz) <= m.r2)
-            idx[i * (size_t)max_nb + c++] = m.slot_vidx[s];
+            idx[i * (size_t)max_nb + c++] = m.grid ? s : m.slot_vidx[s];
     }
     for (int k = c; k < max_nb; ++k) idx[i * (size_t)max_nb + k] = -1;
     cnt[i] = c;

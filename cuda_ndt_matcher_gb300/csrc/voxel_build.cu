@@ -24,11 +24,12 @@
 //                            in FP64; regularisation to the min-ratio and inverse in FP64,
 //                            f32 outputs (Voxel::from_statistics / regularize_covariance,
 //                            src/ndt_cuda/src/voxel_grid/types.rs:54-190).
-//   6. compaction          : valid voxels keep their Morton order.
-//   7. hash insert         : bounded linear probing with atomicCAS, displacement recorded
-//                            (voxel_hash_build_kernel, src/cuda_ffi/csrc/voxel_hash.cu:69-114).
-//   8. dense cell index    : when it fits, {centroid, slot} per cell of the map's box, and
-//                            the neighbourhood masks (one per octant of each cell while they
+//   6. compaction          : valid voxels keep their Morton order; their search records; the
+//                            dense cell index when it fits, {centroid, voxel} per cell of the
+//                            map's box; and hash insert: bounded linear probing with
+//                            atomicCAS, displacement recorded (voxel_hash_build_kernel,
+//                            src/cuda_ffi/csrc/voxel_hash.cu:69-114).
+//   7. masks               : with the dense index, the neighbourhood masks (one per octant of each cell while they
 //                            fit their budget, else one per cell) that list the neighbours a
 //                            point there can accept.
 // Bit-exact parts (cells, keys, counts, means) use no multiply-add: cells are an f32 division,
@@ -1369,56 +1370,76 @@ __global__ void __launch_bounds__(128) k_voxel_stats(
     valid[s] = ok ? 1u : 0u;
 }
 
-__global__ void k_voxel_compact(const SegRec* __restrict__ rec, const uint32_t* __restrict__ valid,
-                                const uint32_t* __restrict__ rank,
-                                const uint32_t* __restrict__ num_seg, int32_t* __restrict__ coord,
-                                float4* __restrict__ mean4, float* __restrict__ cov,
-                                float* __restrict__ icov, uint32_t* __restrict__ count) {
-    uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= *num_seg || !valid[s]) return;
-    uint32_t v = rank[s];
-    const SegRec& r = rec[s];
-    coord[3 * v] = r.coord[0];
-    coord[3 * v + 1] = r.coord[1];
-    coord[3 * v + 2] = r.coord[2];
-    mean4[v] = make_float4(r.mean[0], r.mean[1], r.mean[2], __uint_as_float(r.count));
-    for (int q = 0; q < 9; ++q) cov[9 * (size_t)v + q] = r.cov[q];
-    const float* c = r.icov;
-    float full[9] = {c[0], c[1], c[2], c[1], c[3], c[4], c[2], c[4], c[5]};
-    for (int q = 0; q < 9; ++q) icov[9 * (size_t)v + q] = full[q];
-    count[v] = r.count;
+// Inserts `key` into an open-addressing table of keys (stride words apart): its slot and its
+// displacement from the home slot s, or -1 when the table is full.
+__device__ __forceinline__ int64_t hash_claim(uint32_t* keys, uint32_t stride, uint32_t mask,
+                                              uint32_t key, uint32_t s, uint32_t& disp) {
+    for (uint32_t j = 0; j <= mask; ++j) {
+        if (atomicCAS(keys + (size_t)s * stride, EMPTY_KEY, key) == EMPTY_KEY) {
+            disp = j;
+            return (int64_t)s;
+        }
+        s = (s + 1) & mask;
+    }
+    return -1;
 }
 
-__global__ void k_hash_insert(const int32_t* __restrict__ coord, const float4* __restrict__ mean4,
-                              const float* __restrict__ icov, uint32_t nv, MapView m,
-                              uint4* __restrict__ slots, float4* __restrict__ slot_icov,
-                              int32_t* __restrict__ slot_vidx, uint32_t* __restrict__ max_probe,
-                              uint32_t* __restrict__ status) {
-    const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
+// Valid voxels of the S segment records, in order, into the map's voxel arrays and the search
+// records. With the dense index (grid set) the record of a voxel is written at its own index
+// and its grid entry {centroid, voxel} at its cell, and only its key is inserted into a table
+// of 4-byte keys: no search reads the table then, but the map's description reports its
+// longest probe. Otherwise the voxel goes to its hash slot. On the 50M-point 2 m map (3.1M
+// voxels) writing 52 bytes to each random slot took 607 us and filling the grid from the
+// slots 112 us more; records in voxel order are written by neighbouring threads, and
+// neighbouring voxels share the lines that the searches read.
+__global__ void __launch_bounds__(128) k_voxel_compact(
+    const SegRec* __restrict__ rec, const uint32_t* __restrict__ valid,
+    const uint32_t* __restrict__ rank, uint32_t S, int32_t* __restrict__ coord,
+    float4* __restrict__ mean4, float* __restrict__ cov, float* __restrict__ icov,
+    uint32_t* __restrict__ count, MapView m, float4* __restrict__ icov8,
+    float4* __restrict__ grid, uint32_t* __restrict__ keys, uint4* __restrict__ slots,
+    int32_t* __restrict__ slot_vidx, uint32_t* __restrict__ max_probe,
+    uint32_t* __restrict__ status) {
+    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t disp = 0;  // this voxel's displacement from its home slot
-    if (v < nv) {
-        const int32_t gx = coord[3 * v], gy = coord[3 * v + 1], gz = coord[3 * v + 2];
-        uint32_t key, s;
-        cell_slot(m, gx, gy, gz, key, s);  // every voxel lies inside the map's bounding box
-        bool placed = false;
-        for (uint32_t j = 0; j <= m.mask; ++j) {
-            const uint32_t old = atomicCAS(&slots[s].x, EMPTY_KEY, key);
-            if (old == EMPTY_KEY) {
-                const float4 mu = mean4[v];
-                slots[s].y = __float_as_uint(mu.x);
-                slots[s].z = __float_as_uint(mu.y);
-                slots[s].w = __float_as_uint(mu.z);
-                const float* c = icov + 9 * (size_t)v;
-                slot_icov[2 * (size_t)s] = make_float4(c[0], c[1], c[2], c[4]);
-                slot_icov[2 * (size_t)s + 1] = make_float4(c[5], c[8], 0.f, 0.f);
-                slot_vidx[s] = (int32_t)v;
-                disp = j;
-                placed = true;
-                break;
+    if (s < S && valid[s]) {
+        const uint32_t v = rank[s];
+        const SegRec& r = rec[s];
+        const int32_t g[3] = {r.coord[0], r.coord[1], r.coord[2]};
+        coord[3 * (size_t)v] = g[0];
+        coord[3 * (size_t)v + 1] = g[1];
+        coord[3 * (size_t)v + 2] = g[2];
+        const float mu[3] = {r.mean[0], r.mean[1], r.mean[2]};
+        mean4[v] = make_float4(mu[0], mu[1], mu[2], __uint_as_float(r.count));
+        for (int q = 0; q < 9; ++q) cov[9 * (size_t)v + q] = r.cov[q];
+        float c[6];
+        for (int q = 0; q < 6; ++q) c[q] = r.icov[q];
+        const float full[9] = {c[0], c[1], c[2], c[1], c[3], c[4], c[2], c[4], c[5]};
+        for (int q = 0; q < 9; ++q) icov[9 * (size_t)v + q] = full[q];
+        count[v] = r.count;
+        uint32_t key, home;
+        cell_slot(m, g[0], g[1], g[2], key, home);  // every voxel lies inside the map's box
+        int64_t at;
+        if (grid) {
+            const size_t cell = ((size_t)(g[0] - m.min_cell[0]) * m.ext[1] +
+                                 (g[1] - m.min_cell[1])) * m.ext[2] + (g[2] - m.min_cell[2]);
+            grid[cell] = make_float4(mu[0], mu[1], mu[2], __int_as_float((int32_t)v));
+            at = hash_claim(keys, 1u, m.mask, key, home, disp) < 0 ? -1 : (int64_t)v;
+        } else {
+            at = hash_claim(&slots[0].w, 4u, m.mask, key, home, disp);
+            if (at >= 0) {
+                slots[at].x = __float_as_uint(mu[0]);
+                slots[at].y = __float_as_uint(mu[1]);
+                slots[at].z = __float_as_uint(mu[2]);
+                slot_vidx[at] = (int32_t)v;
             }
-            s = (s + 1) & m.mask;
         }
-        if (!placed) atomicOr(status, ST_HASH_FULL);
+        if (at >= 0) {
+            icov8[2 * at] = make_float4(c[0], c[1], c[2], c[3]);
+            icov8[2 * at + 1] = make_float4(c[4], c[5], 0.f, 0.f);
+        } else {
+            atomicOr(status, ST_HASH_FULL);
+        }
     }
     // the largest displacement: one atomic per warp that has a displaced voxel (3M threads on
     // one counter would queue at its L2 slice)
@@ -1426,27 +1447,14 @@ __global__ void k_hash_insert(const int32_t* __restrict__ coord, const float4* _
     if ((threadIdx.x & 31u) == 0 && disp) atomicMax(max_probe, disp);
 }
 
-// Dense cell index: every occupied hash slot writes {centroid, slot} into the entry of its
-// cell (the grid was set to all-ones first: slot -1 marks an empty cell).
-__global__ void k_grid_fill(MapView m, float4* __restrict__ grid) {
-    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s > m.mask) return;
-    const uint4 v = m.slots[s];
-    if (v.x == EMPTY_KEY) return;
-    const uint32_t lx = v.x & ((1u << m.bits[0]) - 1u);
-    const uint32_t ly = (v.x >> m.bits[0]) & ((1u << m.bits[1]) - 1u);
-    const uint32_t lz = v.x >> (m.bits[0] + m.bits[1]);
-    const size_t idx = ((size_t)lx * m.ext[1] + ly) * m.ext[2] + lz;
-    grid[idx] = make_float4(__uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w),
-                            __int_as_float((int32_t)s));
-}
-
 // Neighbourhood masks (layout in MapView::nmask), scattered from the voxels: the voxel in
 // local cell v is neighbour d = (dx, dy, dz) of cell v - d, so it sets bit
 // 9 (dx + 1) + 3 (dy + 1) + (dz + 1) of that cell's mask (or octant masks), at grown-box
-// position v - d + 1 (always inside the grown box). One thread per hash slot; the masks start
-// at zero, and OR is order-free, so the result does not depend on the threads' order. The
-// work goes with the number of voxels, not with the box.
+// position v - d + 1 (always inside the grown box). One thread per voxel, in Morton order, so
+// a warp's atomics fall on neighbouring words; the masks start at zero, and OR is order-free,
+// so the result does not depend on the threads' order. The work goes with the number of
+// voxels, not with the box. The two octants along z are neighbouring words and are set by one
+// 64-bit atomic (bound: the L2's atomic rate).
 // A bit is set only where the voxel's centroid can pass the radius test from some point of
 // cell v - d (of that octant of it): its distance to the cell's (octant's) box is at most the
 // radius, widened by 1e-5 of it and by 1e-6 cell widths per cell of distance from the origin
@@ -1455,16 +1463,16 @@ __global__ void k_grid_fill(MapView m, float4* __restrict__ grid) {
 // search. On the 5M-point 400 m map at 2 m a scan point tests 16.3 candidates with one mask
 // per cell and 9.0 with octant masks, of which it accepts 5.45.
 template <bool OCT>
-__global__ void k_grid_mask(MapView m, uint32_t* __restrict__ nmask) {
+__global__ void __launch_bounds__(128) k_grid_mask(MapView m, const int32_t* __restrict__ coord,
+                                                   const float4* __restrict__ mean4,
+                                                   uint32_t* __restrict__ nmask) {
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s > m.mask) return;
-    const uint4 sv = m.slots[s];
-    const uint32_t key = sv.x;
-    if (key == EMPTY_KEY) return;
-    const uint32_t v[3] = {key & ((1u << m.bits[0]) - 1u),
-                           (key >> m.bits[0]) & ((1u << m.bits[1]) - 1u),
-                           key >> (m.bits[0] + m.bits[1])};
-    const float mu[3] = {__uint_as_float(sv.y), __uint_as_float(sv.z), __uint_as_float(sv.w)};
+    if (s >= m.num_voxels) return;
+    const uint32_t v[3] = {(uint32_t)(coord[3 * (size_t)s] - m.min_cell[0]),
+                           (uint32_t)(coord[3 * (size_t)s + 1] - m.min_cell[1]),
+                           (uint32_t)(coord[3 * (size_t)s + 2] - m.min_cell[2])};
+    const float4 mv = mean4[s];
+    const float mu[3] = {mv.x, mv.y, mv.z};
     const float res = m.res, half = 0.5f * res;
     // gap[a][d_a + 1][h]: distance along axis a from the centroid to the box of the cell at
     // offset -d (h = 0: the whole cell, or with octants its lower half; h = 1: its upper half)
@@ -1520,11 +1528,15 @@ __global__ void k_grid_mask(MapView m, uint32_t* __restrict__ nmask) {
                                             (v[2] + 2u - dz))
                                            << 3);
 #pragma unroll
-                    for (uint32_t o = 0; o < 8u; ++o) {
+                    for (uint32_t o = 0; o < 8u; o += 2u) {  // octants o (lower z), o + 1
                         const float gx = gap[0][dx][(o >> 2) & 1u],
-                                    gy = gap[1][dy][(o >> 1) & 1u], gz = gap[2][dz][o & 1u];
-                        if (fmaf(gx, gx, fmaf(gy, gy, gz * gz)) > lim2) continue;
-                        atomicOr(w + o, 1u << b);
+                                    gy = gap[1][dy][(o >> 1) & 1u];
+                        const float g0 = gap[2][dz][0], g1 = gap[2][dz][1];
+                        const unsigned long long bit = 1ull << b;
+                        unsigned long long set = 0ull;
+                        if (!(fmaf(gx, gx, fmaf(gy, gy, g0 * g0)) > lim2)) set |= bit;
+                        if (!(fmaf(gx, gx, fmaf(gy, gy, g1 * g1)) > lim2)) set |= bit << 32;
+                        if (set) atomicOr((unsigned long long*)(w + o), set);
                     }
                 }
     }
@@ -1637,14 +1649,12 @@ int finish_map(Map& map, BuildScratch& sc, const SegRec* rec, const uint32_t* va
         (rc = dev_reserve(sc.small, 256)))
         return rc;
     uint32_t* mprobe = (uint32_t*)((char*)sc.small.p + 128);
-    uint32_t* d_S = (uint32_t*)((char*)sc.small.p + 192);
     uint32_t bits[3];
     if ((rc = box_bits(g.mn, g.mx, bits))) return rc;
     if ((rc = exclusive_scan(valid, (uint32_t*)sc.seg_rank.p, S, sc.tmp.p, s))) return rc;
     uint32_t hs[2];
     cudaMemcpyAsync(&hs[0], (uint32_t*)sc.seg_rank.p + (S - 1), 4, cudaMemcpyDeviceToHost, s);
     cudaMemcpyAsync(&hs[1], valid + (S - 1), 4, cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(d_S, &S, 4, cudaMemcpyHostToDevice, s);
     if ((rc = cuda_fail(cudaStreamSynchronize(s), "voxel compaction"))) return rc;
     const uint32_t V = hs[0] + hs[1];
     if (V == 0) {
@@ -1658,30 +1668,16 @@ int finish_map(Map& map, BuildScratch& sc, const SegRec* rec, const uint32_t* va
         set_error("hash capacity exceeds 2^31 slots");
         return NDT_ERR_CAPACITY;
     }
-    if ((rc = dev_reserve(map.vox_coord, (size_t)V * 12)) ||
-        (rc = dev_reserve(map.vox_mean, (size_t)V * 16)) ||
-        (rc = dev_reserve(map.vox_cov, (size_t)V * 36)) ||
-        (rc = dev_reserve(map.vox_icov, (size_t)V * 36)) ||
-        (rc = dev_reserve(map.vox_count, (size_t)V * 4)) ||
-        (rc = dev_reserve(map.slots, cap * 16)) || (rc = dev_reserve(map.slot_icov, cap * 32)) ||
-        (rc = dev_reserve(map.slot_vidx, cap * 4)))
-        return rc;
-    const unsigned blk = (unsigned)((S + 127) / 128);
-    k_voxel_compact<<<blk, 128, 0, s>>>(rec, valid, (uint32_t*)sc.seg_rank.p, d_S,
-                                        (int32_t*)map.vox_coord.p, (float4*)map.vox_mean.p,
-                                        (float*)map.vox_cov.p, (float*)map.vox_icov.p,
-                                        (uint32_t*)map.vox_count.p);
-    cudaMemsetAsync(map.slots.p, 0xFF, cap * 16, s);
-    cudaMemsetAsync(mprobe, 0, 4, s);
     MapView v{};
-    v.slots = (const uint4*)map.slots.p;
-    v.slot_icov = (const float4*)map.slot_icov.p;
-    v.slot_vidx = (const int32_t*)map.slot_vidx.p;
     v.mask = (uint32_t)(cap - 1);
     v.max_probe = 0;
+    uint64_t cells = 1, mcells = 1;
     for (int a = 0; a < 3; ++a) {
         v.min_cell[a] = g.mn[a];
         v.bits[a] = bits[a];
+        v.ext[a] = (uint32_t)((int64_t)g.mx[a] - (int64_t)g.mn[a] + 1);
+        cells *= v.ext[a];
+        mcells *= (uint64_t)v.ext[a] + 2;
     }
     v.res = cfg.resolution;
     v.inv_res = 1.0f / cfg.resolution;
@@ -1692,41 +1688,56 @@ int finish_map(Map& map, BuildScratch& sc, const SegRec* rec, const uint32_t* va
         float fr = frexpf(v.inv_res, &ex);
         v.exact_inv = (fr == 0.5f) ? 1 : 0;
     }
-    k_hash_insert<<<(V + 127) / 128, 128, 0, s>>>(
-        (int32_t*)map.vox_coord.p, (float4*)map.vox_mean.p, (float*)map.vox_icov.p, V, v,
-        (uint4*)map.slots.p, (float4*)map.slot_icov.p, (int32_t*)map.slot_vidx.p, mprobe,
-        d_status);
-    // dense cell index over the bounding box of the map's cells, when it fits the budget
-    uint64_t cells = 1;
-    for (int a = 0; a < 3; ++a) {
-        v.ext[a] = (uint32_t)((int64_t)g.mx[a] - (int64_t)g.mn[a] + 1);
-        cells *= v.ext[a];
-    }
-    v.grid = nullptr;
-    v.nmask = nullptr;
-    v.msh = 0;
-    const uint64_t mcells = (uint64_t)(v.ext[0] + 2) * (v.ext[1] + 2) * (v.ext[2] + 2);
-    uint64_t mwords = 0;
-    if (cfg.cell_index != NDT_CELL_INDEX_HASH && cells * 16 <= DENSE_GRID_MAX_BYTES) {
-        // octant masks (eight words per cell of the grown box) while they fit their budget,
-        // or (NDT_CELL_INDEX_OCTANT) while grid and masks fit the dense index's
-        const bool oct = cfg.cell_index == NDT_CELL_INDEX_OCTANT
-                             ? cells * 16 + mcells * 32 <= DENSE_GRID_MAX_BYTES
-                             : mcells * 32 <= OCTANT_MASK_MAX_BYTES;
-        v.msh = oct ? 3u : 0u;
-        mwords = mcells << v.msh;
-        if ((rc = dev_reserve(map.grid, (size_t)cells * 16)) ||
-            (rc = dev_reserve(map.nmask, (size_t)mwords * 4)))
-            return rc;
-        cudaMemsetAsync(map.grid.p, 0xFF, (size_t)cells * 16, s);
-        cudaMemsetAsync(map.nmask.p, 0, (size_t)mwords * 4, s);
-        k_grid_fill<<<(unsigned)((cap + 255) / 256), 256, 0, s>>>(v, (float4*)map.grid.p);
-        if (v.msh)
-            k_grid_mask<true><<<(unsigned)((cap + 255) / 256), 256, 0, s>>>(v, (uint32_t*)map.nmask.p);
-        else
-            k_grid_mask<false><<<(unsigned)((cap + 255) / 256), 256, 0, s>>>(v, (uint32_t*)map.nmask.p);
+    // dense cell index over the bounding box of the map's cells, when it fits the budget, with
+    // octant masks (eight words per cell of the grown box) while they fit theirs, or
+    // (NDT_CELL_INDEX_OCTANT) while grid and masks fit the dense index's
+    const bool dense =
+        cfg.cell_index != NDT_CELL_INDEX_HASH && cells * 16 <= DENSE_GRID_MAX_BYTES;
+    const bool oct = dense && (cfg.cell_index == NDT_CELL_INDEX_OCTANT
+                                   ? cells * 16 + mcells * 32 <= DENSE_GRID_MAX_BYTES
+                                   : mcells * 32 <= OCTANT_MASK_MAX_BYTES);
+    v.msh = oct ? 3u : 0u;
+    const uint64_t mwords = dense ? mcells << v.msh : 0;
+    if ((rc = dev_reserve(map.vox_coord, (size_t)V * 12)) ||
+        (rc = dev_reserve(map.vox_mean, (size_t)V * 16)) ||
+        (rc = dev_reserve(map.vox_cov, (size_t)V * 36)) ||
+        (rc = dev_reserve(map.vox_icov, (size_t)V * 36)) ||
+        (rc = dev_reserve(map.vox_count, (size_t)V * 4)) ||
+        (rc = dev_reserve(map.slots, cap * (dense ? 4 : 16))) ||
+        (rc = dev_reserve(map.icov8, (dense ? (size_t)V : (size_t)cap) * 32)))
+        return rc;
+    if (dense ? (rc = dev_reserve(map.grid, (size_t)cells * 16)) ||
+                    (rc = dev_reserve(map.nmask, (size_t)mwords * 4))
+              : (rc = dev_reserve(map.slot_vidx, cap * 4)))
+        return rc;
+    v.icov8 = (const float*)map.icov8.p;
+    cudaMemsetAsync(map.slots.p, 0xFF, cap * (dense ? 4 : 16), s);
+    cudaMemsetAsync(mprobe, 0, 4, s);
+    v.rmean = (const float4*)(dense ? map.vox_mean.p : map.slots.p);
+    if (dense) {
         v.grid = (const float4*)map.grid.p;
         v.nmask = (const uint32_t*)map.nmask.p;
+        cudaMemsetAsync(map.grid.p, 0xFF, (size_t)cells * 16, s);
+        cudaMemsetAsync(map.nmask.p, 0, (size_t)mwords * 4, s);
+    } else {
+        v.slots = (const uint4*)map.slots.p;
+        v.slot_vidx = (const int32_t*)map.slot_vidx.p;
+    }
+    k_voxel_compact<<<(S + 127) / 128, 128, 0, s>>>(
+        rec, valid, (uint32_t*)sc.seg_rank.p, S, (int32_t*)map.vox_coord.p,
+        (float4*)map.vox_mean.p, (float*)map.vox_cov.p, (float*)map.vox_icov.p,
+        (uint32_t*)map.vox_count.p, v, (float4*)map.icov8.p, dense ? (float4*)map.grid.p : nullptr,
+        (uint32_t*)map.slots.p, (uint4*)map.slots.p, (int32_t*)map.slot_vidx.p, mprobe, d_status);
+    if (dense) {
+        const unsigned gv = (V + 127) / 128;
+        if (oct)
+            k_grid_mask<true><<<gv, 128, 0, s>>>(v, (const int32_t*)map.vox_coord.p,
+                                                 (const float4*)map.vox_mean.p,
+                                                 (uint32_t*)map.nmask.p);
+        else
+            k_grid_mask<false><<<gv, 128, 0, s>>>(v, (const int32_t*)map.vox_coord.p,
+                                                  (const float4*)map.vox_mean.p,
+                                                  (uint32_t*)map.nmask.p);
     }
     uint32_t hprobe = 0;
     cudaMemcpyAsync(&hprobe, mprobe, 4, cudaMemcpyDeviceToHost, s);
