@@ -37,7 +37,9 @@ namespace cg = cooperative_groups;
 namespace ndtgb {
 
 constexpr int MAX_WARPS = 16;
-constexpr int NFR = 52;           // per-iteration frame: R,t hi (12), R,t lo (12), A_k (27)
+// per-iteration frame, 15 float4 rows: {R row i, t_i} hi parts (3), lo parts (3), then the
+// rows of A_r, A_p, A_y (9, padded), so the point work reads it with 128-bit loads
+constexpr int NFR = NFRAME;
 // line-search candidate sums: score, G[3], G p^T [3x3], correspondence count (14 used)
 constexpr int LS_VALS = 16, LS_USED = 14;
 
@@ -53,27 +55,30 @@ struct SolveScratch {
     int have_w;    // W is set
 };
 
-struct AlignShared {
+// The controller's state of one alignment, in shared memory
+struct CtlShared {
     SolveScratch solve;
-    unsigned long long cyc[4];  // rank 0: points+CTA reduce, cluster wait, control, broadcast
     int n_eigen;
-    double warp_part[MAX_WARPS][NRED];
-    double part[NRED];
     double tot[NRED];
     double pose[6];
     double H[36];
     double g[6];
     double trig[16];            // sin/cos of roll, pitch, yaw, 1 (exact; then small-angle rule)
     double Ad[27], Bd[54];      // dR/dtheta_k and d2R/dtheta_k dtheta_l at `pose` (FP64)
-    float fr[NFR];
-    int done;
-    // rank-0 controller state
+    __align__(16) float fr[NFR];
     double best_pose[6];
     double best_score;
     double last_H[36];
     double prev[3], prev2[3];
     int last_corr;
     int osc, max_osc;
+};
+
+struct AlignShared : CtlShared {
+    unsigned long long cyc[4];  // rank 0: points+CTA reduce, cluster wait, control, broadcast
+    double warp_part[MAX_WARPS][NRED];
+    double part[NRED];
+    int done;
     // line search: direction, start pose, phi(0), phi'(0), candidate step lengths, poses,
     // frames (every rank), A_k at each candidate pose, per-candidate sums. The graph path
     // scores up to 8 candidates; the CPU path's More-Thuente search one trial per round.
@@ -86,7 +91,7 @@ struct AlignShared {
     int mt_open, mt_iter, mt_first;
     double ls_alpha[LS_MAX], ls_pose[LS_MAX][6], ls_phi[LS_MAX], ls_dphi[LS_MAX];
     double ls_Ad[LS_MAX][27], ls_trig[LS_MAX][16];
-    float ls_fr[LS_MAX][NFR];
+    __align__(16) float ls_fr[LS_MAX][NFR];
     double ls_part[LS_MAX][LS_VALS], ls_tot[LS_MAX][LS_VALS];
 };
 
@@ -153,13 +158,14 @@ __device__ __noinline__ void make_frame_warp(const double* pose, bool small, flo
         trig[9 + 2 * lane] = tiny ? 1.0 : c;
         const double t = pose[lane];
         const float h = (float)t;
-        fr[9 + lane] = h;
-        fr[21 + lane] = (float)(t - (double)h);
+        fr[4 * lane + 3] = h;
+        fr[12 + 4 * lane + 3] = (float)(t - (double)h);
     }
     if (lane == 3) {
         trig[6] = 1.0;
         trig[14] = 1.0;
     }
+    if (lane < 9) fr[24 + 4 * lane + 3] = 0.f;  // padding
     __syncwarp();
     // a lane's (up to) three terms are independent: unrolled, their FP64 chains overlap
 #pragma unroll
@@ -175,10 +181,10 @@ __device__ __noinline__ void make_frame_warp(const double* pose, bool small, flo
                          (c1 == 0u ? 0.0 : (c1 == 1u ? t1 : -t1));
         if (e < 9) {
             const float h = (float)v;
-            fr[e] = h;
-            fr[12 + e] = (float)(v - (double)h);
+            fr[4 * (e / 3) + e % 3] = h;
+            fr[12 + 4 * (e / 3) + e % 3] = (float)(v - (double)h);
         } else if (e < 36) {
-            fr[24 + (e - 9)] = (float)v;
+            fr[24 + 4 * ((e - 9) / 3) + e % 3] = (float)v;
             Ad[e - 9] = v;
         } else {
             Bd[e - 36] = v;
@@ -599,17 +605,20 @@ __device__ __forceinline__ void transform_point(const float* fr, const float* pv
                                                 float* ql) {
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-        float hi = fr[9 + i], lo = fr[21 + i];
+        const float4 h4 = reinterpret_cast<const float4*>(fr)[i];
+        const float4 l4 = reinterpret_cast<const float4*>(fr)[3 + i];
+        const float rh[3] = {h4.x, h4.y, h4.z}, rl[3] = {l4.x, l4.y, l4.z};
+        float hi = h4.w, lo = l4.w;
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
-            float r = fr[3 * i + j];
+            float r = rh[j];
             float ph = r * pv[j];
             float pl = fmaf(r, pv[j], -ph);      // exact product error
             float s = hi + ph;                   // TwoSum(hi, ph)
             float bb = s - hi;
             float e = (hi - (s - bb)) + (ph - bb);
             hi = s;
-            lo += e + pl + fr[12 + 3 * i + j] * pv[j];
+            lo += e + pl + rl[j] * pv[j];
         }
         float s = hi + lo;                       // FastTwoSum renormalisation
         ql[i] = lo - (s - hi);
@@ -724,8 +733,8 @@ template <bool CPU_SEM>
 __device__ __forceinline__ void point_terms(const MapView& m, const uint32_t* off27,
                                             float px, float py, float pz,
                                             const float* fr, int max_nb, float d1f, float d2f,
-                                            float* acc, float* sacc, int& ncorr, uint32_t* list,
-                                            int stride) {
+                                            float* acc, float* sacc, int& ncorr,
+                                            uint32_t* list, int stride) {
     const float pv[3] = {px, py, pz};
     float qh[3], ql[3];
     transform_point(fr, pv, qh, ql);
@@ -851,9 +860,10 @@ __device__ __forceinline__ void point_contract(const float* pv, const float* fr,
 #pragma unroll
     for (int k = 0; k < 3; ++k)
 #pragma unroll
-        for (int a = 0; a < 3; ++a)
-            J[k][a] = fmaf(fr[24 + 9 * k + 3 * a], pv[0],
-                           fmaf(fr[25 + 9 * k + 3 * a], pv[1], fr[26 + 9 * k + 3 * a] * pv[2]));
+        for (int a = 0; a < 3; ++a) {
+            const float4 A = reinterpret_cast<const float4*>(fr)[6 + 3 * k + a];
+            J[k][a] = fmaf(A.x, pv[0], fmaf(A.y, pv[1], A.z * pv[2]));
+        }
 #pragma unroll
     for (int k = 0; k < 3; ++k)
 #pragma unroll
@@ -969,7 +979,7 @@ __device__ __noinline__ void finalize_gH(const double* tot, const double* Ad, co
     }
 }
 
-__device__ __forceinline__ void osc_update(AlignShared& sh, const double* pose, int it) {
+__device__ __forceinline__ void osc_update(CtlShared& sh, const double* pose, int it) {
     if (it >= 1) {
         double cv[3], pv[3];
         for (int a = 0; a < 3; ++a) {
@@ -1020,7 +1030,7 @@ __device__ void write_out(AlignOut& o, const double* pose, double score, const d
 // correspondence check, the best score and pose, the singular and converged exits; else the
 // unit ascent direction in x (reversed when g.x <= 0) and the Newton step's norm in *dn.
 // Returns 1 when the alignment is finished (outputs written). Lane 0.
-__device__ int cpu_direction(const AlignParams& P, AlignShared& sh, const AlignJob& job,
+__device__ int cpu_direction(const AlignParams& P, CtlShared& sh, const AlignJob& job,
                              AlignOut& o, int it, double score, int ncorr, double* x,
                              double* dn_out) {
     if (ncorr < P.min_corr) {
@@ -1062,7 +1072,7 @@ __device__ int cpu_direction(const AlignParams& P, AlignShared& sh, const AlignJ
 
 // CPU path, second half: pose += step x (apply_pose_delta, types.rs:183-200), the oscillation
 // history, the max-iteration exit (best pose). Returns 1 when the alignment is finished.
-__device__ int cpu_step(const AlignParams& P, AlignShared& sh, AlignOut& o, int it,
+__device__ int cpu_step(const AlignParams& P, CtlShared& sh, AlignOut& o, int it,
                         const double* x, double step) {
     for (int i = 0; i < 6; ++i) sh.pose[i] += x[i] * step;
     osc_update(sh, sh.pose, it);
@@ -1075,7 +1085,7 @@ __device__ int cpu_step(const AlignParams& P, AlignShared& sh, AlignOut& o, int 
 }
 
 template <bool CPU_SEM>
-__device__ __noinline__ int control_step(const AlignParams& P, AlignShared& sh, const AlignJob& job,
+__device__ __noinline__ int control_step(const AlignParams& P, CtlShared& sh, const AlignJob& job,
                             AlignOut& o, int it, double score, int ncorr) {
     double* pose = sh.pose;
     const double* g = sh.g;
@@ -1504,8 +1514,8 @@ __global__ void __launch_bounds__(THREADS, 65536 / (THREADS * REGCAP))
             float px = __ldg(pts + 3 * (size_t)i), py = __ldg(pts + 3 * (size_t)i + 1),
                   pz = __ldg(pts + 3 * (size_t)i + 2);
             if (!(isfinite(px) && isfinite(py) && isfinite(pz))) continue;
-            point_terms<CPU_SEM>(m, s_off27, px, py, pz, fr, P.max_nb, P.d1f, P.d2f, acc, sacc, nc,
-                                 list_smem + tid, THREADS);
+            point_terms<CPU_SEM>(m, s_off27, px, py, pz, fr, P.max_nb, P.d1f, P.d2f, acc, sacc,
+                                 nc, list_smem + tid, THREADS);
         }
 #pragma unroll
         for (int k = 0; k < NACC - A_HTR; ++k) acc[A_HTR + k] = sacc[k * THREADS];
@@ -1735,13 +1745,24 @@ __global__ void __launch_bounds__(THREADS, 65536 / (THREADS * REGCAP))
 //
 // In k_ndt_align a cluster owns one alignment for all its iterations, so a batch runs in
 // waves: alignments that need many iterations and start late set the batch's makespan, and
-// the cluster's other warps idle while rank 0 runs the FP64 step. Here the unit of work is a
-// chunk of one alignment's points for one iteration. A persistent grid of CTAs (all resident)
-// claims chunks of any open alignment, oldest alignment first; each chunk's sums go to global
-// memory in FP64, and the CTA that finishes the last chunk of an iteration runs that
-// alignment's Newton step (the same controller code) and publishes the next frame. Other
-// alignments' chunks keep every SM busy meanwhile, and the last alignments of a batch spread
-// over the whole GPU.
+// the cluster's other warps idle while rank 0 runs the FP64 step. Here the unit of work is 32
+// lanes' share of one alignment's points for one iteration (a unit: what one warp sums), handed
+// out at two levels: a persistent grid of CTAs (all resident) claims chunks of up to QUNITS
+// units of any open alignment, lowest iteration first, and the warps of a CTA pull the units of
+// its chunks as they become free. Nothing in the loop is a block barrier: a warp that finishes
+// early goes on to the next chunk (claimed by the first warp that finds the last one
+// exhausted) while others still work, and a warp in the FP64 step holds up nobody. (With
+// block barriers around each chunk they were the second largest stall: 2.76 cycles an issued
+// instruction of about 11.) The warp that ends a chunk's last unit sums the chunk's units and
+// writes the sums to global memory in FP64; the warp that ends an iteration's last chunk sums
+// the chunks in order, runs that alignment's Newton step (the same controller code) and
+// publishes the next frame.
+//
+// Which points a lane sums, and in which order, is the launch's partition (QPart below): the
+// ranks and threads of a cluster shape (the default's rule in the host's choose_shape, so a
+// lane's f32 sums are those of k_ndt_align at that shape), or runs of `queue` points per
+// thread. Sums of lanes, units and chunks have a fixed order, so results do not depend on which
+// warp ran what.
 //
 // Claims: QJob.gen_claim packs the alignment's iteration (high word) and the chunks claimed
 // so far (low word), so one atomicAdd both claims a chunk and names its iteration. The
@@ -1749,10 +1770,11 @@ __global__ void __launch_bounds__(THREADS, 65536 / (THREADS * REGCAP))
 // fence after a claim and read shared state through L2 (__ldcg), since L1 is not coherent
 // across SMs. A chunk's partial sums are written behind a fence before its done counter is
 // incremented; the controller, after the increment that completes the iteration, fences and
-// sums the partials in chunk order, so results do not depend on which CTA ran which chunk.
+// sums the partials in chunk order.
 // No CTA ever waits for another; a CTA that finds nothing to claim polls, and gives up with a
 // status bit after P.stall_ns (2 s) without work (every alignment ends within max_iterations
-// steps).
+// steps). Inside a CTA a warp waits only for a warp that is running: for a claim in progress,
+// or for a chunk slot or a controller area to be released.
 // Host batches may still be copying in when the kernel starts (P.qarrive): the points are laid
 // out largest alignment first, in copy chunks that start on 768-byte boundaries, and a copy
 // stream writes the count of resident points after each chunk. An alignment's first
@@ -1780,20 +1802,58 @@ __device__ __forceinline__ uint32_t qw_nch(unsigned long long w) {
     return (uint32_t)(w >> 32) & 0xFFFFu;
 }
 
-// Chunks of iteration `it` of an alignment with n points: n / qchunk for its first
-// QSPLIT_ITER iterations, then QSPLIT_DIV times as many, that much smaller, and from
-// QSPLIT_ITER2 on twice as many again (few alignments run that long). The alignments that
-// run long are the ones that finish a batch, on an otherwise idle GPU: smaller chunks spread
+// Partition of iteration `it` of an alignment with n points into `units` units.
+// P.qranks > 0 (a cluster shape's partition): thread t of rank r sums the points
+// r T + t, r T + t + qranks T, ...; unit r T / 32 + w is warp w of rank r.
+// P.qranks = 0: runs of `size` points, T threads striding each; unit (T / 32) v + w is warp w
+// of run v. `size` is qchunk for the first QSPLIT_ITER iterations, then 1 / QSPLIT_DIV of it,
+// and from QSPLIT_ITER2 on half of that again (few alignments run that long). The alignments
+// that run long are the ones that finish a batch, on an otherwise idle GPU: smaller runs spread
 // each of their iterations over more SMs. The rule depends on the iteration alone, so every
-// run sums an alignment's chunks over the same tree (results are identical run to run). At
-// most QMAXCH.
+// run sums an alignment's points over the same tree (results are identical run to run).
+// Chunks hold P.qunits units; at most QMAXCH chunks.
 constexpr uint32_t QSPLIT_ITER = 10, QSPLIT_ITER2 = 20;
-__device__ __forceinline__ uint32_t queue_chunks(const AlignParams& P, uint32_t n, uint32_t it) {
-    const uint32_t size =
-        it < QSPLIT_ITER ? (uint32_t)P.qchunk
-                         : max(1u, (uint32_t)P.qchunk / (it < QSPLIT_ITER2 ? QSPLIT_DIV
-                                                                          : 2 * QSPLIT_DIV));
-    return min(n ? (n + size - 1u) / size : 1u, QMAXCH);
+struct QPart {
+    uint32_t units, chunks;
+    uint32_t runs, size;  // qranks = 0
+};
+__device__ __forceinline__ QPart queue_part(const AlignParams& P, uint32_t n, uint32_t it) {
+    const uint32_t upr = (uint32_t)P.qthreads / 32u;  // units per rank or run
+    QPart q;
+    if (P.qranks > 0) {
+        q.runs = (uint32_t)P.qranks;
+        q.size = 0u;
+    } else {
+        const uint32_t want =
+            it < QSPLIT_ITER ? (uint32_t)P.qchunk
+                             : max(1u, (uint32_t)P.qchunk / (it < QSPLIT_ITER2 ? QSPLIT_DIV
+                                                                              : 2 * QSPLIT_DIV));
+        q.runs = min(n ? (n + want - 1u) / want : 1u, QMAXCH * (uint32_t)P.qunits / upr);
+        q.size = (n + q.runs - 1u) / q.runs;
+    }
+    q.units = q.runs * upr;
+    // a cluster's partition of a small scan leaves its last warps without points
+    if (P.qranks > 0) q.units = max(1u, min(q.units, (n + 31u) / 32u));
+    q.chunks = (q.units + P.qunits - 1u) / P.qunits;
+    return q;
+}
+
+// The points of lane `lane` of unit u: first, first + step, ... below end
+__device__ __forceinline__ void unit_points(const AlignParams& P, const QPart& q, uint32_t n,
+                                            uint32_t u, int lane, uint32_t& first,
+                                            uint32_t& step, uint32_t& end) {
+    const uint32_t T = (uint32_t)P.qthreads, upr = T / 32u;
+    const uint32_t r = u / upr, t = (u % upr) * 32u + lane;
+    if (P.qranks > 0) {
+        first = r * T + t;
+        step = (uint32_t)P.qranks * T;
+        end = n;
+    } else {
+        const uint32_t f = min(n, r * q.size);
+        first = f + t;
+        step = T;
+        end = min(n, f + q.size);
+    }
 }
 
 // Initial state of every alignment: controller state at the initial pose, the first frame,
@@ -1802,7 +1862,7 @@ template <bool CPU_SEM>
 __global__ void __launch_bounds__(128) k_queue_init(const AlignParams P) {
     __shared__ double s_trig[4][16];
     __shared__ double s_pose[4][6];
-    __shared__ float s_fr[4][NFR];
+    __shared__ __align__(16) float s_fr[4][NFR];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t j = blockIdx.x * 4 + w;
     if (j >= P.num_jobs) return;
@@ -1821,7 +1881,7 @@ __global__ void __launch_bounds__(128) k_queue_init(const AlignParams P) {
         q->point_iters = q->corr_total = 0;
         q->cyc_chunks = q->cyc_ctl = 0;
         q->t_start = 0;
-        const uint32_t nch0 = queue_chunks(P, job.n, 0u);
+        const uint32_t nch0 = queue_part(P, job.n, 0u).chunks;
         // withhold (test hook): every chunk of the first iteration already claimed
         P.qjobs[j].gen_claim = qword(0u, nch0) | (P.withhold ? (unsigned long long)nch0 : 0ull);
         P.qjobs[j].done = 0u;
@@ -1838,7 +1898,7 @@ __global__ void __launch_bounds__(128) k_queue_init(const AlignParams P) {
 // two shuffle rounds add them, lane 0 decides. A dependent FP64 instruction costs about 170
 // cycles on this part, so the three axes in parallel shorten the chain from about 20 such
 // instructions to 6. Same tests as osc_update.
-__device__ __forceinline__ void osc_update_warp(AlignShared& sh, int it, int lane) {
+__device__ __forceinline__ void osc_update_warp(CtlShared& sh, int it, int lane) {
     double cc = 0.0, pp = 0.0, cp = 0.0;
     if (it >= 1 && lane < 3) {
         const double c = sh.pose[lane] - sh.prev[lane];
@@ -1876,7 +1936,7 @@ __device__ __forceinline__ void osc_update_warp(AlignShared& sh, int it, int lan
 // compared on its square, and the clamp's scale step_size / |delta| comes from an f32
 // reciprocal square root refined by one FP64 Newton step (relative error below 1e-14), so the
 // FP64 chain has no square root or division.
-__device__ __noinline__ int control_step_graph_warp(const AlignParams& P, AlignShared& sh,
+__device__ __noinline__ int control_step_graph_warp(const AlignParams& P, CtlShared& sh,
                                                     AlignOut& o, int it, double score,
                                                     int ncorr, int lane) {
     double xi = 0.0, gi = 0.0;
@@ -1918,7 +1978,7 @@ __device__ __noinline__ int control_step_graph_warp(const AlignParams& P, AlignS
 }
 
 // Element e of QCtl's FP64 block, in the controller's shared state
-__device__ __forceinline__ double* qctl_slot(AlignShared& sh, int e) {
+__device__ __forceinline__ double* qctl_slot(CtlShared& sh, int e) {
     if (e < 6) return sh.pose + e;
     if (e < 12) return sh.best_pose + (e - 6);
     if (e < 13) return &sh.best_score;
@@ -1933,9 +1993,9 @@ __device__ __forceinline__ double* qctl_slot(AlignShared& sh, int e) {
 // Newton step of alignment `job` after its iteration `it` (warp 0 of the CTA that finished
 // the iteration's last chunk, once the CTA has summed the chunk partials into sh.tot):
 // state from global memory, the controller of k_ndt_align, then the next frame and claim
-// word (or the outputs) published.
+// word (or the outputs) published. Returns 1 (every lane) when the alignment is finished.
 template <bool CPU_SEM>
-__device__ __noinline__ void queue_control(const AlignParams& P, AlignShared& sh, int job,
+__device__ __noinline__ int queue_control(const AlignParams& P, CtlShared& sh, int job,
                                            uint32_t it, int lane) {
     const unsigned long long c0 = clock64();
     QCtl* q = P.qctl + job;
@@ -2063,328 +2123,465 @@ __device__ __noinline__ void queue_control(const AlignParams& P, AlignShared& sh
     if (lane == 0) {
         if (done) {
             atomicExch(&P.qjobs[job].gen_claim, qword(QDONE, 0u));
-            atomicAdd(P.qcount, 1u);
         } else {
-            atomicExch(&P.qjobs[job].gen_claim, qword(it + 1u, queue_chunks(P, jb.n, it + 1u)));
+            atomicExch(&P.qjobs[job].gen_claim, qword(it + 1u, queue_part(P, jb.n, it + 1u).chunks));
         }
     }
     __syncwarp();
+    return done;
 }
 
-template <int THREADS, bool CPU_SEM, int REGCAP, int NPW>
-__global__ void __launch_bounds__(THREADS, 65536 / (THREADS * REGCAP))
-    k_ndt_queue(const AlignParams P) {
-    constexpr int NW = THREADS / 32;
-    __shared__ AlignShared sh;
-    __shared__ uint32_t s_off27[32];  // neighbour offsets of the dense index
-    __shared__ int s_job, s_lw, s_flag;
-    __shared__ uint32_t s_chunk, s_gen, s_nch;
-    // dynamic shared memory as in k_ndt_align: neighbour lists, then the trailing accumulators
-    extern __shared__ uint32_t list_smem[];
-    float* const sacc =
-        reinterpret_cast<float*>(list_smem + (size_t)P.max_nb * THREADS) + threadIdx.x;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const MapView& m = P.map;
+constexpr int QT = 256;          // threads per CTA
+constexpr int QNW = QT / 32;
+constexpr int QSLOTS = 4;        // chunks a CTA has in hand
+constexpr int QCTLS = 2;         // Newton steps a CTA runs at a time
+constexpr int QREADY = 16;        // more than the alignments a CTA can have in hand
+constexpr uint32_t QSTAY = 152;  // CTAs that stay to the end of a batch: one per SM
+
+// A chunk in a CTA's hands
+struct QSlot {
+    int job;
+    uint32_t chunk, gen, nch;
+    uint32_t unit0, units;       // its first unit, its unit count
+    uint32_t n;
+    QPart part_of;
+    const float* pts;
+    unsigned long long c0;       // clock at the claim
+    int left;                    // units not yet handed out; <= 0: exhausted, or being filled
+    unsigned int done;           // units summed
+    int busy;
+    __align__(16) float fr[NFR];
+    double part[QUNITS][NRED];   // the units' sums
+};
+
+struct QShared {
+    uint32_t off27[32];          // neighbour offsets of the dense index
+    unsigned int head;           // sequence number of the open chunk (slot head % QSLOTS)
+    unsigned int claiming;       // a warp is claiming
+    unsigned int exit_;
+    unsigned int ctl_busy;       // bit c: controller area c in use; from bit 16: steps due
+    int lw;                      // first alignment not known to be finished
+    unsigned long long idle_since;
+    uint32_t seen_arrive;
+    // P.qsolo: alignments of this CTA whose next iteration is ready (0: free entry, else
+    // iteration << 32 | alignment + 1), a ring written by the warps that ran their steps and
+    // read by the claiming warp
+    unsigned long long ready[QREADY];
+    unsigned int ready_put, ready_get;
+    QSlot slot[QSLOTS];
+    CtlShared ctl[QCTLS];
+};
+
+__device__ __forceinline__ unsigned int ld_shared_volatile(const unsigned int* p) {
+    return *reinterpret_cast<const volatile unsigned int*>(p);
+}
+
+// Claims a chunk for the CTA (one warp): lowest iteration first, since alignments that need
+// many iterations form the batch's tail and none may fall behind while others run ahead. Pass
+// 0 finds the lowest iteration (saturated at 255) among the claimable alignments, from the
+// first one not known to be finished; pass 1 tries the claimable ones at that iteration in
+// order (from the oldest); if other CTAs took all of their chunks meanwhile, pass 2 takes any
+// claimable chunk, oldest alignment first. Returns the alignment or -1.
+// With P.qsolo (every iteration of every alignment is one chunk, and all points are resident) a
+// CTA keeps an alignment for all its iterations: it claims the ones whose step it has run, else
+// the next untouched one from a counter. The scan above reads every open alignment's word for
+// each claim: 9 us a claim with 3,200 alignments (16 x 200 particles of 3,200 points: 8.2 ms, 4.2 ms
+// this way).
+__device__ __forceinline__ int queue_claim(const AlignParams& P, QShared& q, int lane,
+                                           uint32_t& chunk, uint32_t& gen, uint32_t& nch) {
     const uint32_t B = P.num_jobs;
-    uint64_t idle_since = 0;    // thread 0
-    uint32_t seen_arrive = 0;   // thread 0: last value of the input counter seen
-    // the chunk's points, staged by one bulk copy (the TMA engine) into shared memory after
-    // the neighbour lists and accumulators: P.qchunk + 4 points (the copy starts on a 16-byte
-    // boundary, up to 3 points early)
-    __shared__ __align__(8) uint64_t s_stage_bar;
-    float* const stage =
-        reinterpret_cast<float*>(list_smem + (size_t)(P.max_nb + NACC - A_HTR) * THREADS);
-    uint32_t stage_phase = 0;
-    if (tid == 0) {
-        s_lw = 0;
-        if (P.qstage) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(
-                (uint32_t)__cvta_generic_to_shared(&s_stage_bar)));
-            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    int job = -1, first_open = -1;
+    if (P.qsolo) {
+        unsigned long long w = 0ull;
+        if (lane == 0) {
+            volatile unsigned long long* const e = &q.ready[q.ready_get % QREADY];
+            if ((w = *e) != 0ull) {
+                *e = 0ull;
+                q.ready_get++;
+            } else if (q.lw == 0) {
+                const uint32_t j = atomicAdd(P.qcount, 1u);
+                if (j < B)
+                    w = (unsigned long long)j + 1ull;
+                else
+                    q.lw = (int)B;
+            }
+        }
+        w = __shfl_sync(0xffffffffu, w, 0);
+        __threadfence();
+        chunk = 0;
+        nch = 1;
+        gen = (uint32_t)(w >> 32);
+        return (int)(uint32_t)w - 1;
+    }
+    // points resident while the batch is still being copied in (all: ~0)
+    uint32_t arrived = 0xFFFFFFFFu;
+    if (P.qarrive) {
+        arrived = ld_volatile32(P.qarrive);
+        if (arrived >= P.qarrive_total) arrived = 0xFFFFFFFFu;
+    }
+    // whether alignment j has a chunk to claim; open: not finished; g: its iteration
+    // (saturated at 255)
+    auto claimable = [&](uint32_t j, bool& open, uint32_t& g) -> bool {
+        const unsigned long long w = ld_volatile(&P.qjobs[j].gen_claim);
+        open = qw_gen(w) != QDONE;
+        g = min(qw_gen(w), 255u);
+        bool ok = open && (uint32_t)w < qw_nch(w);
+        if (ok && arrived != 0xFFFFFFFFu && qw_gen(w) == 0u)
+            ok = P.jobs[j].offset + P.jobs[j].n <= (uint64_t)arrived;
+        return ok;
+    };
+    uint32_t best = 0xFFFFFFFFu;  // min over claimable j of min(iteration, 255) << 24 | j
+#pragma unroll 4
+    for (uint32_t base = (uint32_t)q.lw; base < B; base += 32) {
+        const uint32_t j = base + lane;
+        bool open = false;
+        uint32_t g = 0;
+        if (j < B && claimable(j, open, g)) best = min(best, (g << 24) | j);
+        const unsigned om = __ballot_sync(0xffffffffu, open);
+        if (first_open < 0 && om) first_open = (int)base + __ffs(om) - 1;
+    }
+    best = __reduce_min_sync(0xffffffffu, best);
+    for (int pass = 1; pass <= 2 && job < 0 && best != 0xFFFFFFFFu; ++pass) {
+        const uint32_t gsel = best >> 24;
+        const uint32_t start =
+            pass == 1 ? ((best & 0xFFFFFFu) & ~31u) : (uint32_t)max(first_open, 0);
+        for (uint32_t base = start; base < B && job < 0; base += 32) {
+            const uint32_t j = base + lane;
+            bool ok = false, open = false;
+            uint32_t g = 0;
+            if (j < B) ok = claimable(j, open, g) && (pass == 2 || g == gsel);
+            unsigned okm = __ballot_sync(0xffffffffu, ok);
+            while (okm != 0u && job < 0) {
+                const int src = __ffs(okm) - 1;
+                okm &= okm - 1u;
+                unsigned long long old = 0ull;
+                if (lane == src) old = atomicAdd(&P.qjobs[j].gen_claim, 1ull);
+                old = __shfl_sync(0xffffffffu, old, src);
+                if (qw_gen(old) != QDONE && (uint32_t)old < qw_nch(old)) {
+                    job = (int)base + src;
+                    chunk = (uint32_t)old;
+                    gen = qw_gen(old);
+                    nch = qw_nch(old);
+                }
+            }
         }
     }
-    nbhd_offsets(m, s_off27);  // read after the loop's first barrier
-    for (;;) {
-        __syncthreads();  // the previous chunk (and controller) is finished with shared memory
-        if (warp == 0) {
-            // claim, lowest iteration first: alignments that need many iterations form the
-            // batch's tail, so none may fall behind while others run ahead. Pass 0 finds the
-            // lowest iteration (saturated at 255) among the claimable alignments, from the
-            // first one not known to be finished; pass 1 tries the claimable ones at that
-            // iteration in order (from the oldest); if other CTAs took all of their chunks
-            // meanwhile, pass 2 takes any claimable chunk, oldest alignment first.
-            int job = -1, first_open = -1;
-            uint32_t chunk = 0, gen = 0, nchunks = 0;
-            // points resident while the batch is still being copied in (all: ~0)
-            uint32_t arrived = 0xFFFFFFFFu;
-            if (P.qarrive) {
-                arrived = ld_volatile32(P.qarrive);
-                if (arrived >= P.qarrive_total) arrived = 0xFFFFFFFFu;
-            }
-            // whether alignment j has a chunk to claim; open: not finished; g: its iteration
-            // (saturated at 255)
-            auto claimable = [&](uint32_t j, bool& open, uint32_t& g) -> bool {
-                const unsigned long long w = ld_volatile(&P.qjobs[j].gen_claim);
-                open = qw_gen(w) != QDONE;
-                g = min(qw_gen(w), 255u);
-                bool ok = open && (uint32_t)w < qw_nch(w);
-                if (ok && arrived != 0xFFFFFFFFu && qw_gen(w) == 0u)
-                    ok = P.jobs[j].offset + P.jobs[j].n <= (uint64_t)arrived;
-                return ok;
-            };
-            uint32_t best = 0xFFFFFFFFu;  // min over claimable j of min(iteration, 255) << 24 | j
-#pragma unroll 4
-            for (uint32_t base = (uint32_t)s_lw; base < B; base += 32) {
-                const uint32_t j = base + lane;
-                bool open = false;
-                uint32_t g = 0;
-                if (j < B && claimable(j, open, g)) best = min(best, (g << 24) | j);
-                const unsigned om = __ballot_sync(0xffffffffu, open);
-                if (first_open < 0 && om) first_open = (int)base + __ffs(om) - 1;
-            }
-            best = __reduce_min_sync(0xffffffffu, best);
-            for (int pass = 1; pass <= 2 && job < 0 && best != 0xFFFFFFFFu; ++pass) {
-                const uint32_t gsel = best >> 24;
-                const uint32_t start =
-                    pass == 1 ? ((best & 0xFFFFFFu) & ~31u) : (uint32_t)max(first_open, 0);
-                for (uint32_t base = start; base < B && job < 0; base += 32) {
-                    const uint32_t j = base + lane;
-                    bool ok = false, open = false;
-                    uint32_t g = 0;
-                    if (j < B) ok = claimable(j, open, g) && (pass == 2 || g == gsel);
-                    unsigned okm = __ballot_sync(0xffffffffu, ok);
-                    while (okm != 0u && job < 0) {
-                        const int src = __ffs(okm) - 1;
-                        okm &= okm - 1u;
-                        unsigned long long old = 0ull;
-                        if (lane == src) old = atomicAdd(&P.qjobs[j].gen_claim, 1ull);
-                        old = __shfl_sync(0xffffffffu, old, src);
-                        if (qw_gen(old) != QDONE && (uint32_t)old < qw_nch(old)) {
-                            job = (int)base + src;
-                            chunk = (uint32_t)old;
-                            gen = qw_gen(old);
-                            nchunks = qw_nch(old);
-                        }
-                    }
-                }
-            }
-            __threadfence();  // acquire: the frame of the claimed iteration is published
-            if (lane == 0) {
-                s_lw = first_open >= 0 ? first_open : (int)B;
-                s_job = job;
-                s_chunk = chunk;
-                s_gen = gen;
-                s_nch = nchunks;
-            }
+    __threadfence();  // acquire: the frame of the claimed iteration is published
+    __syncwarp();
+    if (lane == 0) q.lw = first_open >= 0 ? first_open : (int)B;
+    __syncwarp();
+    return job;
+}
+
+// Nothing to claim (lane 0 of the claiming warp): every alignment finished, or the open ones
+// wait for their Newton step. True when the CTA should leave.
+__device__ __forceinline__ bool queue_idle(const AlignParams& P, QShared& q) {
+    // a warp of this CTA still sums or steps: its alignment's next chunks may be this CTA's
+    bool active = ld_shared_volatile(&q.ctl_busy) != 0u;
+    for (int i = 0; i < QSLOTS; ++i)
+        active |= *reinterpret_cast<const volatile int*>(&q.slot[i].busy) != 0;
+    if (q.lw >= (int)P.num_jobs &&
+        !(P.qsolo && (active || *reinterpret_cast<const volatile unsigned long long*>(
+                                    &q.ready[q.ready_get % QREADY]) != 0ull)))
+        return true;
+    const unsigned long long now = global_ns();
+    bool fed = true;  // every point of the batch is resident
+    if (P.qarrive) {
+        const uint32_t a = ld_volatile32(P.qarrive);
+        fed = a >= P.qarrive_total;
+        if (a != q.seen_arrive) {  // input still arriving: not a stall
+            q.seen_arrive = a;
+            q.idle_since = 0;
         }
-        __syncthreads();
-        const int job = s_job;
-        if (job < 0) {
-            // nothing claimable: every alignment finished, or the open ones wait for their
-            // Newton step
-            if (tid == 0) {
-                int stop = s_lw >= (int)B;
-                if (!stop) {
-                    const uint64_t now = global_ns();
-                    bool fed = true;  // every point of the batch is resident
-                    if (P.qarrive) {
-                        const uint32_t a = ld_volatile32(P.qarrive);
-                        fed = a >= P.qarrive_total;
-                        if (a != seen_arrive) {  // input still arriving: not a stall
-                            seen_arrive = a;
-                            idle_since = 0;
-                        }
-                    }
-                    if (idle_since == 0) {
-                        idle_since = now;
-                    } else if (!fed && now - idle_since > QSTARVE_NS) {
-                        stop = 1;  // starved of input: the continuation launch finishes
-                    } else if (now - idle_since > P.stall_ns) {
-                        atomicOr(P.status, ST_QUEUE_STALL);
-                        stop = 1;
-                    } else if (fed && blockIdx.x >= gridDim.x / 4u &&
-                               now - idle_since > 20000ull) {
-                        // near the end of a batch: all but the first quarter of the grid
-                        // (by CTA index) leave after 20 us without work, so a kernel queued
-                        // on another stream (the next asynchronous batch) can take their
-                        // SMs; the quarter that stays serves the remaining iterations (with
-                        // fewer than 4 CTAs none stays idle, and the CTA running a Newton
-                        // step still claims the next iteration's chunks when it ends)
-                        stop = 1;
-                    }
+    }
+    if (active) q.idle_since = 0;
+    if (q.idle_since == 0) {
+        q.idle_since = now;
+    } else if (!fed && now - q.idle_since > QSTARVE_NS) {
+        return true;  // starved of input: the continuation launch finishes
+    } else if (now - q.idle_since > P.stall_ns) {
+        atomicOr(P.status, ST_QUEUE_STALL);
+        return true;
+    } else if (fed && blockIdx.x >= QSTAY && now - q.idle_since > 20000ull) {
+        // near the end of a batch: all but the first QSTAY CTAs leave after 20 us without
+        // work, so a kernel queued on another stream (the next asynchronous batch) can take
+        // their SMs; those that stay serve the remaining iterations
+        return true;
+    }
+    return false;
+}
+
+// Sums of one unit over its points, by one warp, into out[NRED]
+template <bool CPU_SEM, int NPW>
+__device__ __forceinline__ void unit_sums(const AlignParams& P, const QSlot& c,
+                                          const uint32_t* off27, uint32_t* list, float* sacc,
+                                          uint32_t u, int lane, double* out) {
+    const MapView& m = P.map;
+    const float* const pts = c.pts;
+    uint32_t first, step, end;
+    unit_points(P, c.part_of, c.n, u, lane, first, step, end);
+    float acc[NACC];
+#pragma unroll
+    for (int i = 0; i < A_HTR; ++i) acc[i] = 0.f;
+#pragma unroll
+    for (int k = 0; k < NACC - A_HTR; ++k) sacc[k * QT] = 0.f;
+    int nc = 0;
+    if (NPW > 1 && m.grid) {
+        // groups of NPW lanes share each point's neighbour search (search_group); every lane
+        // of the warp runs every round, with or without a point of its own
+        for (uint32_t i0 = first - lane; i0 < end; i0 += step) {
+            const uint32_t i = i0 + lane;
+            float pv[3] = {0.f, 0.f, 0.f}, qh[3] = {0.f, 0.f, 0.f}, ql[3] = {0.f, 0.f, 0.f};
+            uint32_t bits = 0u, corner = 0u;
+            if (i < end) {
+                for (int a = 0; a < 3; ++a) pv[a] = __ldg(pts + 3 * (size_t)i + a);
+                if (isfinite(pv[0]) && isfinite(pv[1]) && isfinite(pv[2])) {
+                    transform_point(c.fr, pv, qh, ql);
+                    int32_t gc[3];
+                    const uint32_t oct = cell_oct_of_sum(m, qh, ql, gc);
+                    bits = nbhd_mask(m, gc, oct, corner);
                 }
-                s_flag = stop;
             }
-            __syncthreads();
-            if (s_flag) break;
-            __nanosleep(500);
+            const int cnt =
+                search_group<NPW>(m, off27, qh, ql, bits, corner, P.max_nb, list, QT, lane);
+            __syncwarp();  // the group's list entries are visible to the point's lane
+            if (cnt > 0) {
+                PointSums ps{};
+                pair_terms<CPU_SEM>(m, qh, ql, cnt, P.d1f, P.d2f, list, QT, ps);
+                nc += cnt;
+                point_contract(pv, c.fr, ps, acc, sacc, QT);
+            }
+            __syncwarp();  // lists are read before the next round rewrites them
+        }
+    } else {
+        for (uint32_t i = first; i < end; i += step) {
+            const float px = __ldg(pts + 3 * (size_t)i), py = __ldg(pts + 3 * (size_t)i + 1),
+                        pz = __ldg(pts + 3 * (size_t)i + 2);
+            if (!(isfinite(px) && isfinite(py) && isfinite(pz))) continue;
+            point_terms<CPU_SEM>(m, off27, px, py, pz, c.fr, P.max_nb, P.d1f, P.d2f, acc, sacc,
+                                 nc, list, QT);
+        }
+        __syncwarp();
+    }
+#pragma unroll
+    for (int k = 0; k < NACC - A_HTR; ++k) acc[A_HTR + k] = sacc[k * QT];
+    warp_sum_acc(acc, lane, out);
+    nc = __reduce_add_sync(0xffffffffu, nc);
+    if (lane == 0) out[NACC] = (double)nc;
+}
+
+template <bool CPU_SEM, int REGCAP, int NPW>
+__global__ void __launch_bounds__(QT, 65536 / (QT * REGCAP)) k_ndt_queue(const AlignParams P) {
+    __shared__ QShared q;
+    // dynamic shared memory as in k_ndt_align: voxel lists, then the trailing accumulators
+    extern __shared__ uint32_t list_smem[];
+    const int tid = threadIdx.x, lane = tid & 31;
+    float* const sacc = reinterpret_cast<float*>(list_smem + (size_t)P.max_nb * QT) + tid;
+    nbhd_offsets(P.map, q.off27);
+    if (tid < QSLOTS) {
+        q.slot[tid].left = 0;
+        q.slot[tid].busy = 0;
+    }
+    if (tid == 0) {
+        q.head = 0;
+        q.claiming = q.exit_ = q.ctl_busy = 0;
+        q.ready_put = q.ready_get = 0;
+        for (int i = 0; i < QREADY; ++i) q.ready[i] = 0ull;
+        q.lw = 0;
+        q.idle_since = 0;
+        q.seen_arrive = 0;
+    }
+    __syncthreads();
+    for (;;) {
+        // a unit of the open chunk: one atomic on the count of units left names it or shows the
+        // chunk exhausted (should the slot have been refilled since `head` was read, the unit
+        // is one of the chunk that it holds now, which is as good)
+        const unsigned int head = ld_shared_volatile(&q.head);
+        QSlot& c = q.slot[head % QSLOTS];
+        int left = 0;
+        if (lane == 0 && *reinterpret_cast<const volatile int*>(&c.left) > 0)
+            left = atomicSub(&c.left, 1);
+        left = __shfl_sync(0xffffffffu, left, 0);
+        __threadfence_block();
+        if (left <= 0) {
+            // exhausted: one warp claims the next chunk, the others wait for it
+            if (ld_shared_volatile(&q.exit_)) break;
+            unsigned int busy = 1;
+            if (lane == 0) busy = atomicCAS(&q.claiming, 0u, 1u);
+            busy = __shfl_sync(0xffffffffu, busy, 0);
+            if (busy) {
+                __nanosleep(100);
+                continue;
+            }
+            __threadfence_block();
+            if (ld_shared_volatile(&q.head) != head) {  // another warp has just claimed
+                __syncwarp();
+                if (lane == 0) atomicExch(&q.claiming, 0u);
+                continue;
+            }
+            QSlot& s = q.slot[(head + 1u) % QSLOTS];
+            // its last chunk's stragglers: running warps (bounded all the same)
+            const unsigned long long t0 = global_ns();
+            bool ok = true;
+            while (*reinterpret_cast<const volatile int*>(&s.busy) != 0) {
+                __nanosleep(100);
+                if (global_ns() - t0 > QSTALL_NS) {
+                    ok = false;
+                    break;
+                }
+            }
+            uint32_t chunk = 0, gen = 0, nch = 0;
+            const int job = ok ? queue_claim(P, q, lane, chunk, gen, nch) : -1;
+            if (job < 0) {
+                if (lane == 0) {
+                    if (!ok) atomicOr(P.status, ST_WAIT_LIMIT);
+                    if (!ok || queue_idle(P, q))
+                        atomicExch(&q.exit_, 1u);
+                }
+                __syncwarp();
+                if (!ld_shared_volatile(&q.exit_)) __nanosleep(200);
+                __threadfence_block();
+                if (lane == 0) atomicExch(&q.claiming, 0u);
+                continue;
+            }
+            const AlignJob& jb = P.jobs[job];
+            for (int i = lane; i < NFR; i += 32)
+                s.fr[i] = __ldcg(P.qframe + (size_t)job * NFR + i);
+            if (lane == 0) {
+                q.idle_since = 0;
+                s.job = job;
+                s.chunk = chunk;
+                s.gen = gen;
+                s.nch = nch;
+                s.n = jb.n;
+                s.part_of = queue_part(P, jb.n, gen);
+                s.unit0 = chunk * (uint32_t)P.qunits;
+                s.pts = P.pts + 3 * jb.offset;
+                s.c0 = clock64();
+                s.done = 0;
+                s.busy = 1;
+                s.units = min((uint32_t)P.qunits, s.part_of.units - s.unit0);
+                if (gen == 0 && chunk == 0) __stcg(&P.qctl[job].t_start, global_ns());
+            }
+            __threadfence_block();
+            __syncwarp();
+            if (lane == 0) {
+                atomicExch(&s.left, (int)s.units);  // opens the slot
+                __threadfence_block();
+                atomicExch(&q.head, head + 1u);
+                atomicExch(&q.claiming, 0u);
+            }
+            __syncwarp();
             continue;
         }
-        if (tid == 0) idle_since = 0;
-        const unsigned long long c0 = clock64();
-        const uint32_t chunk = s_chunk, gen = s_gen, nchunks = s_nch;
-        const AlignJob& jb = P.jobs[job];
-        if (tid < NFR) sh.fr[tid] = __ldcg(P.qframe + (size_t)job * NFR + tid);
-        if (tid == 0 && gen == 0 && chunk == 0) __stcg(&P.qctl[job].t_start, global_ns());
-        __syncthreads();
-        const float* pts = P.pts + 3 * jb.offset;
-        const uint32_t csize = (jb.n + nchunks - 1u) / nchunks;  // this iteration's chunk size
-        const uint32_t first = min(jb.n, chunk * csize);
-        const uint32_t last = min(jb.n, first + csize);
-        // staged points: job-local indices below stage_end come from shared memory (point i
-        // at stage[3 (i - stage_first)]); the rest of the chunk (a ragged tail of less than
-        // 16 bytes, or every point when staging is off) from global memory
-        int64_t stage_first = 0, stage_end = 0;
-        if (P.qstage && last > first) {
-            const uint64_t g0 = (jb.offset + first) & ~3ull;  // 16-byte aligned point index
-            const uint64_t gend = jb.offset + last;
-            const uint32_t bytes = (uint32_t)(((gend - g0) * 12ull) & ~15ull);
-            if (bytes >= 16 && gend - g0 <= (uint64_t)P.qchunk + 4) {
-                const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&s_stage_bar);
-                if (tid == 0) {
-                    // the CTA's reads of the previous chunk (generic proxy) precede this write
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
-                                     bar),
-                                 "r"(bytes)
-                                 : "memory");
-                    asm volatile(
-                        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes "
-                        "[%0], [%1], %2, [%3];" ::"r"((uint32_t)__cvta_generic_to_shared(stage)),
-                        "l"(P.pts + 3 * g0), "r"(bytes), "r"(bar)
-                        : "memory");
-                }
-                // bounded wait (1 s of the global timer); a copy from global memory that does
-                // not land means the device is in trouble: report it and stop this CTA
-                const uint64_t t0 = global_ns();
-                bool done = false;
-                while (!done) {
-                    uint32_t ok;
-                    asm volatile(
-                        "{\n\t.reg .pred p;\n\t"
-                        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                        "selp.u32 %0, 1, 0, p;\n\t}"
-                        : "=r"(ok)
-                        : "r"(bar), "r"(stage_phase)
-                        : "memory");
-                    done = ok != 0;
-                    if (!done && global_ns() - t0 > 1000000000ull) break;
-                }
-                if (!__syncthreads_and(done ? 1 : 0)) {
-                    if (tid == 0) atomicOr(P.status, ST_STAGE_TIMEOUT);
-                    return;
-                }
-                stage_phase ^= 1u;
-                stage_first = (int64_t)g0 - (int64_t)jb.offset;
-                stage_end = stage_first + (int64_t)(bytes / 12u);
+        const uint32_t nunits = c.units, u = (uint32_t)left - 1u;
+        unit_sums<CPU_SEM, NPW>(P, c, q.off27, list_smem + tid, sacc, c.unit0 + u, lane,
+                                c.part[u]);
+        __threadfence_block();
+        __syncwarp();
+        unsigned int d = 0;
+        if (lane == 0) d = atomicAdd(&c.done, 1u);
+        d = __shfl_sync(0xffffffffu, d, 0);
+        if (d + 1u != nunits) continue;
+        // the chunk's last unit: its sums to global memory
+        __threadfence_block();
+        const int job = c.job;
+        const uint32_t gen = c.gen, nch = c.nch;
+        {
+            double* const part = P.qpart + ((size_t)P.qpart_off[job] + c.chunk) * NRED;
+            double s0 = 0.0, s1 = 0.0;
+            const int k1 = lane < NRED - 32 ? 32 + lane : lane;
+            for (uint32_t w = 0; w < nunits; ++w) {
+                s0 += c.part[w][lane];
+                s1 += c.part[w][k1];
             }
-        }
-        auto load_point = [&](uint32_t i, float* pv) {
-            if ((int64_t)i < stage_end) {
-                const float* q = stage + 3 * ((int64_t)i - stage_first);
-                pv[0] = q[0];
-                pv[1] = q[1];
-                pv[2] = q[2];
-            } else {
-                pv[0] = __ldg(pts + 3 * (size_t)i);
-                pv[1] = __ldg(pts + 3 * (size_t)i + 1);
-                pv[2] = __ldg(pts + 3 * (size_t)i + 2);
-            }
-        };
-        float acc[NACC];
-#pragma unroll
-        for (int i = 0; i < A_HTR; ++i) acc[i] = 0.f;
-#pragma unroll
-        for (int k = 0; k < NACC - A_HTR; ++k) sacc[k * THREADS] = 0.f;
-        int nc = 0;
-        if (NPW > 1 && m.grid) {
-            // groups of NPW lanes share each point's neighbour search (search_group); every
-            // lane of a warp runs every round, with or without a point of its own
-            for (uint32_t i0 = first; i0 < last; i0 += THREADS) {
-                const uint32_t i = i0 + tid;
-                float pv[3] = {0.f, 0.f, 0.f}, qh[3] = {0.f, 0.f, 0.f}, ql[3] = {0.f, 0.f, 0.f};
-                uint32_t bits = 0u, corner = 0u;
-                if (i < last) {
-                    load_point(i, pv);
-                    if (isfinite(pv[0]) && isfinite(pv[1]) && isfinite(pv[2])) {
-                        transform_point(sh.fr, pv, qh, ql);
-                        int32_t gc[3];
-                        const uint32_t oct = cell_oct_of_sum(m, qh, ql, gc);
-                        bits = nbhd_mask(m, gc, oct, corner);
-                    }
-                }
-                const int cnt = search_group<NPW>(m, s_off27, qh, ql, bits, corner, P.max_nb,
-                                                  list_smem + tid, THREADS, lane);
-                __syncwarp();  // the group's list entries are visible to the point's lane
-                if (cnt > 0) {
-                    PointSums ps{};
-                    pair_terms<CPU_SEM>(m, qh, ql, cnt, P.d1f, P.d2f, list_smem + tid, THREADS, ps);
-                    nc += cnt;
-                    point_contract(pv, sh.fr, ps, acc, sacc, THREADS);
-                }
-                __syncwarp();  // lists are read before the next round rewrites them
-            }
-        } else {
-            for (uint32_t i = first + tid; i < last; i += THREADS) {
-                float pv[3];
-                load_point(i, pv);
-                if (!(isfinite(pv[0]) && isfinite(pv[1]) && isfinite(pv[2]))) continue;
-                point_terms<CPU_SEM>(m, s_off27, pv[0], pv[1], pv[2], sh.fr, P.max_nb, P.d1f,
-                                     P.d2f, acc, sacc, nc, list_smem + tid, THREADS);
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < NACC - A_HTR; ++k) acc[A_HTR + k] = sacc[k * THREADS];
-        warp_sum_acc(acc, lane, sh.warp_part[warp]);
-        nc = __reduce_add_sync(0xffffffffu, nc);
-        if (lane == 0) sh.warp_part[warp][NACC] = (double)nc;
-        __syncthreads();
-        double* part = P.qpart + ((size_t)P.qpart_off[job] + chunk) * NRED;
-        for (int k = tid; k < NRED; k += THREADS) {
-            double s = 0.0;
-            for (int w = 0; w < NW; ++w) s += sh.warp_part[w][k];
-            __stcg(part + k, s);
+            __stcg(part + lane, s0);
+            if (lane < NRED - 32) __stcg(part + 32 + lane, s1);
         }
         __threadfence();
-        __syncthreads();
-        if (tid == 0) {
-            const uint32_t prev = atomicAdd(&P.qjobs[job].done, 1u);
-            s_flag = prev + 1u == nchunks;
-            atomicAdd(&P.qctl[job].cyc_chunks, (unsigned long long)(clock64() - c0));
+        __syncwarp();
+        unsigned int prev = 0;
+        if (lane == 0) {
+            prev = atomicAdd(&P.qjobs[job].done, 1u);
+            atomicAdd(&P.qctl[job].cyc_chunks, (unsigned long long)(clock64() - c.c0));
+            // a step to come keeps the CTA from leaving (bit 16 up count warps on their way)
+            if (prev + 1u == nch) atomicAdd(&q.ctl_busy, 0x10000u);
+            __threadfence_block();
+            *reinterpret_cast<volatile int*>(&c.busy) = 0;
         }
-        __syncthreads();
-        if (!s_flag) continue;
+        prev = __shfl_sync(0xffffffffu, prev, 0);
+        if (prev + 1u != nch) continue;
         __threadfence();  // acquire: every chunk's partials of this iteration are visible
-        // the iteration's sums, by the whole CTA in a fixed order: thread (value k, segment s)
-        // sums a contiguous run of chunks, then the segments are added in order
-        {
-            constexpr int NSEG = (THREADS / NRED) < MAX_WARPS ? (THREADS / NRED) : MAX_WARPS;
-            const uint32_t seg = (nchunks + NSEG - 1u) / NSEG;
-            const double* part0 = P.qpart + (size_t)P.qpart_off[job] * NRED;
-            if (tid < NSEG * NRED) {
-                const int k = tid % NRED, s = tid / NRED;
-                const uint32_t c_lo = min(nchunks, (uint32_t)s * seg);
-                const uint32_t c_hi = min(nchunks, c_lo + seg);
-                double v = 0.0;
-                for (uint32_t c = c_lo; c < c_hi; ++c) v += __ldcg(part0 + (size_t)c * NRED + k);
-                sh.warp_part[s][k] = v;
+        // the Newton step, in a free controller area (another warp's step at most ahead)
+        int area = -1;
+        const unsigned long long t0 = global_ns();
+        while (area < 0) {
+            if (lane == 0) {
+                const unsigned int b = ld_shared_volatile(&q.ctl_busy);
+                for (int i = 0; i < QCTLS && area < 0; ++i)
+                    if (!(b >> i & 1u) && !(atomicOr(&q.ctl_busy, 1u << i) >> i & 1u)) area = i;
             }
-            __syncthreads();
-            if (tid < NRED) {
-                double v = 0.0;
-                for (int s = 0; s < NSEG; ++s) v += sh.warp_part[s][tid];
-                sh.tot[tid] = v;
+            area = __shfl_sync(0xffffffffu, area, 0);
+            if (area >= 0) break;
+            __nanosleep(100);
+            if (global_ns() - t0 > QSTALL_NS) {
+                if (lane == 0) {
+                    atomicOr(P.status, ST_WAIT_LIMIT);
+                    atomicExch(&q.exit_, 1u);
+                }
+                break;
             }
-            __syncthreads();
         }
-        if (warp == 0) queue_control<CPU_SEM>(P, sh, job, gen, lane);
+        if (area < 0) break;
+        __threadfence_block();
+        CtlShared& ctl = q.ctl[area];
+        {
+            // the iteration's sums, chunks in order, four chains
+            const double* part0 = P.qpart + (size_t)P.qpart_off[job] * NRED;
+            const int k1 = lane < NRED - 32 ? 32 + lane : lane;
+            double a[4] = {0.0, 0.0, 0.0, 0.0}, b[4] = {0.0, 0.0, 0.0, 0.0};
+            uint32_t ch = 0;
+            for (; ch + 4 <= nch; ch += 4) {
+                double v[4], w[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    v[i] = __ldcg(part0 + (size_t)(ch + i) * NRED + lane);
+                    w[i] = __ldcg(part0 + (size_t)(ch + i) * NRED + k1);
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    a[i] += v[i];
+                    b[i] += w[i];
+                }
+            }
+            for (int i = 0; ch < nch; ++ch, ++i) {
+                a[0] += __ldcg(part0 + (size_t)ch * NRED + lane);
+                b[0] += __ldcg(part0 + (size_t)ch * NRED + k1);
+            }
+            ctl.tot[lane] = (a[0] + a[1]) + (a[2] + a[3]);
+            if (lane < NRED - 32) ctl.tot[32 + lane] = (b[0] + b[1]) + (b[2] + b[3]);
+            __syncwarp();
+        }
+        const int done = queue_control<CPU_SEM>(P, ctl, job, gen, lane);
+        __threadfence_block();
+        __syncwarp();
+        if (lane == 0) {
+            if (P.qsolo && !done) {
+                const unsigned int e = atomicAdd(&q.ready_put, 1u) % QREADY;
+                atomicExch(&q.ready[e], (unsigned long long)(gen + 1u) << 32 |
+                                            (unsigned long long)((uint32_t)job + 1u));
+                __threadfence_block();
+            }
+            atomicAnd(&q.ctl_busy, ~(1u << area));
+            atomicSub(&q.ctl_busy, 0x10000u);
+        }
     }
 }
 
-template <int T, bool SEM, int CAP, int NPW>
-static cudaError_t launch_queue_k(const AlignParams& p, size_t smem, uint32_t chunks,
+template <bool SEM, int CAP, int NPW>
+static cudaError_t launch_queue_k(const AlignParams& p, size_t smem, uint64_t units,
                                   cudaStream_t s) {
-    auto kern = k_ndt_queue<T, SEM, CAP, NPW>;
+    auto kern = k_ndt_queue<SEM, CAP, NPW>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     // persistent grid: every CTA resident (the kernel's CTAs never wait for each other, so
     // residency is a matter of speed only), at most one CTA per chunk of the batch
@@ -2400,7 +2597,7 @@ static cudaError_t launch_queue_k(const AlignParams& p, size_t smem, uint32_t ch
             ctas = it->second;
         } else {
             int per_sm = 0, sms = 0;
-            cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, T, smem);
+            cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, QT, smem);
             if (e != cudaSuccess) return e;
             if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)))
                 return e;
@@ -2408,31 +2605,30 @@ static cudaError_t launch_queue_k(const AlignParams& p, size_t smem, uint32_t ch
             cache[{dev, smem}] = ctas;
         }
     }
-    // at most one CTA per chunk of the batch at the late-iteration chunk size
+    // at most one CTA per chunk of the batch, counted at the late iterations' run size
+    const uint64_t chunks = (units + p.qunits - 1) / p.qunits;
     const unsigned grid = (unsigned)std::min<uint64_t>(
-        (uint64_t)ctas, (uint64_t)QSPLIT_DIV * std::max(1u, chunks));
+        (uint64_t)ctas, (p.qranks > 0 ? 1u : QSPLIT_DIV) * std::max<uint64_t>(1u, chunks));
     AlignParams q = p;
     q.qgrid = grid;
     if (!q.qresume) k_queue_init<SEM><<<(q.num_jobs + 3) / 4, 128, 0, s>>>(q);
-    kern<<<grid, T, smem, s>>>(q);
+    kern<<<grid, QT, smem, s>>>(q);
     return cudaGetLastError();
 }
 
-template <int T, int CAP>
-static int launch_queue_t(const AlignParams& p, uint32_t chunks, cudaStream_t s, int npw) {
-    // neighbour lists, trailing accumulators, then (staging) the chunk's points
-    const size_t smem = (size_t)T * (p.max_nb + NACC - A_HTR) * sizeof(uint32_t) +
-                        (p.qstage ? ((size_t)p.qchunk + 4) * 12 : 0);
+template <int CAP>
+static int launch_queue_t(const AlignParams& p, uint64_t units, cudaStream_t s, int npw) {
+    // voxel lists, trailing accumulators
+    const size_t smem = (size_t)QT * (p.max_nb + NACC - A_HTR) * sizeof(uint32_t);
     cudaError_t e;
-    if (p.semantics == NDT_SEMANTICS_CPU) {
-        e = launch_queue_k<T, true, CAP, 1>(p, smem, chunks, s);
-    } else if (T == 256 && CAP == 64 && npw == 2) {
-        e = launch_queue_k<T, false, CAP, 2>(p, smem, chunks, s);
-    } else if (T == 256 && CAP == 64 && npw == 4) {
-        e = launch_queue_k<T, false, CAP, 4>(p, smem, chunks, s);
-    } else {
-        e = launch_queue_k<T, false, CAP, 1>(p, smem, chunks, s);
-    }
+    if (p.semantics == NDT_SEMANTICS_CPU)
+        e = launch_queue_k<true, CAP, 1>(p, smem, units, s);
+    else if (CAP == 64 && npw == 2)
+        e = launch_queue_k<false, 64, 2>(p, smem, units, s);
+    else if (CAP == 64 && npw == 4)
+        e = launch_queue_k<false, 64, 4>(p, smem, units, s);
+    else
+        e = launch_queue_k<false, CAP, 1>(p, smem, units, s);
     return cuda_fail(e, "work-queue align launch");
 }
 
@@ -2486,26 +2682,23 @@ int launch_align(const AlignParams& p, LaunchShape shape, cudaStream_t s) {
             set_error("the work-queue kernel takes no line search and needs its buffers");
             return NDT_ERR_INVALID_ARGUMENT;
         }
-        q.qchunk = shape.threads * shape.queue;
-        // staging needs a 16-byte aligned points buffer (the bulk copy's rule)
-        q.qstage = shape.stage > 0 && ((uintptr_t)p.pts & 15u) == 0 ? 1 : 0;
-        const int npw = shape.npw;
-        if (npw > 1 && !(shape.threads == 256 && R != 80 && (npw == 2 || npw == 4) &&
+        const int npw = shape.npw, T = shape.threads;
+        if (T != 128 && T != 256 && T != 512) {
+            set_error("threads per CTA must be 128, 256 or 512");
+            return NDT_ERR_INVALID_ARGUMENT;
+        }
+        if (npw > 1 && !(T == 256 && R != 80 && (npw == 2 || npw == 4) &&
                          p.semantics != NDT_SEMANTICS_CPU)) {
             set_error("lanes per point 2 or 4 are built for the graph semantics' 256-thread, "
                       "64-register work-queue kernel");
             return NDT_ERR_INVALID_ARGUMENT;
         }
-        switch (shape.threads) {
-            case 128: return launch_queue_t<128, 64>(q, p.qchunks_total, s, 1);
-            case 256:
-                return R == 80 ? launch_queue_t<256, 80>(q, p.qchunks_total, s, 1)
-                               : launch_queue_t<256, 64>(q, p.qchunks_total, s, npw);
-            case 512: return launch_queue_t<512, 128>(q, p.qchunks_total, s, 1);
-            default:
-                set_error("threads per CTA must be 128, 256 or 512");
-                return NDT_ERR_INVALID_ARGUMENT;
-        }
+        q.qthreads = T;
+        q.qranks = shape.ranks;
+        q.qchunk = T * shape.queue;
+        q.qunits = shape.units;
+        return R == 80 ? launch_queue_t<80>(q, p.qunits_total, s, 1)
+                       : launch_queue_t<64>(q, p.qunits_total, s, npw);
     }
     switch (shape.threads) {
         case 128:

@@ -868,9 +868,18 @@ static int log2_bucket(uint64_t v) {
 // Launch shape: an explicit configuration wins, then an autotuned entry for this
 // (batch size, scan size) bucket, then the default: 512-thread CTAs for large scans, and
 // clusters doubled until the launch covers about three CTAs per SM while keeping at least
-// two points per thread per CTA.
-// The work-queue kernel is used when the configuration asks for it (work_queue > 0) or the
-// autotuner picked it, never with line search.
+// two points per thread per CTA. That is the partition of the points over threads; batches of
+// more than CLUSTER_JOBS run it on the work-queue kernel, smaller ones (and line search) as
+// clusters. The work-queue kernel with its own partition is used when the configuration asks
+// for it (work_queue > 0) or the autotuner picked it, never with line search.
+static int queue_units(int threads) { return std::min<int>(QUNITS, threads / 32); }
+
+// Largest batch that takes one cluster per alignment by default. Few alignments leave most SMs
+// idle on either kernel, and the hardware cluster barrier is quicker than the queue's claims
+// through L2 (one 20k-point scan: 0.30 ms on the cluster, 0.34 on the queue); a batch of 64 fills
+// the GPU and spends its waves' tails idle (0.75 ms on clusters, 0.53 on the queue).
+constexpr uint32_t CLUSTER_JOBS = 8;
+
 static LaunchShape choose_shape(ndt_ctx* c, uint32_t jobs, uint32_t max_n) {
     LaunchShape sh{0, 0, 128, 0};
     if (c->forced.cluster > 0) return c->forced;
@@ -878,10 +887,12 @@ static LaunchShape choose_shape(ndt_ctx* c, uint32_t jobs, uint32_t max_n) {
     if (c->cfg.work_queue > 0 && !ls) {
         sh.cluster = 1;
         sh.threads = c->cfg.threads_per_cta > 0 ? c->cfg.threads_per_cta : 256;
-        sh.regcap = c->cfg.max_registers > 0 ? c->cfg.max_registers : (sh.threads == 512 ? 128 : 64);
+        sh.regcap = c->cfg.max_registers > 0 ? c->cfg.max_registers : 80;
+        if (c->cfg.lanes_per_point > 1 && c->cfg.max_registers <= 0) sh.regcap = 64;
         sh.queue = c->cfg.work_queue;
         sh.npw = c->cfg.lanes_per_point > 1 ? c->cfg.lanes_per_point : 1;
         sh.stage = c->cfg.stage_points > 0 ? 1 : 0;
+        sh.units = queue_units(sh.threads);
         return sh;
     }
     auto it = c->tuned.find({log2_bucket(jobs), log2_bucket(max_n)});
@@ -900,6 +911,21 @@ static LaunchShape choose_shape(ndt_ctx* c, uint32_t jobs, uint32_t max_n) {
     while (K < 8 && (uint64_t)jobs * K < 3ull * (uint64_t)c->num_sms &&
            max_n / (uint32_t)(2 * K) >= (uint32_t)sh.threads * 2)
         K *= 2;
+    if (jobs > CLUSTER_JOBS && c->cfg.work_queue == 0 && !ls && c->cfg.threads_per_cta <= 0 &&
+        c->cfg.max_registers <= 0) {
+        // this cluster's partition of the points on the work-queue kernel: every lane's f32
+        // sums are the cluster kernel's
+        sh.cluster = 1;
+        sh.ranks = K;
+        sh.queue = 1;
+        sh.npw = 1;
+        sh.units = queue_units(sh.threads);
+        // 64 registers (four CTAs an SM) where a CTA keeps its alignments and steps hide
+        // behind other alignments' points, else 80 (three CTAs, no spills in the point work):
+        // 16 x 200 particles 4.17 and 4.27 ms, 64 scans of 2k-40k points 0.58 and 0.53 ms
+        sh.regcap = K * sh.threads <= (int)QUNITS * 32 ? 64 : 80;
+        return sh;
+    }
     sh.cluster = K;
     return sh;
 }
@@ -983,6 +1009,8 @@ static int run_align_enqueue(ndt_ctx* c, const float* d_pts, std::vector<AlignJo
     uint32_t* hq = nullptr;
     if (shape.queue > 0) {
         const uint32_t chunk = (uint32_t)(shape.threads * shape.queue);
+        const uint32_t upr = (uint32_t)shape.threads / 32, U = (uint32_t)shape.units;
+        const uint64_t max_runs = (uint64_t)QMAXCH * U / upr;
         qob = (size_t)nj * sizeof(uint32_t);
         if ((rc = pin_reserve(c->h_jobs, jb + sjb + qob))) return rc;
         hj = (AlignJob*)c->h_jobs.p;  // the block may have moved: refill it
@@ -997,15 +1025,20 @@ static int run_align_enqueue(ndt_ctx* c, const float* d_pts, std::vector<AlignJo
             hs[j] = s;
         }
         hq = (uint32_t*)((char*)c->h_jobs.p + jb + sjb);
-        // partial-sum slots per alignment: its chunk count at the smallest (last iterations')
-        // chunk size, the most an iteration uses, capped at the 16-bit count of the claim word
+        // partial-sum slots per alignment: its chunk count, at the smallest (last iterations')
+        // run size the most an iteration uses, capped at the claim word's 16-bit count
         const uint32_t small = std::max(1u, chunk / (2 * QSPLIT_DIV));
         uint64_t total = 0, full = 0;
         for (uint32_t j = 0; j < nj; ++j) {
             hq[j] = (uint32_t)total;
             const uint64_t n = jobs[j].n;
-            total += std::min<uint64_t>(n ? (n + small - 1) / small : 1, QMAXCH);
-            full += std::min<uint64_t>(n ? (n + chunk - 1) / chunk : 1, QMAXCH);
+            uint64_t most = (uint64_t)shape.ranks, runs = most;
+            if (shape.ranks == 0) {
+                most = std::min<uint64_t>(n ? (n + small - 1) / small : 1, max_runs);
+                runs = std::min<uint64_t>(n ? (n + chunk - 1) / chunk : 1, max_runs);
+            }
+            total += (most * upr + U - 1) / U;
+            full += runs * upr;
         }
         if (total > 0xFFFFFFFFull) {
             set_error("too many chunks in one batch");
@@ -1013,7 +1046,7 @@ static int run_align_enqueue(ndt_ctx* c, const float* d_pts, std::vector<AlignJo
         }
         if ((rc = dev_reserve(c->d_qjobs, (size_t)nj * sizeof(QJob))) ||
             (rc = dev_reserve(c->d_qctl, (size_t)nj * sizeof(QCtl))) ||
-            (rc = dev_reserve(c->d_qframe, (size_t)nj * 52 * sizeof(float))) ||
+            (rc = dev_reserve(c->d_qframe, (size_t)nj * NFRAME * sizeof(float))) ||
             (rc = dev_reserve(c->d_qoff, qob)) ||
             (rc = dev_reserve(c->d_qpart, (size_t)total * NRED * sizeof(double))))
             return rc;
@@ -1023,7 +1056,8 @@ static int run_align_enqueue(ndt_ctx* c, const float* d_pts, std::vector<AlignJo
         p.qpart = (double*)c->d_qpart.p;
         p.qpart_off = (const uint32_t*)c->d_qoff.p;
         p.qcount = (uint32_t*)c->d_status.p + 2;  // word 2 of the status block
-        p.qchunks_total = (uint32_t)full;
+        p.qunits_total = full;
+        p.qsolo = total == nj && !p.withhold ? 1 : 0;
         c->stats.h2d_bytes += qob;
     }
     AlignOut* ho = (AlignOut*)c->h_aout.p;
@@ -1040,6 +1074,7 @@ static int run_align_enqueue(ndt_ctx* c, const float* d_pts, std::vector<AlignJo
         d_arrive = (uint32_t*)c->d_status.p + 3;
         p.qarrive = d_arrive;
         p.qarrive_total = (uint32_t)plan->total;
+        p.qsolo = 0;
     }
     // the batch on the stream: job tables in, Newton kernel, NVTL scoring, results out (the
     // events are graph nodes when captured)
@@ -1082,7 +1117,7 @@ static int run_align_enqueue(ndt_ctx* c, const float* d_pts, std::vector<AlignJo
     if (c->cfg.cuda_graph && !c->trace && !stream_in) {
         const std::vector<uint64_t> key = {
             nj, max_n, (uint64_t)shape.cluster, (uint64_t)shape.threads, (uint64_t)shape.regcap,
-            (uint64_t)shape.queue, (uint64_t)shape.npw, (uint64_t)shape.stage,
+            (uint64_t)shape.queue, (uint64_t)shape.npw, (uint64_t)shape.ranks, (uint64_t)shape.units,
             (uint64_t)(uintptr_t)c->d_qjobs.p,
             (uint64_t)(uintptr_t)c->d_qctl.p, (uint64_t)(uintptr_t)c->d_qframe.p,
             (uint64_t)(uintptr_t)c->d_qpart.p, (uint64_t)(uintptr_t)c->d_qoff.p,
@@ -1874,7 +1909,7 @@ int ndt_autotune(ndt_ctx* c, const float* d_xyz, const uint64_t* offsets, const 
     const int TC[8][2] = {{128, 128}, {128, 80}, {128, 64}, {256, 128},
                           {256, 80},  {256, 64}, {256, 48}, {512, 128}};
     // work-queue candidates: (threads, registers, points per thread per chunk, lanes sharing
-    // each point's neighbour search, chunk points staged in shared memory)
+    // each point's neighbour search, stage_points: no effect)
     const int QC[14][5] = {{256, 64, 2, 1, 0}, {256, 64, 4, 1, 0}, {256, 64, 8, 1, 0},
                            {256, 80, 4, 1, 0}, {128, 64, 4, 1, 0}, {512, 128, 2, 1, 0},
                            {256, 64, 4, 2, 0}, {256, 64, 4, 4, 0}, {256, 64, 8, 4, 0},
@@ -1889,7 +1924,8 @@ int ndt_autotune(ndt_ctx* c, const float* d_xyz, const uint64_t* offsets, const 
     if (c->cfg.work_queue >= 0 && !ls)
         for (const auto& qc : QC)
             if (qc[3] == 1 || graph_sem)
-                cands.push_back(LaunchShape{1, qc[0], qc[1], qc[2], qc[3], qc[4]});
+                cands.push_back(LaunchShape{1, qc[0], qc[1], qc[2], qc[3], qc[4], 0,
+                                            queue_units(qc[0])});
     LaunchShape best{0, 0, 128, 0};
     double best_ms = 1e300;
     int tried = 0;

@@ -183,17 +183,21 @@ struct AlignParams {
     int32_t ls_cands;      // graph-path line search: candidates per iteration (0: off)
     double ls_mu, ls_nu;   // strong Wolfe constants
     // work-queue kernel (k_ndt_queue): per-alignment claim words, controller state, frames,
-    // per-chunk partial sums (offsets by alignment), counters {alignments finished}
+    // per-chunk partial sums (offsets by alignment), counter of alignments taken (qsolo)
     struct QJob* qjobs;
     struct QCtl* qctl;
     float* qframe;
     double* qpart;
     const uint32_t* qpart_off;
     uint32_t* qcount;
-    int32_t qchunk;        // points per chunk (set by the launch from the shape); chunks of
-                           // 1/QSPLIT_DIV of it in an alignment's late iterations
-    uint32_t qchunks_total;  // chunks of one iteration of every alignment (at full size)
-    uint32_t qgrid;          // CTAs of the launch (set by the launch)
+    // partition (set by the launch from the shape): qranks ranks of qthreads threads, or runs
+    // of qchunk points (fewer in an alignment's late iterations) strided by qthreads threads;
+    // qunits units of 32 threads per chunk
+    int32_t qthreads, qranks, qchunk, qunits;
+    uint64_t qunits_total;  // units of one iteration of every alignment (early iterations)
+    int32_t qsolo;          // every iteration of every alignment is one chunk, and all points
+                            // are resident: CTAs keep their alignments
+    uint32_t qgrid;         // CTAs of the launch (set by the launch)
     // points copied in while the work-queue kernel runs: the device word counts the points of
     // the batch resident so far (a prefix of pts, written by the copy stream after each
     // chunk); an alignment is claimable once its last point is resident. nullptr: all are.
@@ -210,9 +214,6 @@ struct AlignParams {
     // withhold, every chunk starts out claimed (a test hook: no CTA finds work)
     uint64_t stall_ns;
     int32_t withhold;
-    // work-queue kernel: each chunk's points staged into shared memory by one bulk copy
-    // (needs the points' buffer 16-byte aligned)
-    int32_t qstage;
 };
 constexpr unsigned long long QSTARVE_NS = 2000000ull;
 constexpr unsigned long long QSTALL_NS = 2000000000ull;
@@ -221,6 +222,7 @@ constexpr unsigned long long QSTALL_NS = 2000000000ull;
 // Hessian terms), reduced in FP64, plus the correspondence count.
 constexpr int NACC = 34;
 constexpr int NRED = NACC + 1;
+constexpr int NFRAME = 60;  // floats of a frame (ndt_align.cu)
 
 // Work-queue kernel state, one per alignment (global memory).
 struct QJob {
@@ -232,7 +234,8 @@ struct QJob {
 };
 constexpr uint32_t QDONE = 0xFFFFu;
 constexpr uint32_t QMAXCH = 0xFFFFu;  // chunks per iteration at most (16-bit count)
-// Chunks of an alignment's late iterations are 1/QSPLIT_DIV of the launch's chunk size, and
+constexpr uint32_t QUNITS = 8;        // units (warps' shares) per chunk at most
+// Runs of an alignment's late iterations are 1/QSPLIT_DIV of the launch's run size, and
 // 1/(2 QSPLIT_DIV) in its last ones (the partial-sum slots are sized for those). At the
 // 20k-point bench batch, 2 and 8 were slower as the first split.
 constexpr uint32_t QSPLIT_DIV = 4;
@@ -269,9 +272,11 @@ struct LaunchShape {
     int cluster;
     int threads;
     int regcap;  // 128 (default); 80, 64, 48: denser residency for 128/256-thread CTAs
-    int queue;   // > 0: work-queue kernel, chunks of `queue` points per thread (cluster 1)
+    int queue;   // > 0: work-queue kernel, runs of `queue` points per thread (cluster 1)
     int npw;     // work-queue kernel: lanes sharing each point's neighbour search (0, 1: one)
-    int stage;   // work-queue kernel: 1 stages each chunk's points in shared memory (bulk copy)
+    int stage;   // the stage_points option (no effect)
+    int ranks;   // work-queue kernel: > 0, the partition of a cluster of `ranks` CTAs
+    int units;   // work-queue kernel: units per chunk
 };
 
 int launch_align(const AlignParams& p, LaunchShape shape, cudaStream_t s);

@@ -96,17 +96,16 @@ typedef struct ndt_config {
     int32_t work_queue;            /* Newton-kernel form: n > 0 the work-queue kernel (a
                                       persistent grid claiming chunks of n points per thread
                                       of any alignment's iteration); -1 one thread-block
-                                      cluster per alignment; 0 autotuned (cluster kernel
-                                      until tuned). Line search always uses the cluster
+                                      cluster per alignment; 0 autotuned (until tuned, by
+                                      the batch's size). Line search always uses the cluster
                                       kernel. */
     int32_t lanes_per_point;       /* work-queue kernel, graph semantics, 256 threads at 64
                                       registers: 2 or 4 lanes share each point's neighbour
                                       search (the occupied cells among its 27); 0 or 1: each
                                       lane searches its own point. The autotuner chooses it. */
-    int32_t stage_points;          /* work-queue kernel: 1 stages each chunk's points in shared
-                                      memory with one bulk copy (the TMA engine) before the
-                                      chunk's work; 0 reads them from global memory. The
-                                      autotuner chooses it. */
+    int32_t stage_points;          /* 0 or 1; no effect: the work-queue kernel reads each point
+                                      once, in order, through L1 (staging its chunks in shared
+                                      memory first cost more than it saved) */
 } ndt_config;
 
 /* AlignResult (src/ndt_cuda/src/ndt.rs:219-248) with the pose as a vector. */
@@ -275,8 +274,7 @@ typedef struct ndt_tune_result {
                                       work-queue kernel, else 0 */
     int32_t lanes_per_point;       /* lanes sharing each point's neighbour search in the
                                       winning work-queue kernel (1, 2, 4), else 0 */
-    int32_t stage_points;          /* 1 when the winning work-queue kernel stages its chunks'
-                                      points in shared memory */
+    int32_t stage_points;          /* stage_points of the winning candidate (no effect) */
     int32_t reserved;
 } ndt_tune_result;
 int ndt_autotune(ndt_ctx* ctx, const float* d_xyz, const uint64_t* offsets,
