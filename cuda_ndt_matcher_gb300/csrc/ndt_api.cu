@@ -535,7 +535,7 @@ int ndt_ctx_destroy(ndt_ctx* c) {
                       &c->d_qcnt, &c->d_trace, &c->d_qjobs, &c->d_qctl, &c->d_qframe,
                       &c->d_qpart, &c->d_qoff})
         dev_free(*b);
-    for (PinBuf* b : {&c->h_pts, &c->h_jobs, &c->h_aout, &c->h_sjobs, &c->h_sout, &c->h_misc,
+    for (PinBuf* b : {&c->bs.host, &c->bs_b.host, &c->bs_tile.host, &c->h_pts, &c->h_jobs, &c->h_aout, &c->h_sjobs, &c->h_sout, &c->h_misc,
                       &c->h_arrive})
         pin_free(*b);
     for (cudaEvent_t ev : {c->ev0, c->ev1, c->ev2, c->ev3, c->ev_in0, c->ev_in1})
@@ -628,10 +628,7 @@ static int set_target_dev(ndt_ctx* c, const float* d_xyz, uint64_t n) {
     int rc = build_map(c->map, c->bs, d_xyz, (size_t)n, c->cfg, (uint32_t*)c->d_status.p,
                        c->stream, &ms);
     if (rc) return rc;
-    uint32_t st = 0;
-    cudaMemcpyAsync(&st, c->d_status.p, 4, cudaMemcpyDeviceToHost, c->stream);
-    if ((rc = cuda_fail(cudaStreamSynchronize(c->stream), "set_target"))) return rc;
-    if ((rc = check_status(c, st))) {
+    if ((rc = check_status(c, c->map.status))) {
         c->map.valid = false;
         return rc;
     }
@@ -769,11 +766,7 @@ int ndt_tiles_commit(ndt_ctx* c, int32_t wait) {
         float ms = 0.f;
         int r = merge_tiles(c->map_b, c->bs_b, refs, c->d_tile_refs, cfg,
                             (uint32_t*)c->d_status_b.p, c->bstream, &ms);
-        uint32_t st = 0;
-        if (!r) {
-            cudaMemcpyAsync(&st, c->d_status_b.p, 4, cudaMemcpyDeviceToHost, c->bstream);
-            r = cuda_fail(cudaStreamSynchronize(c->bstream), "tile rebuild");
-        }
+        const uint32_t st = r ? 0u : c->map_b.status;
         if (!r && st) {
             uint32_t zero = 0;
             cudaMemcpyAsync(c->d_status_b.p, &zero, 4, cudaMemcpyHostToDevice, c->bstream);

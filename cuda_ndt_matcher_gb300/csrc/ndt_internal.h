@@ -56,6 +56,7 @@ struct Map {
     DevBuf vox_coord, vox_mean, vox_cov, vox_icov, vox_count;
     MapView view{};
     ndt_map_info info{};
+    uint32_t status = 0;  // the status word at the end of the last build
     bool valid = false;
 };
 
@@ -63,6 +64,7 @@ struct Map {
 struct BuildScratch {
     DevBuf keys_a, keys_b, vals_a, vals_b, tmp;
     DevBuf seg_ids, seg_starts, seg_valid, seg_rank, seg_rec, small;
+    PinBuf host;  // sizes read back between stages
 };
 
 // Temporary-storage sizing of the sort / scan primitives (two-phase convention).
@@ -70,8 +72,6 @@ size_t radix_sort_temp_bytes(size_t n);
 size_t scan_temp_bytes(size_t n);
 int radix_sort_pairs(uint64_t* keys, uint32_t* vals, size_t n, int begin_bit, int end_bit,
                      void* temp, size_t temp_bytes, cudaStream_t s);
-int radix_sort_pairs32(uint32_t* keys, uint32_t* vals, size_t n, int begin_bit, int end_bit,
-                       void* temp, size_t temp_bytes, cudaStream_t s);
 int detect_segments(const uint64_t* sorted, size_t n, uint32_t* seg_ids, uint32_t* seg_starts,
                     uint32_t* num_segments, void* temp, size_t temp_bytes, cudaStream_t s);
 size_t detect_segments_temp_bytes(size_t n);

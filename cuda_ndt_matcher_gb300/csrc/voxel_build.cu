@@ -5,13 +5,13 @@
 //   1. cells + bounds      : cell = floor(p / res) per finite point (f32 IEEE division, the
 //                            membership rule of VoxelCoord::from_point,
 //                            src/ndt_cuda/src/voxel_grid/types.rs:206-212); min/max cell.
-//   2. Morton keys         : key = morton(cell - min cell), 21 bits per axis
-//                            (src/ndt_cuda/src/voxel_grid/gpu/morton.rs:45-95 layout); the
-//                            non-finite points get key ~0 and sort last.
-//   3. LSD radix sort      : stable, 8-bit digits, only the significant key bits, 32-bit
-//                            keys when they fit (replaces cub::DeviceRadixSort,
-//                            src/cuda_ffi/csrc/radix_sort.cu).
-//   4. segments            : per-tile counts of key changes, scanned, then the starts
+//   2. Morton keys         : the order of morton(cell - min cell), 21 bits per axis
+//                            (src/ndt_cuda/src/voxel_grid/gpu/morton.rs:45-95), as a 32-bit key of
+//                            the bits that the map's box has; non-finite points sort last.
+//   3. LSD radix sort      : stable, digits of up to 8 bits, the key's bits shared evenly by
+//                            the passes (replaces cub::DeviceRadixSort,
+//                            src/cuda_ffi/csrc/radix_sort.cu); 64-bit keys from 2^30 points on.
+//   4. segments            : starts of the runs of equal keys, one launch with look-back
 //                            (src/cuda_ffi/csrc/segment_detect.cu:27-146; the API's
 //                            ndt_detect_segments keeps flags + scan for the segment ids).
 //   5. voxel statistics    : segments visited largest first; segments of 48 points or more
@@ -29,12 +29,12 @@
 //                            map's box; and hash insert: bounded linear probing with
 //                            atomicCAS, displacement recorded (voxel_hash_build_kernel,
 //                            src/cuda_ffi/csrc/voxel_hash.cu:69-114).
-//   7. masks               : with the dense index, the neighbourhood masks (one per octant of each cell while they
-//                            fit their budget, else one per cell) that list the neighbours a
-//                            point there can accept.
-// Bit-exact parts (cells, keys, counts, means) use no multiply-add: cells are an f32 division,
-// means an FP64 division of an exact sum (or a running sum of adds), so FMA contraction
-// cannot change them; the regularised covariances, compared in f32 ULPs, use FMAs freely.
+//   7. masks               : with the dense index, the neighbourhood masks (one per octant of
+//                            each cell while they fit their budget, else one per cell) that
+//                            list the neighbours a point there can accept.
+// Bit-exact parts (cells, keys, counts, means) do not depend on FMA contraction: cells are an
+// f32 quotient, means the correctly rounded FP64 quotient of an exact sum (or a running sum of
+// adds); the regularised covariances, compared in f32 ULPs, use FMAs freely.
 #include <algorithm>
 #include <cstdio>
 #include <mutex>
@@ -82,52 +82,65 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* w
     return pre + x - v;
 }
 
-__global__ void __launch_bounds__(BT) k_tile_reduce(const uint32_t* __restrict__ in, size_t n,
-                                                    uint32_t* __restrict__ bsum) {
-    __shared__ uint32_t ws[BT / 32];
-    size_t base = (size_t)blockIdx.x * TILE;
-    uint32_t s = 0;
-#pragma unroll
-    for (int r = 0; r < ITEMS; ++r) {
-        size_t i = base + (size_t)r * BT + threadIdx.x;
-        if (i < n) s += in[i];
-    }
-    uint32_t tot;
-    block_exclusive_scan(s, ws, &tot);
-    if (threadIdx.x == 0) bsum[blockIdx.x] = tot;
+// ---------------------------------------------------------------------------------------
+// Decoupled look-back (Merrill and Garland 2016): the tiles of a launch take their numbers from
+// a ticket, so every earlier tile is running or done; each publishes its own sum, then walks
+// back over the earlier tiles' words until it meets an inclusive prefix. A word holds state
+// (top two bits: 0 not there yet, 1 the tile's sum, 2 the inclusive prefix) and value, so it
+// is read and written whole and needs no fence.
+// ---------------------------------------------------------------------------------------
+constexpr unsigned long long LB_LIMIT_NS = 1000000000ull;  // bounded waits: 1 s
+
+__device__ __forceinline__ unsigned long long lb_now() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
 }
 
-__global__ void __launch_bounds__(BT) k_scan_bsums(uint32_t* __restrict__ bsum, uint32_t nb) {
-    __shared__ uint32_t ws[BT / 32];
-    uint32_t carry = 0;
-    for (uint32_t base = 0; base < nb; base += TILE) {
-        uint32_t v[ITEMS];
-        uint32_t s = 0;
-#pragma unroll
-        for (int k = 0; k < ITEMS; ++k) {
-            uint32_t i = base + threadIdx.x * ITEMS + k;
-            v[k] = i < nb ? bsum[i] : 0u;
-            s += v[k];
+// Exclusive prefix of tile `tile` over 64-bit words w[0 .. tile), whose own sum is `sum`, by one
+// warp (32 earlier tiles at a time); publishes the tile's inclusive prefix. False when a word
+// did not arrive within the limit.
+__device__ __forceinline__ bool lookback_warp(unsigned long long* w, uint32_t tile,
+                                              unsigned long long sum, int lane,
+                                              unsigned long long& excl) {
+    constexpr unsigned long long ONE = 1ull << 62, TWO = 2ull << 62, VAL = ONE - 1ull;
+    if (lane == 0) atomicExch(w + tile, (tile == 0 ? TWO : ONE) | sum);
+    excl = 0ull;
+    if (tile == 0) return true;
+    const unsigned long long t0 = lb_now();
+    int64_t at = (int64_t)tile - 1 - lane;
+    for (;;) {
+        unsigned long long v = at >= 0 ? *(volatile unsigned long long*)(w + at) : TWO;
+        while (__any_sync(0xffffffffu, (v >> 62) == 0ull)) {
+            if (lb_now() - t0 > LB_LIMIT_NS) return false;
+            if ((v >> 62) == 0ull) v = *(volatile unsigned long long*)(w + at);
         }
-        uint32_t tot;
-        uint32_t run = carry + block_exclusive_scan(s, ws, &tot);
+        // the nearest inclusive prefix among these 32, and the sums after it
+        const unsigned full = __ballot_sync(0xffffffffu, (v >> 62) == 2ull);
+        const int stop = full ? __ffs(full) - 1 : 32;
+        unsigned long long x = lane <= stop ? (v & VAL) : 0ull;
 #pragma unroll
-        for (int k = 0; k < ITEMS; ++k) {
-            uint32_t i = base + threadIdx.x * ITEMS + k;
-            if (i < nb) bsum[i] = run;
-            run += v[k];
-        }
-        carry += tot;
-        __syncthreads();
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        excl += x;
+        if (full) break;
+        at -= 32;
     }
+    if (lane == 0) atomicExch(w + tile, TWO | (excl + sum));
+    return true;
 }
 
-// exclusive scan of a tile; element order: thread t holds items t*ITEMS .. t*ITEMS+15
-__global__ void __launch_bounds__(BT) k_tile_scan(const uint32_t* __restrict__ in,
-                                                  uint32_t* __restrict__ out, size_t n,
-                                                  const uint32_t* __restrict__ bsum) {
+// Exclusive scan in one launch, element order (thread t of a tile holds items t * ITEMS ..).
+// tmp: one ticket, then a word per tile, all zero at the start. In place allowed.
+__global__ void __launch_bounds__(BT) k_scan(const uint32_t* __restrict__ in,
+                                             uint32_t* __restrict__ out, size_t n,
+                                             unsigned long long* __restrict__ tmp) {
     __shared__ uint32_t ws[BT / 32];
-    size_t base = (size_t)blockIdx.x * TILE + (size_t)threadIdx.x * ITEMS;
+    __shared__ uint32_t s_tile, s_excl;
+    __shared__ bool s_ok;
+    if (threadIdx.x == 0) s_tile = atomicAdd((unsigned int*)tmp, 1u);
+    __syncthreads();
+    const uint32_t tile = s_tile;
+    const size_t base = (size_t)tile * TILE + (size_t)threadIdx.x * ITEMS;
     uint32_t v[ITEMS];
     uint32_t s = 0;
 #pragma unroll
@@ -136,7 +149,18 @@ __global__ void __launch_bounds__(BT) k_tile_scan(const uint32_t* __restrict__ i
         s += v[k];
     }
     uint32_t tot;
-    uint32_t run = bsum[blockIdx.x] + block_exclusive_scan(s, ws, &tot);
+    const uint32_t pre = block_exclusive_scan(s, ws, &tot);
+    if (threadIdx.x < 32) {
+        unsigned long long e;
+        const bool ok = lookback_warp(tmp + 1, tile, tot, (int)threadIdx.x, e);
+        if (threadIdx.x == 0) {
+            s_excl = (uint32_t)e;
+            s_ok = ok;
+        }
+    }
+    __syncthreads();
+    if (!s_ok) return;
+    uint32_t run = s_excl + pre;
 #pragma unroll
     for (int k = 0; k < ITEMS; ++k) {
         if (base + k < n) out[base + k] = run;
@@ -144,17 +168,15 @@ __global__ void __launch_bounds__(BT) k_tile_scan(const uint32_t* __restrict__ i
     }
 }
 
-size_t scan_temp_bytes(size_t n) { return align_up((size_t)ntiles(n) * 4 + 4, 256); }
+size_t scan_temp_bytes(size_t n) { return align_up((size_t)ntiles(n) * 8 + 8, 256); }
 
-// exclusive scan in -> out (may alias); temp >= scan_temp_bytes(n)
+// exclusive scan in -> out (may alias); temp >= scan_temp_bytes(n), 8-byte aligned
 static int exclusive_scan(const uint32_t* in, uint32_t* out, size_t n, void* temp,
                           cudaStream_t s) {
     if (n == 0) return 0;
-    uint32_t nb = ntiles(n);
-    uint32_t* bsum = (uint32_t*)temp;
-    k_tile_reduce<<<nb, BT, 0, s>>>(in, n, bsum);
-    k_scan_bsums<<<1, BT, 0, s>>>(bsum, nb);
-    k_tile_scan<<<nb, BT, 0, s>>>(in, out, n, bsum);
+    const uint32_t nb = ntiles(n);
+    cudaMemsetAsync(temp, 0, (size_t)nb * 8 + 8, s);
+    k_scan<<<nb, BT, 0, s>>>(in, out, n, (unsigned long long*)temp);
     return cuda_fail(cudaGetLastError(), "scan launch");
 }
 
@@ -350,9 +372,205 @@ int radix_sort_pairs(uint64_t* keys, uint32_t* vals, size_t n, int begin_bit, in
     return radix_sort_t(keys, vals, n, begin_bit, end_bit, temp, temp_bytes, s);
 }
 
-int radix_sort_pairs32(uint32_t* keys, uint32_t* vals, size_t n, int begin_bit, int end_bit,
-                       void* temp, size_t temp_bytes, cudaStream_t s) {
-    return radix_sort_t(keys, vals, n, begin_bit, std::min(end_bit, 32), temp, temp_bytes, s);
+// ---------------------------------------------------------------------------------------
+// Stable LSD sort of (u32 key, u32 value) pairs with digits of up to 8 bits, the map build's
+// form. Against the form above: the key's bits shared evenly by the passes (fewer digits make
+// longer runs), the first pass's tile counts taken while the keys are made, and one search for
+// each key's peers instead of two (that form was bound by the instructions of its ballots: 58%
+// issue, math pipe throttled). 50M pairs: 277 us a pass, 225 this way. Slower: 9-bit digits (460
+// us a pass: a tile's runs are 32 bytes), and a one-sweep form with look-back over the earlier
+// tiles instead of scanned counts (545 us: 600 tiles in flight walk over one another's sums).
+// ---------------------------------------------------------------------------------------
+constexpr int SP_BINS = 256;
+constexpr size_t SP_MAX_PAIRS = size_t(1) << 30;
+
+// Passes over `bits` key bits and the digit width of each
+struct SortPlan {
+    int passes, width;
+};
+static SortPlan sort_plan(int bits) {
+    SortPlan o;
+    o.passes = std::max(1, (bits + 7) / 8);
+    o.width = std::max(1, (bits + o.passes - 1) / o.passes);
+    return o;
+}
+// Workspace of a sort: tile counts [bins][tiles], then the scan's
+static size_t sort_counts(size_t n, SortPlan o) { return (size_t)ntiles(n) << o.width; }
+static size_t sort_bytes(size_t n, SortPlan o) {
+    return align_up(sort_counts(n, o) * 4, 256) + scan_temp_bytes(sort_counts(n, o));
+}
+
+// Digit counts of a tile: shared-memory atomics into one counter set per warp, so keys of one
+// digit queue only within their warp
+struct TileCounts {
+    uint32_t c[BT / 32][SP_BINS];
+};
+__device__ __forceinline__ void tile_counts_clear(TileCounts& t, uint32_t bins) {
+    for (uint32_t i = threadIdx.x; i < (BT / 32) * SP_BINS; i += BT)
+        if (i % SP_BINS < bins) t.c[i / SP_BINS][i % SP_BINS] = 0;
+}
+__device__ __forceinline__ void tile_counts_add(TileCounts& t, uint32_t d, bool valid) {
+    if (valid) atomicAdd(&t.c[threadIdx.x >> 5][d], 1u);
+}
+__device__ __forceinline__ void tile_counts_store(const TileCounts& t, uint32_t bins,
+                                                  uint32_t* __restrict__ hist, uint32_t tile,
+                                                  uint32_t nb) {
+    for (uint32_t d = threadIdx.x; d < bins; d += BT) {
+        uint32_t c = 0;
+#pragma unroll
+        for (int w = 0; w < BT / 32; ++w) c += t.c[w][d];
+        hist[(size_t)d * nb + tile] = c;
+    }
+}
+
+__global__ void __launch_bounds__(BT) k_tile_digits(const uint32_t* __restrict__ keys, uint32_t n,
+                                                    int shift, int width,
+                                                    uint32_t* __restrict__ hist) {
+    __shared__ TileCounts t;
+    const uint32_t bins = 1u << width;
+    tile_counts_clear(t, bins);
+    const uint32_t base = blockIdx.x * (uint32_t)TILE;
+    uint32_t kv[ITEMS];
+#pragma unroll
+    for (int r = 0; r < ITEMS; ++r) {
+        const uint32_t i = base + (uint32_t)r * BT + threadIdx.x;
+        kv[r] = i < n ? keys[i] : 0u;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < ITEMS; ++r)
+        tile_counts_add(t, (kv[r] >> shift) & (bins - 1u),
+                        base + (uint32_t)r * BT + threadIdx.x < n);
+    __syncthreads();
+    tile_counts_store(t, bins, hist, blockIdx.x, gridDim.x);
+}
+
+// One pass. A block takes one TILE-key tile; warp w holds the tile's keys [w * 512, (w + 1) *
+// 512) as 16 rounds of 32. Each round finds every key's peers (same digit) by ballots, and its
+// rank from the warp's counter: tile order within a digit, so the sort is stable. The digits'
+// tile positions (scanned over the block) and global positions (the scanned tile counts, offs)
+// then give each key's place; the tile leaves through shared memory as one contiguous run per
+// digit. vin null: the values are the positions.
+__global__ void __launch_bounds__(BT, 4) k_sort_pass(
+    const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin,
+    uint32_t* __restrict__ kout, uint32_t* __restrict__ vout, uint32_t n, int shift, int width,
+    const uint32_t* __restrict__ offs) {
+    constexpr int NWARP = BT / 32, ROUNDS = TILE / BT, PER = SP_BINS / BT;
+    __shared__ TileCounts wc;          // per warp: digit counts, then first positions
+    __shared__ uint32_t base[SP_BINS]; // global position minus tile position of a digit
+    __shared__ uint32_t skey[TILE], sval[TILE];  // the tile on its way out
+    __shared__ uint32_t ws[NWARP];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t bins = 1u << width, dmask = bins - 1u;
+    const uint32_t tbase = blockIdx.x * (uint32_t)TILE;
+    const uint32_t tn = min((uint32_t)TILE, n - tbase);
+    const uint32_t wbase = (uint32_t)warp * (ROUNDS * 32);
+    uint32_t key[ROUNDS];
+    uint32_t rank[ROUNDS / 2];  // two 16-bit ranks a word
+#pragma unroll
+    for (int r = 0; r < ROUNDS; ++r) {
+        const uint32_t li = wbase + (uint32_t)r * 32 + lane;
+        key[r] = li < tn ? kin[tbase + li] : 0u;
+    }
+    tile_counts_clear(wc, bins);
+    __syncthreads();
+    const uint32_t lt = (1u << lane) - 1u;
+    uint32_t* const wcnt = wc.c[warp];
+#pragma unroll
+    for (int r = 0; r < ROUNDS; ++r) {
+        const uint32_t li = wbase + (uint32_t)r * 32 + lane;
+        const bool valid = li < tn;
+        const uint32_t d = (key[r] >> shift) & dmask;
+        uint32_t peers = tn == (uint32_t)TILE ? 0xffffffffu : __ballot_sync(0xffffffffu, valid);
+        for (int k = 0; k < width; ++k) {
+            const bool bit = (d >> k) & 1u;
+            const uint32_t b = __ballot_sync(0xffffffffu, bit);
+            peers &= bit ? b : ~b;
+        }
+        uint32_t rk = 0;
+        if (valid) rk = wcnt[d];
+        __syncwarp();
+        if (valid && (peers & lt) == 0u) wcnt[d] = rk + (uint32_t)__popc(peers);
+        __syncwarp();
+        rk += (uint32_t)__popc(peers & lt);
+        if (r & 1)
+            rank[r / 2] |= rk << 16;
+        else
+            rank[r / 2] = rk;
+    }
+    __syncthreads();
+    // thread t owns the digits t * PER .. (only the first `bins` exist)
+    uint32_t cnt[PER], tot, mine = 0;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        const uint32_t d = threadIdx.x * PER + j;
+        uint32_t run = 0;
+        if (d < bins) {
+#pragma unroll
+            for (int w = 0; w < NWARP; ++w) {
+                const uint32_t c = wc.c[w][d];
+                wc.c[w][d] = run;
+                run += c;
+            }
+            base[d] = offs[(size_t)d * gridDim.x + blockIdx.x];
+        }
+        cnt[j] = run;
+        mine += run;
+    }
+    uint32_t lo = block_exclusive_scan(mine, ws, &tot);
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        const uint32_t d = threadIdx.x * PER + j;
+        if (d < bins) {
+#pragma unroll
+            for (int w = 0; w < NWARP; ++w) wc.c[w][d] += lo;
+            base[d] -= lo;
+        }
+        lo += cnt[j];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < ROUNDS; ++r) {
+        const uint32_t li = wbase + (uint32_t)r * 32 + lane;
+        if (li < tn) {
+            const uint32_t rk = (rank[r / 2] >> (16 * (r & 1))) & 0xFFFFu;
+            const uint32_t pos = wcnt[(key[r] >> shift) & dmask] + rk;
+            skey[pos] = key[r];
+            sval[pos] = vin ? vin[tbase + li] : tbase + li;
+        }
+    }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < tn; i += BT) {
+        const uint32_t k = skey[i];
+        const uint32_t at = base[(k >> shift) & dmask] + i;
+        kout[at] = k;
+        vout[at] = sval[i];
+    }
+}
+
+// Sorts n pairs (keys k0, values: the positions); counted: the first pass's tile counts are in
+// the workspace already; alternate buffers k1 and v1, values through v0 and v1. On return *kout and *vout
+// are the buffers that hold the result: v0 after an even number of passes, else v1.
+static int sort_positions(uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* v1, size_t n,
+                          SortPlan o, bool counted, void* work, uint32_t** kout,
+                          uint32_t** vout, cudaStream_t s) {
+    uint32_t* hist = (uint32_t*)work;
+    void* stemp = (char*)work + align_up(sort_counts(n, o) * 4, 256);
+    const uint32_t nb = ntiles(n);
+    uint32_t *ki = k0, *vi = v0, *ko = k1, *vo = v1;
+    int rc;
+    for (int p = 0; p < o.passes; ++p) {
+        if (p > 0 || !counted)
+            k_tile_digits<<<nb, BT, 0, s>>>(ki, (uint32_t)n, p * o.width, o.width, hist);
+        if ((rc = exclusive_scan(hist, hist, sort_counts(n, o), stemp, s))) return rc;
+        k_sort_pass<<<nb, BT, 0, s>>>(ki, p == 0 ? nullptr : vi, ko, vo, (uint32_t)n,
+                                      p * o.width, o.width, hist);
+        std::swap(ki, ko);
+        std::swap(vi, vo);
+    }
+    *kout = ki;
+    *vout = vi;
+    return cuda_fail(cudaGetLastError(), "sort");
 }
 
 // ---------------------------------------------------------------------------------------
@@ -487,69 +705,72 @@ size_t detect_segments_temp_bytes(size_t n) {
     return 2 * align_up(n * 4 + 4, 256) + scan_temp_bytes(n);
 }
 
-// Segment starts without per-key flags (the map build's form, no segment ids): one block
-// per TILE keys counts the tile's segment starts (key != previous key), the tile counts are
-// scanned, and the blocks write their starts at the scanned offsets in key order.
+// Segment starts without per-key flags (the map build's form, no segment ids), in one launch:
+// a block counts its tile's segment starts (key != previous key), finds the earlier tiles'
+// count by look-back and writes its starts there, in key order. tmp as for k_scan.
 template <typename K>
-__global__ void __launch_bounds__(BT) k_seg_count(const K* __restrict__ keys, size_t n,
-                                                  uint32_t* __restrict__ tile_cnt) {
+__global__ void __launch_bounds__(BT) k_seg_starts(const K* __restrict__ keys, size_t n,
+                                                   unsigned long long* __restrict__ tmp,
+                                                   uint32_t* __restrict__ starts,
+                                                   uint32_t* __restrict__ num) {
     __shared__ uint32_t ws[BT / 32];
-    const size_t base = (size_t)blockIdx.x * TILE + (size_t)threadIdx.x * ITEMS;
-    uint32_t c = 0;
-    K prev = base > 0 && base - 1 < n ? keys[base - 1] : K(0);
+    __shared__ uint32_t s_tile, s_excl;
+    __shared__ bool s_ok;
+    constexpr int ROUNDS = TILE / BT;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) s_tile = atomicAdd((unsigned int*)tmp, 1u);
+    __syncthreads();
+    const uint32_t tile = s_tile;
+    // warp w holds the tile's keys [w * 512, (w + 1) * 512) as 16 rounds of 32
+    const size_t wbase = (size_t)tile * TILE + (size_t)warp * (ROUNDS * 32);
+    uint32_t start[ROUNDS], mine = 0;  // a round's segment starts, by lane
+    K last = lane == 0 && wbase > 0 && wbase - 1 < n ? keys[wbase - 1] : K(0);
+    last = __shfl_sync(0xffffffffu, last, 0);
 #pragma unroll
-    for (int k = 0; k < ITEMS; ++k) {
-        const size_t i = base + k;
-        if (i < n) {
-            const K key = keys[i];
-            c += (i == 0 || key != prev) ? 1u : 0u;
-            prev = key;
+    for (int r = 0; r < ROUNDS; ++r) {
+        const size_t i = wbase + (size_t)r * 32 + lane;
+        const K key = i < n ? keys[i] : K(0);
+        K prev = __shfl_up_sync(0xffffffffu, key, 1);
+        if (lane == 0) prev = last;
+        last = __shfl_sync(0xffffffffu, key, 31);
+        start[r] = __ballot_sync(0xffffffffu, i < n && (i == 0 || key != prev));
+        mine += (uint32_t)__popc(start[r]);
+    }
+    uint32_t tot;
+    uint32_t r0 = block_exclusive_scan(lane == 0 ? mine : 0u, ws, &tot);
+    r0 = __shfl_sync(0xffffffffu, r0, 0);
+    if (threadIdx.x < 32) {
+        unsigned long long e;
+        const bool ok = lookback_warp(tmp + 1, tile, tot, (int)threadIdx.x, e);
+        if (threadIdx.x == 0) {
+            s_excl = (uint32_t)e;
+            s_ok = ok;
         }
     }
-    uint32_t tot;
-    block_exclusive_scan(c, ws, &tot);
-    if (threadIdx.x == 0) tile_cnt[blockIdx.x] = tot;
-}
-
-template <typename K>
-__global__ void __launch_bounds__(BT) k_seg_write(const K* __restrict__ keys, size_t n,
-                                                  const uint32_t* __restrict__ tile_off,
-                                                  uint32_t* __restrict__ starts,
-                                                  uint32_t* __restrict__ num) {
-    __shared__ uint32_t ws[BT / 32];
-    const size_t base = (size_t)blockIdx.x * TILE + (size_t)threadIdx.x * ITEMS;
-    K kv[ITEMS];
-    uint32_t flags = 0, c = 0;
-    K prev = base > 0 && base - 1 < n ? keys[base - 1] : K(0);
+    __syncthreads();
+    if (!s_ok) return;
+    r0 += s_excl;
 #pragma unroll
-    for (int k = 0; k < ITEMS; ++k) {
-        const size_t i = base + k;
-        kv[k] = i < n ? keys[i] : K(0);
-        const bool f = i < n && (i == 0 || kv[k] != prev);
-        prev = kv[k];
-        flags |= (f ? 1u : 0u) << k;
-        c += f ? 1u : 0u;
+    for (int r = 0; r < ROUNDS; ++r) {
+        if (start[r] >> lane & 1u)
+            starts[r0 + __popc(start[r] & ((1u << lane) - 1u))] =
+                (uint32_t)(wbase + (size_t)r * 32 + lane);
+        r0 += (uint32_t)__popc(start[r]);
     }
-    uint32_t tot;
-    uint32_t r = tile_off[blockIdx.x] + block_exclusive_scan(c, ws, &tot);
-#pragma unroll
-    for (int k = 0; k < ITEMS; ++k)
-        if (flags >> k & 1u) starts[r++] = (uint32_t)(base + k);
-    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *num = tile_off[blockIdx.x] + tot;
+    if (tile == gridDim.x - 1 && threadIdx.x == 0) *num = s_excl + tot;
 }
 
-// starts of the runs of equal keys in sorted[0..n), their count in *num_segments;
-// temp >= ntiles(n) * 4 bytes
+// starts of the runs of equal keys in sorted[0..n), their count in *num_segments (0 when a
+// wait ran out); temp >= scan_temp_bytes(n), 8-byte aligned
 template <typename K>
 static int segment_starts(const K* sorted, size_t n, uint32_t* seg_starts,
                           uint32_t* num_segments, void* temp, cudaStream_t s) {
     cudaMemsetAsync(num_segments, 0, 4, s);
     if (n == 0) return cuda_fail(cudaGetLastError(), "segments");
     const uint32_t nb = ntiles(n);
-    uint32_t* cnt = (uint32_t*)temp;
-    k_seg_count<K><<<nb, BT, 0, s>>>(sorted, n, cnt);
-    k_scan_bsums<<<1, BT, 0, s>>>(cnt, nb);
-    k_seg_write<K><<<nb, BT, 0, s>>>(sorted, n, cnt, seg_starts, num_segments);
+    cudaMemsetAsync(temp, 0, (size_t)nb * 8 + 8, s);
+    k_seg_starts<K><<<nb, BT, 0, s>>>(sorted, n, (unsigned long long*)temp, seg_starts,
+                                      num_segments);
     return cuda_fail(cudaGetLastError(), "segments");
 }
 
@@ -594,39 +815,94 @@ __device__ __forceinline__ void cell_of(const float* p, float res, int32_t* c) {
     c[2] = sat_i32(floorf(p[2] / res));
 }
 
-// mm: [0..2] min cell, [3..5] max cell, [6] finite count
-__global__ void __launch_bounds__(BT) k_cells_minmax(const float* __restrict__ pts, size_t n,
-                                                     float res, int32_t* __restrict__ mm) {
-    int32_t mn[3] = {INT32_MAX, INT32_MAX, INT32_MAX}, mx[3] = {INT32_MIN, INT32_MIN, INT32_MIN};
-    uint32_t cnt = 0;
-    for (size_t i = (size_t)blockIdx.x * BT + threadIdx.x; i < n; i += (size_t)gridDim.x * BT) {
-        float p[3] = {pts[3 * i], pts[3 * i + 1], pts[3 * i + 2]};
-        if (!finite3(p[0], p[1], p[2])) continue;
-        int32_t c[3];
+// The same by a multiplication with inv = 1 / res where res is a power of two (inv exact, so
+// the product is the quotient, rounded alike), else by the division (inv 0)
+__device__ __forceinline__ void cell_of_inv(const float* p, float res, float inv, int32_t* c) {
+    if (inv == 0.f) {
         cell_of(p, res, c);
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            mn[a] = min(mn[a], c[a]);
-            mx[a] = max(mx[a], c[a]);
-        }
-        cnt++;
+        return;
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
+    for (int a = 0; a < 3; ++a) c[a] = sat_i32(floorf(__fmul_rn(p[a], inv)));
+}
+static float exact_inverse(float res) {
+    int e = 0;
+    const float f = std::frexp(res, &e);
+    const float inv = 1.0f / res;
+    return f == 0.5f && std::isnormal(inv) ? inv : 0.f;
+}
+
+// Point i of pts, four consecutive points (i a multiple of 4) as three 16-byte loads when `vec`
+// (pts 16-byte aligned) and all four exist; returns how many of the four there are.
+__device__ __forceinline__ int load4(const float* __restrict__ pts, size_t n, size_t i, bool vec,
+                                     float (*p)[3]) {
+    if (vec && i + 4 <= n) {
+        const float4* q = reinterpret_cast<const float4*>(pts + 3 * i);
+        const float4 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2);
+        const float v[12] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y, c.z, c.w};
 #pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            mn[a] = min(mn[a], __shfl_xor_sync(0xffffffffu, mn[a], o));
-            mx[a] = max(mx[a], __shfl_xor_sync(0xffffffffu, mx[a], o));
-        }
-        cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+        for (int k = 0; k < 12; ++k) p[k / 3][k % 3] = v[k];
+        return 4;
     }
-    if ((threadIdx.x & 31) == 0) {
+    int m = 0;
 #pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            atomicMin(&mm[a], mn[a]);
-            atomicMax(&mm[3 + a], mx[a]);
+    for (int k = 0; k < 4; ++k)
+        if (i + k < n) {
+            m = k + 1;
+            for (int a = 0; a < 3; ++a) p[k][a] = pts[3 * (i + k) + a];
         }
-        atomicAdd(&mm[6], (int32_t)cnt);
+    return m;
+}
+
+// mm: [0..2] min cell, [3..5] max cell, [6] finite count. Bound: reading the points once; a
+// block adds its seven values with one atomic each (one per warp queued at seven addresses:
+// 58 us on 5M points, 17 now).
+__global__ void __launch_bounds__(BT) k_cells_minmax(const float* __restrict__ pts, size_t n,
+                                                     float res, float inv, bool vec,
+                                                     int32_t* __restrict__ mm) {
+    __shared__ int32_t red[BT / 32][7];
+    int32_t v[6] = {INT32_MAX, INT32_MAX, INT32_MAX, INT32_MIN, INT32_MIN, INT32_MIN};
+    uint32_t cnt = 0;
+    for (size_t i = 4 * ((size_t)blockIdx.x * BT + threadIdx.x); i < n;
+         i += 4 * (size_t)gridDim.x * BT) {
+        float p[4][3];
+        const int m = load4(pts, n, i, vec, p);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (k >= m || !finite3(p[k][0], p[k][1], p[k][2])) continue;
+            int32_t c[3];
+            cell_of_inv(p[k], res, inv, c);
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                v[a] = min(v[a], c[a]);
+                v[3 + a] = max(v[3 + a], c[a]);
+            }
+            cnt++;
+        }
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        v[a] = __reduce_min_sync(0xffffffffu, v[a]);
+        v[3 + a] = __reduce_max_sync(0xffffffffu, v[3 + a]);
+    }
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
+    if (lane == 0) {
+#pragma unroll
+        for (int a = 0; a < 6; ++a) red[warp][a] = v[a];
+        red[warp][6] = (int32_t)cnt;
+    }
+    __syncthreads();
+    if (threadIdx.x < 7) {
+        const int a = threadIdx.x;
+        int32_t x = red[0][a];
+        for (int w = 1; w < BT / 32; ++w) {
+            const int32_t y = red[w][a];
+            x = a < 3 ? min(x, y) : (a < 6 ? max(x, y) : x + y);
+        }
+        if (a < 3) atomicMin(&mm[a], x);
+        else if (a < 6) atomicMax(&mm[a], x);
+        else atomicAdd(&mm[6], x);
     }
 }
 
@@ -662,12 +938,103 @@ __global__ void __launch_bounds__(BT) k_morton(const float* __restrict__ pts, si
     idx[i] = (uint32_t)i;
 }
 
+// Order-preserving 32-bit form of the Morton key of a cell offset inside a box with b[a] bits
+// per axis (b0 + b1 + b2 <= 31): the interleaved bits that can be set. Up to the shortest
+// axis's bits all three interleave, above them the two longer ones, above those the longest.
+struct CompactKey {
+    uint32_t lo, mid;         // bits of the shortest and of the middle axis
+    uint32_t ax_hi, ax_lo;    // the two longer axes, the earlier of x, y, z first
+    uint32_t ax_long;         // the longest
+    uint32_t total;           // key bits
+};
+static CompactKey compact_key(const uint32_t* b) {
+    uint32_t o[3] = {0, 1, 2};  // axes by bits, ascending (stable)
+    std::stable_sort(o, o + 3, [&](uint32_t x, uint32_t y) { return b[x] < b[y]; });
+    CompactKey c;
+    c.lo = b[o[0]];
+    c.mid = b[o[1]];
+    c.ax_hi = std::min(o[1], o[2]);
+    c.ax_lo = std::max(o[1], o[2]);
+    c.ax_long = o[2];
+    c.total = b[0] + b[1] + b[2];
+    return c;
+}
+__host__ __device__ __forceinline__ uint32_t spread16(uint32_t v) {
+    v &= 0xFFFFu;
+    v = (v | (v << 8)) & 0x00FF00FFu;
+    v = (v | (v << 4)) & 0x0F0F0F0Fu;
+    v = (v | (v << 2)) & 0x33333333u;
+    return (v | (v << 1)) & 0x55555555u;
+}
+__host__ __device__ __forceinline__ uint32_t spread10(uint32_t v) {
+    v &= 0x3FFu;
+    v = (v | (v << 16)) & 0x030000FFu;
+    v = (v | (v << 8)) & 0x0300F00Fu;
+    v = (v | (v << 4)) & 0x030C30C3u;
+    return (v | (v << 2)) & 0x09249249u;
+}
+__host__ __device__ __forceinline__ uint32_t compact_morton(const CompactKey& c,
+                                                            const uint32_t* q) {
+    const uint32_t lm = (1u << c.lo) - 1u;  // lo <= 10, mid - lo <= 15
+    uint32_t key = (spread10(q[0] & lm) << 2) | (spread10(q[1] & lm) << 1) | spread10(q[2] & lm);
+    const uint32_t qh = c.ax_hi == 0u ? q[0] : q[1], ql = c.ax_lo == 1u ? q[1] : q[2];
+    const uint32_t qx = c.ax_long == 0u ? q[0] : (c.ax_long == 1u ? q[1] : q[2]);
+    const uint32_t w = c.mid - c.lo, wm = (1u << w) - 1u;
+    key |= ((spread16((qh >> c.lo) & wm) << 1) | spread16((ql >> c.lo) & wm)) << (3u * c.lo);
+    const uint32_t up = 3u * c.lo + 2u * w;
+    return up < 32u ? key | ((qx >> c.mid) << up) : key;
+}
+
+// Compact Morton key of every point (non-finite points: the first value past every cell's, so
+// they sort last) and the first sort pass's tile counts. A block takes one tile, four points a
+// thread at a time.
+__global__ void __launch_bounds__(BT) k_compact_keys(const float* __restrict__ pts, uint32_t n,
+                                                     float res, float inv, bool vec,
+                                                     const int32_t* __restrict__ mm,
+                                                     CompactKey ck, int width,
+                                                     uint32_t* __restrict__ keys,
+                                                     uint32_t* __restrict__ hist) {
+    __shared__ TileCounts t;
+    const uint32_t bins = 1u << width;
+    tile_counts_clear(t, bins);
+    __syncthreads();
+    const int32_t mn[3] = {mm[0], mm[1], mm[2]};
+#pragma unroll 1
+    for (uint32_t r = 0; r < TILE / (4 * BT); ++r) {
+        const size_t i = (size_t)blockIdx.x * TILE + 4 * (r * BT + threadIdx.x);
+        float p[4][3];
+        const int m = i < n ? load4(pts, n, i, vec, p) : 0;
+        uint32_t key[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            key[k] = 1u << ck.total;
+            if (k < m && finite3(p[k][0], p[k][1], p[k][2])) {
+                int32_t c[3];
+                cell_of_inv(p[k], res, inv, c);
+                const uint32_t q[3] = {(uint32_t)c[0] - (uint32_t)mn[0],
+                                       (uint32_t)c[1] - (uint32_t)mn[1],
+                                       (uint32_t)c[2] - (uint32_t)mn[2]};
+                key[k] = compact_morton(ck, q);
+            }
+            tile_counts_add(t, key[k] & (bins - 1u), k < m);
+        }
+        if (m == 4) {
+            *reinterpret_cast<uint4*>(keys + i) = make_uint4(key[0], key[1], key[2], key[3]);
+        } else {
+            for (int k = 0; k < m; ++k) keys[i + k] = key[k];
+        }
+    }
+    __syncthreads();
+    tile_counts_store(t, bins, hist, blockIdx.x, gridDim.x);
+}
+
 // min / max cell and finite count of the points into mm
 static void cell_bounds(const float* pts, size_t n, float res, int32_t* mm, cudaStream_t s) {
     k_minmax_init<<<1, 32, 0, s>>>(mm);
     if (n) {
-        unsigned g = (unsigned)std::min<size_t>((n + BT - 1) / BT, 152 * 8);
-        k_cells_minmax<<<g, BT, 0, s>>>(pts, n, res, mm);
+        unsigned g = (unsigned)std::min<size_t>((n + 4 * BT - 1) / (4 * BT), 152 * 8);
+        k_cells_minmax<<<g, BT, 0, s>>>(pts, n, res, exact_inverse(res),
+                                        ((uintptr_t)pts & 15u) == 0, mm);
     }
 }
 
@@ -684,7 +1051,9 @@ int morton_codes(const float* pts, size_t n, float res, uint64_t* codes, uint32_
 
 // Cyclic Jacobi for a symmetric 3x3 in f32 (row-major a, eigenvectors in the columns of v).
 // It only has to find the eigenvector directions to f32 accuracy: the eigenvalues and the
-// regularised covariance and inverse are then formed in FP64 (k_voxel_stats).
+// regularised covariance and inverse are then formed in FP64 (k_voxel_stats), so the rotations
+// use the approximate reciprocals. The caller scales the matrix to a largest diagonal entry of
+// about 1.
 __device__ void jacobi3f(float* a, float* v) {
     for (int i = 0; i < 3; ++i)
         for (int j = 0; j < 3; ++j) v[i * 3 + j] = (i == j) ? 1.f : 0.f;
@@ -698,10 +1067,16 @@ __device__ void jacobi3f(float* a, float* v) {
             const int p = pq == 2 ? 1 : 0, q = pq == 0 ? 1 : 2;
             const float apq = a[p * 3 + q];
             if (apq == 0.f) continue;
-            const float theta = (a[q * 3 + q] - a[p * 3 + p]) / (2.f * apq);
-            float t = 1.f / (fabsf(theta) + sqrtf(theta * theta + 1.f));
-            if (theta < 0.f) t = -t;
-            const float c = 1.f / sqrtf(t * t + 1.f);
+            // t = tan of the angle, |d + sqrt(d^2 + (2 a_pq)^2)| scaled clear of under- and
+            // overflow by the larger of the two
+            const float d = a[q * 3 + q] - a[p * 3 + p], o2 = 2.f * apq;
+            const float sc = fmaxf(fabsf(d), fabsf(o2));
+            if (!(sc > 1e-30f)) continue;  // (the largest entry is about 1)
+            const float dn = __fdividef(d, sc), on = __fdividef(o2, sc);
+            const float h = dn * dn + on * on;
+            float t = __fdividef(fabsf(on), fabsf(dn) + h * rsqrtf(h));
+            if ((d < 0.f) != (apq < 0.f)) t = -t;
+            const float c = rsqrtf(t * t + 1.f);
             const float sn = t * c;
             a[p * 3 + p] -= t * apq;
             a[q * 3 + q] += t * apq;
@@ -754,6 +1129,24 @@ __device__ void jacobi3_refine(double* B, double* V, int max_sweeps) {
     }
 }
 
+// v 2^e, v and the result zero or normal: an addition to the exponent field. (A warp's FP64
+// instruction occupies the SM's FP64 unit for 16 cycles; integer ones are free beside it.)
+__device__ __forceinline__ double scale2(double v, int e) {
+    const long long b = __double_as_longlong(v);
+    return __longlong_as_double(b == 0ll ? b : b + ((long long)e << 52));
+}
+
+// 1 / d for a normal d: the f32 reciprocal and two Newton steps (error 2^-52 or so)
+__device__ __forceinline__ double recip2(double d) {
+    // d scaled into f32's range by its exponent, the reciprocal scaled back
+    const int e = (int)((__double_as_longlong(d) >> 52) & 0x7FF) - 1023;
+    const double m = scale2(d, -e);
+    double r = (double)(1.f / (float)m);
+    r = fma(r, fma(-m, r, 1.0), r);
+    r = fma(r, fma(-m, r, 1.0), r);
+    return scale2(r, -e);
+}
+
 // FP64 Rayleigh quotient v^T A v / v^T v of an f32 unit vector v (|v|^2 = 1 +- 1e-7, so
 // 1 / v^T v = 2 - v^T v to FP64 rounding): FP64-accurate for an eigenvalue, since its error
 // is quadratic in v's direction error. *w receives 1 / v^T v.
@@ -776,7 +1169,7 @@ __device__ __forceinline__ bool inverse_sym3(const double* C, float* icov6) {
     const double c22 = C[0] * C[4] - C[1] * C[1];
     const double det = C[0] * c00 + C[1] * c01 + C[2] * c02;
     if (!(det > 0.0)) return false;
-    const double id = 1.0 / det;
+    const double id = recip2(det);
     icov6[0] = (float)(c00 * id);
     icov6[1] = (float)(c01 * id);
     icov6[2] = (float)(c02 * id);
@@ -825,8 +1218,9 @@ __device__ __forceinline__ void refine_vector(const double* A, double* v, double
 // (Gram-Schmidt), Jacobi sweeps on V^T A V to the reference's stopping rule, and the
 // reconstruction from the eigen-decomposition. Every route is FP64-accurate, so the f32
 // outputs agree with an FP64 eigen-decomposition to f32 rounding.
-__device__ bool regularize(const double* A, const float* a32, const float* V32, float ratio,
-                           SegRec& r) {
+// a32 carries the scale 2^-e32x of voxel_finish.
+__device__ bool regularize(const double* A, const float* a32, const float* V32, int e32x,
+                           float ratio, SegRec& r) {
     const float e32[3] = {a32[0], a32[4], a32[8]};
     const float mx32 = fmaxf(e32[0], fmaxf(e32[1], e32[2]));
     bool fast = mx32 > 0.f;
@@ -850,21 +1244,33 @@ __device__ bool regularize(const double* A, const float* a32, const float* V32, 
             for (int q = 0; q < 9; ++q) r.cov[q] = (float)A[q];
             return inverse_sym3(A, r.icov);
         }
+        // FP64 eigenvalues of the largest eigenvector (the threshold) and of the one to refine
+        // (t); the others only enter as f32 gaps of the first-order correction
         double v[3][3], w[3], lam[3];
+        const int one = __popc(clamp) == 1;
+        const int t = one ? __ffs(clamp) - 1 : __ffs(7 & ~clamp) - 1;
+        const int top = e32[0] >= e32[1] ? (e32[0] >= e32[2] ? 0 : 2) : (e32[1] >= e32[2] ? 1 : 2);
+#pragma unroll
         for (int i = 0; i < 3; ++i) {
             for (int k = 0; k < 3; ++k) v[i][k] = (double)V32[k * 3 + i];
-            lam[i] = rayleigh(A, v[i], &w[i]);
+            lam[i] = scale2((double)e32[i], e32x);
+            w[i] = 1.0;
         }
-        const double mx = fmax(lam[0], fmax(lam[1], lam[2]));
+        double mx = 0.0, lt = 0.0;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            if (i != top && i != t) continue;
+            lam[i] = rayleigh(A, v[i], &w[i]);
+            if (i == top) mx = lam[i];
+            if (i == t) lt = lam[i];
+        }
         if (!(mx > 0.0)) return false;
         const double thr = mx * (double)ratio;
-        const int one = __popc(clamp) == 1;
-        const int t = one ? __ffs(clamp) - 1 : __ffs(7 & ~clamp) - 1;  // the vector to refine
         double u[3] = {v[t][0], v[t][1], v[t][2]};
-        refine_vector(A, u, lam[t], v, lam, w, 7 & ~(1 << t));
+        refine_vector(A, u, lt, v, lam, w, 7 & ~(1 << t));
         const double wu = 2.0 - (u[0] * u[0] + u[1] * u[1] + u[2] * u[2]);
         double C[9];
-        const double c = one ? (thr - lam[t]) * wu : (lam[t] - thr) * wu;
+        const double c = one ? (thr - lt) * wu : (lt - thr) * wu;
         for (int rr = 0; rr < 3; ++rr)
             for (int cc = rr; cc < 3; ++cc) {  // upper triangle, mirrored: C stays symmetric
                 const double base = one ? A[rr * 3 + cc] : (rr == cc ? thr : 0.0);
@@ -1028,11 +1434,6 @@ __device__ __forceinline__ void exact_add(ExactMoments& em, const float* p) {
     add_prod128(em.s2h[5], em.s2l[5], d[2], d[2]);
 }
 
-// 2^e as an FP64 (normal range)
-__device__ __forceinline__ double pow2d(int e) {
-    return __longlong_as_double((long long)(e + 1023) << 52);
-}
-
 // A signed 128-bit integer (hi, lo) rounded once to the nearest FP64 (ties to even)
 __device__ __forceinline__ double i128_to_double(long long hi, unsigned long long lo) {
     const bool neg = hi < 0;
@@ -1049,7 +1450,7 @@ __device__ __forceinline__ double i128_to_double(long long hi, unsigned long lon
     unsigned long long top = lz ? (uh << lz) | (ul >> (64 - lz)) : uh;
     const unsigned long long rest = lz ? ul << lz : ul;
     if (rest != 0ull) top |= 1ull;  // sticky: the discarded bits decide ties and halves
-    const double v = __ull2double_rn(top) * pow2d(64 - lz);
+    const double v = scale2(__ull2double_rn(top), 64 - lz);
     return neg ? -v : v;
 }
 
@@ -1058,6 +1459,7 @@ __device__ __forceinline__ double i128_to_double(long long hi, unsigned long lon
 __device__ __forceinline__ int exact_finish(const ExactMoments& em, uint32_t n, double* mean,
                                             double* A) {
     const double nn = (double)n;
+    const double rn = 1.0 / nn;  // correctly rounded
     int redo = 0;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
@@ -1065,12 +1467,17 @@ __device__ __forceinline__ int exact_finish(const ExactMoments& em, uint32_t n, 
         const unsigned long long mag = tot < 0 ? (unsigned long long)(-tot) : (unsigned long long)tot;
         const int sig = mag ? 64 - __clzll((long long)mag) - min(em.tz[a], 63) : 0;
         if (em.rep[a] && sig <= 53) {
-            mean[a] = (__ll2double_rn(tot) * pow2d(em.e0[a])) / nn;
+            // tot / n from the rounded reciprocal: q = tot rn is corrected by its exact
+            // remainder, which gives the correctly rounded quotient (Markstein 1990); the
+            // scaling by 2^e0 is exact
+            const double t = __ll2double_rn(tot);
+            const double q = t * rn;
+            mean[a] = scale2(fma(fma(-q, nn, t), rn, q), em.e0[a]);
         } else {
             redo |= 1 << a;
         }
     }
-    const double inv_den = 1.0 / (nn * (double)(n - 1u));
+    const double inv_den = recip2(nn * (double)(n - 1u));
     const int ia[6] = {0, 0, 0, 1, 1, 2}, ib[6] = {0, 1, 2, 1, 2, 2};
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
@@ -1084,7 +1491,7 @@ __device__ __forceinline__ int exact_finish(const ExactMoments& em, uint32_t n, 
         const unsigned long long rl = nl - ql;
         const long long rh = nh - qh - (nl < ql ? 1ll : 0ll);
         const double v =
-            i128_to_double(rh, rl) * pow2d(em.e0[ia[k]] + em.e0[ib[k]]) * inv_den;
+            scale2(i128_to_double(rh, rl) * inv_den, em.e0[ia[k]] + em.e0[ib[k]]);
         A[ia[k] * 3 + ib[k]] = A[ib[k] * 3 + ia[k]] = v;
     }
     return redo;
@@ -1144,12 +1551,20 @@ __device__ __noinline__ void moments_two_pass(Each each, uint32_t cnt, double* m
 __device__ __forceinline__ bool voxel_finish(const double* mean, const double* A, float ratio,
                                              SegRec& r) {
     float a32[9], V32[9];
-    for (int q = 0; q < 9; ++q) a32[q] = (float)A[q];
+    // scaled by the power of two of the largest diagonal entry (0 for a zero matrix)
+    int e = 0;
+    for (int q = 0; q < 9; q += 4)
+        e = max(e, (int)((__double_as_longlong(A[q]) >> 52) & 0x7FF));
+    e = e ? e - 1023 : 0;
+    const double dn = __longlong_as_double((long long)(1023 - min(e, 1000)) << 52);
+    for (int q = 0; q < 9; ++q) a32[q] = (float)(A[q] * dn);
     jacobi3f(a32, V32);
-    if (!regularize(A, a32, V32, ratio, r)) return false;
+    if (!regularize(A, a32, V32, min(e, 1000), ratio, r)) return false;
     for (int q = 0; q < 3; ++q) r.mean[q] = (float)mean[q];
     return true;
 }
+
+constexpr uint32_t SIZE_KEY_MAX = 255;
 
 // Largest voxel whose sums stay exact (S1 below 2^57, S2 below 2^98 with |d| < 2^41)
 constexpr uint32_t EXACT_MAX_POINTS = 65536;
@@ -1181,21 +1596,20 @@ __device__ __forceinline__ bool voxel_stats(Each each, const float* first, uint3
     return voxel_finish(mean, A, ratio, r);
 }
 
-// Segment sizes as sort keys: segments visited largest first (key 0xFFFF - min(count,
-// 0xFFFF)), so the threads of a warp take segments of nearly equal size and the longest
-// start first.
+// Segment sizes as 8-bit sort keys: segments visited largest first (key 255 - min(count, 255)),
+// so the threads of a warp take segments of nearly equal size and the longest start first.
 __global__ void k_seg_size_keys(const uint32_t* __restrict__ starts, uint32_t S, uint32_t nf,
-                                uint32_t* __restrict__ keys, uint32_t* __restrict__ order) {
+                                uint32_t* __restrict__ keys) {
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= S) return;
     const uint32_t e = s + 1 < S ? starts[s + 1] : nf;
-    keys[s] = 0xFFFFu - min(e - starts[s], 0xFFFFu);
-    order[s] = s;
+    keys[s] = SIZE_KEY_MAX - min(e - starts[s], SIZE_KEY_MAX);
 }
 
 // Voxels of at least WARP_SEG_MIN points are summed by a whole warp (exact sums of the lanes'
 // strided shares, added over the lanes in 128-bit), up to EXACT_MAX_POINTS points.
 constexpr uint32_t WARP_SEG_MIN = 48;
+static_assert(WARP_SEG_MIN < SIZE_KEY_MAX, "the size keys tell large segments apart");
 
 // 128-bit (hi, lo) sum over the warp's lanes (every lane ends with the total)
 __device__ __forceinline__ void warp_sum128(long long& hi, unsigned long long& lo) {
@@ -1244,7 +1658,7 @@ struct SegSums {
 // Number of visit-order segments with at least WARP_SEG_MIN points (sorted size keys ascend)
 __device__ __forceinline__ uint32_t large_segments(const uint32_t* __restrict__ skey, uint32_t S) {
     uint32_t lo = 0, hi = S;
-    const uint32_t lim = 0xFFFFu - WARP_SEG_MIN;
+    const uint32_t lim = SIZE_KEY_MAX - WARP_SEG_MIN;
     while (lo < hi) {
         const uint32_t mid = (lo + hi) >> 1;
         if (skey[mid] <= lim) lo = mid + 1;
@@ -1392,7 +1806,12 @@ __device__ __forceinline__ int64_t hash_claim(uint32_t* keys, uint32_t stride, u
 // voxels) writing 52 bytes to each random slot took 607 us and filling the grid from the
 // slots 112 us more; records in voxel order are written by neighbouring threads, and
 // neighbouring voxels share the lines that the searches read.
-__global__ void __launch_bounds__(128) k_voxel_compact(
+// A block reads its 128 records and writes its voxels (consecutive ones: ranks are a scan)
+// through shared memory, so 88-byte records and 36-byte matrices move as whole lines (a thread
+// each was bound by the load-store unit's replays). Compaction, hash insert and grid of the
+// 50M-point 2 m map together: 0.88 ms as three kernels, 0.36 now.
+constexpr int VC = 128;
+__global__ void __launch_bounds__(VC) k_voxel_compact(
     const SegRec* __restrict__ rec, const uint32_t* __restrict__ valid,
     const uint32_t* __restrict__ rank, uint32_t S, int32_t* __restrict__ coord,
     float4* __restrict__ mean4, float* __restrict__ cov, float* __restrict__ icov,
@@ -1400,22 +1819,30 @@ __global__ void __launch_bounds__(128) k_voxel_compact(
     float4* __restrict__ grid, uint32_t* __restrict__ keys, uint4* __restrict__ slots,
     int32_t* __restrict__ slot_vidx, uint32_t* __restrict__ max_probe,
     uint32_t* __restrict__ status) {
-    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+    constexpr int RW = sizeof(SegRec) / 4;
+    static_assert(sizeof(SegRec) == RW * 4, "records move as words");
+    __shared__ uint32_t in[VC * RW];
+    __shared__ float o_cov[VC * 9], o_icov[VC * 9];
+    __shared__ int32_t o_coord[VC * 3];
+    const uint32_t s0 = blockIdx.x * VC, s = s0 + threadIdx.x, ns = min((uint32_t)VC, S - s0);
+    for (uint32_t i = threadIdx.x; i < ns * RW; i += VC)
+        in[i] = __ldg(reinterpret_cast<const uint32_t*>(rec + s0) + i);
+    const bool ok = s < S && valid[s];
+    const uint32_t v0 = rank[s0], v = s < S ? rank[s] : 0u;
+    const uint32_t nv = (uint32_t)__syncthreads_count(ok);
     uint32_t disp = 0;  // this voxel's displacement from its home slot
-    if (s < S && valid[s]) {
-        const uint32_t v = rank[s];
-        const SegRec& r = rec[s];
+    if (ok) {
+        const SegRec& r = *reinterpret_cast<const SegRec*>(in + threadIdx.x * RW);
+        const uint32_t lv = v - v0;
         const int32_t g[3] = {r.coord[0], r.coord[1], r.coord[2]};
-        coord[3 * (size_t)v] = g[0];
-        coord[3 * (size_t)v + 1] = g[1];
-        coord[3 * (size_t)v + 2] = g[2];
+        for (int a = 0; a < 3; ++a) o_coord[3 * lv + a] = g[a];
         const float mu[3] = {r.mean[0], r.mean[1], r.mean[2]};
         mean4[v] = make_float4(mu[0], mu[1], mu[2], __uint_as_float(r.count));
-        for (int q = 0; q < 9; ++q) cov[9 * (size_t)v + q] = r.cov[q];
+        for (int q = 0; q < 9; ++q) o_cov[9 * lv + q] = r.cov[q];
         float c[6];
         for (int q = 0; q < 6; ++q) c[q] = r.icov[q];
         const float full[9] = {c[0], c[1], c[2], c[1], c[3], c[4], c[2], c[4], c[5]};
-        for (int q = 0; q < 9; ++q) icov[9 * (size_t)v + q] = full[q];
+        for (int q = 0; q < 9; ++q) o_icov[9 * lv + q] = full[q];
         count[v] = r.count;
         uint32_t key, home;
         cell_slot(m, g[0], g[1], g[2], key, home);  // every voxel lies inside the map's box
@@ -1441,105 +1868,135 @@ __global__ void __launch_bounds__(128) k_voxel_compact(
             atomicOr(status, ST_HASH_FULL);
         }
     }
-    // the largest displacement: one atomic per warp that has a displaced voxel (3M threads on
-    // one counter would queue at its L2 slice)
+    // the largest displacement: an atomic only where it grows (one per warp queued at the
+    // counter's L2 slice: 90k atomics, 0.5 ms of the 50M-point build)
     disp = __reduce_max_sync(0xffffffffu, disp);
-    if ((threadIdx.x & 31u) == 0 && disp) atomicMax(max_probe, disp);
+    if ((threadIdx.x & 31u) == 0 && disp > *(volatile uint32_t*)max_probe)
+        atomicMax(max_probe, disp);
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < nv * 9; i += VC) {
+        cov[9 * (size_t)v0 + i] = o_cov[i];
+        icov[9 * (size_t)v0 + i] = o_icov[i];
+    }
+    for (uint32_t i = threadIdx.x; i < nv * 3; i += VC) coord[3 * (size_t)v0 + i] = o_coord[i];
 }
 
-// Neighbourhood masks (layout in MapView::nmask), scattered from the voxels: the voxel in
-// local cell v is neighbour d = (dx, dy, dz) of cell v - d, so it sets bit
-// 9 (dx + 1) + 3 (dy + 1) + (dz + 1) of that cell's mask (or octant masks), at grown-box
-// position v - d + 1 (always inside the grown box). One thread per voxel, in Morton order, so
-// a warp's atomics fall on neighbouring words; the masks start at zero, and OR is order-free,
-// so the result does not depend on the threads' order. The work goes with the number of
-// voxels, not with the box. The two octants along z are neighbouring words and are set by one
-// 64-bit atomic (bound: the L2's atomic rate).
-// A bit is set only where the voxel's centroid can pass the radius test from some point of
-// cell v - d (of that octant of it): its distance to the cell's (octant's) box is at most the
-// radius, widened by 1e-5 of it and by 1e-6 cell widths per cell of distance from the origin
-// (the f32 rounding of a point's cell and octant and of the f32 distance test). A cleared bit
-// names a neighbour no point there accepts, so neighbour lists are those of the full 27-cell
-// search. On the 5M-point 400 m map at 2 m a scan point tests 16.3 candidates with one mask
-// per cell and 9.0 with octant masks, of which it accepts 5.45.
-template <bool OCT>
+// Neighbourhood masks (layout in MapView::nmask). Bit 9 (dx + 1) + 3 (dy + 1) + (dz + 1) of a
+// cell's mask (or octant's) stands for the voxel in cell + d. It is set only where that voxel's
+// centroid can pass the radius test from some point of the cell (of the octant): its distance
+// to the cell's (octant's) box is at most the radius, widened by 1e-5 of it and by 1e-6 cell
+// widths per cell of distance from the origin (the f32 rounding of a point's cell and octant
+// and of the f32 distance test). A cleared bit names a neighbour no point there accepts, so
+// neighbour lists are those of the full 27-cell search. On the 5M-point 400 m map at 2 m a scan
+// point tests 16.3 candidates with one mask per cell and 9.0 with octant masks, of which it
+// accepts 5.45.
+
+// Distance along an axis from a voxel's centroid mu (in cell c of that axis) to the box of the
+// cell at offset -d (dk = d + 1): h = 0 the lower half, 1 the upper half, or (whole) the cell
+__device__ __forceinline__ float mask_gap(float mu, int32_t c, float res, uint32_t dk, uint32_t h,
+                                          bool whole) {
+    const float half = 0.5f * res;
+    const float lo = fmaxf(mu - (float)c * res, 0.f);           // above the voxel's cell floor
+    const float hi = fmaxf(((float)c + 1.f) * res - mu, 0.f);   // below its ceiling
+    if (whole) return dk == 2u ? lo : (dk == 0u ? hi : 0.f);
+    if (dk == 2u) return h ? lo : lo + half;  // the cell below the voxel's
+    if (dk == 0u) return h ? hi + half : hi;  // the cell above
+    return h ? fmaxf(hi - half, 0.f) : fmaxf(lo - half, 0.f);  // its own slab: the other half
+}
+
+// Squared limit of the distance test for a voxel in cell c. f32 evaluation: the cell corners
+// and gaps carry at most a few ulps of far * res, well inside the 1e-6 far * res widening.
+__device__ __forceinline__ float mask_limit2(const int32_t* c, float res) {
+    float far = 0.f;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) far = fmaxf(far, fabsf((float)c[a]) + 2.f);
+    const float lim = res * (1.f + 1e-5f) + 1e-6f * far * res;
+    return lim * lim;
+}
+
+// One mask per cell (m.msh = 0), scattered from the voxels: the voxel in local cell v is
+// neighbour d of cell v - d, at grown-box position v - d + 1. One thread per voxel, in Morton
+// order, so a warp's atomics fall on neighbouring words; the masks start at zero, and OR is
+// order-free. The work goes with the number of voxels: these are the maps whose box is large.
 __global__ void __launch_bounds__(128) k_grid_mask(MapView m, const int32_t* __restrict__ coord,
                                                    const float4* __restrict__ mean4,
                                                    uint32_t* __restrict__ nmask) {
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= m.num_voxels) return;
-    const uint32_t v[3] = {(uint32_t)(coord[3 * (size_t)s] - m.min_cell[0]),
-                           (uint32_t)(coord[3 * (size_t)s + 1] - m.min_cell[1]),
-                           (uint32_t)(coord[3 * (size_t)s + 2] - m.min_cell[2])};
+    const int32_t c[3] = {coord[3 * (size_t)s], coord[3 * (size_t)s + 1],
+                          coord[3 * (size_t)s + 2]};
+    const uint32_t v[3] = {(uint32_t)(c[0] - m.min_cell[0]), (uint32_t)(c[1] - m.min_cell[1]),
+                           (uint32_t)(c[2] - m.min_cell[2])};
     const float4 mv = mean4[s];
-    const float mu[3] = {mv.x, mv.y, mv.z};
-    const float res = m.res, half = 0.5f * res;
-    // gap[a][d_a + 1][h]: distance along axis a from the centroid to the box of the cell at
-    // offset -d (h = 0: the whole cell, or with octants its lower half; h = 1: its upper half)
-    float gap[3][3][2], far = 0.f;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        const float c = (float)((int64_t)v[a] + m.min_cell[a]);
-        const float lo = fmaxf(mu[a] - c * res, 0.f);          // above the voxel's cell floor
-        const float hi = fmaxf((c + 1.f) * res - mu[a], 0.f);  // below its ceiling
-        far = fmaxf(far, fabsf(c) + 2.f);
-        if constexpr (!OCT) {
-            gap[a][2][0] = gap[a][2][1] = lo;  // d_a = +1: the cell below the voxel's
-            gap[a][0][0] = gap[a][0][1] = hi;  // d_a = -1: the cell above
-            gap[a][1][0] = gap[a][1][1] = 0.f;
-        } else {
-            gap[a][2][0] = lo + half;
-            gap[a][2][1] = lo;
-            gap[a][0][0] = hi;
-            gap[a][0][1] = hi + half;
-            gap[a][1][0] = fmaxf(lo - half, 0.f);  // the voxel's own slab: the other half
-            gap[a][1][1] = fmaxf(hi - half, 0.f);
-        }
-    }
-    // f32 evaluation: the cell corners and gaps carry at most a few ulps of far * res, well
-    // inside the 1e-6 far * res widening
-    const float lim = res * (1.f + 1e-5f) + 1e-6f * far * res;
-    const float lim2 = lim * lim;
+    const float lim2 = mask_limit2(c, m.res);
     const uint32_t E1 = m.ext[1] + 2u, E2 = m.ext[2] + 2u;
-    if constexpr (!OCT) {  // one mask per cell (m.msh = 0): a rolled loop over the 27 neighbours
 #pragma unroll 1
-        for (uint32_t b = 0; b < 27u; ++b) {
-            const uint32_t dx = b / 9u, dy = b / 3u % 3u, dz = b % 3u;
-            const float gx = dx == 2u ? gap[0][2][0] : (dx == 0u ? gap[0][0][0] : 0.f);
-            const float gy = dy == 2u ? gap[1][2][0] : (dy == 0u ? gap[1][0][0] : 0.f);
-            const float gz = dz == 2u ? gap[2][2][0] : (dz == 0u ? gap[2][0][0] : 0.f);
-            if (fmaf(gx, gx, fmaf(gy, gy, gz * gz)) > lim2) continue;
-            atomicOr(nmask + ((size_t)(v[0] + 2u - dx) * E1 + (v[1] + 2u - dy)) * E2 +
-                         (v[2] + 2u - dz),
-                     1u << b);
-        }
-    } else {
-        // octant masks (m.msh = 3): every loop unrolled, so the gap table stays in registers
-#pragma unroll
-        for (uint32_t dx = 0; dx < 3u; ++dx)  // d + 1 per axis
-#pragma unroll
-            for (uint32_t dy = 0; dy < 3u; ++dy)
-#pragma unroll
-                for (uint32_t dz = 0; dz < 3u; ++dz) {
-                    const uint32_t b = dx * 9u + dy * 3u + dz;
-                    // grown-box position of cell v - d, plus one: v + 2 - (d + 1)
-                    uint32_t* w = nmask + ((((size_t)(v[0] + 2u - dx) * E1 + (v[1] + 2u - dy)) *
-                                                E2 +
-                                            (v[2] + 2u - dz))
-                                           << 3);
-#pragma unroll
-                    for (uint32_t o = 0; o < 8u; o += 2u) {  // octants o (lower z), o + 1
-                        const float gx = gap[0][dx][(o >> 2) & 1u],
-                                    gy = gap[1][dy][(o >> 1) & 1u];
-                        const float g0 = gap[2][dz][0], g1 = gap[2][dz][1];
-                        const unsigned long long bit = 1ull << b;
-                        unsigned long long set = 0ull;
-                        if (!(fmaf(gx, gx, fmaf(gy, gy, g0 * g0)) > lim2)) set |= bit;
-                        if (!(fmaf(gx, gx, fmaf(gy, gy, g1 * g1)) > lim2)) set |= bit << 32;
-                        if (set) atomicOr((unsigned long long*)(w + o), set);
-                    }
-                }
+    for (uint32_t b = 0; b < 27u; ++b) {
+        const uint32_t dx = b / 9u, dy = b / 3u % 3u, dz = b % 3u;
+        const float gx = mask_gap(mv.x, c[0], m.res, dx, 0u, true);
+        const float gy = mask_gap(mv.y, c[1], m.res, dy, 0u, true);
+        const float gz = mask_gap(mv.z, c[2], m.res, dz, 0u, true);
+        if (fmaf(gx, gx, fmaf(gy, gy, gz * gz)) > lim2) continue;
+        atomicOr(nmask + ((size_t)(v[0] + 2u - dx) * E1 + (v[1] + 2u - dy)) * E2 +
+                     (v[2] + 2u - dz),
+                 1u << b);
     }
+}
+
+// Octant masks (m.msh = 3), gathered: one thread per cell of the grown box tests the voxels of
+// its 27 cells against its eight octants and writes the eight words. The boxes are small enough
+// (256 MiB of masks), a warp's cells share columns of the grid, and every word is written: no
+// atomics (about 70 words a voxel, bound by the L2's atomic rate) and no clear. Bound: the ALU
+// (70% busy) on half-empty warps; 56 -> 53 us on the 5M-point map, and the clear saved.
+__global__ void __launch_bounds__(128) k_grid_mask_oct(MapView m, uint4* __restrict__ nmask) {
+    const uint32_t E1 = m.ext[1] + 2u, E2 = m.ext[2] + 2u;
+    const size_t cells = (size_t)(m.ext[0] + 2u) * E1 * E2;
+    const size_t u = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (u >= cells) return;
+    // local cell + 1 of this cell
+    const uint32_t uz = (uint32_t)(u % E2), uy = (uint32_t)(u / E2 % E1),
+                   ux = (uint32_t)(u / E2 / E1);
+    uint32_t w[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+#pragma unroll
+    for (uint32_t dx = 0; dx < 3u; ++dx) {
+        const uint32_t x = ux + dx - 2u;
+        if (x >= m.ext[0]) continue;
+#pragma unroll
+        for (uint32_t dy = 0; dy < 3u; ++dy) {
+            const uint32_t y = uy + dy - 2u;
+            if (y >= m.ext[1]) continue;
+            const float4* const col = m.grid + ((size_t)x * m.ext[1] + y) * m.ext[2];
+            float4 e[3];
+#pragma unroll
+            for (uint32_t dz = 0; dz < 3u; ++dz) {
+                const uint32_t z = uz + dz - 2u;
+                e[dz] = z < m.ext[2] ? __ldg(col + z)
+                                     : make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
+            }
+#pragma unroll
+            for (uint32_t dz = 0; dz < 3u; ++dz) {
+                if (__float_as_int(e[dz].w) < 0) continue;
+                const int32_t c[3] = {(int32_t)x + m.min_cell[0], (int32_t)y + m.min_cell[1],
+                                      (int32_t)(uz + dz - 2u) + m.min_cell[2]};
+                const float lim2 = mask_limit2(c, m.res);
+                float gx[2], gy[2], gz[2];
+#pragma unroll
+                for (uint32_t h = 0; h < 2u; ++h) {
+                    gx[h] = mask_gap(e[dz].x, c[0], m.res, dx, h, false);
+                    gy[h] = mask_gap(e[dz].y, c[1], m.res, dy, h, false);
+                    gz[h] = mask_gap(e[dz].z, c[2], m.res, dz, h, false);
+                }
+                const uint32_t bit = 1u << (dx * 9u + dy * 3u + dz);
+#pragma unroll
+                for (uint32_t o = 0; o < 8u; ++o) {
+                    const float x0 = gx[(o >> 2) & 1u], y0 = gy[(o >> 1) & 1u], z0 = gz[o & 1u];
+                    if (!(fmaf(x0, x0, fmaf(y0, y0, z0 * z0)) > lim2)) w[o] |= bit;
+                }
+            }
+        }
+    }
+    nmask[2 * u] = make_uint4(w[0], w[1], w[2], w[3]);
+    nmask[2 * u + 1] = make_uint4(w[4], w[5], w[6], w[7]);
 }
 
 static uint32_t bit_width(uint32_t x) {
@@ -1574,18 +2031,18 @@ int build_segments(BuildScratch& sc, const float* d_pts, size_t n, const ndt_con
     if ((rc = dev_reserve(sc.keys_a, n * 8)) || (rc = dev_reserve(sc.vals_a, n * 4)) ||
         (rc = dev_reserve(sc.small, 256)) || (rc = dev_reserve(sc.seg_starts, n * 4 + 4)) ||
         (rc = dev_reserve(sc.seg_valid, n * 4 + 4)) || (rc = dev_reserve(sc.seg_rank, n * 4 + 4)) ||
-        (rc = dev_reserve(sc.seg_rec, n * sizeof(SegRec))))
+        (rc = dev_reserve(sc.seg_rec, n * sizeof(SegRec))) || (rc = pin_reserve(sc.host, 256)))
         return rc;
     size_t tmp = std::max(radix_sort_temp_bytes(n), detect_segments_temp_bytes(n));
-    tmp = std::max(tmp, scan_temp_bytes(n));
+    tmp = std::max(tmp, sort_bytes(n, SortPlan{1, 8}) + 2 * align_up(n * 4, 256));
     if ((rc = dev_reserve(sc.tmp, tmp))) return rc;
-    uint32_t* vals = (uint32_t*)sc.vals_a.p;
     int32_t* mm = (int32_t*)sc.small.p;
     uint32_t* nseg = (uint32_t*)((char*)sc.small.p + 64);
+    int32_t* hmm = (int32_t*)sc.host.p;
+    uint32_t* hseg = (uint32_t*)sc.host.p + 16;
 
     cell_bounds(d_pts, n, cfg.resolution, mm, s);
-    int32_t hmm[7];
-    cudaMemcpyAsync(hmm, mm, sizeof hmm, cudaMemcpyDeviceToHost, s);
+    cudaMemcpyAsync(hmm, mm, 28, cudaMemcpyDeviceToHost, s);
     if ((rc = cuda_fail(cudaStreamSynchronize(s), "map bounds"))) return rc;
     g.nf = (size_t)(uint32_t)hmm[6];
     if (g.nf == 0) {
@@ -1598,45 +2055,68 @@ int build_segments(BuildScratch& sc, const float* d_pts, size_t n, const ndt_con
     }
     uint32_t bits[3];
     if ((rc = box_bits(g.mn, g.mx, bits))) return rc;
-    const uint32_t lv = std::max(bits[0], std::max(bits[1], bits[2]));
-    const int end_bit = std::min(64, (int)(3 * lv + 1));
-    const unsigned gp = (unsigned)((n + BT - 1) / BT);
-    if (end_bit <= 32) {
-        // the keys fit 32 bits (the non-finite key, all ones, still sorts last)
-        uint32_t* keys = (uint32_t*)sc.keys_a.p;
-        k_morton<uint32_t><<<gp, BT, 0, s>>>(d_pts, n, cfg.resolution, mm, keys, vals);
-        if ((rc = radix_sort_pairs32(keys, vals, n, 0, end_bit, sc.tmp.p, sc.tmp.bytes, s)) ||
-            (rc = segment_starts(keys, g.nf, (uint32_t*)sc.seg_starts.p, nseg, sc.tmp.p, s)))
+    // workspace of the sorts in front of sc.tmp, their alternate values behind it
+    uint32_t* vals = (uint32_t*)sc.vals_a.p;  // ends with the point indices in key order
+    const CompactKey ck = compact_key(bits);
+    if (n < SP_MAX_PAIRS) {
+        const SortPlan o = sort_plan((int)ck.total + (g.nf < n ? 1 : 0));
+        uint32_t* k0 = (uint32_t*)sc.keys_a.p;
+        uint32_t* k1 = k0 + n;
+        uint32_t* v1 = (uint32_t*)((char*)sc.tmp.p + sort_bytes(n, o));
+        k_compact_keys<<<ntiles(n), BT, 0, s>>>(d_pts, (uint32_t)n, cfg.resolution,
+                                                exact_inverse(cfg.resolution),
+                                                ((uintptr_t)d_pts & 15u) == 0, mm, ck, o.width,
+                                                k0, (uint32_t*)sc.tmp.p);
+        uint32_t *ks, *vs;
+        // the last pass writes the values to vals_a: an even number of passes starts there
+        uint32_t *va = vals, *vb = v1;
+        if (o.passes & 1) std::swap(va, vb);
+        if ((rc = sort_positions(k0, va, k1, vb, n, o, true, sc.tmp.p, &ks, &vs, s)) ||
+            (rc = segment_starts(ks, g.nf, (uint32_t*)sc.seg_starts.p, nseg, sc.tmp.p, s)))
             return rc;
     } else {
+        const uint32_t lv = std::max(bits[0], std::max(bits[1], bits[2]));
         uint64_t* keys = (uint64_t*)sc.keys_a.p;
-        k_morton<uint64_t><<<gp, BT, 0, s>>>(d_pts, n, cfg.resolution, mm, keys, vals);
-        if ((rc = radix_sort_pairs(keys, vals, n, 0, end_bit, sc.tmp.p, sc.tmp.bytes, s)) ||
+        k_morton<uint64_t><<<(unsigned)((n + BT - 1) / BT), BT, 0, s>>>(d_pts, n, cfg.resolution,
+                                                                        mm, keys, vals);
+        if ((rc = radix_sort_pairs(keys, vals, n, 0, std::min(64, (int)(3 * lv + 1)), sc.tmp.p,
+                                   sc.tmp.bytes, s)) ||
             (rc = segment_starts(keys, g.nf, (uint32_t*)sc.seg_starts.p, nseg, sc.tmp.p, s)))
             return rc;
     }
-    cudaMemcpyAsync(&g.S, nseg, 4, cudaMemcpyDeviceToHost, s);
+    cudaMemcpyAsync(hseg, nseg, 4, cudaMemcpyDeviceToHost, s);
     if ((rc = cuda_fail(cudaStreamSynchronize(s), "segments"))) return rc;
+    g.S = hseg[0];
+    if (g.S == 0) {
+        set_error("map build: a look-back wait ran out");
+        return NDT_ERR_DEVICE;
+    }
     // visit order of the segments, largest first (the keys' buffer is free again: the
     // segments are recorded by their starts)
+    const SortPlan oz = {1, 8};
     uint32_t* skeys = (uint32_t*)sc.keys_a.p;
     uint32_t* order = (uint32_t*)sc.seg_rank.p;
+    const size_t oz_bytes = sort_bytes(g.S, oz);
+    uint32_t* sorted = skeys + g.S;
+    uint32_t *kz, *vz;
     k_seg_size_keys<<<(g.S + 255) / 256, 256, 0, s>>>((const uint32_t*)sc.seg_starts.p, g.S,
-                                                      (uint32_t)g.nf, skeys, order);
-    if ((rc = radix_sort_pairs32(skeys, order, g.S, 0, 16, sc.tmp.p, sc.tmp.bytes, s))) return rc;
-    // the large segments' sums into the sort's temporary storage (free again): at most
-    // nf / WARP_SEG_MIN segments of SegSums, well inside its 12 bytes per point
-    SegSums* sums = (SegSums*)sc.tmp.p;
+                                                      (uint32_t)g.nf, skeys);
+    if ((rc = sort_positions(skeys, nullptr, sorted, order, g.S, oz, false, sc.tmp.p, &kz, &vz,
+                             s)))
+        return rc;
+    // the large segments' sums behind the sort's workspace: at most nf / WARP_SEG_MIN segments
+    // of SegSums, well inside its 8 bytes per point
+    SegSums* sums = (SegSums*)((char*)sc.tmp.p + oz_bytes);
     const uint32_t wmax = (uint32_t)std::min<size_t>(g.S, g.nf / WARP_SEG_MIN + 1);
     const unsigned gs = (unsigned)std::min<uint32_t>((wmax + 3) / 4, 152u * 64u);
-    k_segment_sums<<<gs, 128, 0, s>>>(d_pts, vals, (uint32_t*)sc.seg_starts.p, order, skeys,
-                                      g.S, (uint32_t)g.nf, cfg.resolution,
-                                      cfg.min_points_per_voxel, sums);
+    k_segment_sums<<<gs, 128, 0, s>>>(d_pts, vals, (uint32_t*)sc.seg_starts.p, order, kz, g.S,
+                                      (uint32_t)g.nf, cfg.resolution, cfg.min_points_per_voxel,
+                                      sums);
     k_voxel_stats<<<(g.S + 127) / 128, 128, 0, s>>>(
-        d_pts, vals, (uint32_t*)sc.seg_starts.p, order, skeys, sums, g.S, (uint32_t)g.nf,
+        d_pts, vals, (uint32_t*)sc.seg_starts.p, order, kz, sums, g.S, (uint32_t)g.nf,
         cfg.resolution, cfg.min_points_per_voxel, cfg.eigenvalue_ratio, (SegRec*)sc.seg_rec.p,
         (uint32_t*)sc.seg_valid.p);
-    return cuda_fail(cudaStreamSynchronize(s), "voxel statistics");
+    return cuda_fail(cudaGetLastError(), "voxel statistics");
 }
 
 // Stages 6-7: valid voxels of the S records (in Morton order of their cells) compacted into
@@ -1652,7 +2132,8 @@ int finish_map(Map& map, BuildScratch& sc, const SegRec* rec, const uint32_t* va
     uint32_t bits[3];
     if ((rc = box_bits(g.mn, g.mx, bits))) return rc;
     if ((rc = exclusive_scan(valid, (uint32_t*)sc.seg_rank.p, S, sc.tmp.p, s))) return rc;
-    uint32_t hs[2];
+    if ((rc = pin_reserve(sc.host, 256))) return rc;
+    uint32_t* hs = (uint32_t*)sc.host.p + 24;
     cudaMemcpyAsync(&hs[0], (uint32_t*)sc.seg_rank.p + (S - 1), 4, cudaMemcpyDeviceToHost, s);
     cudaMemcpyAsync(&hs[1], valid + (S - 1), 4, cudaMemcpyDeviceToHost, s);
     if ((rc = cuda_fail(cudaStreamSynchronize(s), "voxel compaction"))) return rc;
@@ -1718,30 +2199,27 @@ int finish_map(Map& map, BuildScratch& sc, const SegRec* rec, const uint32_t* va
         v.grid = (const float4*)map.grid.p;
         v.nmask = (const uint32_t*)map.nmask.p;
         cudaMemsetAsync(map.grid.p, 0xFF, (size_t)cells * 16, s);
-        cudaMemsetAsync(map.nmask.p, 0, (size_t)mwords * 4, s);
+        if (!oct) cudaMemsetAsync(map.nmask.p, 0, (size_t)mwords * 4, s);
     } else {
         v.slots = (const uint4*)map.slots.p;
         v.slot_vidx = (const int32_t*)map.slot_vidx.p;
     }
-    k_voxel_compact<<<(S + 127) / 128, 128, 0, s>>>(
+    k_voxel_compact<<<(S + VC - 1) / VC, VC, 0, s>>>(
         rec, valid, (uint32_t*)sc.seg_rank.p, S, (int32_t*)map.vox_coord.p,
         (float4*)map.vox_mean.p, (float*)map.vox_cov.p, (float*)map.vox_icov.p,
         (uint32_t*)map.vox_count.p, v, (float4*)map.icov8.p, dense ? (float4*)map.grid.p : nullptr,
         (uint32_t*)map.slots.p, (uint4*)map.slots.p, (int32_t*)map.slot_vidx.p, mprobe, d_status);
-    if (dense) {
-        const unsigned gv = (V + 127) / 128;
-        if (oct)
-            k_grid_mask<true><<<gv, 128, 0, s>>>(v, (const int32_t*)map.vox_coord.p,
-                                                 (const float4*)map.vox_mean.p,
-                                                 (uint32_t*)map.nmask.p);
-        else
-            k_grid_mask<false><<<gv, 128, 0, s>>>(v, (const int32_t*)map.vox_coord.p,
-                                                  (const float4*)map.vox_mean.p,
-                                                  (uint32_t*)map.nmask.p);
-    }
-    uint32_t hprobe = 0;
-    cudaMemcpyAsync(&hprobe, mprobe, 4, cudaMemcpyDeviceToHost, s);
+    if (oct)
+        k_grid_mask_oct<<<(unsigned)((mcells + 127) / 128), 128, 0, s>>>(v, (uint4*)map.nmask.p);
+    else if (dense)
+        k_grid_mask<<<(V + 127) / 128, 128, 0, s>>>(v, (const int32_t*)map.vox_coord.p,
+                                                    (const float4*)map.vox_mean.p,
+                                                    (uint32_t*)map.nmask.p);
+    cudaMemcpyAsync(&hs[2], mprobe, 4, cudaMemcpyDeviceToHost, s);
+    cudaMemcpyAsync(&hs[3], d_status, 4, cudaMemcpyDeviceToHost, s);
     if ((rc = cuda_fail(cudaStreamSynchronize(s), "hash insert"))) return rc;
+    const uint32_t hprobe = hs[2];
+    map.status = hs[3];
     v.max_probe = hprobe;
     map.view = v;
     ndt_map_info& info = map.info;
@@ -1766,26 +2244,20 @@ int finish_map(Map& map, BuildScratch& sc, const SegRec* rec, const uint32_t* va
 // ---------------------------------------------------------------------------------------
 // Map tiles: segments built once per tile, merged per commit.
 // ---------------------------------------------------------------------------------------
-// Keys of every tile's segments for the merged map: Morton code of the cell relative to the
-// merged box's minimum cell (the key set_target of the concatenated points would give each of
-// its points), value = the segment's index in tile order.
-__global__ void k_merge_keys(const TileSegRef* __restrict__ tiles, int nt, uint64_t total,
-                             int32_t mn0, int32_t mn1, int32_t mn2, uint64_t* __restrict__ keys,
-                             uint32_t* __restrict__ vals) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// Keys of every tile's segments for the merged map: compact Morton key of the cell in the
+// merged box (the key set_target of the concatenated points would give each of its points);
+// the values of the sort are the segments' indices in tile order.
+__global__ void k_merge_keys(const TileSegRef* __restrict__ tiles, int nt, uint32_t total,
+                             int32_t mn0, int32_t mn1, int32_t mn2, CompactKey ck,
+                             uint32_t* __restrict__ keys) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
     int t = 0;
     while (t + 1 < nt && i >= tiles[t + 1].seg_off) ++t;
     const int32_t* c = tiles[t].rec[i - tiles[t].seg_off].coord;
-    const int32_t mn[3] = {mn0, mn1, mn2};
-    uint32_t q[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        const int64_t d = (int64_t)c[a] - (int64_t)mn[a];
-        q[a] = d > 0x1FFFFF ? 0x1FFFFFu : (uint32_t)d;
-    }
-    keys[i] = morton3(q[0], q[1], q[2]);
-    vals[i] = (uint32_t)i;
+    const uint32_t q[3] = {(uint32_t)c[0] - (uint32_t)mn0, (uint32_t)c[1] - (uint32_t)mn1,
+                           (uint32_t)c[2] - (uint32_t)mn2};
+    keys[i] = compact_morton(ck, q);
 }
 
 // One thread per cell of the merged map (a group of equal keys: the segments of that cell in
@@ -1858,7 +2330,7 @@ int merge_tiles(Map& map, BuildScratch& sc, const std::vector<TileSegRef>& refs,
         set_error("Target point cloud is empty");
         return NDT_ERR_EMPTY_INPUT;
     }
-    if (total >= 0xFFFFFFF0ull) {
+    if (total >= SP_MAX_PAIRS) {
         set_error("too many occupied cells in the tiles");
         return NDT_ERR_CAPACITY;
     }
@@ -1873,34 +2345,42 @@ int merge_tiles(Map& map, BuildScratch& sc, const std::vector<TileSegRef>& refs,
     for (const auto& t : refs)
         if (t.S) used.push_back(t);
     const int nt = (int)used.size();
-    size_t tmp = std::max(radix_sort_temp_bytes(total), detect_segments_temp_bytes(total));
+    const CompactKey ck = compact_key(bits);
+    const SortPlan o = sort_plan((int)ck.total);
+    const size_t ob = sort_bytes(total, o);
     if ((rc = dev_reserve(d_refs, used.size() * sizeof(TileSegRef))) ||
         (rc = dev_reserve(sc.keys_a, total * 8)) || (rc = dev_reserve(sc.vals_a, total * 4)) ||
         (rc = dev_reserve(sc.small, 256)) || (rc = dev_reserve(sc.seg_starts, total * 4 + 4)) ||
         (rc = dev_reserve(sc.seg_valid, total * 4 + 4)) ||
         (rc = dev_reserve(sc.seg_rec, total * sizeof(SegRec))) ||
-        (rc = dev_reserve(sc.tmp, std::max(tmp, scan_temp_bytes(total)))))
+        (rc = pin_reserve(sc.host, 256)) ||
+        (rc = dev_reserve(sc.tmp, std::max(ob + align_up(total * 4, 256), scan_temp_bytes(total)))))
         return rc;
     cudaMemcpyAsync(d_refs.p, used.data(), used.size() * sizeof(TileSegRef),
                     cudaMemcpyHostToDevice, s);
-    uint64_t* keys = (uint64_t*)sc.keys_a.p;
-    uint32_t* vals = (uint32_t*)sc.vals_a.p;
+    uint32_t* keys = (uint32_t*)sc.keys_a.p;
     uint32_t* ngroups = (uint32_t*)((char*)sc.small.p + 64);
     const TileSegRef* dref = (const TileSegRef*)d_refs.p;
-    k_merge_keys<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(dref, nt, total, g.mn[0],
-                                                                 g.mn[1], g.mn[2], keys, vals);
-    const uint32_t lv = std::max(bits[0], std::max(bits[1], bits[2]));
-    const int end_bit = std::min(64, (int)(3 * lv + 1));
-    if ((rc = radix_sort_pairs(keys, vals, total, 0, end_bit, sc.tmp.p, sc.tmp.bytes, s)) ||
-        (rc = detect_segments(keys, total, nullptr, (uint32_t*)sc.seg_starts.p, ngroups,
-                              sc.tmp.p, sc.tmp.bytes, s)))
+    k_merge_keys<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(
+        dref, nt, (uint32_t)total, g.mn[0], g.mn[1], g.mn[2], ck, keys);
+    uint32_t *ks, *vals;
+    if ((rc = sort_positions(keys, (uint32_t*)sc.vals_a.p, keys + total,
+                             (uint32_t*)((char*)sc.tmp.p + ob), total, o, false, sc.tmp.p, &ks,
+                             &vals, s)) ||
+        (rc = segment_starts(ks, total, (uint32_t*)sc.seg_starts.p, ngroups, sc.tmp.p, s)))
         return rc;
     k_merge_groups<<<(unsigned)((total + 127) / 128), 128, 0, s>>>(
         dref, nt, vals, (const uint32_t*)sc.seg_starts.p, ngroups, (uint32_t)total,
         cfg.min_points_per_voxel, cfg.eigenvalue_ratio, cfg.resolution, (SegRec*)sc.seg_rec.p,
         (uint32_t*)sc.seg_valid.p);
-    cudaMemcpyAsync(&g.S, ngroups, 4, cudaMemcpyDeviceToHost, s);
+    uint32_t* hseg = (uint32_t*)sc.host.p + 16;
+    cudaMemcpyAsync(hseg, ngroups, 4, cudaMemcpyDeviceToHost, s);
     if ((rc = cuda_fail(cudaStreamSynchronize(s), "tile merge"))) return rc;
+    g.S = hseg[0];
+    if (g.S == 0) {
+        set_error("map merge: a look-back wait ran out");
+        return NDT_ERR_DEVICE;
+    }
     rc = finish_map(map, sc, (const SegRec*)sc.seg_rec.p, (const uint32_t*)sc.seg_valid.p, g.S,
                     g, cfg, d_status, s);
     cudaEventRecord(e1, s);
