@@ -20,15 +20,17 @@
 //      src/ndt_cuda/src/optimization/newton.rs:160-176 for the CPU semantics, with an FP64
 //      Cholesky fast path when H is definite and well conditioned), applies the reference's
 //      step control and convergence test, and broadcasts the next pose through DSMEM.
-// k_ndt_align uses only hardware cluster barriers: no global-memory spin waits. The
-// work-queue variant k_ndt_queue (below) splits iterations into chunks claimed by a
-// persistent grid; its only waits are bounded polls for work.
+// k_ndt_align uses only hardware cluster barriers: no global-memory spin waits. Two more kernels
+// run the same partition of the points (below): k_ndt_queue splits iterations into chunks claimed
+// by a persistent grid, for large batches; k_ndt_few spreads a few alignments over all SMs. Their
+// waits on global memory are bounded.
 #include <cooperative_groups.h>
 
 #include <algorithm>
 #include <cstdio>
 #include <map>
 #include <mutex>
+#include <queue>
 
 #include "ndt_internal.h"
 
@@ -138,16 +140,20 @@ __device__ const uint32_t FRAME_TERMS[90] = {
 // A_k, B_kl in FP64 for assembling g and H at this pose. `small` applies the CPU path's
 // |angle| < 1e-5 rule (sin = 0, cos = 1) to A_k and B_kl (angular.rs), not to R. With Bd
 // null the B_kl entries are skipped (a line-search candidate needs the gradient only).
-__device__ __noinline__ void make_frame_warp(const double* pose, bool small, float* fr,
-                                             double* trig, double* Ad, double* Bd, int lane) {
+// One table entry at the trigonometric values f = trig + (0 for R, 8 for its derivatives)
+__device__ __forceinline__ double frame_term(uint32_t w, const double* f) {
+    const double t0 = f[w & 7u] * f[(w >> 3) & 7u] * f[(w >> 6) & 7u];
+    const double t1 = f[(w >> 9) & 7u] * f[(w >> 12) & 7u] * f[(w >> 15) & 7u];
+    const uint32_t c0 = (w >> 18) & 3u, c1 = (w >> 20) & 3u;
+    return (c0 == 0u ? 0.0 : (c0 == 1u ? t0 : -t0)) + (c1 == 0u ? 0.0 : (c1 == 1u ? t1 : -t1));
+}
+
+// What the point work reads (fr) and A_k; trig is left for frame_second
+__device__ __forceinline__ void frame_first(const double* pose, bool small, float* fr,
+                                            double* trig, double* Ad, int lane) {
     // each lane's term words first: their loads overlap the sines and cosines
-    const int nterms = Bd ? 90 : 36;
-    uint32_t words[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const int e = lane + 32 * k;
-        words[k] = e < nterms ? __ldg(FRAME_TERMS + e) : 0u;
-    }
+    const uint32_t w0 = __ldg(FRAME_TERMS + lane);
+    const uint32_t w1 = lane < 4 ? __ldg(FRAME_TERMS + 32 + lane) : 0u;
     if (lane < 3) {
         double s, c;
         sincos(pose[3 + lane], &s, &c);
@@ -167,30 +173,37 @@ __device__ __noinline__ void make_frame_warp(const double* pose, bool small, flo
     }
     if (lane < 9) fr[24 + 4 * lane + 3] = 0.f;  // padding
     __syncwarp();
-    // a lane's (up to) three terms are independent: unrolled, their FP64 chains overlap
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const int e = lane + 32 * k;
-        if (e >= nterms) break;
-        const uint32_t w = words[k];
-        const double* f = e < 9 ? trig : trig + 8;
-        const double t0 = f[w & 7u] * f[(w >> 3) & 7u] * f[(w >> 6) & 7u];
-        const double t1 = f[(w >> 9) & 7u] * f[(w >> 12) & 7u] * f[(w >> 15) & 7u];
-        const uint32_t c0 = (w >> 18) & 3u, c1 = (w >> 20) & 3u;
-        const double v = (c0 == 0u ? 0.0 : (c0 == 1u ? t0 : -t0)) +
-                         (c1 == 0u ? 0.0 : (c1 == 1u ? t1 : -t1));
-        if (e < 9) {
-            const float h = (float)v;
-            fr[4 * (e / 3) + e % 3] = h;
-            fr[12 + 4 * (e / 3) + e % 3] = (float)(v - (double)h);
-        } else if (e < 36) {
-            fr[24 + 4 * ((e - 9) / 3) + e % 3] = (float)v;
-            Ad[e - 9] = v;
-        } else {
-            Bd[e - 36] = v;
-        }
+    const double v0 = frame_term(w0, lane < 9 ? trig : trig + 8);
+    const double v1 = lane < 4 ? frame_term(w1, trig + 8) : 0.0;
+    if (lane < 9) {
+        const float h = (float)v0;
+        fr[4 * (lane / 3) + lane % 3] = h;
+        fr[12 + 4 * (lane / 3) + lane % 3] = (float)(v0 - (double)h);
+    } else {
+        fr[24 + 4 * ((lane - 9) / 3) + lane % 3] = (float)v0;
+        Ad[lane - 9] = v0;
+    }
+    if (lane < 4) {
+        const int e = 32 + lane;
+        fr[24 + 4 * ((e - 9) / 3) + e % 3] = (float)v1;
+        Ad[e - 9] = v1;
     }
     __syncwarp();
+}
+
+// B_kl at the pose of the frame_first before it
+__device__ __forceinline__ void frame_second(const double* trig, double* Bd, int lane) {
+    const uint32_t w0 = __ldg(FRAME_TERMS + 36 + lane);
+    const uint32_t w1 = lane < 22 ? __ldg(FRAME_TERMS + 68 + lane) : 0u;
+    Bd[lane] = frame_term(w0, trig + 8);
+    if (lane < 22) Bd[32 + lane] = frame_term(w1, trig + 8);
+    __syncwarp();
+}
+
+__device__ __noinline__ void make_frame_warp(const double* pose, bool small, float* fr,
+                                             double* trig, double* Ad, double* Bd, int lane) {
+    frame_first(pose, small, fr, trig, Ad, lane);
+    if (Bd) frame_second(trig, Bd, lane);
 }
 
 // ------------------------------------------------------------------------------------
@@ -330,7 +343,7 @@ __device__ __noinline__ int jacobi6_warp(T* A, T* V, T* cs, int lane, bool init_
     return sweeps;
 }
 
-// f32 Cholesky of s*H (s = +1 or -1; H symmetric FP64) by one lane. Every index is a
+// f32 Cholesky of s*H (s = +1 or -1; H symmetric, rounded to f32) by a lane. Every index is a
 // compile-time constant, so the factor stays in registers: L lower triangular, packed by
 // rows, and rinv[j] = 1 / L_jj. False if a pivot is not positive or the pivot ratio falls
 // below 1e-6 (the caller then takes the eigen path).
@@ -341,11 +354,11 @@ struct Chol32 {
 
 __device__ __forceinline__ constexpr int tri(int i, int j) { return i * (i + 1) / 2 + j; }
 
-__device__ __forceinline__ bool chol6f(const double* H, float sgn, Chol32& C) {
+__device__ __forceinline__ bool chol6f(const float* H, float sgn, Chol32& C) {
     float dmin = 3.0e38f, dmax = 0.f;
 #pragma unroll
     for (int j = 0; j < 6; ++j) {
-        float s = sgn * (float)H[j * 6 + j];
+        float s = sgn * H[j * 6 + j];
 #pragma unroll
         for (int k = 0; k < j; ++k) s = fmaf(-C.L[tri(j, k)], C.L[tri(j, k)], s);
         if (!(s > 0.f)) return false;
@@ -356,7 +369,7 @@ __device__ __forceinline__ bool chol6f(const double* H, float sgn, Chol32& C) {
         C.L[tri(j, j)] = s * r;
 #pragma unroll
         for (int i = j + 1; i < 6; ++i) {
-            float t = sgn * (float)H[i * 6 + j];
+            float t = sgn * H[i * 6 + j];
 #pragma unroll
             for (int k = 0; k < j; ++k) t = fmaf(-C.L[tri(i, k)], C.L[tri(j, k)], t);
             C.L[tri(i, j)] = t * r;
@@ -420,62 +433,81 @@ template <bool CPU_SEM>
 __device__ __noinline__ void solve_warp(const double* H, const double* g, SolveScratch& S,
                                         int lane) {
     // Definite fast path: f32 Cholesky factor of (s H), then mixed-precision iterative
-    // refinement — the residual r = b - (s H) x in FP64 (lane i owns row i), the correction
-    // solved with the f32 factor — until the last correction is below 1e-13 of x (four f32
-    // solves reach FP64 accuracy while cond(H) stays below about 1e4; worse-conditioned
-    // definite Hessians take the eigen path).
+    // refinement of H x = s b: the residual s b - H x in FP64 (lanes i and 8 + i hold half of
+    // row i each), the correction solved with the f32 factor by every lane alike. A correction
+    // of relative size d after one of size p leaves an error of about d^2 / p: it stops once
+    // that is below 1e-16 (two or three residuals reach FP64 accuracy while cond(H) stays below
+    // about 1e4; worse-conditioned definite Hessians take the eigen path).
     Chol32 C;
     int sgn = 0;
+    const int row = lane & 7, half = lane >> 3;  // lanes 0-5 and 8-13 own half rows
+    const bool own = row < 6 && half < 2;
+    double h[3] = {0.0, 0.0, 0.0};
+    if (own) {
+#pragma unroll
+        for (int j = 0; j < 3; ++j) h[j] = H[row * 6 + 3 * half + j];
+    }
+    S.A32[lane] = (float)H[lane];
+    if (lane < 4) S.A32[32 + lane] = (float)H[32 + lane];
     if (lane == 0) {
         S.ok = 0;
         S.path = 1;
         S.sweeps = 0;
-        for (int s = -1; s <= 1; s += 2) {
-            if (CPU_SEM && s == 1) continue;  // only the negative-definite fast path
-            if (chol6f(H, (float)s, C)) {
-                sgn = s;
-                break;
-            }
-        }
     }
-    sgn = __shfl_sync(0xffffffffu, sgn, 0);
+    __syncwarp();
+    for (int s = -1; s <= 1 && sgn == 0; s += 2) {
+        if (CPU_SEM && s == 1) continue;  // only the negative-definite fast path
+        if (chol6f(S.A32, (float)s, C)) sgn = s;  // every lane alike
+    }
     if (sgn != 0) {
-        const double b = lane < 6 ? (CPU_SEM ? g[lane] : -g[lane]) : 0.0;
-        double x = 0.0, r = b;
+        // (s H) x = b with b = -g (graph) or g (CPU): H x = s b
+        double b = 0.0;
+        if (lane < 6) b = CPU_SEM ? g[lane] : -g[lane];
+        const double sb = sgn > 0 ? b : -b;
+        double x = 0.0, r = sb;
+        float prev = 0.f;
         bool conv = false;
         for (int ref = 0; ref < 4; ++ref) {
-            if (lane < 6) S.cs[lane] = r;
-            __syncwarp();
-            if (lane == 0) {
-                float rf[6], dx[6];
+            const float rf = (float)(sgn > 0 ? r : -r);  // the factor is of s H
+            float rr[6], dx[6];
 #pragma unroll
-                for (int i = 0; i < 6; ++i) rf[i] = (float)S.cs[i];
-                chol6f_solve(C, rf, dx);
+            for (int i = 0; i < 6; ++i) rr[i] = __shfl_sync(0xffffffffu, rf, i);
+            chol6f_solve(C, rr, dx);
+            float ax = 0.f, ad = 0.f, mine = 0.f;
 #pragma unroll
-                for (int i = 0; i < 6; ++i) S.T[i] = (double)dx[i];
+            for (int i = 0; i < 6; ++i) {
+                ad = fmaxf(ad, fabsf(dx[i]));
+                if (i == lane) mine = dx[i];
             }
-            __syncwarp();
-            float adx = 0.f, ax = 0.f;
-            if (lane < 6) {
-                const double d = S.T[lane];
-                x += d;
-                S.x[lane] = x;
-                adx = fabsf((float)d);
-                ax = fabsf((float)x);
+            if (ref == 0) {
+                x = (double)mine;
+            } else {
+                x += (double)mine;
             }
+            ax = lane < 6 ? fabsf((float)x) : 0.f;
 #pragma unroll
             for (int o = 4; o > 0; o >>= 1) ax = fmaxf(ax, __shfl_xor_sync(0xffffffffu, ax, o));
             ax = __shfl_sync(0xffffffffu, ax, 0);
-            conv = __all_sync(0xffffffffu, adx <= 1e-13f * ax);
-            if (conv) break;
+            // |correction|^2 / |last correction| against 1e-16 |x| (b = 0: x = 0 exactly)
+            conv = ax == 0.f || (ref > 0 && prev > 0.f && ad / prev < 1e-3f &&
+                                 (ad / ax) * (ad / prev) <= 1e-16f) ||
+                   (ref > 0 && ad == 0.f);
+            if (conv || ref == 3) break;
+            prev = ad;
+            if (lane < 6) S.x[lane] = x;
             __syncwarp();
-            if (lane < 6) {
-                double t = b;
-                for (int j = 0; j < 6; ++j) t = fma(-(double)sgn * H[lane * 6 + j], S.x[j], t);
-                r = t;
+            double t = 0.0;
+            if (own) {
+                t = half == 0 ? sb : 0.0;
+#pragma unroll
+                for (int j = 0; j < 3; ++j) t = fma(-h[j], S.x[3 * half + j], t);
             }
+            t += __shfl_xor_sync(0xffffffffu, t, 8);
+            r = t;  // lanes 0-5
+            __syncwarp();
         }
         if (conv) {
+            if (lane < 6) S.x[lane] = x;
             if (lane == 0) {
                 S.ok = 1;
                 S.path = 0;
@@ -631,6 +663,7 @@ __device__ __forceinline__ void transform_point(const float* fr, const float* pv
 // max_nb) are listed in shared memory (nbl[k * nbl_stride]), so the search runs with all
 // lanes busy and the pair work runs once per listed voxel rather than once per cell.
 // Returns the number listed. off27: the CTA's table of neighbour offsets (nbhd_offsets).
+template <int NB_BATCH = 4>
 __device__ __forceinline__ int search_point(const MapView& m, const uint32_t* off27,
                                             const float* qh, const float* ql, int max_nb,
                                             uint32_t* nbl, int nbl_stride) {
@@ -642,7 +675,6 @@ __device__ __forceinline__ int search_point(const MapView& m, const uint32_t* of
         // occupied cells among the 27 that it can accept, in search order; their
         // {centroid, slot} entries are loaded NB_BATCH at a time (independent loads in flight
         // together), then tested in order
-        constexpr int NB_BATCH = 4;
         uint32_t corner;
         uint32_t bits = nbhd_mask(m, gc, oct, corner);
 #pragma unroll 1
@@ -721,7 +753,7 @@ struct PointSums {
     float S, G0, G1, G2, M0, M1, M2, M3, M4, M5;
 };
 
-template <bool CPU_SEM>
+template <bool CPU_SEM, int AHEAD = 1>
 __device__ __forceinline__ void pair_terms(const MapView& m, const float* qh, const float* ql,
                                            int cnt, float d1f, float d2f, const uint32_t* list,
                                            int stride, PointSums& p);
@@ -811,14 +843,14 @@ __device__ __forceinline__ int search_group(const MapView& m, const uint32_t* of
 // k2 = -d2 log2(e) / 2 carried as two floats (the constant -log2(e) / 2 split into two floats,
 // then an exact product split: k2h + k2l), so the argument is as accurate as the product d2 sq
 // itself: two operations and the base-2 exponential per pair.
-template <bool CPU_SEM>
+template <bool CPU_SEM, int AHEAD>
 __device__ __forceinline__ void pair_terms(const MapView& m, const float* qh, const float* ql,
                                            int cnt, float d1f, float d2f, const uint32_t* list,
                                            int stride, PointSums& p) {
     const float d1d2 = d1f * d2f;
     const float k2h = d2f * -0.72134751081466674805f;
     const float k2l = fmaf(d2f, -0.72134751081466674805f, -k2h) + d2f * -9.6298151675000554e-09f;
-#pragma unroll 1
+#pragma unroll AHEAD  // voxels whose loads are in flight together
     for (int j = 0; j < cnt; ++j) {
         float x[3], C[6];
         load_voxel(m, list[j * stride], qh, ql, x, C);
@@ -940,42 +972,41 @@ __device__ __forceinline__ void point_terms_ls(const MapView& m, const uint32_t*
 }
 
 // g (6) and H (6x6) in FP64 from the reduced accumulators; lanes of one warp share the work.
-// Ad / Bd: A_k and B_kl at the pose the accumulators were taken at (make_frame_warp).
-__device__ __noinline__ void finalize_gH(const double* tot, const double* Ad, const double* Bd,
-                                         double* g, double* H, int lane) {
-    const double(*A)[9] = reinterpret_cast<const double(*)[9]>(Ad);
-    const double(*B)[9] = reinterpret_cast<const double(*)[9]>(Bd);
+// Ad / Bd: A_k and B_kl at the pose the accumulators were taken at (make_frame_warp). Nine
+// entries are 9-term dot products with G p^T (g's rotation part with A_k, H's rotation block
+// with B_kl): three lanes each take three terms of one (dependent FP64 instructions cost 60 to
+// 130 cycles, so a chain of nine would be most of this step).
+__device__ __forceinline__ void finalize_gH(const double* tot, const double* Ad,
+                                            const double* Bd, double* g, double* H, int lane) {
     const double* GP = tot + A_GP;
-    if (lane < 6) {
-        double v;
-        if (lane < 3) {
-            v = tot[A_G + lane];
-        } else {
-            v = 0.0;
-            for (int q = 0; q < 9; ++q) v += A[lane - 3][q] * GP[q];
-        }
-        g[lane] = v;
+    double v = 0.0;
+    const int e = lane / 3, s = lane % 3;  // entry (0-2: A_k, 3-8: B_kl), third of its terms
+    if (lane < 27) {
+        const double* m = (e < 3 ? Ad + 9 * e : Bd + 9 * (e - 3)) + 3 * s;
+        const double* q = GP + 3 * s;
+        v = fma(m[2], q[2], fma(m[1], q[1], m[0] * q[0]));
     }
-    if (lane < 21) {
-        int i = 0, j = lane;
-        while (j >= 6 - i) {
-            j -= 6 - i;
-            ++i;
-        }
-        j += i;
-        double v;
-        if (j < 3) {
-            v = tot[A_M + sym3(i, j)];
-        } else if (i < 3) {
-            v = tot[A_HTR + 3 * i + (j - 3)];
+    const double v1 = __shfl_down_sync(0xffffffffu, v, 1);
+    const double v2 = __shfl_down_sync(0xffffffffu, v, 2);
+    if (lane < 27 && s == 0) {
+        const double d = v + v1 + v2;
+        if (e < 3) {
+            g[3 + e] = d;
         } else {
-            int k = i - 3, l = j - 3;
-            int kl = (k == 0) ? l : (k == 1 ? 2 + l : 5);  // rr rp ry pp py yy
-            v = tot[A_HRR + kl];
-            for (int q = 0; q < 9; ++q) v += B[kl][q] * GP[q];
+            const int kl = e - 3;  // rr rp ry pp py yy
+            const int k = kl < 3 ? 0 : (kl < 5 ? 1 : 2), l = kl < 3 ? kl : (kl < 5 ? kl - 2 : 2);
+            const double w = tot[A_HRR + kl] + d;
+            H[(3 + k) * 6 + 3 + l] = w;
+            H[(3 + l) * 6 + 3 + k] = w;
         }
-        H[i * 6 + j] = v;
-        H[j * 6 + i] = v;
+    }
+    // the entries that are sums themselves: g's translation part, H's first three rows
+    if (lane < 3) g[lane] = tot[A_G + lane];
+    if (lane < 18) {
+        const int i = lane / 6, j = lane % 6;
+        const double w = j < 3 ? tot[A_M + sym3(i, j)] : tot[A_HTR + 3 * i + (j - 3)];
+        H[i * 6 + j] = w;
+        if (j >= 3) H[j * 6 + i] = w;
     }
 }
 
@@ -1930,15 +1961,26 @@ __device__ __forceinline__ void osc_update_warp(CtlShared& sh, int it, int lane)
     __syncwarp();
 }
 
+// The end of the graph path (converged, or out of iterations): the outputs. Returns 1 (every
+// lane) when the alignment is finished.
+__device__ __forceinline__ int graph_finish(const AlignParams& P, CtlShared& sh, AlignOut& o,
+                                            int it, double score, int ncorr, bool conv, int lane) {
+    if (!conv && it + 1 < P.max_iter) return 0;
+    if (lane == 0) {
+        const int status = ncorr == 0 ? NDT_STATUS_NO_CORRESPONDENCES
+                                      : (conv ? NDT_STATUS_CONVERGED : NDT_STATUS_MAX_ITERATIONS);
+        write_out(o, sh.pose, score, sh.H, it + 1, conv && ncorr > 0, ncorr, sh.max_osc, status);
+    }
+    return 1;
+}
+
 // The graph path's step (K5, ndt_graph_kernels.cu:618-847) by the warp: delta = the solve's
 // x (or -1e-4 g when it failed), reversed when g . delta <= 0; step = min(|delta|, step_size);
 // the pose moves by delta scaled to that step; converged when step < eps. The length is
 // compared on its square, and the clamp's scale step_size / |delta| comes from an f32
 // reciprocal square root refined by one FP64 Newton step (relative error below 1e-14), so the
 // FP64 chain has no square root or division.
-__device__ __noinline__ int control_step_graph_warp(const AlignParams& P, CtlShared& sh,
-                                                    AlignOut& o, int it, double score,
-                                                    int ncorr, int lane) {
+__device__ __forceinline__ bool graph_step_warp(const AlignParams& P, CtlShared& sh, int lane) {
     double xi = 0.0, gi = 0.0;
     if (lane < 6) {
         gi = sh.g[lane];
@@ -1966,15 +2008,17 @@ __device__ __noinline__ int control_step_graph_warp(const AlignParams& P, CtlSha
     }
     if (lane < 6) sh.pose[lane] += scale * xi;
     __syncwarp();
+    return conv != 0;
+}
+
+// The step, the oscillation history and, at the end, the outputs. Returns 1 (every lane) when
+// the alignment is finished.
+__device__ __noinline__ int control_step_graph_warp(const AlignParams& P, CtlShared& sh,
+                                                    AlignOut& o, int it, double score,
+                                                    int ncorr, int lane) {
+    const bool conv = graph_step_warp(P, sh, lane);
     osc_update_warp(sh, it, lane);
-    int done = 0;
-    if (lane == 0 && (conv || it + 1 >= P.max_iter)) {
-        const int status = ncorr == 0 ? NDT_STATUS_NO_CORRESPONDENCES
-                                      : (conv ? NDT_STATUS_CONVERGED : NDT_STATUS_MAX_ITERATIONS);
-        write_out(o, sh.pose, score, sh.H, it + 1, conv && ncorr > 0, ncorr, sh.max_osc, status);
-        done = 1;
-    }
-    return __shfl_sync(0xffffffffu, done, 0);
+    return graph_finish(P, sh, o, it, score, ncorr, conv, lane);
 }
 
 // Element e of QCtl's FP64 block, in the controller's shared state
@@ -2632,6 +2676,412 @@ static int launch_queue_t(const AlignParams& p, uint64_t units, cudaStream_t s, 
     return cuda_fail(e, "work-queue align launch");
 }
 
+// ------------------------------------------------------------------------------------
+// Few alignments, spread over the whole GPU
+//
+// A live tracker aligns one scan at a time. On clusters that scan had 2 to 8 SMs and every
+// thread worked through its three to five points one after another (a point's chain of dependent
+// loads takes about 5 us), and the FP64 step ran between two barriers. Here the SMs are shared
+// among the alignments by their work (few_share), a CTA of FT threads each, and a warp takes one
+// point per lane: an item (o, k) is the k-th points of the 32 lanes of warp o of the partition
+// (the cluster shape's, as in queue_part). Items leave each point's sums S, G, M in shared
+// memory; then one warp per o contracts them into its lanes' accumulators in the order k = 0, 1,
+// ..., so the f32 sums are the cluster kernel's bit for bit. Per iteration a CTA adds its warps'
+// sums in FP64 and writes them to global memory; the alignment's first CTA reads all CTAs' sums
+// as they arrive, adds them, runs the Newton step (one warp) and publishes the next frame, which
+// the others poll for. The launch is cooperative, so all CTAs are resident together; every wait
+// is bounded (P.stall_ns).
+// Kernel time, clusters and now: a 20k-point scan over 7 iterations 297 and 127 us, a 1,500-point
+// scan over 10 301 and 154 us, eight 20k-point scans over 5 310 and 272 us, a 400k-point scan over
+// 5 1563 and 368 us. Latency bounds it: an iteration of one small scan is about 12k cycles of
+// points (one per lane), 2k of exchange and 14k of Newton step (FP64 and dependent).
+// ------------------------------------------------------------------------------------
+constexpr int FT = 512, FNW = FT / 32;
+constexpr int FITEMS = 20;        // items in shared memory at a time
+constexpr int FOWN = FNW - 1;     // partition warps a CTA works on at a time
+constexpr int FVAL = 14;          // S, G (3), M (6), the point (3), its voxel count
+constexpr int FSEG = 8;           // segments of the sum over CTAs
+
+struct FewShared {
+    CtlShared ctl;                // the alignment's controller state (its first CTA)
+    __align__(16) float fr[NFR];
+    uint32_t off27[32];
+    double wpart[FNW][NRED];      // the warps' sums
+    double seg[FSEG][NRED];
+    int stop;                     // finished, or a wait ran out
+    int failed;
+    unsigned long long cyc[4];
+};
+
+// A word of the exchange: a 32-bit value and the iteration it belongs to (from 1), read and
+// written whole (64 bits), so a reader that finds the iteration has the value: no fence and no
+// second read behind a flag (each about 700 cycles of L2 latency).
+__device__ __forceinline__ unsigned long long few_word(uint32_t it, uint32_t v) {
+    return (unsigned long long)it << 32 | v;
+}
+__device__ __forceinline__ void few_put2(ulonglong2* p, unsigned long long a,
+                                         unsigned long long b) {
+    asm volatile("st.volatile.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(a), "l"(b) : "memory");
+}
+__device__ __forceinline__ ulonglong2 few_get2(const ulonglong2* p) {
+    ulonglong2 v;
+    asm volatile("ld.volatile.global.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p)
+                 : "memory");
+    return v;
+}
+__device__ __forceinline__ bool few_there(const ulonglong2& v, uint32_t it) {
+    return (uint32_t)(v.x >> 32) == it && (uint32_t)(v.y >> 32) == it;
+}
+// Waits for both words at p to reach iteration `it`, v as already read; false when the limit
+// runs out.
+__device__ __forceinline__ bool few_wait2(const ulonglong2* p, uint32_t it, ulonglong2& v,
+                                          unsigned long long limit_ns) {
+    if (few_there(v, it)) return true;
+    const unsigned long long t0 = global_ns();
+    do {
+        v = few_get2(p);
+        if (few_there(v, it)) return true;
+    } while (global_ns() - t0 < limit_ns);
+    return false;
+}
+
+// The frame of iteration `it` (or, with the last word set, the end) to the alignment's CTAs:
+// lane l writes words 2 l and 2 l + 1 of 64 (60 frame values, the end mark, unused)
+__device__ __forceinline__ void few_publish(FewJob* fj, const float* fr, uint32_t it, bool end,
+                                            int lane) {
+    uint32_t v[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int w = 2 * lane + i;
+        v[i] = w < NFR ? __float_as_uint(fr[w]) : (end ? 1u : 0u);
+    }
+    few_put2(fj->frame + lane, few_word(it, v[0]), few_word(it, v[1]));
+}
+
+// The Newton step of the alignment whose state is in `ctl` (one warp): as queue_control, with
+// the next frame in ctl.fr, published as soon as it is there. Left for few_after: what only the
+// next step reads. Returns 1 (every lane) when the alignment is finished.
+template <bool CPU_SEM>
+__device__ __noinline__ int few_control(const AlignParams& P, CtlShared& ctl, FewJob* fj, int job,
+                                        int it, int lane) {
+    finalize_gH(ctl.tot, ctl.Ad, ctl.Bd, ctl.g, ctl.H, lane);
+    __syncwarp();
+    solve_warp<CPU_SEM>(ctl.H, ctl.g, ctl.solve, lane);
+    if (lane == 0) ctl.n_eigen += ctl.solve.path;
+    const int ncorr = (int)ctl.tot[NACC];
+    AlignOut& o = P.out[job];
+    int done = 0;
+    if (CPU_SEM) {
+        if (lane == 0)
+            done = control_step<CPU_SEM>(P, ctl, P.jobs[job], o, it, ctl.tot[A_SC], ncorr);
+        done = __shfl_sync(0xffffffffu, done, 0);
+        __syncwarp();
+    } else {
+        const bool conv = graph_step_warp(P, ctl, lane);
+        done = conv || it + 1 >= P.max_iter;
+        if (done) {
+            osc_update_warp(ctl, it, lane);
+            graph_finish(P, ctl, o, it, ctl.tot[A_SC], ncorr, conv, lane);
+        }
+    }
+    if (!done) frame_first(ctl.pose, CPU_SEM, ctl.fr, ctl.trig, ctl.Ad, lane);
+    few_publish(fj, ctl.fr, (uint32_t)(it + 1), done != 0, lane);
+    return done;
+}
+
+// The rest of a step that goes on: B_kl and the oscillation history
+template <bool CPU_SEM>
+__device__ __forceinline__ void few_after(CtlShared& ctl, int it, int lane) {
+    frame_second(ctl.trig, ctl.Bd, lane);
+    if (!CPU_SEM) osc_update_warp(ctl, it, lane);
+}
+
+// S, G, M of one point at the frame, into out[FVAL][32] of its lane
+template <bool CPU_SEM>
+__device__ __forceinline__ void few_item(const AlignParams& P, const float* fr,
+                                         const uint32_t* off27, bool there, const float* pv,
+                                         uint32_t* list, float* out) {
+    const MapView& m = P.map;
+    PointSums p{};
+    int cnt = 0;
+    if (there && isfinite(pv[0]) && isfinite(pv[1]) && isfinite(pv[2])) {
+        float qh[3], ql[3];
+        transform_point(fr, pv, qh, ql);
+        cnt = search_point<8>(m, off27, qh, ql, P.max_nb, list, FT);
+        if (cnt) pair_terms<CPU_SEM, 4>(m, qh, ql, cnt, P.d1f, P.d2f, list, FT, p);
+    }
+    const float v[FVAL] = {p.S,  p.G0, p.G1, p.G2,  p.M0,  p.M1,  p.M2,
+                           p.M3, p.M4, p.M5, pv[0], pv[1], pv[2], __int_as_float(cnt)};
+#pragma unroll
+    for (int j = 0; j < FVAL; ++j) out[j * 32] = v[j];
+}
+
+template <bool CPU_SEM>
+__global__ void __launch_bounds__(FT, 1) k_ndt_few(const AlignParams P) {
+    __shared__ FewShared sh;
+    // dynamic shared memory: [FITEMS][FVAL][32] item sums, then voxel lists [max_nb][FT]
+    extern __shared__ uint32_t list_smem[];
+    float* const sums = reinterpret_cast<float*>(list_smem);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    uint32_t* const list = list_smem + FITEMS * FVAL * 32 + tid;
+    const FewCta me_cta = P.few_ctas[blockIdx.x];
+    const int G = (int)me_cta.ctas, r = (int)me_cta.rank, job = (int)me_cta.job;
+    const AlignJob jb = P.jobs[job];
+    FewJob* const fj = P.few + job;
+    ulonglong2* const part = P.few_part + (size_t)(blockIdx.x - r) * NRED;
+    const MapView& m = P.map;
+    const float* const pts = P.pts + 3 * jb.offset;
+    const QPart q = queue_part(P, jb.n, 0u);
+    // this CTA's partition warps [o0, o0 + owners), up to FOWN of them at a time
+    const int owners = max(0, min((int)me_cta.owners, (int)q.units - r * (int)me_cta.owners));
+    const uint32_t o0 = (uint32_t)r * me_cta.owners;
+    const uint32_t step = (uint32_t)P.qranks * (uint32_t)P.qthreads;
+    const int slices = (int)((jb.n + step - 1u) / step);    // points of a lane at most
+    // the warps that take items: all, but in the first CTA not the one that runs the steps
+    const int w0 = r == 0 ? 1 : 0;
+    const uint64_t t_start = global_ns();
+    nbhd_offsets(m, sh.off27);
+    if (tid < 6) sh.ctl.pose[tid] = sh.ctl.best_pose[tid] = jb.pose[tid];
+    if (tid < 3) sh.ctl.prev[tid] = sh.ctl.prev2[tid] = jb.pose[tid];
+    if (tid < 36) sh.ctl.last_H[tid] = 0.0;
+    if (tid == 0) {
+        sh.ctl.best_score = -INFINITY;
+        sh.ctl.last_corr = sh.ctl.osc = sh.ctl.max_osc = sh.ctl.n_eigen = 0;
+        sh.ctl.solve.have_w = 0;
+        sh.stop = sh.failed = 0;
+        sh.cyc[0] = sh.cyc[1] = sh.cyc[2] = sh.cyc[3] = 0ull;
+    }
+    auto load_item = [&](int o, int k, float* pv) -> bool {
+        uint32_t first, st, end;
+        unit_points(P, q, jb.n, o0 + o, lane, first, st, end);
+        const uint64_t at = first + (uint64_t)k * st;
+        pv[0] = pv[1] = pv[2] = 0.f;
+        if (at >= end) return false;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) pv[a] = __ldg(pts + 3 * at + a);
+        return true;
+    };
+    // slices whose items fit in shared memory together, for `no` partition warps
+    auto slices_for = [&](int no) { return min(max(1, FITEMS / max(1, no)), slices); };
+    // a warp's first item keeps its points in registers over the iterations
+    const int me = warp - w0;
+    float pv0[3];
+    bool there0 = false;
+    {
+        const int no = min(owners, FOWN), ks = slices_for(no);
+        if (me >= 0 && me < no * ks) there0 = load_item(me / ks, me % ks, pv0);
+    }
+    __syncthreads();
+    if (warp == 0) {
+        frame_first(sh.ctl.pose, CPU_SEM, sh.ctl.fr, sh.ctl.trig, sh.ctl.Ad, lane);
+        for (int i = lane; i < NFR; i += 32) sh.fr[i] = sh.ctl.fr[i];
+    }
+    __syncthreads();
+    uint64_t point_iters = 0, corr_total = 0;  // CTA 0, thread 0
+    for (int it = 0;; ++it) {
+        const unsigned long long c0 = clock64();
+        if (r == 0 && warp == 0) {
+            if (it == 0)
+                frame_second(sh.ctl.trig, sh.ctl.Bd, lane);
+            else
+                few_after<CPU_SEM>(sh.ctl, it - 1, lane);
+        }
+        double sum = 0.0;  // thread k: the CTA's value k
+        for (int ob = 0; ob < owners; ob += FOWN) {
+            const int no = min(FOWN, owners - ob), batch = slices_for(no);
+            float acc[NACC];  // of lane `lane` of partition warp o0 + ob + me (me < no)
+#pragma unroll
+            for (int i = 0; i < NACC; ++i) acc[i] = 0.f;
+            int nc = 0;
+            for (int k0 = 0; k0 < slices; k0 += batch) {
+                const int ks = min(batch, slices - k0);
+                if (ob + k0 > 0) __syncthreads();  // the last items have been read
+                for (int i = me; i >= 0 && i < no * ks; i += FNW - w0) {
+                    float* const out = sums + (size_t)i * FVAL * 32 + lane;
+                    if (ob + k0 == 0 && i == me) {
+                        few_item<CPU_SEM>(P, sh.fr, sh.off27, there0, pv0, list, out);
+                    } else {
+                        float pv[3];
+                        const bool there = load_item(ob + i / ks, k0 + i % ks, pv);
+                        few_item<CPU_SEM>(P, sh.fr, sh.off27, there, pv, list, out);
+                    }
+                }
+                __syncthreads();
+                if (me < 0 || me >= no) continue;
+                for (int k = 0; k < ks; ++k) {
+                    const float* in = sums + (size_t)(me * ks + k) * FVAL * 32 + lane;
+                    const int cnt = __float_as_int(in[13 * 32]);
+                    if (cnt == 0) continue;
+                    const PointSums p{in[0],       in[1 * 32], in[2 * 32], in[3 * 32], in[4 * 32],
+                                      in[5 * 32],  in[6 * 32], in[7 * 32], in[8 * 32], in[9 * 32]};
+                    const float pv[3] = {in[10 * 32], in[11 * 32], in[12 * 32]};
+                    nc += cnt;
+                    point_contract(pv, sh.fr, p, acc, acc + A_HTR, 1);
+                }
+                __syncwarp();
+            }
+            if (me >= 0 && me < no) {
+                warp_sum_acc(acc, lane, sh.wpart[me]);
+                nc = __reduce_add_sync(0xffffffffu, nc);
+                if (lane == 0) sh.wpart[me][NACC] = (double)nc;
+            }
+            __syncthreads();
+            if (tid < NRED)
+                for (int w = 0; w < no; ++w) sum += sh.wpart[w][tid];
+        }
+        const uint32_t now = (uint32_t)(it + 1);
+        if (tid < NRED) {
+            const unsigned long long b = (unsigned long long)__double_as_longlong(sum);
+            few_put2(part + (size_t)r * NRED + tid, few_word(now, (uint32_t)b),
+                     few_word(now, (uint32_t)(b >> 32)));
+        }
+        const unsigned long long c1 = clock64();
+        if (r == 0) {
+            // the sum over CTAs: FSEG segments, then the segments as a tree
+            const int k = tid % NRED, sg = tid / NRED;
+            if (sg < FSEG) {
+                double s = 0.0;
+                constexpr int A = 4;
+                for (int c = sg; c < G; c += A * FSEG) {
+                    ulonglong2 v[A];
+#pragma unroll
+                    for (int i = 0; i < A; ++i)
+                        if (c + i * FSEG < G)
+                            v[i] = few_get2(part + (size_t)(c + i * FSEG) * NRED + k);
+#pragma unroll
+                    for (int i = 0; i < A; ++i)
+                        if (c + i * FSEG < G) {
+                            if (!few_wait2(part + (size_t)(c + i * FSEG) * NRED + k, now, v[i],
+                                           P.stall_ns))
+                                sh.failed = 1;
+                            s += __longlong_as_double((long long)(v[i].y << 32 |
+                                                                  (uint32_t)v[i].x));
+                        }
+                }
+                sh.seg[sg][k] = s;
+            }
+            __syncthreads();
+            const unsigned long long c2 = clock64();
+            if (!sh.failed) {
+                if (warp < 2 && tid < NRED) {
+                    double v[FSEG];
+#pragma unroll
+                    for (int i = 0; i < FSEG; ++i) v[i] = sh.seg[i][tid];
+                    sh.ctl.tot[tid] =
+                        ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+                }
+                __syncthreads();
+                if (warp == 0) {
+                    const int done = few_control<CPU_SEM>(P, sh.ctl, fj, job, it, lane);
+                    for (int i = lane; i < NFR; i += 32) sh.fr[i] = sh.ctl.fr[i];
+                    if (lane == 0) {
+                        const unsigned long long c3 = clock64();
+                        sh.cyc[0] += c1 - c0;
+                        sh.cyc[1] += c2 - c1;
+                        sh.cyc[2] += c3 - c2;
+                        point_iters += jb.n;
+                        corr_total += (uint64_t)sh.ctl.tot[NACC];
+                        sh.stop = done;
+                        if (done) {
+                            AlignOut& o = P.out[job];
+                            o.point_iters = point_iters;
+                            o.corr_total = corr_total;
+                            for (int i = 0; i < 4; ++i) o.cycles[i] = sh.cyc[i];
+                            o.n_eigen = sh.ctl.n_eigen;
+                            o.t_start = t_start;
+                            o.t_end = global_ns();
+                        }
+                    }
+                }
+            } else if (warp == 0) {
+                if (lane == 0) {
+                    atomicOr(P.status, ST_WAIT_LIMIT);
+                    sh.stop = 1;
+                }
+                few_publish(fj, sh.fr, now, true, lane);  // the others leave too
+            }
+        } else if (warp == 0) {
+            ulonglong2 v = few_get2(fj->frame + lane);
+            const bool ok = few_wait2(fj->frame + lane, now, v, P.stall_ns);
+            const bool all = __all_sync(0xffffffffu, ok);
+            const uint32_t end = __shfl_sync(0xffffffffu, (uint32_t)v.x, NFR / 2);
+            if (2 * lane < NFR) {
+                sh.fr[2 * lane] = __uint_as_float((uint32_t)v.x);
+                sh.fr[2 * lane + 1] = __uint_as_float((uint32_t)v.y);
+            }
+            if (lane == 0) {
+                sh.stop = !all || end != 0u;
+                if (!all) atomicOr(P.status, ST_WAIT_LIMIT);
+            }
+        }
+        __syncthreads();
+        if (sh.stop) break;
+    }
+}
+
+size_t few_bytes(uint32_t jobs, uint32_t ctas) {
+    return (size_t)jobs * sizeof(FewJob) + (size_t)ctas * NRED * sizeof(ulonglong2);
+}
+
+template <bool SEM>
+static cudaError_t launch_few_k(const AlignParams& p, size_t smem, cudaStream_t s) {
+    auto kern = k_ndt_few<SEM>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)smem);
+    if (e != cudaSuccess) return e;
+    // the exchange words: no iteration there yet
+    cudaMemsetAsync(p.few, 0, few_bytes(p.num_jobs, p.qgrid), s);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(p.qgrid, 1, 1);
+    cfg.blockDim = dim3(FT, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, p);
+}
+
+// Shares `sms` CTAs among the alignments of n[j] points (partition: `ranks` ranks of `threads`
+// threads): every alignment gets one, then the alignment with the most items per CTA another,
+// until the CTAs are used up or each alignment has a warp for every item in at least 16 CTAs
+// (more SMs shorten the point work of a small scan). Appends the CTAs, alignment by alignment;
+// false when there are more alignments than CTAs.
+bool few_share(const uint32_t* n, uint32_t jobs, int ranks, int threads, int sms,
+               std::vector<FewCta>& out) {
+    if (jobs > (uint32_t)sms) return false;
+    const uint64_t step = (uint64_t)ranks * threads;
+    std::vector<uint32_t> units(jobs), ctas(jobs, 1u);
+    std::vector<uint64_t> slices(jobs);
+    for (uint32_t j = 0; j < jobs; ++j) {
+        units[j] = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(step / 32, (n[j] + 31ull) / 32));
+        slices[j] = std::max<uint64_t>(1, (n[j] + step - 1) / step);
+    }
+    // the alignments by items per CTA, most first (ties: the earlier)
+    auto load = [&](uint32_t j) {
+        return std::make_pair((uint64_t)units[j] * slices[j] * 1024 / ctas[j], ~j);
+    };
+    std::priority_queue<std::pair<uint64_t, uint32_t>> by_load;
+    for (uint32_t j = 0; j < jobs; ++j) by_load.push(load(j));
+    for (int left = sms - (int)jobs; left > 0 && !by_load.empty();) {
+        const uint32_t j = ~by_load.top().second;
+        by_load.pop();
+        const uint64_t own = (units[j] + ctas[j] - 1) / ctas[j];
+        if (ctas[j] >= units[j] || (own * slices[j] <= (uint64_t)FOWN && ctas[j] >= 16)) continue;
+        ctas[j]++;
+        --left;
+        by_load.push(load(j));
+    }
+    for (uint32_t j = 0; j < jobs; ++j) {
+        const uint32_t own = (units[j] + ctas[j] - 1) / ctas[j];
+        const uint32_t g = (units[j] + own - 1) / own;  // CTAs with work
+        for (uint32_t r = 0; r < g; ++r) out.push_back(FewCta{j, r, g, own});
+    }
+    return true;
+}
+
 template <int T, bool SEM, int CAP, bool LS>
 static cudaError_t launch_k(cudaLaunchConfig_t& cfg, const AlignParams& p, int K) {
     auto kern = k_ndt_align<T, SEM, CAP, LS>;
@@ -2677,6 +3127,16 @@ int launch_align(const AlignParams& p, LaunchShape shape, cudaStream_t s) {
     AlignParams q = p;
     q.cluster = K;
     const int R = shape.regcap;
+    if (shape.few > 0) {
+        q.qthreads = shape.threads;
+        q.qranks = shape.ranks;
+        q.qunits = (int32_t)QUNITS;
+        q.few_part = (ulonglong2*)(p.few + p.num_jobs);
+        const size_t smem = ((size_t)FITEMS * FVAL * 32 + (size_t)FT * p.max_nb) * 4;
+        return cuda_fail(p.semantics == NDT_SEMANTICS_CPU ? launch_few_k<true>(q, smem, s)
+                                                          : launch_few_k<false>(q, smem, s),
+                         "align launch");
+    }
     if (shape.queue > 0) {
         if (p.ls_cands > 0 || !p.qjobs) {
             set_error("the work-queue kernel takes no line search and needs its buffers");

@@ -212,7 +212,8 @@ struct ndt_ctx {
     bool profile = false;
     bool trace = false;
     DevBuf d_trace;
-    DevBuf d_qjobs, d_qctl, d_qframe, d_qpart, d_qoff;  // work-queue kernel
+    DevBuf d_qjobs, d_qctl, d_qframe, d_qpart;          // work-queue kernel
+    DevBuf d_few;                                       // few-alignments kernel
     std::vector<double> h_trace;       // last call's records, by job order
     std::vector<uint32_t> trace_slot;  // job index -> caller's result index
     int trace_iters = 0;
@@ -383,6 +384,10 @@ static int check_status(ndt_ctx* c, uint32_t st) {
                   std::to_string(c->stall_ns / 1000000ull) + " ms with alignments open");
         return NDT_ERR_DEVICE;
     }
+    if (st & ST_WAIT_LIMIT) {
+        set_error("a wait inside a Newton kernel ran out");
+        return NDT_ERR_DEVICE;
+    }
     set_error("device reported status " + std::to_string(st));
     return NDT_ERR_DEVICE;
 }
@@ -533,7 +538,7 @@ int ndt_ctx_destroy(ndt_ctx* c) {
                       &c->bs.seg_rec, &c->bs.small, &c->d_in, &c->d_jobs, &c->d_aout,
                       &c->d_sjobs, &c->d_sout, &c->d_part, &c->d_sdone, &c->d_status, &c->d_q, &c->d_qidx,
                       &c->d_qcnt, &c->d_trace, &c->d_qjobs, &c->d_qctl, &c->d_qframe,
-                      &c->d_qpart, &c->d_qoff})
+                      &c->d_qpart, &c->d_few})
         dev_free(*b);
     for (PinBuf* b : {&c->bs.host, &c->bs_b.host, &c->bs_tile.host, &c->h_pts, &c->h_jobs, &c->h_aout, &c->h_sjobs, &c->h_sout, &c->h_misc,
                       &c->h_arrive})
@@ -861,19 +866,33 @@ static int log2_bucket(uint64_t v) {
 // Launch shape: an explicit configuration wins, then an autotuned entry for this
 // (batch size, scan size) bucket, then the default: 512-thread CTAs for large scans, and
 // clusters doubled until the launch covers about three CTAs per SM while keeping at least
-// two points per thread per CTA. That is the partition of the points over threads; batches of
-// more than CLUSTER_JOBS run it on the work-queue kernel, smaller ones (and line search) as
-// clusters. The work-queue kernel with its own partition is used when the configuration asks
-// for it (work_queue > 0) or the autotuner picked it, never with line search.
+// two points per thread per CTA. That is the partition of the points over threads; which kernel
+// runs it is the next rule. The work-queue kernel with its own partition is used when the
+// configuration asks for it (work_queue > 0) or the autotuner picked it, never with line search.
 static int queue_units(int threads) { return std::min<int>(QUNITS, threads / 32); }
 
-// Largest batch that takes one cluster per alignment by default. Few alignments leave most SMs
-// idle on either kernel, and the hardware cluster barrier is quicker than the queue's claims
-// through L2 (one 20k-point scan: 0.30 ms on the cluster, 0.34 on the queue); a batch of 64 fills
-// the GPU and spends its waves' tails idle (0.75 ms on clusters, 0.53 on the queue).
-constexpr uint32_t CLUSTER_JOBS = 8;
+// The kernel that runs a default batch's partition (calls from pinned host memory, a 1M-point
+// map, 5 iterations, in us: few / cluster / queue):
+//   Up to FEW_JOBS scans, or FEW_POINTS_PER_SM points per SM: k_ndt_few, all SMs on every scan.
+//       1 x 1.5k points 167/216/-, 8 x 20k 395/421/425, 8 x 400k 2412/2791/2717, 48 x 1.5k
+//       347/354/464, 12 x 6k 324/353/424; beyond, a scan has too few SMs to make up for the
+//       exchange: 64 x 1.5k 408/380/492, 32 x 6k 452/406/520, 12 x 20k 500/453/553. FEW_POINTS
+//       bounds an iteration, and with it the waits inside the kernel, to a small part of their
+//       limit.
+//   Batches whose clusters need more than 1.75 waves of the GPU: k_ndt_queue, which has no last
+//       wave to fill and takes scans as they are copied in: 80 x 4.2k (2.1 waves) -/683/584,
+//       64 x 2k-40k (3.4) -/953/728, 152 x 20k -/2013/1496; 24 x 20k (1.3 waves) -/597/657. But
+//       when a few alignments go on alone, an iteration of theirs is about 23 us longer than on a
+//       cluster, and a wave saves about 85: hence also more waves than max_iterations / 4 (64 x
+//       20k device-resident, up to 30 iterations: 1493 on clusters, 1797). Alignments of 1,024 to
+//       4,095 points only where a CTA keeps them for all iterations (K = 1): 600 x 1.5k
+//       device-resident 658 -> 586, but 300 x 2.5k (K = 2) 614 -> 657. Below 1,024 points a
+//       step weighs more than its points and clusters step faster: 3,200 x 200 935 -> 1336.
+constexpr uint64_t FEW_POINTS_PER_SM = 500;
+constexpr uint32_t FEW_JOBS = 8;
+constexpr uint64_t FEW_POINTS = 1ull << 26;
 
-static LaunchShape choose_shape(ndt_ctx* c, uint32_t jobs, uint32_t max_n) {
+static LaunchShape choose_shape(ndt_ctx* c, uint32_t jobs, uint32_t max_n, uint64_t total) {
     LaunchShape sh{0, 0, 128, 0};
     if (c->forced.cluster > 0) return c->forced;
     const bool ls = c->cfg.use_line_search != 0;
@@ -904,20 +923,33 @@ static LaunchShape choose_shape(ndt_ctx* c, uint32_t jobs, uint32_t max_n) {
     while (K < 8 && (uint64_t)jobs * K < 3ull * (uint64_t)c->num_sms &&
            max_n / (uint32_t)(2 * K) >= (uint32_t)sh.threads * 2)
         K *= 2;
-    if (jobs > CLUSTER_JOBS && c->cfg.work_queue == 0 && !ls && c->cfg.threads_per_cta <= 0 &&
+    if (c->cfg.work_queue == 0 && !ls && c->cfg.threads_per_cta <= 0 &&
         c->cfg.max_registers <= 0) {
-        // this cluster's partition of the points on the work-queue kernel: every lane's f32
-        // sums are the cluster kernel's
-        sh.cluster = 1;
-        sh.ranks = K;
-        sh.queue = 1;
-        sh.npw = 1;
-        sh.units = queue_units(sh.threads);
-        // 64 registers (four CTAs an SM) where a CTA keeps its alignments and steps hide
-        // behind other alignments' points, else 80 (three CTAs, no spills in the point work):
-        // 16 x 200 particles 4.17 and 4.27 ms, 64 scans of 2k-40k points 0.58 and 0.53 ms
-        sh.regcap = K * sh.threads <= (int)QUNITS * 32 ? 64 : 80;
-        return sh;
+        // this cluster's partition of the points on another kernel: every lane's f32 sums are
+        // the cluster kernel's
+        if (!c->trace && jobs <= (uint32_t)c->num_sms &&
+            total <= (jobs <= FEW_JOBS ? FEW_POINTS : FEW_POINTS_PER_SM * (uint64_t)c->num_sms)) {
+            sh.cluster = 1;
+            sh.ranks = K;
+            sh.few = 1;
+            return sh;
+        }
+        const uint64_t resident = (uint64_t)c->num_sms * (512 / sh.threads);  // CTAs of a wave
+        const uint64_t quarters = 4 * (uint64_t)jobs * K / resident;         // of waves
+        if ((sh.threads == 512 || (sh.threads == 256 && K == 1)) &&
+            quarters >= (uint64_t)std::max(7, c->cfg.max_iterations + 1)) {
+            sh.cluster = 1;
+            sh.ranks = K;
+            sh.queue = 1;
+            sh.npw = 1;
+            sh.units = queue_units(sh.threads);
+            // 64 registers (four CTAs an SM) where a CTA keeps its alignments and steps hide
+            // behind other alignments' points, else 80 (three CTAs, no spills in the point
+            // work): 16 x 200 particles 4.17 and 4.27 ms, 64 scans of 2k-40k points 0.58 and
+            // 0.53 ms
+            sh.regcap = K * sh.threads <= (int)QUNITS * 32 ? 64 : 80;
+            return sh;
+        }
     }
     sh.cluster = K;
     return sh;
@@ -941,21 +973,28 @@ static int run_align_enqueue(ndt_ctx* c, const float* d_pts, std::vector<AlignJo
     int rc;
     size_t jb = nj * sizeof(AlignJob), ob = nj * sizeof(AlignOut), sjb = nj * sizeof(ScoreJob),
            sob = nj * sizeof(ScoreOut);
-    if ((rc = dev_reserve(c->d_jobs, jb)) || (rc = dev_reserve(c->d_aout, ob)) ||
-        (rc = dev_reserve(c->d_sjobs, sjb)) || (rc = dev_reserve(c->d_sout, sob)) ||
-        (rc = score_reserve(c, nj, max_n)) || (rc = pin_reserve(c->h_jobs, jb + sjb)) || (rc = pin_reserve(c->h_aout, ob + sob + 16)))
+    // tables in one block each way (a copy costs a small call about 3 us): alignment jobs,
+    // scoring jobs and partial-sum offsets in; alignment and scoring results out
+    if ((rc = dev_reserve(c->d_jobs, jb + sjb)) || (rc = dev_reserve(c->d_aout, ob + sob)) ||
+        (rc = score_reserve(c, nj, max_n)) || (rc = pin_reserve(c->h_jobs, jb + sjb)) ||
+        (rc = pin_reserve(c->h_aout, ob + sob + 16)))
         return rc;
-    AlignJob* hj = (AlignJob*)c->h_jobs.p;
-    ScoreJob* hs = (ScoreJob*)((char*)c->h_jobs.p + jb);
-    for (uint32_t j = 0; j < nj; ++j) {
-        hj[j] = jobs[j];
-        ScoreJob s{};
-        s.offset = jobs[j].offset;
-        s.n = jobs[j].n;
-        s.pose_src = 1;
-        s.out_index = j;
-        hs[j] = s;
-    }
+    AlignJob* hj = nullptr;
+    ScoreJob* hs = nullptr;
+    auto fill_jobs = [&]() {
+        hj = (AlignJob*)c->h_jobs.p;
+        hs = (ScoreJob*)((char*)c->h_jobs.p + jb);
+        for (uint32_t j = 0; j < nj; ++j) {
+            hj[j] = jobs[j];
+            ScoreJob s{};
+            s.offset = jobs[j].offset;
+            s.n = jobs[j].n;
+            s.pose_src = 1;
+            s.out_index = j;
+            hs[j] = s;
+        }
+    };
+    fill_jobs();
     cudaStream_t st = c->stream;
     c->stats.h2d_bytes += jb + sjb;
     AlignParams p{};
@@ -995,10 +1034,12 @@ static int run_align_enqueue(ndt_ctx* c, const float* d_pts, std::vector<AlignJo
         cudaMemsetAsync(c->d_trace.p, 0xFF, tb, st);  // NaN marks iterations not run
         p.trace = (double*)c->d_trace.p;
     }
-    LaunchShape shape = choose_shape(c, nj, max_n);
+    uint64_t points = 0;
+    for (uint32_t j = 0; j < nj; ++j) points += jobs[j].n;
+    LaunchShape shape = choose_shape(c, nj, max_n, points);
     // work-queue kernel: chunk counts and partial-sum offsets per alignment (host, in the
     // pinned job block), per-alignment state and the partials (device)
-    size_t qob = 0;
+    size_t qob = 0;  // bytes behind the two job tables: partial-sum offsets, or the CTA table
     uint32_t* hq = nullptr;
     if (shape.queue > 0) {
         const uint32_t chunk = (uint32_t)(shape.threads * shape.queue);
@@ -1006,17 +1047,7 @@ static int run_align_enqueue(ndt_ctx* c, const float* d_pts, std::vector<AlignJo
         const uint64_t max_runs = (uint64_t)QMAXCH * U / upr;
         qob = (size_t)nj * sizeof(uint32_t);
         if ((rc = pin_reserve(c->h_jobs, jb + sjb + qob))) return rc;
-        hj = (AlignJob*)c->h_jobs.p;  // the block may have moved: refill it
-        hs = (ScoreJob*)((char*)c->h_jobs.p + jb);
-        for (uint32_t j = 0; j < nj; ++j) {
-            hj[j] = jobs[j];
-            ScoreJob s{};
-            s.offset = jobs[j].offset;
-            s.n = jobs[j].n;
-            s.pose_src = 1;
-            s.out_index = j;
-            hs[j] = s;
-        }
+        fill_jobs();  // the block may have moved
         hq = (uint32_t*)((char*)c->h_jobs.p + jb + sjb);
         // partial-sum slots per alignment: its chunk count, at the smallest (last iterations')
         // run size the most an iteration uses, capped at the claim word's 16-bit count
@@ -1040,25 +1071,47 @@ static int run_align_enqueue(ndt_ctx* c, const float* d_pts, std::vector<AlignJo
         if ((rc = dev_reserve(c->d_qjobs, (size_t)nj * sizeof(QJob))) ||
             (rc = dev_reserve(c->d_qctl, (size_t)nj * sizeof(QCtl))) ||
             (rc = dev_reserve(c->d_qframe, (size_t)nj * NFRAME * sizeof(float))) ||
-            (rc = dev_reserve(c->d_qoff, qob)) ||
+            (rc = dev_reserve(c->d_jobs, jb + sjb + qob)) ||
             (rc = dev_reserve(c->d_qpart, (size_t)total * NRED * sizeof(double))))
             return rc;
         p.qjobs = (QJob*)c->d_qjobs.p;
         p.qctl = (QCtl*)c->d_qctl.p;
         p.qframe = (float*)c->d_qframe.p;
         p.qpart = (double*)c->d_qpart.p;
-        p.qpart_off = (const uint32_t*)c->d_qoff.p;
+        p.jobs = (const AlignJob*)c->d_jobs.p;  // the block may have moved
+        p.qpart_off = (const uint32_t*)((char*)c->d_jobs.p + jb + sjb);
         p.qcount = (uint32_t*)c->d_status.p + 2;  // word 2 of the status block
         p.qunits_total = full;
         p.qsolo = total == nj && !p.withhold ? 1 : 0;
         c->stats.h2d_bytes += qob;
+    }
+    if (shape.few > 0) {
+        std::vector<uint32_t> sizes(nj);
+        std::vector<FewCta> ctas;
+        for (uint32_t j = 0; j < nj; ++j) sizes[j] = jobs[j].n;
+        few_share(sizes.data(), nj, shape.ranks, shape.threads, c->num_sms, ctas);
+        qob = (size_t)c->num_sms * sizeof(FewCta);
+        const size_t at = (jb + sjb + 15) & ~(size_t)15;  // the table's place in the block
+        qob += at - (jb + sjb);
+        if ((rc = pin_reserve(c->h_jobs, jb + sjb + qob)) ||
+            (rc = dev_reserve(c->d_jobs, jb + sjb + qob)) ||
+            (rc = dev_reserve(c->d_few, few_bytes(nj, (uint32_t)c->num_sms))))
+            return rc;
+        fill_jobs();  // the block may have moved
+        std::memcpy((char*)c->h_jobs.p + at, ctas.data(), ctas.size() * sizeof(FewCta));
+        p.jobs = (const AlignJob*)c->d_jobs.p;
+        p.few = (FewJob*)c->d_few.p;
+        p.few_ctas = (const FewCta*)((char*)c->d_jobs.p + at);
+        p.qgrid = (uint32_t)ctas.size();
     }
     AlignOut* ho = (AlignOut*)c->h_aout.p;
     ScoreOut* hso = (ScoreOut*)((char*)c->h_aout.p + ob);
     uint32_t* hst = (uint32_t*)((char*)c->h_aout.p + ob + sob);
     // host batch copied in during the launch: the kernel reads the resident-point count from
     // word 3 of the status block (32-bit: the batch holds fewer than 2^32 points)
-    const bool stream_in = plan && shape.queue > 0 && !c->trace &&
+    // (not where CTAs keep their alignments, which are taken in order: 600 x 1.5k points 1015 us
+    // on clusters, 1335 streamed in)
+    const bool stream_in = plan && shape.queue > 0 && !c->trace && !(shape.ranks && p.qsolo) &&
                            plan->chunk_job.size() > 2 && plan->total < 0xFFFFFFFFull;
     if (plan && !stream_in) stage_plan(c, *plan, jobs, st, nullptr);
     uint32_t* d_arrive = nullptr;
@@ -1072,12 +1125,8 @@ static int run_align_enqueue(ndt_ctx* c, const float* d_pts, std::vector<AlignJo
     // the batch on the stream: job tables in, Newton kernel, NVTL scoring, results out (the
     // events are graph nodes when captured)
     auto enqueue = [&](unsigned evf) -> int {
-        cudaMemcpyAsync(c->d_jobs.p, hj, jb, cudaMemcpyHostToDevice, st);
-        cudaMemcpyAsync(c->d_sjobs.p, hs, sjb, cudaMemcpyHostToDevice, st);
-        if (shape.queue > 0) {
-            cudaMemcpyAsync(c->d_qoff.p, hq, qob, cudaMemcpyHostToDevice, st);
-            cudaMemsetAsync(p.qcount, 0, d_arrive ? 8 : 4, st);  // words 2 (and 3)
-        }
+        cudaMemcpyAsync(c->d_jobs.p, hj, jb + sjb + qob, cudaMemcpyHostToDevice, st);
+        if (shape.queue > 0) cudaMemsetAsync(p.qcount, 0, d_arrive ? 8 : 4, st);  // words 2 (, 3)
         if (d_arrive) cudaEventRecord(c->ev_in0, st);  // the counter is reset
         cudaEventRecordWithFlags(c->ev0, st, evf);
         int r = launch_align(p, shape, st);
@@ -1097,13 +1146,13 @@ static int run_align_enqueue(ndt_ctx* c, const float* d_pts, std::vector<AlignJo
             if ((r = launch_align(pr, shape, st))) return r;
             cudaEventRecordWithFlags(c->ev1, st, evf);
         }
-        r = launch_score(c->map.view, d_pts, (const ScoreJob*)c->d_sjobs.p, nj, max_n,
-                         (const AlignOut*)c->d_aout.p, c->d_part.p, (uint32_t*)c->d_sdone.p,
-                         (ScoreOut*)c->d_sout.p, (float)c->d1, (float)c->d2, st);
+        r = launch_score(c->map.view, d_pts, (const ScoreJob*)((char*)c->d_jobs.p + jb), nj,
+                         max_n, (const AlignOut*)c->d_aout.p, c->d_part.p,
+                         (uint32_t*)c->d_sdone.p, (ScoreOut*)((char*)c->d_aout.p + ob),
+                         (float)c->d1, (float)c->d2, st);
         if (r) return r;
         cudaEventRecordWithFlags(c->ev2, st, evf);
-        cudaMemcpyAsync(ho, c->d_aout.p, ob, cudaMemcpyDeviceToHost, st);
-        cudaMemcpyAsync(hso, c->d_sout.p, sob, cudaMemcpyDeviceToHost, st);
+        cudaMemcpyAsync(ho, c->d_aout.p, ob + sob, cudaMemcpyDeviceToHost, st);
         cudaMemcpyAsync(hst, c->d_status.p, 4, cudaMemcpyDeviceToHost, st);
         return cuda_fail(cudaGetLastError(), "align enqueue");
     };
@@ -1111,12 +1160,12 @@ static int run_align_enqueue(ndt_ctx* c, const float* d_pts, std::vector<AlignJo
         const std::vector<uint64_t> key = {
             nj, max_n, (uint64_t)shape.cluster, (uint64_t)shape.threads, (uint64_t)shape.regcap,
             (uint64_t)shape.queue, (uint64_t)shape.npw, (uint64_t)shape.ranks, (uint64_t)shape.units,
+            (uint64_t)shape.few, (uint64_t)p.qgrid, (uint64_t)(uintptr_t)c->d_few.p,
             (uint64_t)(uintptr_t)c->d_qjobs.p,
             (uint64_t)(uintptr_t)c->d_qctl.p, (uint64_t)(uintptr_t)c->d_qframe.p,
-            (uint64_t)(uintptr_t)c->d_qpart.p, (uint64_t)(uintptr_t)c->d_qoff.p,
+            (uint64_t)(uintptr_t)c->d_qpart.p, (uint64_t)qob,
             c->map_gen, c->cfg_gen, (uint64_t)(uintptr_t)d_pts, (uint64_t)(uintptr_t)c->d_jobs.p,
-            (uint64_t)(uintptr_t)c->d_aout.p, (uint64_t)(uintptr_t)c->d_sjobs.p,
-            (uint64_t)(uintptr_t)c->d_sout.p, (uint64_t)(uintptr_t)c->d_part.p,
+            (uint64_t)(uintptr_t)c->d_aout.p, (uint64_t)(uintptr_t)c->d_part.p,
             (uint64_t)(uintptr_t)c->d_sdone.p,
             (uint64_t)(uintptr_t)c->h_jobs.p, (uint64_t)(uintptr_t)c->h_aout.p};
         size_t gi = c->graphs.size();

@@ -30,7 +30,7 @@ constexpr uint32_t ST_HASH_FULL = 1u << 0;
 constexpr uint32_t ST_PROBE_LIMIT = 1u << 1;
 constexpr uint32_t ST_BAD_INPUT = 1u << 2;
 constexpr uint32_t ST_QUEUE_STALL = 1u << 3;  // work-queue kernel found no progress for 2 s
-constexpr uint32_t ST_WAIT_LIMIT = 1u << 4;   // a wait inside a work-queue CTA ran out (2 s)
+constexpr uint32_t ST_WAIT_LIMIT = 1u << 4;   // a wait inside a Newton kernel ran out (2 s)
 
 struct MapView {
     const uint4* slots;      // null when the dense index serves

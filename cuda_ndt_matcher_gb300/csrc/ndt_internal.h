@@ -194,10 +194,13 @@ struct AlignParams {
     // of qchunk points (fewer in an alignment's late iterations) strided by qthreads threads;
     // qunits units of 32 threads per chunk
     int32_t qthreads, qranks, qchunk, qunits;
+    struct FewJob* few;     // few-alignments kernel: frames, and the CTAs' sums
+    ulonglong2* few_part;   // (set by the launch)
+    const struct FewCta* few_ctas;  // qgrid CTAs
     uint64_t qunits_total;  // units of one iteration of every alignment (early iterations)
     int32_t qsolo;          // every iteration of every alignment is one chunk, and all points
                             // are resident: CTAs keep their alignments
-    uint32_t qgrid;         // CTAs of the launch (set by the launch)
+    uint32_t qgrid;         // CTAs of the launch
     // points copied in while the work-queue kernel runs: the device word counts the points of
     // the batch resident so far (a prefix of pts, written by the copy stream after each
     // chunk); an alignment is claimable once its last point is resident. nullptr: all are.
@@ -239,6 +242,20 @@ constexpr uint32_t QUNITS = 8;        // units (warps' shares) per chunk at most
 // 1/(2 QSPLIT_DIV) in its last ones (the partial-sum slots are sized for those). At the
 // 20k-point bench batch, 2 and 8 were slower as the first split.
 constexpr uint32_t QSPLIT_DIV = 4;
+// Few-alignments kernel, one per alignment (global memory, zero at the start of a launch): the
+// frame of the next iteration and the end mark, as words {value, iteration}; behind all of them
+// the CTAs' sums, the same way.
+struct FewJob {
+    ulonglong2 frame[32];
+};
+size_t few_bytes(uint32_t jobs, uint32_t ctas);
+// A CTA of the few-alignments kernel: its alignment (launch order), its rank among the
+// alignment's CTAs, their number, and the partition warps each takes
+struct FewCta {
+    uint32_t job, rank, ctas, owners;
+};
+bool few_share(const uint32_t* n, uint32_t jobs, int ranks, int threads, int sms,
+               std::vector<FewCta>& out);
 // Controller state of an alignment between iterations (FP64; read and written only by the
 // controller of the alignment's current iteration).
 struct QCtl {
@@ -275,8 +292,9 @@ struct LaunchShape {
     int queue;   // > 0: work-queue kernel, runs of `queue` points per thread (cluster 1)
     int npw;     // work-queue kernel: lanes sharing each point's neighbour search (0, 1: one)
     int stage;   // the stage_points option (no effect)
-    int ranks;   // work-queue kernel: > 0, the partition of a cluster of `ranks` CTAs
+    int ranks;   // work-queue and few-alignments kernels: > 0, a cluster's partition (its CTAs)
     int units;   // work-queue kernel: units per chunk
+    int few;     // 1: few-alignments kernel (partition: ranks, threads)
 };
 
 int launch_align(const AlignParams& p, LaunchShape shape, cudaStream_t s);
