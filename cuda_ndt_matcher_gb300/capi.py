@@ -244,6 +244,38 @@ def as_xyz(points):
     return a
 
 
+def _plain_xyz(a):
+    """Whether an array already is what as_xyz makes of it."""
+    return (type(a) is np.ndarray and a.ndim == 2 and a.shape[1] == 3 and a.dtype == np.float32
+            and a.flags.c_contiguous)
+
+
+def scan_array(scans, poses):
+    """The C array of a list of scans and their poses, the number of scans, and the arrays that
+    must outlive it. Filled by columns: element by element, 256 scans took about 0.7 ms."""
+    scans = [s if _plain_xyz(s) else as_xyz(s) for s in scans]
+    m = len(scans)
+    try:
+        p = np.asarray(poses)
+    except ValueError:  # rows of different lengths
+        p = None
+    if m and p is not None and p.dtype.kind in "fiu" and p.ndim == 2 and p.shape[1] >= 6 \
+            and len(p) >= m:
+        rows = np.empty((m, 8))
+        heads = rows.view(np.uint64)
+        heads[:, 0] = [s.__array_interface__["data"][0] for s in scans]
+        heads[:, 1] = [len(s) for s in scans]
+        rows[:, 2:] = p[:m, :6]
+        return (Scan * m).from_buffer(rows), m, scans
+    arr = (Scan * m)()
+    for i, (s, pose) in enumerate(zip(scans, poses)):
+        arr[i].xyz = s.ctypes.data
+        arr[i].num_points = len(s)
+        for k in range(6):
+            arr[i].initial_pose[k] = float(pose[k])
+    return arr, m, scans
+
+
 def result_dict(r: Result):
     return {
         "pose": np.array(r.pose[:], dtype=np.float64),
@@ -366,15 +398,7 @@ class Context:
 
     @staticmethod
     def _scan_array(scans, poses):
-        scans = [as_xyz(s) for s in scans]
-        m = len(scans)
-        arr = (Scan * m)()
-        for i, (s, pose) in enumerate(zip(scans, poses)):
-            arr[i].xyz = s.ctypes.data
-            arr[i].num_points = len(s)
-            for k in range(6):
-                arr[i].initial_pose[k] = float(pose[k])
-        return arr, m, scans
+        return scan_array(scans, poses)
 
     def align_batch(self, scans, poses):
         arr, m, keep = self._scan_array(scans, poses)
@@ -586,14 +610,7 @@ class PNet:
         return {k: getattr(st, k) for k, _ in st._fields_}
 
     def propose(self, map_id, queries, coarse):
-        qs = [as_xyz(q) for q in queries]
-        m = len(qs)
-        arr = (Scan * m)()
-        for i, (s, pose) in enumerate(zip(qs, coarse)):
-            arr[i].xyz = s.ctypes.data
-            arr[i].num_points = len(s)
-            for k in range(6):
-                arr[i].initial_pose[k] = float(pose[k])
+        arr, m, keep = scan_array(queries, coarse)
         P = self.cfg.proposals
         poses = np.zeros((m, P, 6))
         logits = np.zeros((m, P))
