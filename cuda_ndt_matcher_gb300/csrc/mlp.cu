@@ -4,12 +4,12 @@
 // particles of the initial-pose search. Network: input 64x64x8 scan occupancy + 64x64 map
 // height crop (36,864 features, bf16) -> 4 hidden layers of 512 (GELU) -> 16 proposals of
 // (dx, dy, dyaw, logit). Every matrix product is the tcgen05 GEMM of tc_gemm.cu
-// (D = A B^T, both operands K-major bf16, f32 accumulate):
-//   forward   Z_l   = X_l  W_l^T          A = X_l  [B x in],  B = W_l    [out x in]
-//   dW_l            = dZ_l^T X_l          A = dZ_l^T [out x B], B = X_l^T [in x B]
-//   dX_l            = dZ_l W_l            A = dZ_l [B x out],  B = W_l^T  [in x out]
-// so activations and output gradients are written in both layouts by the elementwise kernels,
-// and each weight keeps a bf16 copy and a bf16 transposed copy next to its f32 master.
+// (D = A B^T over bf16 operands in either layout, f32 accumulate), on row-major arrays as they are:
+//   forward   Z_l   = X_l  W_l^T          A = X_l  [B x in],         B = W_l [out x in]
+//   dX_l            = dZ_l W_l            A = dZ_l [B x out],        B = W_l (MN-major)
+//   dW_l            = dZ_l^T X_l          A = dZ_l (MN-major),       B = X_l (MN-major)
+// Each weight keeps a bf16 copy next to its f32 master; the Adam update is the epilogue of the dW
+// product, so weight gradients never reach memory while training.
 //
 // Features (per sample, on the device):
 //   scan grid : sensor points rotated by the coarse yaw (world-aligned, centred on the sensor),
@@ -36,8 +36,6 @@
 
 namespace ndtgb {
 
-int gemm_bf16_tn(const void* A, const void* B, float* D, int M, int N, int K, int ldd,
-                 uint32_t* d_err, cudaStream_t s, int splits, const GemmEpilogue* epi);
 constexpr int PN_MAX_SPLITS = 16;
 
 constexpr int PN_GRID = 64, PN_ZB = 8;
@@ -64,39 +62,49 @@ __device__ __forceinline__ float wrap_pi(float a) {
 }
 
 // ---- elementwise kernels ----------------------------------------------------------
-// Z [B x N] f32 (+ bias) -> X [B x N] bf16 and XT [N x B] bf16 (GELU unless `linear`);
-// with split-K partials Zp (splits x [B x N]) Z is their sum
+// Z [B x N] f32 = sum of the split-K partials Zp (splits x [B x N]) + bias, and X [B x N] bf16 =
+// GELU(Z) (Z itself if `linear`); four elements a thread (N is a multiple of 64). The partials
+// are summed in the order of the splits.
 __global__ void k_bias_act(float* __restrict__ Z, const float* __restrict__ Zp, int splits,
                            const float* __restrict__ bias, int B, int N, int linear,
-                           __nv_bfloat16* __restrict__ X, __nv_bfloat16* __restrict__ XT) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= B * N) return;
-    const int b = i / N, n = i % N;
-    float acc;
-    if (Zp) {
-        acc = 0.f;
-        for (int s = 0; s < splits; ++s) acc += Zp[(size_t)s * B * N + i];
-    } else {
-        acc = Z[i];
+                           __nv_bfloat16* __restrict__ X) {
+    const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
+    const size_t n = (size_t)B * N;
+    if (i >= n) return;
+    float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+    for (int s = 0; s < splits; ++s) {
+        const float4 p = *reinterpret_cast<const float4*>(Zp + (size_t)s * n + i);
+        z.x += p.x;
+        z.y += p.y;
+        z.z += p.z;
+        z.w += p.w;
     }
-    const float z = acc + bias[n];
-    Z[i] = z;
+    const float4 b = *reinterpret_cast<const float4*>(bias + i % N);
+    z.x += b.x;
+    z.y += b.y;
+    z.z += b.z;
+    z.w += b.w;
+    *reinterpret_cast<float4*>(Z + i) = z;
     if (X) {
-        const __nv_bfloat16 h = __float2bfloat16(linear ? z : gelu(z));
-        X[i] = h;
-        if (XT) XT[(size_t)n * B + b] = h;
+        if (!linear) z = make_float4(gelu(z.x), gelu(z.y), gelu(z.z), gelu(z.w));
+        __nv_bfloat162 h[2] = {__floats2bfloat162_rn(z.x, z.y), __floats2bfloat162_rn(z.z, z.w)};
+        *reinterpret_cast<uint2*>(X + i) = *reinterpret_cast<uint2*>(h);
     }
 }
 
 // Bias gradients of every layer in one launch: column sums over the batch of each layer's
-// output gradient (one thread per column of the concatenated layers, fixed summation order)
-constexpr int PN_MAX_LAYERS = 16;
+// output gradient (one thread per column of the concatenated layers, fixed summation order),
+// and with `update` the biases' Adam update
+constexpr int PN_MAX_LAYERS = GEMM_ADAM_MAX;
 struct ColsumTable {
     const float* g[PN_MAX_LAYERS];
     float* out[PN_MAX_LAYERS];
     int n[PN_MAX_LAYERS];
     int start[PN_MAX_LAYERS + 1];
     int layers;
+    int update;
+    AdamState adam[PN_MAX_LAYERS];
 };
 // One block of 32 x 32 threads per 32 columns: lane x takes column c0 + x, row group y the
 // rows y, y + 32, ... (coalesced 128-byte rows), then the 32 row-group sums of a column are
@@ -123,132 +131,82 @@ __global__ void __launch_bounds__(32 * PN_CS_ROWS) k_colsum_all(const ColsumTabl
         float tot = 0.f;
         for (int r = 0; r < PN_CS_ROWS; ++r) tot += part[r][x];
         t.out[l][n] = tot;
+        if (t.update) {
+            const AdamState& a = t.adam[l];
+            float c[2];
+            adam_corrections(a, c);
+            float m = a.m[n], v = a.v[n], w = a.w[n];
+            adam_update(a, tot, m, v, w, c[0], c[1]);
+            a.m[n] = m;
+            a.v[n] = v;
+            a.w[n] = w;
+        }
     }
 }
 
-// loss and output gradient, one thread per sample; O [B x P*4] (biased), T [B x 3]
+// loss and output gradient, one warp per sample, lane j the proposals j, j + 32, ...; O [B x P*4]
+// (biased), T [B x 3]. Sums over proposals run in order over all lanes' values, in every lane. (One
+// thread per sample left 8 blocks of dependent loads: 28 us for 1,024 samples.)
 __global__ void k_loss(const float* __restrict__ O, const float* __restrict__ T, int B, int P,
                        float yw, float* __restrict__ loss, float* __restrict__ dOf,
-                       __nv_bfloat16* __restrict__ dO, __nv_bfloat16* __restrict__ dOT) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+                       __nv_bfloat16* __restrict__ dO) {
+    const int b = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (b >= B) return;
-    const float* o = O + (size_t)b * P * PN_OUT_PER;
+    const float4* o4 = reinterpret_cast<const float4*>(O + (size_t)b * P * PN_OUT_PER);
     const float tx = T[3 * b] / PN_XY_SCALE, ty = T[3 * b + 1] / PN_XY_SCALE, tyaw = T[3 * b + 2];
     float best = INFINITY, mx = -INFINITY, esum = 0.f;
     int jb = 0;
-    for (int j = 0; j < P; ++j) {
-        const float ex = o[4 * j] - tx, ey = o[4 * j + 1] - ty;
-        const float ea = yw * wrap_pi(PN_PI * o[4 * j + 2] - tyaw) / PN_PI;
-        const float e = ex * ex + ey * ey + ea * ea;
-        esum += e;
-        if (e < best) {
-            best = e;
-            jb = j;
+    for (int j0 = 0; j0 < P; j0 += 32) {
+        const int cnt = min(32, P - j0);
+        float e = 0.f;
+        if (lane < cnt) {
+            const float4 o = o4[j0 + lane];
+            const float ex = o.x - tx, ey = o.y - ty;
+            const float ea = yw * wrap_pi(PN_PI * o.z - tyaw) / PN_PI;
+            e = ex * ex + ey * ey + ea * ea;
+            mx = fmaxf(mx, o.w);
         }
-        mx = fmaxf(mx, o[4 * j + 3]);
+        for (int k = 0; k < cnt; ++k) {
+            const float ek = __shfl_sync(0xffffffffu, e, k);
+            esum += ek;
+            if (ek < best) {
+                best = ek;
+                jb = j0 + k;
+            }
+        }
     }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, d));
     float z = 0.f;
-    for (int j = 0; j < P; ++j) z += expf(o[4 * j + 3] - mx);
+    for (int j0 = 0; j0 < P; j0 += 32) {
+        const int cnt = min(32, P - j0);
+        const float x = lane < cnt ? expf(o4[j0 + lane].w - mx) : 0.f;
+        for (int k = 0; k < cnt; ++k) z += __shfl_sync(0xffffffffu, x, k);
+    }
     const float lse = mx + logf(z);
     const float w_other = P > 1 ? PN_EPS_WTA / (float)(P - 1) : 0.f;
-    loss[b] = best + (lse - o[4 * jb + 3]) + w_other * (esum - best);
+    if (lane == 0) loss[b] = best + (lse - o4[jb].w) + w_other * (esum - best);
     const float inv_b = 1.f / (float)B;
-    const int ld = P * PN_OUT_PER;
-    for (int j = 0; j < P; ++j) {
+    for (int j = lane; j < P; j += 32) {
         const float w = (j == jb ? 1.f : w_other) * inv_b;
-        const float ex = o[4 * j] - tx, ey = o[4 * j + 1] - ty;
-        const float ea = yw * wrap_pi(PN_PI * o[4 * j + 2] - tyaw) / PN_PI;
-        float g[4];
-        g[0] = 2.f * ex * w;
-        g[1] = 2.f * ey * w;
-        g[2] = 2.f * ea * yw * w;
-        g[3] = (expf(o[4 * j + 3] - lse) - (j == jb ? 1.f : 0.f)) * inv_b;
-        for (int q = 0; q < 4; ++q) {
-            const int c = 4 * j + q;
-            dOf[(size_t)b * ld + c] = g[q];
-            const __nv_bfloat16 h = __float2bfloat16(g[q]);
-            dO[(size_t)b * ld + c] = h;
-            dOT[(size_t)c * B + b] = h;
-        }
+        const float4 o = o4[j];
+        const float ex = o.x - tx, ey = o.y - ty;
+        const float ea = yw * wrap_pi(PN_PI * o.z - tyaw) / PN_PI;
+        float4 g;
+        g.x = 2.f * ex * w;
+        g.y = 2.f * ey * w;
+        g.z = 2.f * ea * yw * w;
+        g.w = (expf(o.w - lse) - (j == jb ? 1.f : 0.f)) * inv_b;
+        const size_t at = (size_t)b * P + j;
+        reinterpret_cast<float4*>(dOf)[at] = g;
+        __nv_bfloat162 h[2] = {__floats2bfloat162_rn(g.x, g.y), __floats2bfloat162_rn(g.z, g.w)};
+        reinterpret_cast<uint2*>(dO)[at] = *reinterpret_cast<uint2*>(h);
     }
 }
 
-// Adam on the f32 masters of every parameter tensor in one launch (weights and biases of all
-// layers, concatenated), refreshing each weight's bf16 copy and bf16 transposed copy. The
-// step count t comes from the device counter the step's sampling kernel advanced, so a
-// captured training step replays without host updates.
-struct AdamTable {
-    float* w[2 * PN_MAX_LAYERS];
-    const float* g[2 * PN_MAX_LAYERS];
-    float* m[2 * PN_MAX_LAYERS];
-    float* v[2 * PN_MAX_LAYERS];
-    __nv_bfloat16* wb[2 * PN_MAX_LAYERS];
-    __nv_bfloat16* wbt[2 * PN_MAX_LAYERS];
-    int cols[2 * PN_MAX_LAYERS];   // C of a [R x C] weight (the transposed copy's index rule)
-    int rows[2 * PN_MAX_LAYERS];
-    uint64_t start[2 * PN_MAX_LAYERS + 1];
-    int tensors;
-};
-// Four consecutive elements per thread (every tensor's size and start is a multiple of 4):
-// 16-byte loads and stores of the f32 state, 8-byte stores of the bf16 copy. The bias
-// corrections are formed once per block.
-__global__ void k_adam_all(const AdamTable t, const uint64_t* __restrict__ step_ctr, float lr,
-                           float b1, float b2, float eps) {
-    __shared__ float s_c[2];
-    if (threadIdx.x == 0) {
-        const float step = (float)*step_ctr;
-        s_c[0] = lr / (1.f - powf(b1, step));  // lr / (1 - b1^t)
-        s_c[1] = 1.f / (1.f - powf(b2, step));  // 1 / (1 - b2^t)
-    }
-    __syncthreads();
-    const uint64_t i = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4ull;
-    if (i >= t.start[t.tensors]) return;
-    int k = 0;
-    while (i >= t.start[k + 1]) ++k;
-    const size_t j = (size_t)(i - t.start[k]);
-    const float lc1 = s_c[0], ic2 = s_c[1];
-    const float4 g4 = *reinterpret_cast<const float4*>(t.g[k] + j);
-    float4 m4 = *reinterpret_cast<const float4*>(t.m[k] + j);
-    float4 v4 = *reinterpret_cast<const float4*>(t.v[k] + j);
-    float4 w4 = *reinterpret_cast<const float4*>(t.w[k] + j);
-    float* const gm[4] = {&m4.x, &m4.y, &m4.z, &m4.w};
-    float* const gv[4] = {&v4.x, &v4.y, &v4.z, &v4.w};
-    float* const gw[4] = {&w4.x, &w4.y, &w4.z, &w4.w};
-    const float gg[4] = {g4.x, g4.y, g4.z, g4.w};
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const float mi = b1 * *gm[q] + (1.f - b1) * gg[q];
-        const float vi = b2 * *gv[q] + (1.f - b2) * gg[q] * gg[q];
-        *gm[q] = mi;
-        *gv[q] = vi;
-        *gw[q] -= lc1 * mi / (sqrtf(vi * ic2) + eps);
-    }
-    *reinterpret_cast<float4*>(t.m[k] + j) = m4;
-    *reinterpret_cast<float4*>(t.v[k] + j) = v4;
-    *reinterpret_cast<float4*>(t.w[k] + j) = w4;
-    if (t.wb[k]) {
-        const __nv_bfloat162 h01 = __floats2bfloat162_rn(w4.x, w4.y);
-        const __nv_bfloat162 h23 = __floats2bfloat162_rn(w4.z, w4.w);
-        __nv_bfloat162* wb2 = reinterpret_cast<__nv_bfloat162*>(t.wb[k] + j);
-        wb2[0] = h01;
-        wb2[1] = h23;
-        if (t.wbt[k]) {
-            const int C = t.cols[k];
-            const __nv_bfloat16 hs[4] = {h01.x, h01.y, h23.x, h23.y};
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-                t.wbt[k][(size_t)((j + q) % C) * t.rows[k] + (j + q) / C] = hs[q];
-        }
-    }
-}
-
-__global__ void k_to_bf16(const float* __restrict__ w, size_t n, int C, int R,
-                          __nv_bfloat16* __restrict__ wb, __nv_bfloat16* __restrict__ wbt) {
+__global__ void k_to_bf16(const float* __restrict__ w, size_t n, __nv_bfloat16* __restrict__ wb) {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const __nv_bfloat16 h = __float2bfloat16(w[i]);
-    wb[i] = h;
-    if (wbt) wbt[(size_t)(i % C) * R + i / C] = h;
+    if (i < n) wb[i] = __float2bfloat16(w[i]);
 }
 
 // ---- features ----------------------------------------------------------------------
@@ -287,45 +245,67 @@ struct PnScan {
 
 constexpr int EMPTY_ORD = (int)0x80808080;  // the memset byte 0x80: below every finite height
 
-// scan grid + map crop of every sample into X [B x F] and XT [F x B] (both zeroed first)
-__global__ void k_features(const float* __restrict__ scan_pts, const PnScan* __restrict__ scans,
-                           const PnSample* __restrict__ smp, const PnMap* __restrict__ maps,
-                           int B, int F, __nv_bfloat16* __restrict__ X,
-                           __nv_bfloat16* __restrict__ XT) {
-    const int b = blockIdx.y;
-    if (b >= B) return;
+// Scan grid and map crop of every sample into X [B x F], one block per sample: the scan's cells
+// are bits in shared memory (a byte per column of eight z cells), so that every row is written
+// once, in order, 16 bytes a thread; features beyond the two grids are 0. Bound by the 74 KB
+// write of a row. (Zeroing X and its transpose and scattering ones into both took 76 us for 1,024
+// samples.)
+__global__ void __launch_bounds__(256)
+    k_features(const float* __restrict__ scan_pts, const PnScan* __restrict__ scans,
+               const PnSample* __restrict__ smp, const PnMap* __restrict__ maps, int F,
+               __nv_bfloat16* __restrict__ X) {
+    __shared__ uint32_t bits[PN_SCAN_FEATS / 32];
+    const int b = blockIdx.x, tid = threadIdx.x;
     const PnSample s = smp[b];
     const PnScan sc = scans[s.scan];
-    const __nv_bfloat16 one = __float2bfloat16(1.f);
     float sy, cy;
     sincosf(s.cyaw, &sy, &cy);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < sc.n; i += gridDim.x * blockDim.x) {
+    for (int i = tid; i < PN_SCAN_FEATS / 32; i += 256) bits[i] = 0u;
+    __syncthreads();
+#pragma unroll 4
+    for (uint32_t i = tid; i < sc.n; i += 256) {
         const float* p = scan_pts + 3 * (sc.offset + i);
         const float px = p[0], py = p[1], pz = p[2];
         const float wx = cy * px - sy * py, wy = sy * px + cy * py;
-        const int gx = (int)floorf(wx + 32.f), gy = (int)floorf(wy + 32.f), gz = (int)floorf(pz + 2.f);
+        const int gx = (int)floorf(wx + 32.f), gy = (int)floorf(wy + 32.f);
+        const int gz = (int)floorf(pz + 2.f);
         if (gx < 0 || gy < 0 || gz < 0 || gx >= PN_GRID || gy >= PN_GRID || gz >= PN_ZB) continue;
         const int f = (gx * PN_GRID + gy) * PN_ZB + gz;
-        X[(size_t)b * F + f] = one;
-        if (XT) XT[(size_t)f * B + b] = one;
+        atomicOr(&bits[f >> 5], 1u << (f & 31));
     }
+    __syncthreads();
     const PnMap m = maps[s.map];
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < PN_MAP_FEATS; c += gridDim.x * blockDim.x) {
-        const int u = c / PN_GRID, v = c % PN_GRID;
-        const float wx = s.cx - 32.f + (float)u + 0.5f, wy = s.cy - 32.f + (float)v + 0.5f;
-        const int ix = (int)floorf(wx - m.ox), iy = (int)floorf(wy - m.oy);
-        float val = 0.f;
-        if (ix >= 0 && iy >= 0 && ix < m.W && iy < m.H) {
-            const int hv = m.img[(size_t)ix * m.H + iy];
-            if (hv != EMPTY_ORD) {
-                const float h = ord2f(hv);
-                val = 0.1f + fminf(fmaxf((h - s.cz + 2.f) / 10.f, 0.f), 0.9f);
+    uint4* const row = reinterpret_cast<uint4*>(X + (size_t)b * F);
+    const uint32_t one = 0x3F80u;  // 1 in bf16
+    for (int q = tid; q < F / 8; q += 256) {
+        uint32_t h[4] = {0u, 0u, 0u, 0u};
+        if (q < PN_SCAN_FEATS / 8) {
+            const uint32_t c = bits[q >> 2] >> (8 * (q & 3));
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                h[k] = (c >> (2 * k) & 1u ? one : 0u) | (c >> (2 * k + 1) & 1u ? one << 16 : 0u);
+        } else if (q < (PN_SCAN_FEATS + PN_MAP_FEATS) / 8) {
+            const int c0 = 8 * q - PN_SCAN_FEATS;
+            float val[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const int u = (c0 + k) / PN_GRID, v = (c0 + k) % PN_GRID;
+                const float wx = s.cx - 32.f + (float)u + 0.5f, wy = s.cy - 32.f + (float)v + 0.5f;
+                const int ix = (int)floorf(wx - m.ox), iy = (int)floorf(wy - m.oy);
+                val[k] = 0.f;
+                if (ix >= 0 && iy >= 0 && ix < m.W && iy < m.H) {
+                    const int hv = m.img[(size_t)ix * m.H + iy];
+                    if (hv != EMPTY_ORD)
+                        val[k] = 0.1f + fminf(fmaxf((ord2f(hv) - s.cz + 2.f) / 10.f, 0.f), 0.9f);
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                __nv_bfloat162 v2 = __floats2bfloat162_rn(val[2 * k], val[2 * k + 1]);
+                h[k] = *reinterpret_cast<uint32_t*>(&v2);
             }
         }
-        const __nv_bfloat16 h = __float2bfloat16(val);
-        const int f = PN_SCAN_FEATS + c;
-        X[(size_t)b * F + f] = h;
-        if (XT) XT[(size_t)f * B + b] = h;
+        row[q] = make_uint4(h[0], h[1], h[2], h[3]);
     }
 }
 
@@ -410,7 +390,7 @@ using namespace ndtgb;
 // ------------------------------------------------------------------------------------
 struct PnLayer {
     int in = 0, out = 0;
-    DevBuf w, b, wb, wbt, mw, vw, mb, vb, gw, gb;
+    DevBuf w, b, wb, mw, vw, mb, vb, gw, gb;
 };
 
 struct ndt_pnet {
@@ -420,7 +400,7 @@ struct ndt_pnet {
     std::vector<PnLayer> L;
     // batch buffers (capacity cap_b samples)
     int cap_b = 0;
-    std::vector<DevBuf> X, XT, Z, dZ, dZT, dZf;  // per layer
+    std::vector<DevBuf> X, Z, dZ, dZf;  // per layer
     DevBuf loss, T, smp, coarse, poses, logits, err;
     DevBuf Zp;              // split-K partial products
     DevBuf q_pts, q_scans;  // inference queries
@@ -438,6 +418,8 @@ struct ndt_pnet {
     // host copies: a query call's tables and results, and two halves of PN_STAGE bytes through
     // which points go in and parameters come out
     PinBuf h_query, h_stage;
+    cudaStream_t side = nullptr;  // bias gradients beside the chain of input gradients
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     cudaEvent_t ev_half[2] = {nullptr, nullptr};  // the half's last copy has finished
     HostPool pool;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;  // CUDA-event timing on the network's stream
@@ -553,19 +535,15 @@ static int pn_reserve_batch(ndt_pnet* p, int B) {
     if (B <= p->cap_b) return 0;
     const int nl = (int)p->L.size();
     p->X.resize(nl + 1);
-    p->XT.resize(nl + 1);
     p->Z.resize(nl);
     p->dZ.resize(nl);
-    p->dZT.resize(nl);
     p->dZf.resize(nl);
     int rc;
     for (int l = 0; l < nl; ++l) {
         const size_t in = p->L[l].in, out = p->L[l].out;
         if ((rc = dev_reserve(p->X[l], (size_t)B * in * 2)) ||
-            (rc = dev_reserve(p->XT[l], (size_t)B * in * 2)) ||
             (rc = dev_reserve(p->Z[l], (size_t)B * out * 4)) ||
             (rc = dev_reserve(p->dZ[l], (size_t)B * out * 2)) ||
-            (rc = dev_reserve(p->dZT[l], (size_t)B * out * 2)) ||
             (rc = dev_reserve(p->dZf[l], (size_t)B * out * 4)))
             return rc;
     }
@@ -618,10 +596,9 @@ static inline unsigned blocks(size_t n, int t = 256) { return (unsigned)((n + t 
 
 // forward over X[0] (already filled) for B samples; leaves the biased output in Z[last].
 // Layers after the first add their bias and activation in the GEMM's epilogue, which also
-// writes the next layer's bf16 input (and, for training, its transposed copy). The input
-// layer's long K is split so every SM streams a share of the operands; its partial products
-// are summed by k_bias_act.
-static int pn_forward(ndt_pnet* p, int B, bool need_t) {
+// writes the next layer's bf16 input. The input layer's long K is split so every SM streams a
+// share of the operands; its partial products are summed by k_bias_act.
+static int pn_forward(ndt_pnet* p, int B) {
     const int nl = (int)p->L.size();
     cudaStream_t s = p->stream;
     int rc;
@@ -632,135 +609,129 @@ static int pn_forward(ndt_pnet* p, int B, bool need_t) {
         int splits = 1;
         if (tiles < 64 && L.in >= 4096) splits = std::min(PN_MAX_SPLITS, L.in / 64 / 8);
         if (splits > 1) {
-            if ((rc = gemm_bf16_tn(p->X[l].p, L.wb.p, (float*)p->Zp.p, B, L.out, L.in, L.out,
-                                   (uint32_t*)p->err.p, s, splits, nullptr)))
+            if ((rc = gemm_bf16({p->X[l].p, 0}, {L.wb.p, 0}, (float*)p->Zp.p, B, L.out, L.in,
+                                L.out, (uint32_t*)p->err.p, s, splits, nullptr)))
                 return rc;
-            k_bias_act<<<blocks((size_t)B * L.out), 256, 0, s>>>(
+            k_bias_act<<<blocks((size_t)B * L.out / 4), 256, 0, s>>>(
                 (float*)p->Z[l].p, (const float*)p->Zp.p, splits, (const float*)L.b.p, B, L.out,
-                last ? 1 : 0, last ? nullptr : (__nv_bfloat16*)p->X[l + 1].p,
-                last || !need_t ? nullptr : (__nv_bfloat16*)p->XT[l + 1].p);
+                last ? 1 : 0, last ? nullptr : (__nv_bfloat16*)p->X[l + 1].p);
             continue;
         }
         GemmEpilogue e{};
         e.mode = last ? GEMM_EPI_BIAS : GEMM_EPI_BIAS_GELU;
         e.bias = (const float*)L.b.p;
         e.x = last ? nullptr : (__nv_bfloat16*)p->X[l + 1].p;
-        e.xt = last || !need_t ? nullptr : (__nv_bfloat16*)p->XT[l + 1].p;
-        if ((rc = gemm_bf16_tn(p->X[l].p, L.wb.p, (float*)p->Z[l].p, B, L.out, L.in, L.out,
-                               (uint32_t*)p->err.p, s, 1, &e)))
+        if ((rc = gemm_bf16({p->X[l].p, 0}, {L.wb.p, 0}, (float*)p->Z[l].p, B, L.out, L.in, L.out,
+                            (uint32_t*)p->err.p, s, 1, &e)))
             return rc;
     }
     return cuda_fail(cudaGetLastError(), "proposal forward");
 }
 
-// backward from the loss gradient in dZ*[last]; fills every layer's gw, gb. The input
-// gradient's GEMM applies GELU' of the layer below in its epilogue and writes that layer's
-// output gradient in f32 and in both bf16 layouts; the bias gradients are one launch.
-static int pn_backward(ndt_pnet* p, int B) {
+static AdamState pn_adam(const ndt_pnet* p, const DevBuf& w, const DevBuf& m, const DevBuf& v,
+                         const DevBuf* wb) {
+    AdamState a{};
+    a.w = (float*)w.p;
+    a.m = (float*)m.p;
+    a.v = (float*)v.p;
+    a.wb = wb ? (__nv_bfloat16*)wb->p : nullptr;
+    a.step = (const uint64_t*)p->step_ctr.p;
+    a.lr = p->cfg.learning_rate;
+    a.b1 = 0.9f;
+    a.b2 = 0.999f;
+    a.eps = 1e-8f;
+    return a;
+}
+
+// bias gradients (and with `update` their Adam step) of layers [l0, l1)
+static void pn_biases(ndt_pnet* p, int B, int l0, int l1, bool update, cudaStream_t s) {
+    ColsumTable ct{};
+    ct.layers = l1 - l0;
+    ct.update = update ? 1 : 0;
+    for (int k = 0; k < l1 - l0; ++k) {
+        PnLayer& L = p->L[l0 + k];
+        ct.g[k] = (const float*)p->dZf[l0 + k].p;
+        ct.out[k] = (float*)L.gb.p;
+        ct.n[k] = L.out;
+        ct.start[k + 1] = ct.start[k] + L.out;
+        ct.adam[k] = pn_adam(p, L.b, L.mb, L.vb, nullptr);
+    }
+    k_colsum_all<<<(unsigned)((ct.start[ct.layers] + 31) / 32), 32 * PN_CS_ROWS, 0, s>>>(ct, B);
+}
+
+// backward from the loss gradient in dZ*[last]: with `update` one Adam step of every parameter,
+// else every layer's gradient into gw, gb. The input gradient's GEMM applies GELU' of the layer
+// below in its epilogue and writes that layer's output gradient in f32 and bf16. The biases of
+// the layers above the first run on the side stream, beside the chain of input gradients.
+static int pn_backward(ndt_pnet* p, int B, bool update) {
     const int nl = (int)p->L.size();
     cudaStream_t s = p->stream;
     int rc;
-    ColsumTable ct{};
-    ct.layers = nl;
-    ct.start[0] = 0;
-    for (int l = nl - 1; l >= 0; --l) {
+    for (int l = nl - 1; l > 0; --l) {
         PnLayer& L = p->L[l];
-        // dW = dZ^T X  (A = dZ^T [out x B], B-operand = X^T [in x B])
-        if ((rc = gemm_bf16_tn(p->dZT[l].p, p->XT[l].p, (float*)L.gw.p, L.out, L.in, B, L.in,
-                               (uint32_t*)p->err.p, s, 1, nullptr)))
+        if (l == 1) {  // the output gradients of layers 1.. are there
+            cudaEventRecord(p->ev_fork, s);
+            cudaStreamWaitEvent(p->side, p->ev_fork, 0);
+            pn_biases(p, B, 1, nl, update, p->side);
+            cudaEventRecord(p->ev_join, p->side);
+        }
+        GemmEpilogue e{};
+        e.mode = GEMM_EPI_GELU_BACK;
+        e.zin = (const float*)p->Z[l - 1].p;
+        e.x = (__nv_bfloat16*)p->dZ[l - 1].p;
+        if ((rc = gemm_bf16({p->dZ[l].p, 0}, {L.wb.p, 1}, (float*)p->dZf[l - 1].p, B, L.in, L.out,
+                            L.in, (uint32_t*)p->err.p, s, 1, &e)))
             return rc;
-        if (l > 0) {
-            // dX = dZ W  (A = dZ [B x out], B-operand = W^T [in x out]), then * GELU'(Z_{l-1})
-            GemmEpilogue e{};
-            e.mode = GEMM_EPI_GELU_BACK;
-            e.zin = (const float*)p->Z[l - 1].p;
-            e.x = (__nv_bfloat16*)p->dZ[l - 1].p;
-            e.xt = (__nv_bfloat16*)p->dZT[l - 1].p;
-            if ((rc = gemm_bf16_tn(p->dZ[l].p, L.wbt.p, (float*)p->dZf[l - 1].p, B, L.in, L.out,
-                                   L.in, (uint32_t*)p->err.p, s, 1, &e)))
+    }
+    pn_biases(p, B, 0, 1, update, s);
+    cudaStreamWaitEvent(s, p->ev_join, 0);
+    if (update) {
+        GemmAdam w[PN_MAX_LAYERS];
+        for (int l = 0; l < nl; ++l) {
+            PnLayer& L = p->L[l];
+            w[l] = {p->dZ[l].p, p->X[l].p, L.out, L.in, pn_adam(p, L.w, L.mw, L.vw, &L.wb)};
+        }
+        if ((rc = gemm_adam(w, nl, B, (uint32_t*)p->err.p, s))) return rc;
+    } else {
+        for (int l = 0; l < nl; ++l) {
+            PnLayer& L = p->L[l];
+            if ((rc = gemm_bf16({p->dZ[l].p, 1}, {p->X[l].p, 1}, (float*)L.gw.p, L.out, L.in, B,
+                                L.in, (uint32_t*)p->err.p, s, 1, nullptr)))
                 return rc;
         }
     }
-    for (int l = 0; l < nl; ++l) {
-        ct.g[l] = (const float*)p->dZf[l].p;
-        ct.out[l] = (float*)p->L[l].gb.p;
-        ct.n[l] = p->L[l].out;
-        ct.start[l + 1] = ct.start[l] + p->L[l].out;
-    }
-    k_colsum_all<<<(unsigned)((ct.start[nl] + 31) / 32), 32 * PN_CS_ROWS, 0, s>>>(ct, B);
     return cuda_fail(cudaGetLastError(), "proposal backward");
 }
 
 static int pn_loss(ndt_pnet* p, int B) {
     const int nl = (int)p->L.size();
-    k_loss<<<blocks(B, 128), 128, 0, p->stream>>>(
+    k_loss<<<blocks((size_t)B * 32, 128), 128, 0, p->stream>>>(
         (const float*)p->Z[nl - 1].p, (const float*)p->T.p, B, p->cfg.proposals,
         p->cfg.yaw_weight, (float*)p->loss.p, (float*)p->dZf[nl - 1].p,
-        (__nv_bfloat16*)p->dZ[nl - 1].p,
-        (__nv_bfloat16*)p->dZT[nl - 1].p);
+        (__nv_bfloat16*)p->dZ[nl - 1].p);
     return cuda_fail(cudaGetLastError(), "proposal loss");
 }
 
-// Adam over every parameter tensor in one launch; the step count is the device counter
-static int pn_adam(ndt_pnet* p) {
-    AdamTable t{};
-    int k = 0;
-    t.start[0] = 0;
-    for (size_t l = 0; l < p->L.size(); ++l) {
-        PnLayer& L = p->L[l];
-        const size_t nw = (size_t)L.in * L.out;
-        t.w[k] = (float*)L.w.p;
-        t.g[k] = (const float*)L.gw.p;
-        t.m[k] = (float*)L.mw.p;
-        t.v[k] = (float*)L.vw.p;
-        t.wb[k] = (__nv_bfloat16*)L.wb.p;
-        t.wbt[k] = l > 0 ? (__nv_bfloat16*)L.wbt.p : nullptr;
-        t.cols[k] = L.in;
-        t.rows[k] = L.out;
-        t.start[k + 1] = t.start[k] + nw;
-        ++k;
-        t.w[k] = (float*)L.b.p;
-        t.g[k] = (const float*)L.gb.p;
-        t.m[k] = (float*)L.mb.p;
-        t.v[k] = (float*)L.vb.p;
-        t.wb[k] = nullptr;
-        t.wbt[k] = nullptr;
-        t.cols[k] = L.out;
-        t.rows[k] = 1;
-        t.start[k + 1] = t.start[k] + (uint64_t)L.out;
-        ++k;
-    }
-    t.tensors = k;
-    k_adam_all<<<blocks((t.start[k] + 3) / 4), 256, 0, p->stream>>>(
-        t, (const uint64_t*)p->step_ctr.p, p->cfg.learning_rate, 0.9f, 0.999f, 1e-8f);
-    return cuda_fail(cudaGetLastError(), "proposal update");
-}
-
-// input features of B samples into X[0] (and, for training, the transposed copy XT[0])
-static int pn_features(ndt_pnet* p, int B, const void* pts, const void* scans, bool need_t) {
-    const size_t F = (size_t)p->L[0].in;
-    cudaMemsetAsync(p->X[0].p, 0, (size_t)B * F * 2, p->stream);
-    if (need_t) cudaMemsetAsync(p->XT[0].p, 0, (size_t)B * F * 2, p->stream);
-    k_features<<<dim3(8, B), 256, 0, p->stream>>>(
-        (const float*)pts, (const PnScan*)scans, (const PnSample*)p->smp.p,
-        (const PnMap*)p->maps_d.p, B, (int)F, (__nv_bfloat16*)p->X[0].p,
-        need_t ? (__nv_bfloat16*)p->XT[0].p : nullptr);
+// input features of B samples into X[0]
+static int pn_features(ndt_pnet* p, int B, const void* pts, const void* scans) {
+    k_features<<<B, 256, 0, p->stream>>>((const float*)pts, (const PnScan*)scans,
+                                         (const PnSample*)p->smp.p, (const PnMap*)p->maps_d.p,
+                                         p->L[0].in, (__nv_bfloat16*)p->X[0].p);
     return cuda_fail(cudaGetLastError(), "proposal features");
 }
 
-// One training step on the network's stream: sample a batch (advancing the device step
-// counter), features, forward, loss, backward, Adam. Stream-ordered only, so it can be
-// captured into a graph.
+// One training step on the network's stream (and its side stream, forked and joined within the
+// step): sample a batch (advancing the device step counter), features, forward, loss, backward
+// with the Adam updates. Stream-ordered only, so it can be captured into a graph.
 static int pn_train_step(ndt_pnet* p, int B) {
     cudaStream_t s = p->stream;
-    k_sample<<<1, 256, 0, s>>>(p->cfg.seed, (uint64_t*)p->step_ctr.p, B,
+    k_sample<<<1, 1024, 0, s>>>(p->cfg.seed, (uint64_t*)p->step_ctr.p, B,
                                (uint32_t)p->scans_h.size(), (const PnScan*)p->scans_d.p,
                                (const double*)p->conv_d.p, p->cfg.xy_range, (PnSample*)p->smp.p,
                                (float*)p->T.p);
     int rc;
-    if ((rc = pn_features(p, B, p->scan_pts_d.p, p->scans_d.p, true)) ||
-        (rc = pn_forward(p, B, true)) || (rc = pn_loss(p, B)) || (rc = pn_backward(p, B)) ||
-        (rc = pn_adam(p)))
+    if ((rc = pn_features(p, B, p->scan_pts_d.p, p->scans_d.p)) || (rc = pn_forward(p, B)) ||
+        (rc = pn_loss(p, B)) || (rc = pn_backward(p, B, true)))
         return rc;
     return 0;
 }
@@ -811,6 +782,9 @@ int ndt_pnet_create(const ndt_pnet_config* cfg, int32_t device, ndt_pnet** out) 
     p->cfg = c;
     p->device = device;
     cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking);
+    cudaStreamCreateWithFlags(&p->side, cudaStreamNonBlocking);
+    cudaEventCreateWithFlags(&p->ev_fork, cudaEventDisableTiming);
+    cudaEventCreateWithFlags(&p->ev_join, cudaEventDisableTiming);
     cudaEventCreate(&p->ev0);
     for (auto& e : p->ev_half) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
     cudaEventCreate(&p->ev1);
@@ -829,7 +803,7 @@ int ndt_pnet_create(const ndt_pnet_config* cfg, int32_t device, ndt_pnet** out) 
         L.out = dims[l + 1];
         const size_t nw = (size_t)L.in * L.out;
         if ((rc = dev_reserve(L.w, nw * 4)) || (rc = dev_reserve(L.b, L.out * 4)) ||
-            (rc = dev_reserve(L.wb, nw * 2)) || (rc = dev_reserve(L.wbt, nw * 2)) ||
+            (rc = dev_reserve(L.wb, nw * 2)) ||
             (rc = dev_reserve(L.mw, nw * 4)) || (rc = dev_reserve(L.vw, nw * 4)) ||
             (rc = dev_reserve(L.mb, L.out * 4)) || (rc = dev_reserve(L.vb, L.out * 4)) ||
             (rc = dev_reserve(L.gw, nw * 4)) || (rc = dev_reserve(L.gb, L.out * 4)))
@@ -849,9 +823,8 @@ int ndt_pnet_create(const ndt_pnet_config* cfg, int32_t device, ndt_pnet** out) 
         cudaMemsetAsync(L.vw.p, 0, nw * 4, p->stream);
         cudaMemsetAsync(L.mb.p, 0, L.out * 4, p->stream);
         cudaMemsetAsync(L.vb.p, 0, L.out * 4, p->stream);
-        k_to_bf16<<<blocks(nw), 256, 0, p->stream>>>((const float*)L.w.p, nw, L.in, L.out,
-                                                     (__nv_bfloat16*)L.wb.p,
-                                                     (__nv_bfloat16*)L.wbt.p);
+        k_to_bf16<<<blocks(nw), 256, 0, p->stream>>>((const float*)L.w.p, nw,
+                                                     (__nv_bfloat16*)L.wb.p);
         rc = cuda_fail(cudaStreamSynchronize(p->stream), "proposal network init");
     }
     if (!rc) rc = pn_reserve_batch(p, std::max(c.batch, c.train_batch));
@@ -874,10 +847,11 @@ int ndt_pnet_destroy(ndt_pnet* p) {
     if (!p) return NDT_OK;
     cudaSetDevice(p->device);
     if (p->stream) cudaStreamSynchronize(p->stream);
+    if (p->side) cudaStreamSynchronize(p->side);
     for (auto& L : p->L)
-        for (DevBuf* b : {&L.w, &L.b, &L.wb, &L.wbt, &L.mw, &L.vw, &L.mb, &L.vb, &L.gw, &L.gb})
+        for (DevBuf* b : {&L.w, &L.b, &L.wb, &L.mw, &L.vw, &L.mb, &L.vb, &L.gw, &L.gb})
             dev_free(*b);
-    for (auto* v : {&p->X, &p->XT, &p->Z, &p->dZ, &p->dZT, &p->dZf})
+    for (auto* v : {&p->X, &p->Z, &p->dZ, &p->dZf})
         for (auto& b : *v) dev_free(b);
     for (auto& b : p->map_imgs) dev_free(b);
     for (DevBuf* b : {&p->loss, &p->T, &p->smp, &p->coarse, &p->poses, &p->logits, &p->err,
@@ -893,6 +867,9 @@ int ndt_pnet_destroy(ndt_pnet* p) {
     dev_free(p->step_ctr);
     if (p->ev0) cudaEventDestroy(p->ev0);
     if (p->ev1) cudaEventDestroy(p->ev1);
+    if (p->ev_fork) cudaEventDestroy(p->ev_fork);
+    if (p->ev_join) cudaEventDestroy(p->ev_join);
+    if (p->side) cudaStreamDestroy(p->side);
     if (p->stream) cudaStreamDestroy(p->stream);
     delete p;
     return NDT_OK;
@@ -1071,8 +1048,7 @@ int ndt_pnet_propose(ndt_pnet* p, int32_t map_id, const ndt_scan* q, uint64_t nq
         cudaMemcpyAsync(p->smp.p, smp, B * sizeof(PnSample), cudaMemcpyHostToDevice, s);
         cudaMemcpyAsync(p->coarse.p, coarse, B * 48, cudaMemcpyHostToDevice, s);
         cudaEventRecord(p->ev0, s);
-        if ((rc = pn_features(p, B, p->q_pts.p, p->q_scans.p, false)) ||
-            (rc = pn_forward(p, B, false)))
+        if ((rc = pn_features(p, B, p->q_pts.p, p->q_scans.p)) || (rc = pn_forward(p, B)))
             break;
         k_decode<<<blocks((size_t)B * P), 256, 0, s>>>(
             (const float*)p->Z[p->L.size() - 1].p, (const PnSample*)p->smp.p,
@@ -1111,7 +1087,7 @@ int ndt_pnet_debug_grad(ndt_pnet* p, const float* x, const float* targets, uint6
     const int B = (int)b;
     const size_t F = (size_t)p->L[0].in;
     cudaStream_t s = p->stream;
-    std::vector<uint16_t> xb(B * F), xt(B * F);
+    std::vector<uint16_t> xb(B * F);
     for (int i = 0; i < B; ++i)
         for (size_t f = 0; f < F; ++f) {
             float v = x[(size_t)i * F + f];
@@ -1120,13 +1096,11 @@ int ndt_pnet_debug_grad(ndt_pnet* p, const float* x, const float* targets, uint6
             u += 0x7FFFu + ((u >> 16) & 1u);  // round to nearest even
             const uint16_t h = (uint16_t)(u >> 16);
             xb[(size_t)i * F + f] = h;
-            xt[f * B + i] = h;
         }
     cudaMemcpyAsync(p->X[0].p, xb.data(), xb.size() * 2, cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(p->XT[0].p, xt.data(), xt.size() * 2, cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(p->T.p, targets, (size_t)B * 12, cudaMemcpyHostToDevice, s);
     int rc;
-    if ((rc = pn_forward(p, B, true)) || (rc = pn_loss(p, B)) || (rc = pn_backward(p, B)))
+    if ((rc = pn_forward(p, B)) || (rc = pn_loss(p, B)) || (rc = pn_backward(p, B, false)))
         return rc;
     std::vector<float> lb(B);
     cudaMemcpyAsync(lb.data(), p->loss.p, (size_t)B * 4, cudaMemcpyDeviceToHost, s);
@@ -1164,9 +1138,8 @@ int ndt_pnet_params(ndt_pnet* p, float* out, uint64_t* count, int32_t set) {
         if (set) {
             cudaMemcpyAsync(L.w.p, out + off, nw * 4, cudaMemcpyHostToDevice, p->stream);
             cudaMemcpyAsync(L.b.p, out + off + nw, L.out * 4, cudaMemcpyHostToDevice, p->stream);
-            k_to_bf16<<<blocks(nw), 256, 0, p->stream>>>(
-                (const float*)L.w.p, nw, L.in, L.out, (__nv_bfloat16*)L.wb.p,
-                (__nv_bfloat16*)L.wbt.p);
+            k_to_bf16<<<blocks(nw), 256, 0, p->stream>>>((const float*)L.w.p, nw,
+                                                         (__nv_bfloat16*)L.wb.p);
         } else {
             parts.push_back({L.w.p, (uint64_t)nw * 4});
             parts.push_back({L.b.p, (uint64_t)L.out * 4});

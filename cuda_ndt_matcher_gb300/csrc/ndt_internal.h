@@ -14,25 +14,70 @@
 
 namespace ndtgb {
 
-// Grow-only device allocation owned by a context.
-// Elementwise work fused into the tcgen05 GEMM's epilogue (tc_gemm.cu), per element (row m,
-// column n) of the accumulator acc:
+// One operand of the tcgen05 GEMM: bf16, row-major [rows x K] (K-major) or [K x rows] (MN-major).
+struct GemmOperand {
+    const void* p;
+    int mn_major;
+};
+// A parameter tensor under Adam: f32 master, moments, bf16 copy (weights) and the step count t,
+// a device counter, so that a captured training step replays without host updates.
+struct AdamState {
+    float *w, *m, *v;
+    __nv_bfloat16* wb;
+    const uint64_t* step;
+    float lr, b1, b2, eps;
+};
+#ifdef __CUDACC__
+// lc1 = lr / (1 - b1^t), ic2 = 1 / (1 - b2^t)
+__device__ __forceinline__ void adam_update(const AdamState& a, float g, float& m, float& v,
+                                            float& w, float lc1, float ic2) {
+    // the contractions are spelled out: moments and weights must not depend on what else the
+    // compiler finds in the kernel around them
+    const float mi = __fmaf_rn(a.b1, m, __fmul_rn(1.f - a.b1, g));
+    const float vi = __fmaf_rn(a.b2, v, __fmul_rn(__fmul_rn(1.f - a.b2, g), g));
+    m = mi;
+    v = vi;
+    w -= lc1 * mi / (sqrtf(vi * ic2) + a.eps);
+}
+__device__ __forceinline__ void adam_corrections(const AdamState& a, float* out) {
+    const float step = (float)*a.step;
+    out[0] = a.lr / (1.f - powf(a.b1, step));
+    out[1] = 1.f / (1.f - powf(a.b2, step));
+}
+#endif
+// Work fused into the tcgen05 GEMM's epilogue (tc_gemm.cu), per element (row m, column n) of the
+// accumulator acc:
 //   GEMM_EPI_STORE        D = acc
-//   GEMM_EPI_BIAS_GELU    z = acc + bias[n]: D = z, x = GELU(z) as bf16 into x [M x N] and
-//                         xt [N x M] (the next layer's input in both operand layouts)
+//   GEMM_EPI_BIAS_GELU    z = acc + bias[n]: D = z, x = GELU(z) as bf16 into x [M x N] (the next
+//                         layer's input)
 //   GEMM_EPI_BIAS         z = acc + bias[n]: D = z (the output layer)
-//   GEMM_EPI_GELU_BACK    g = acc * GELU'(zin[m][n]): D = g, bf16 g into x [M x N] and
-//                         xt [N x M] (the previous layer's output gradient)
+//   GEMM_EPI_GELU_BACK    g = acc * GELU'(zin[m][n]): D = g, bf16 g into x [M x N] (the
+//                         previous layer's output gradient)
 // Not with split-K (a partial product has no bias and no activation).
-enum { GEMM_EPI_STORE = 0, GEMM_EPI_BIAS_GELU = 1, GEMM_EPI_BIAS = 2, GEMM_EPI_GELU_BACK = 3 };
+enum {
+    GEMM_EPI_STORE = 0,
+    GEMM_EPI_BIAS_GELU = 1,
+    GEMM_EPI_BIAS = 2,
+    GEMM_EPI_GELU_BACK = 3
+};
 struct GemmEpilogue {
     int mode;
     const float* bias;
     const float* zin;
     __nv_bfloat16* x;
-    __nv_bfloat16* xt;
 };
+// A weight [m x n] and the operands of its gradient, a [k x m] and b [k x n]
+struct GemmAdam {
+    const void *a, *b;
+    int m, n;
+    AdamState st;
+};
+constexpr int GEMM_ADAM_MAX = 16;
+int gemm_adam(const GemmAdam* w, int count, int k, uint32_t* d_err, cudaStream_t s);
+int gemm_bf16(GemmOperand A, GemmOperand B, float* D, int M, int N, int K, int ldd,
+              uint32_t* d_err, cudaStream_t s, int splits, const GemmEpilogue* epi);
 
+// Grow-only device allocation owned by a context.
 struct DevBuf {
     void* p = nullptr;
     size_t bytes = 0;
