@@ -172,6 +172,7 @@ struct ndt_ctx {
         float seg_ratio = 0.f;
     };
     std::vector<Tile> tiles;
+    Tile spare{};            // buffers of the last removed tile, for the next new one
     Map map_b;
     BuildScratch bs_b, bs_tile;
     DevBuf d_gather, d_status_b, d_tile_refs;
@@ -203,13 +204,14 @@ static int score_reserve(ndt_ctx* c, uint32_t nj, uint32_t max_n) {
                      "score counters");
 }
 
-// Finishes a background rebuild: joins its thread and, when it succeeded, makes the standby
-// map the active one (alignment work on the old map has completed: every call synchronises,
-// and asynchronous batches are drained first).
-static void tiles_settle(ndt_ctx* c, bool wait) {
-    if (!c->builder.joinable()) return;
-    if (!wait && c->build_state.load() != 2) return;
-    c->builder.join();
+static void tile_free(ndt_ctx::Tile& t) {
+    for (DevBuf* b : {&t.pts, &t.segs.idx, &t.segs.starts, &t.segs.rec, &t.segs.valid})
+        dev_free(*b);
+}
+
+// After a rebuild: when it succeeded, the standby map becomes the active one (alignment work on
+// the old map has completed: every call synchronises, and asynchronous batches are drained first).
+static void tiles_adopt(ndt_ctx* c) {
     c->build_state.store(0);
     if (c->build_rc == 0) {
         async_drain(c);
@@ -219,6 +221,14 @@ static void tiles_settle(ndt_ctx* c, bool wait) {
         c->stats.build_launches++;
         c->stats.build_ms += c->build_ms_b;
     }
+}
+
+// Finishes a background rebuild: joins its thread and adopts its map.
+static void tiles_settle(ndt_ctx* c, bool wait) {
+    if (!c->builder.joinable()) return;
+    if (!wait && c->build_state.load() != 2) return;
+    c->builder.join();
+    tiles_adopt(c);
 }
 
 // Packs host scans into the pinned staging buffer with the context's host threads and copies
@@ -443,9 +453,8 @@ int ndt_ctx_destroy(ndt_ctx* c) {
     if (c->stream) cudaStreamSynchronize(c->stream);
     if (c->cstream) cudaStreamSynchronize(c->cstream);
     if (c->builder.joinable()) c->builder.join();
-    for (auto& t : c->tiles)
-        for (DevBuf* b : {&t.pts, &t.segs.idx, &t.segs.starts, &t.segs.rec, &t.segs.valid})
-            dev_free(*b);
+    for (auto& t : c->tiles) tile_free(t);
+    tile_free(c->spare);
     for (DevBuf* b : {&c->bs_tile.keys_a, &c->bs_tile.keys_b, &c->bs_tile.vals_a,
                       &c->bs_tile.vals_b, &c->bs_tile.tmp, &c->bs_tile.seg_ids,
                       &c->bs_tile.seg_starts, &c->bs_tile.seg_valid, &c->bs_tile.seg_rank,
@@ -632,17 +641,24 @@ int ndt_tile_put(ndt_ctx* c, uint64_t tile_id, const float* xyz, uint64_t n) {
     if (t) {
         tiles_settle(c, true);  // a running merge reads this tile's buffers
     } else {
-        c->tiles.push_back(ndt_ctx::Tile{});
+        // a new tile, in the last removed one's buffers
+        ndt_ctx::Tile fresh{};
+        fresh.id = tile_id;
+        fresh.pts = c->spare.pts;
+        fresh.segs = c->spare.segs;
+        fresh.segs.geo = SegGeometry{};
+        c->spare = ndt_ctx::Tile{};
+        c->tiles.push_back(fresh);
         t = &c->tiles.back();
-        t->id = tile_id;
     }
     int rc = dev_reserve(t->pts, n * 12);
     if (rc) return rc;
     t->n = n;
     cudaMemcpyAsync(t->pts.p, xyz, n * 12, cudaMemcpyHostToDevice, c->bstream);
     c->stats.h2d_bytes += n * 12;
-    if ((rc = cuda_fail(cudaStreamSynchronize(c->bstream), "tile upload"))) return rc;
-    return tile_segments(c, *t);
+    // (the segments' build waits for the stream: the caller's array is free on return)
+    if ((rc = tile_segments(c, *t))) cudaStreamSynchronize(c->bstream);
+    return rc;
 }
 
 int ndt_tile_remove(ndt_ctx* c, uint64_t tile_id) {
@@ -650,9 +666,10 @@ int ndt_tile_remove(ndt_ctx* c, uint64_t tile_id) {
     for (size_t i = 0; i < c->tiles.size(); ++i)
         if (c->tiles[i].id == tile_id) {
             tiles_settle(c, true);  // a running merge reads the tile's buffers
-            ndt_ctx::Tile& t = c->tiles[i];
-            for (DevBuf* b : {&t.pts, &t.segs.idx, &t.segs.starts, &t.segs.rec, &t.segs.valid})
-                dev_free(*b);
+            // its buffers wait for the next put (one tile's at most are kept): five cudaFree and
+            // five cudaMalloc cost a tile that follows the vehicle about 170 us
+            tile_free(c->spare);
+            c->spare = c->tiles[i];
             c->tiles.erase(c->tiles.begin() + (long)i);
             return NDT_OK;
         }
@@ -698,7 +715,7 @@ int ndt_tiles_commit(ndt_ctx* c, int32_t wait) {
     }
     c->build_state.store(1);
     const ndt_config cfg = c->cfg;
-    c->builder = std::thread([c, refs, cfg]() {
+    auto rebuild = [c, refs, cfg]() {
         cudaSetDevice(c->device);
         float ms = 0.f;
         int r = merge_tiles(c->map_b, c->bs_b, refs, c->d_tile_refs, cfg,
@@ -715,9 +732,12 @@ int ndt_tiles_commit(ndt_ctx* c, int32_t wait) {
         c->build_ms_b = ms;
         c->build_err = r ? std::string(ndt_last_error_string()) : std::string();
         c->build_state.store(2);
-    });
-    if (wait) {
-        tiles_settle(c, true);
+    };
+    if (!wait) {
+        c->builder = std::thread(rebuild);
+    } else {  // here and now: starting and joining a thread takes about 60 us
+        rebuild();
+        tiles_adopt(c);
         if (c->build_rc) {
             set_error(c->build_err);
             return c->build_rc;
