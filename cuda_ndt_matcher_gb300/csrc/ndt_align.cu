@@ -2713,7 +2713,7 @@ struct FewShared {
     unsigned long long cyc[4];
 };
 
-// A word of the exchange: a 32-bit value and the iteration it belongs to (from 1), read and
+// A word of the exchange: a 32-bit value and the iteration it belongs to (FewCta), read and
 // written whole (64 bits), so a reader that finds the iteration has the value: no fence and no
 // second read behind a flag (each about 700 cycles of L2 latency).
 __device__ __forceinline__ unsigned long long few_word(uint32_t it, uint32_t v) {
@@ -2763,7 +2763,7 @@ __device__ __forceinline__ void few_publish(FewJob* fj, const float* fr, uint32_
 // next step reads. Returns 1 (every lane) when the alignment is finished.
 template <bool CPU_SEM>
 __device__ __noinline__ int few_control(const AlignParams& P, CtlShared& ctl, FewJob* fj, int job,
-                                        int it, int lane) {
+                                        int it, uint32_t tag, int lane) {
     finalize_gH(ctl.tot, ctl.Ad, ctl.Bd, ctl.g, ctl.H, lane);
     __syncwarp();
     solve_warp<CPU_SEM>(ctl.H, ctl.g, ctl.solve, lane);
@@ -2785,7 +2785,7 @@ __device__ __noinline__ int few_control(const AlignParams& P, CtlShared& ctl, Fe
         }
     }
     if (!done) frame_first(ctl.pose, CPU_SEM, ctl.fr, ctl.trig, ctl.Ad, lane);
-    few_publish(fj, ctl.fr, (uint32_t)(it + 1), done != 0, lane);
+    few_publish(fj, ctl.fr, tag + (uint32_t)(it + 1), done != 0, lane);
     return done;
 }
 
@@ -2929,7 +2929,7 @@ __global__ void __launch_bounds__(FT, 1) k_ndt_few(const AlignParams P) {
             if (tid < NRED)
                 for (int w = 0; w < no; ++w) sum += sh.wpart[w][tid];
         }
-        const uint32_t now = (uint32_t)(it + 1);
+        const uint32_t now = me_cta.tag + (uint32_t)(it + 1);
         if (tid < NRED) {
             const unsigned long long b = (unsigned long long)__double_as_longlong(sum);
             few_put2(part + (size_t)r * NRED + tid, few_word(now, (uint32_t)b),
@@ -2972,7 +2972,8 @@ __global__ void __launch_bounds__(FT, 1) k_ndt_few(const AlignParams P) {
                 }
                 __syncthreads();
                 if (warp == 0) {
-                    const int done = few_control<CPU_SEM>(P, sh.ctl, fj, job, it, lane);
+                    const int done = few_control<CPU_SEM>(P, sh.ctl, fj, job, it, me_cta.tag,
+                                                          lane);
                     for (int i = lane; i < NFR; i += 32) sh.fr[i] = sh.ctl.fr[i];
                     if (lane == 0) {
                         const unsigned long long c3 = clock64();
@@ -3029,8 +3030,6 @@ static cudaError_t launch_few_k(const AlignParams& p, size_t smem, cudaStream_t 
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
     if (e != cudaSuccess) return e;
-    // the exchange words: no iteration there yet
-    cudaMemsetAsync(p.few, 0, few_bytes(p.num_jobs, p.qgrid), s);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(p.qgrid, 1, 1);
     cfg.blockDim = dim3(FT, 1, 1);
@@ -3077,7 +3076,7 @@ bool few_share(const uint32_t* n, uint32_t jobs, int ranks, int threads, int sms
     for (uint32_t j = 0; j < jobs; ++j) {
         const uint32_t own = (units[j] + ctas[j] - 1) / ctas[j];
         const uint32_t g = (units[j] + own - 1) / own;  // CTAs with work
-        for (uint32_t r = 0; r < g; ++r) out.push_back(FewCta{j, r, g, own});
+        for (uint32_t r = 0; r < g; ++r) out.push_back(FewCta{j, r, g, own, 0u, {}});
     }
     return true;
 }

@@ -145,7 +145,8 @@ struct ndt_ctx {
     bool trace = false;
     DevBuf d_trace;
     DevBuf d_qjobs, d_qctl, d_qframe, d_qpart;          // work-queue kernel
-    DevBuf d_few;                                       // few-alignments kernel
+    DevBuf d_few;                                       // few-alignments kernel's exchange words,
+    uint32_t few_tag = 0;                               // and the last launch's last tag
     std::vector<double> h_trace;       // last call's records, by job order
     std::vector<uint32_t> trace_slot;  // job index -> caller's result index
     int trace_iters = 0;
@@ -843,6 +844,7 @@ static int queue_units(int threads) { return std::min<int>(QUNITS, threads / 32)
 constexpr uint64_t FEW_POINTS_PER_SM = 500;
 constexpr uint32_t FEW_JOBS = 8;
 constexpr uint64_t FEW_POINTS = 1ull << 26;
+constexpr uint64_t FEW_INLINE_POINTS = 32768;
 
 static LaunchShape choose_shape(ndt_ctx* c, uint32_t jobs, uint32_t max_n, uint64_t total) {
     LaunchShape sh{0, 0, 128, 0};
@@ -1042,15 +1044,36 @@ static int run_align_enqueue(ndt_ctx* c, const float* d_pts, std::vector<AlignJo
         std::vector<FewCta> ctas;
         for (uint32_t j = 0; j < nj; ++j) sizes[j] = jobs[j].n;
         few_share(sizes.data(), nj, shape.ranks, shape.threads, c->num_sms, ctas);
-        qob = (size_t)c->num_sms * sizeof(FewCta);
+        const uint32_t tags = (uint32_t)c->cfg.max_iterations + 1;
+        const size_t few_size = few_bytes(nj, (uint32_t)c->num_sms);
+        if (few_size > c->d_few.bytes || c->few_tag > 0xFFFFFFFFu - tags) {
+            if ((rc = dev_reserve(c->d_few, few_size))) return rc;
+            cudaMemsetAsync(c->d_few.p, 0, c->d_few.bytes, st);
+            c->few_tag = 0;
+        }
+        for (auto& f : ctas) f.tag = c->few_tag;
+        c->few_tag += tags;
         const size_t at = (jb + sjb + 15) & ~(size_t)15;  // the table's place in the block
-        qob += at - (jb + sjb);
-        if ((rc = pin_reserve(c->h_jobs, jb + sjb + qob)) ||
-            (rc = dev_reserve(c->d_jobs, jb + sjb + qob)) ||
-            (rc = dev_reserve(c->d_few, few_bytes(nj, (uint32_t)c->num_sms))))
-            return rc;
+        size_t end = at + (size_t)c->num_sms * sizeof(FewCta);
+        // the points of a small call go in with the tables: a copy of its own costs it about 6 us
+        // (not under a graph, which is kept by the block's size)
+        const size_t pts_at = end;
+        const bool pts_in = plan && plan->total <= FEW_INLINE_POINTS && !c->cfg.cuda_graph;
+        if (pts_in) end += plan->total * 12 + 16;
+        qob = end - (jb + sjb);
+        if ((rc = pin_reserve(c->h_jobs, end)) || (rc = dev_reserve(c->d_jobs, end))) return rc;
         fill_jobs();  // the block may have moved
         std::memcpy((char*)c->h_jobs.p + at, ctas.data(), ctas.size() * sizeof(FewCta));
+        if (pts_in) {
+            for (const AlignJob& j : jobs)
+                if (j.n)
+                    std::memcpy((char*)c->h_jobs.p + pts_at + j.offset * 12,
+                                plan->scans[j.slot].xyz, (size_t)j.n * 12);
+            d_pts = (const float*)((char*)c->d_jobs.p + pts_at);
+            p.pts = d_pts;
+            c->stats.h2d_bytes += plan->total * 12;
+            plan = nullptr;
+        }
         p.jobs = (const AlignJob*)c->d_jobs.p;
         p.few = (FewJob*)c->d_few.p;
         p.few_ctas = (const FewCta*)((char*)c->d_jobs.p + at);

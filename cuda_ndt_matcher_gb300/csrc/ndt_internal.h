@@ -295,9 +295,11 @@ struct FewJob {
 };
 size_t few_bytes(uint32_t jobs, uint32_t ctas);
 // A CTA of the few-alignments kernel: its alignment (launch order), its rank among the
-// alignment's CTAs, their number, and the partition warps each takes
+// alignment's CTAs, their number, and the partition warps each takes. tag + 1, tag + 2, ... mark
+// the exchange words of the launch's iterations: values that no earlier launch on the same
+// words has used, so they need no clearing between launches.
 struct FewCta {
-    uint32_t job, rank, ctas, owners;
+    uint32_t job, rank, ctas, owners, tag, pad[3];
 };
 bool few_share(const uint32_t* n, uint32_t jobs, int ranks, int threads, int sms,
                std::vector<FewCta>& out);
