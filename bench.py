@@ -168,32 +168,29 @@ class ClockSampler:
 
 def build_bytes(info):
     """Algorithmic DRAM bytes of one map build as the pipeline runs it (set_target):
-    per point: bounds pass (12 B read), key pass (12 B read, key + index written), one
-    histogram read and one key+value read and write per 8-bit radix pass over the significant
-    key bits (32-bit keys when 3 x max key bits + 1 <= 32, else 64-bit), two key reads for the
+    per point: bounds pass (12 B read), key pass (12 B read, 4 B key written, first digit
+    counted), first sort pass (key read, key and position written), each further pass of up to 8
+    key bits (key read for the counts, key and position read and written), one key read for the
     segment starts, and the statistics' index and point gather (16 B); per segment: its start,
-    size key and visit order, the two 16-bit size-sort passes, its record (88 B) and validity;
-    per voxel: the record read back, the voxel arrays written (104 B), the hash insert's
-    reads (64 B) and slot writes (52 B); per slot: the 16 B clear; the dense index: one clear
-    and one fill of 16 B per cell; the neighbourhood masks (4 B each, one or eight per cell of
-    the grown box): one clear, and one write-back of the words the voxels' atomic ORs set in
-    L2."""
+    size key and visit order with their sort pass, its record (88 B) and validity; per voxel: the
+    record read back, the voxel arrays (104 B), the search record (32 B) and its hash key; per
+    slot: the clear (4 B with the dense index, else 16); the dense index: one clear and one fill of
+    16 B per cell; the neighbourhood masks: written once when gathered (one per octant), cleared
+    and written back when scattered (one per cell). (Maps of 2^30 points and more sort 64-bit
+    keys; not counted here.)"""
     n, S, V, cap = (int(info.num_points), int(info.num_segments), int(info.num_voxels),
                     int(info.hash_capacity))
-    lv = max(int(b) for b in info.key_bits)
-    end_bit = min(64, 3 * lv + 1)
-    kw = 4 if end_bit <= 32 else 8
-    passes = (end_bit + 7) // 8
-    per_point = 12 + 12 + kw + 4 + passes * (kw + 2 * (kw + 4)) + 2 * kw + 16
-    per_seg = 4 + 8 + 2 * 3 * 8 + 88 + 4
-    per_vox = 88 + 104 + 64 + 52
-    # dense index: the grid (16 B per cell of the box: cleared, then filled) and the
-    # neighbourhood masks (the rest of dense_grid_mib: cleared, then written back)
+    passes = max(1, (sum(int(b) for b in info.key_bits) + 7) // 8)
+    per_point = 12 + 12 + 4 + 12 + 20 * (passes - 1) + 4 + 16
+    per_seg = 4 + 4 + 4 + 4 + 8 + 12 + 88 + 4
+    per_vox = 88 + 104 + 32 + 8
+    # dense index: the grid (16 B per cell of the box) and the masks (the rest of dense_grid_mib)
     dense = float(info.dense_grid_mib) * 1024 * 1024
     cells = float(np.prod([int(info.max_coord[a]) - int(info.min_coord[a]) + 1
                            for a in range(3)])) if dense > 0 else 0.0
-    grid_bytes = 2 * 16 * cells + 2 * max(dense - 16 * cells, 0.0)
-    return int(per_point * n + per_seg * S + per_vox * V + 16 * cap + grid_bytes)
+    masks = max(dense - 16 * cells, 0.0) * (1 if int(info.masks_per_cell) > 1 else 2)
+    return int(per_point * n + per_seg * S + per_vox * V + (4 if dense > 0 else 16) * cap
+               + 2 * 16 * cells + masks)
 
 
 def peaks():
@@ -409,7 +406,7 @@ def learned_bench(steps=15000, n_maps=50, n_train=400, n_test=200, nvtl_tol=0.01
                         "seconds": train_s,
                         "device_ms": nst["train_ms"], "prep_seconds": prep,
                         "final_loss": float(loss.mean()),
-                        "roofline": {"bound": "tensor", "kernel": "k_gemm_bf16_tn (training step)",
+                        "roofline": {"bound": "tensor", "kernel": "k_gemm_bf16, k_gemm_adam (training step)",
                                      "achieved": flops_step * steps / (nst["train_ms"] / 1e3) / 1e12,
                                      "peak": peaks()[0].get("bf16_tflops_sustained"),
                                      "unit": "TFLOP/s",

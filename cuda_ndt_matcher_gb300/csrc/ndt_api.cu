@@ -3,7 +3,7 @@
 // A context owns one CUDA stream, the device voxel map, grow-only device buffers, pinned
 // host staging buffers and a few host threads. An alignment call packs the host scans into
 // pinned memory with those threads, copying each packed chunk to the device while the next
-// is packed, launches the Newton kernel (one cluster per alignment, longest scans first) and
+// is packed, launches a Newton kernel (choose_shape; longest scans first) and
 // the NVTL kernel on the final poses (as a CUDA graph when configured), copies the
 // per-alignment records back and synchronises once.
 #include <algorithm>
@@ -1080,7 +1080,6 @@ static int run_align_enqueue(ndt_ctx* c, const float* d_pts, std::vector<AlignJo
         p.qgrid = (uint32_t)ctas.size();
     }
     AlignOut* ho = (AlignOut*)c->h_aout.p;
-    ScoreOut* hso = (ScoreOut*)((char*)c->h_aout.p + ob);
     uint32_t* hst = (uint32_t*)((char*)c->h_aout.p + ob + sob);
     // host batch copied in during the launch: the kernel reads the resident-point count from
     // word 3 of the status block (32-bit: the batch holds fewer than 2^32 points)

@@ -277,7 +277,7 @@ struct QJob {
     // iteration << 48 | the iteration's chunk count << 32 | chunks claimed (iteration QDONE:
     // the alignment is finished)
     unsigned long long gen_claim;
-    uint32_t done;                 // chunks of the current iteration finished
+    uint32_t done;                 // chunks of the current iteration finished, and the step before
     uint32_t pad;
 };
 constexpr uint32_t QDONE = 0xFFFFu;
