@@ -2176,11 +2176,13 @@ __device__ __noinline__ int queue_control(const AlignParams& P, CtlShared& sh, i
 }
 
 constexpr int QT = 256;          // threads per CTA
-constexpr int QSLOTS = 4;        // chunks a CTA has in hand
+constexpr int QSLOTS = 2;        // chunks a CTA has in hand
 constexpr int QCTLS = 2;         // Newton steps a CTA runs at a time
-// From the iteration QLATE on (the lowest to claim) a CTA that runs a step claims nothing: its
-// chunk would wait for the stepping warp's share, and late in a batch there are free CTAs. 256
-// scans of up to 30 iterations 3,396 -> 3,322 us; from 0 on 3,330, from 10 on 3,364.
+// From the iteration QLATE on (the lowest to claim) a CTA with a chunk in hand or a step to run
+// claims nothing: late in a batch there are free CTAs, and a chunk claimed by a busy one waits for
+// warps. 256 scans of 20k points, up to 30 iterations: 3,396 us without the rule, 3,051 with it
+// (from 3 on 3,108, from 6 on 3,066; only CTAs with a step 3,227); up to 5 iterations 1,312 and
+// 1,300. Four chunks in hand instead of two: 3,104.
 constexpr uint32_t QLATE = 5;
 constexpr int QREADY = 16;        // more than the alignments a CTA can have in hand
 constexpr uint32_t QSTAY = 152;  // CTAs that stay to the end of a batch: one per SM
@@ -2288,9 +2290,13 @@ __device__ __forceinline__ int queue_claim(const AlignParams& P, QShared& q, int
         if (first_open < 0 && om) first_open = (int)base + __ffs(om) - 1;
     }
     best = __reduce_min_sync(0xffffffffu, best);
-    // late in a batch a CTA that runs a step leaves the chunks to the others
-    if (best != 0xFFFFFFFFu && (best >> 24) >= QLATE && ld_shared_volatile(&q.ctl_busy) != 0u)
-        best = 0xFFFFFFFFu;
+    // late in a batch a CTA with a chunk in hand or a step leaves the chunks to the others
+    if (best != 0xFFFFFFFFu && (best >> 24) >= QLATE) {
+        bool busy = ld_shared_volatile(&q.ctl_busy) != 0u;
+        for (int i = 0; i < QSLOTS; ++i)
+            busy |= *reinterpret_cast<const volatile int*>(&q.slot[i].busy) != 0;
+        if (busy) best = 0xFFFFFFFFu;
+    }
     for (int pass = 1; pass <= 2 && job < 0 && best != 0xFFFFFFFFu; ++pass) {
         const uint32_t gsel = best >> 24;
         const uint32_t start =
@@ -2352,7 +2358,7 @@ __device__ __forceinline__ bool queue_idle(const AlignParams& P, QShared& q) {
     } else if (now - q.idle_since > P.stall_ns) {
         atomicOr(P.status, ST_QUEUE_STALL);
         return true;
-    } else if (fed && blockIdx.x >= QSTAY && now - q.idle_since > 20000ull) {
+    } else if (fed && !P.qstay && blockIdx.x >= QSTAY && now - q.idle_since > 20000ull) {
         // near the end of a batch: all but the first QSTAY CTAs leave after 20 us without
         // work, so a kernel queued on another stream (the next asynchronous batch) can take
         // their SMs; those that stay serve the remaining iterations

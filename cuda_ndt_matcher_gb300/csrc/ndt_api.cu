@@ -1094,6 +1094,10 @@ static int run_align_enqueue(ndt_ctx* c, const float* d_pts, std::vector<AlignJo
         d_arrive = (uint32_t*)c->d_status.p + 3;
         p.qarrive = d_arrive;
         p.qarrive_total = (uint32_t)plan->total;
+        // a call that waits keeps every CTA for the scans still to come; an asynchronous batch
+        // leaves SMs to the next one: 256 x 20k points 65.6k against 68.0k aligns/s waiting, two
+        // asynchronous batches in flight 83k against 75k
+        p.qstay = c->borrowed_map ? 0 : 1;
         p.qsolo = 0;
     }
     // the batch on the stream: job tables in, Newton kernel, NVTL scoring, results out (the

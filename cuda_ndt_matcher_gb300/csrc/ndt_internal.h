@@ -243,6 +243,7 @@ struct AlignParams {
     ulonglong2* few_part;   // (set by the launch)
     const struct FewCta* few_ctas;  // qgrid CTAs
     uint64_t qunits_total;  // units of one iteration of every alignment (early iterations)
+    int32_t qstay;          // idle CTAs stay to the end of the batch
     int32_t qsolo;          // every iteration of every alignment is one chunk, and all points
                             // are resident: CTAs keep their alignments
     uint32_t qgrid;         // CTAs of the launch
