@@ -1916,6 +1916,7 @@ __global__ void __launch_bounds__(128) k_queue_init(const AlignParams P) {
         // withhold (test hook): every chunk of the first iteration already claimed
         P.qjobs[j].gen_claim = qword(0u, nch0) | (P.withhold ? (unsigned long long)nch0 : 0ull);
         P.qjobs[j].done = 1u;  // the step before the first iteration: there
+        P.out[j].status = ALIGN_NOT_FINISHED;
     }
 }
 
@@ -2217,6 +2218,9 @@ struct QShared {
     // read by the claiming warp
     unsigned long long ready[QREADY];
     unsigned int ready_put, ready_get;
+    // P.qsolo: alignments that this CTA has taken and not finished. Only the claiming warp adds,
+    // so while it holds the claim the count can only fall: at zero the CTA has nothing left.
+    unsigned int kept;
     QSlot slot[QSLOTS];
     CtlShared ctl[QCTLS];
 };
@@ -2249,10 +2253,12 @@ __device__ __forceinline__ int queue_claim(const AlignParams& P, QShared& q, int
                 q.ready_get++;
             } else if (q.lw == 0) {
                 const uint32_t j = atomicAdd(P.qcount, 1u);
-                if (j < B)
+                if (j < B) {
                     w = (unsigned long long)j + 1ull;
-                else
+                    atomicAdd(&q.kept, 1u);
+                } else {
                     q.lw = (int)B;
+                }
             }
         }
         w = __shfl_sync(0xffffffffu, w, 0);
@@ -2332,14 +2338,15 @@ __device__ __forceinline__ int queue_claim(const AlignParams& P, QShared& q, int
 // Nothing to claim (lane 0 of the claiming warp): every alignment finished, or the open ones
 // wait for their Newton step. True when the CTA should leave.
 __device__ __forceinline__ bool queue_idle(const AlignParams& P, QShared& q) {
-    // a warp of this CTA still sums or steps: its alignment's next chunks may be this CTA's
-    bool active = ld_shared_volatile(&q.ctl_busy) != 0u;
+    const bool keeps = P.qsolo && ld_shared_volatile(&q.kept) != 0u;
+    if (q.lw >= (int)P.num_jobs && !keeps) return true;
+    // a warp of this CTA still sums or steps: its alignment's next chunks may be this CTA's. (A
+    // warp that ends a chunk enters ctl_busy before it releases the slot: slots first, here too.)
+    bool active = false;
     for (int i = 0; i < QSLOTS; ++i)
         active |= *reinterpret_cast<const volatile int*>(&q.slot[i].busy) != 0;
-    if (q.lw >= (int)P.num_jobs &&
-        !(P.qsolo && (active || *reinterpret_cast<const volatile unsigned long long*>(
-                                    &q.ready[q.ready_get % QREADY]) != 0ull)))
-        return true;
+    __threadfence_block();
+    active |= ld_shared_volatile(&q.ctl_busy) != 0u;
     const unsigned long long now = global_ns();
     bool fed = true;  // every point of the batch is resident
     if (P.qarrive) {
@@ -2358,7 +2365,8 @@ __device__ __forceinline__ bool queue_idle(const AlignParams& P, QShared& q) {
     } else if (now - q.idle_since > P.stall_ns) {
         atomicOr(P.status, ST_QUEUE_STALL);
         return true;
-    } else if (fed && !P.qstay && blockIdx.x >= QSTAY && now - q.idle_since > 20000ull) {
+    } else if (fed && !keeps && !P.qstay && blockIdx.x >= QSTAY &&
+               now - q.idle_since > 20000ull) {
         // near the end of a batch: all but the first QSTAY CTAs leave after 20 us without
         // work, so a kernel queued on another stream (the next asynchronous batch) can take
         // their SMs; those that stay serve the remaining iterations
@@ -2441,7 +2449,7 @@ __global__ void __launch_bounds__(QT, 65536 / (QT * REGCAP)) k_ndt_queue(const A
     if (tid == 0) {
         q.head = 0;
         q.claiming = q.exit_ = q.ctl_busy = 0;
-        q.ready_put = q.ready_get = 0;
+        q.ready_put = q.ready_get = q.kept = 0;
         for (int i = 0; i < QREADY; ++i) q.ready[i] = 0ull;
         q.lw = 0;
         q.idle_since = 0;
@@ -2632,7 +2640,9 @@ __global__ void __launch_bounds__(QT, 65536 / (QT * REGCAP)) k_ndt_queue(const A
         __threadfence_block();
         __syncwarp();
         if (lane == 0) {
-            if (P.qsolo && !done) {
+            if (P.qsolo && done) {
+                atomicSub(&q.kept, 1u);  // (its outputs are written)
+            } else if (P.qsolo) {
                 const unsigned int e = atomicAdd(&q.ready_put, 1u) % QREADY;
                 atomicExch(&q.ready[e], (unsigned long long)(gen + 1u) << 32 |
                                             (unsigned long long)((uint32_t)job + 1u));

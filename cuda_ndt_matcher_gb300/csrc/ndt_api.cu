@@ -1224,7 +1224,13 @@ static int run_align_finish(ndt_ctx* c, ndt_result* out) {
     c->stats.score_launches++;
     c->stats.score_kernel_ms += sms;
     uint64_t t0 = UINT64_MAX;
-    for (uint32_t j = 0; j < nj; ++j) t0 = std::min(t0, ho[j].t_start);
+    for (uint32_t j = 0; j < nj; ++j) {
+        if (ho[j].status == ALIGN_NOT_FINISHED) {
+            set_error("an alignment of the batch was not finished");
+            return NDT_ERR_DEVICE;
+        }
+        t0 = std::min(t0, ho[j].t_start);
+    }
     c->t_start_ms.assign(nj, 0.0);
     c->t_finish_ms.assign(nj, 0.0);
     for (uint32_t j = 0; j < nj; ++j) {

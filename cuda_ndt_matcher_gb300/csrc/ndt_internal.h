@@ -194,6 +194,8 @@ struct AlignOut {
     int32_t pad2;
     uint64_t t_start, t_end;  // global timer (ns) when the alignment started / finished
 };
+// AlignOut::status of an alignment that the work-queue kernel has not finished
+constexpr int32_t ALIGN_NOT_FINISHED = -1;
 
 // Per-iteration trace record (doubles): it, score, correspondences, pose before the step (6),
 // gradient (6), Hessian upper triangle (21), raw solver output (6), solver path, solver ok,
