@@ -2298,10 +2298,13 @@ __device__ __forceinline__ int queue_claim(const AlignParams& P, QShared& q, int
     best = __reduce_min_sync(0xffffffffu, best);
     // late in a batch a CTA with a chunk in hand or a step leaves the chunks to the others
     if (best != 0xFFFFFFFFu && (best >> 24) >= QLATE) {
-        bool busy = ld_shared_volatile(&q.ctl_busy) != 0u;
-        for (int i = 0; i < QSLOTS; ++i)
-            busy |= *reinterpret_cast<const volatile int*>(&q.slot[i].busy) != 0;
-        if (busy) best = 0xFFFFFFFFu;
+        bool busy = false;
+        if (lane == 0) {
+            busy = ld_shared_volatile(&q.ctl_busy) != 0u;
+            for (int i = 0; i < QSLOTS; ++i)
+                busy |= *reinterpret_cast<const volatile int*>(&q.slot[i].busy) != 0;
+        }
+        if (__shfl_sync(0xffffffffu, (int)busy, 0)) best = 0xFFFFFFFFu;
     }
     for (int pass = 1; pass <= 2 && job < 0 && best != 0xFFFFFFFFu; ++pass) {
         const uint32_t gsel = best >> 24;
@@ -2456,56 +2459,69 @@ __global__ void __launch_bounds__(QT, 65536 / (QT * REGCAP)) k_ndt_queue(const A
         q.seen_arrive = 0;
     }
     __syncthreads();
+    // What other warps write (head, left, exit_, claiming, a slot's busy flag, the areas) lane 0
+    // alone reads, and the warp acts on its reading: nothing keeps 32 lanes' readings of such a
+    // word alike, nor the lanes together after a branch that depends on one.
     for (;;) {
         // a unit of the open chunk: one atomic on the count of units left names it or shows the
         // chunk exhausted (should the slot have been refilled since `head` was read, the unit
         // is one of the chunk that it holds now, which is as good)
-        const unsigned int head = ld_shared_volatile(&q.head);
-        QSlot& c = q.slot[head % QSLOTS];
+        unsigned int head = 0;
         int left = 0;
-        if (lane == 0 && *reinterpret_cast<const volatile int*>(&c.left) > 0)
-            left = atomicSub(&c.left, 1);
+        if (lane == 0) {
+            head = ld_shared_volatile(&q.head);
+            int* const l = &q.slot[head % QSLOTS].left;
+            if (*reinterpret_cast<const volatile int*>(l) > 0) left = atomicSub(l, 1);
+            __threadfence_block();
+        }
+        head = __shfl_sync(0xffffffffu, head, 0);
         left = __shfl_sync(0xffffffffu, left, 0);
-        __threadfence_block();
+        __syncwarp();
+        QSlot& c = q.slot[head % QSLOTS];
         if (left <= 0) {
             // exhausted: one warp claims the next chunk, the others wait for it
-            if (ld_shared_volatile(&q.exit_)) break;
-            unsigned int busy = 1;
-            if (lane == 0) busy = atomicCAS(&q.claiming, 0u, 1u);
-            busy = __shfl_sync(0xffffffffu, busy, 0);
-            if (busy) {
+            enum { LEAVE, WAIT, AGAIN, STUCK, CLAIM };
+            int act = LEAVE;
+            QSlot& s = q.slot[(head + 1u) % QSLOTS];
+            if (lane == 0 && !ld_shared_volatile(&q.exit_)) {
+                act = WAIT;
+                if (atomicCAS(&q.claiming, 0u, 1u) == 0u) {
+                    __threadfence_block();
+                    act = CLAIM;
+                    if (ld_shared_volatile(&q.head) != head) {  // another warp has just claimed
+                        act = AGAIN;
+                        atomicExch(&q.claiming, 0u);
+                    }
+                    // its last chunk's stragglers: running warps (bounded all the same)
+                    const unsigned long long t0 = global_ns();
+                    while (act == CLAIM && *reinterpret_cast<const volatile int*>(&s.busy) != 0) {
+                        __nanosleep(100);
+                        if (global_ns() - t0 > QSTALL_NS) act = STUCK;
+                    }
+                    __threadfence_block();
+                }
+            }
+            act = __shfl_sync(0xffffffffu, act, 0);
+            __syncwarp();
+            if (act == LEAVE) break;
+            if (act == WAIT) {
                 __nanosleep(400);
                 continue;
             }
-            __threadfence_block();
-            if (ld_shared_volatile(&q.head) != head) {  // another warp has just claimed
-                __syncwarp();
-                if (lane == 0) atomicExch(&q.claiming, 0u);
-                continue;
-            }
-            QSlot& s = q.slot[(head + 1u) % QSLOTS];
-            // its last chunk's stragglers: running warps (bounded all the same)
-            const unsigned long long t0 = global_ns();
-            bool ok = true;
-            while (*reinterpret_cast<const volatile int*>(&s.busy) != 0) {
-                __nanosleep(100);
-                if (global_ns() - t0 > QSTALL_NS) {
-                    ok = false;
-                    break;
-                }
-            }
+            if (act == AGAIN) continue;
             uint32_t chunk = 0, gen = 0, nch = 0;
-            const int job = ok ? queue_claim(P, q, lane, chunk, gen, nch) : -1;
+            const int job = act == CLAIM ? queue_claim(P, q, lane, chunk, gen, nch) : -1;
             if (job < 0) {
                 if (lane == 0) {
-                    if (!ok) atomicOr(P.status, ST_WAIT_LIMIT);
-                    if (!ok || queue_idle(P, q))
+                    if (act == STUCK) atomicOr(P.status, ST_WAIT_LIMIT);
+                    if (act == STUCK || queue_idle(P, q))
                         atomicExch(&q.exit_, 1u);
+                    else
+                        __nanosleep(250);
+                    __threadfence_block();
+                    atomicExch(&q.claiming, 0u);
                 }
                 __syncwarp();
-                if (!ld_shared_volatile(&q.exit_)) __nanosleep(250);
-                __threadfence_block();
-                if (lane == 0) atomicExch(&q.claiming, 0u);
                 continue;
             }
             const AlignJob& jb = P.jobs[job];
@@ -2549,6 +2565,7 @@ __global__ void __launch_bounds__(QT, 65536 / (QT * REGCAP)) k_ndt_queue(const A
         if (d + 1u != nunits) continue;
         // the chunk's last unit: its sums to global memory
         __threadfence_block();
+        __syncwarp();
         const int job = c.job;
         uint32_t gen = c.gen, nch = c.nch;
         {
@@ -2577,26 +2594,28 @@ __global__ void __launch_bounds__(QT, 65536 / (QT * REGCAP)) k_ndt_queue(const A
         // nch chunks and the step before arrive; the last of them runs the step
         if (prev != nch) continue;
         __threadfence();  // acquire: every chunk's partials of this iteration are visible
+        __syncwarp();
         // the Newton step, in a free controller area (another warp's step at most ahead)
         int area = -1;
-        const unsigned long long t0 = global_ns();
-        while (area < 0) {
-            if (lane == 0) {
+        if (lane == 0) {
+            const unsigned long long t0 = global_ns();
+            for (bool late = false; area < 0 && !late;) {
                 const unsigned int b = ld_shared_volatile(&q.ctl_busy);
                 for (int i = 0; i < QCTLS && area < 0; ++i)
                     if (!(b >> i & 1u) && !(atomicOr(&q.ctl_busy, 1u << i) >> i & 1u)) area = i;
-            }
-            area = __shfl_sync(0xffffffffu, area, 0);
-            if (area >= 0) break;
-            __nanosleep(100);
-            if (global_ns() - t0 > QSTALL_NS) {
-                if (lane == 0) {
-                    atomicOr(P.status, ST_WAIT_LIMIT);
-                    atomicExch(&q.exit_, 1u);
+                if (area < 0) {
+                    __nanosleep(100);
+                    late = global_ns() - t0 > QSTALL_NS;
                 }
-                break;
             }
+            if (area < 0) {
+                atomicOr(P.status, ST_WAIT_LIMIT);
+                atomicExch(&q.exit_, 1u);
+            }
+            __threadfence_block();
         }
+        area = __shfl_sync(0xffffffffu, area, 0);
+        __syncwarp();
         if (area < 0) break;
         __threadfence_block();
         CtlShared& ctl = q.ctl[area];
@@ -2635,6 +2654,7 @@ __global__ void __launch_bounds__(QT, 65536 / (QT * REGCAP)) k_ndt_queue(const A
             prev = __shfl_sync(0xffffffffu, prev, 0);
             if (prev != nch) break;
             __threadfence();
+            __syncwarp();
             gen += 1u;
         }
         __threadfence_block();
