@@ -527,6 +527,16 @@ int ndt_debug_queue_stall(ndt_ctx* c, uint64_t limit_ns, int32_t withhold_next) 
     return NDT_OK;
 }
 
+int ndt_debug_lookback_stall(ndt_ctx* c, uint64_t limit_ns, int32_t withhold) {
+    if (!c || withhold < 0 || withhold > 4) return NDT_ERR_INVALID_ARGUMENT;
+    tiles_settle(c, true);  // a rebuild in the background reads the scratch
+    for (BuildScratch* b : {&c->bs, &c->bs_b, &c->bs_tile}) {
+        b->lb_limit_ns = limit_ns ? limit_ns : LB_LIMIT_NS;
+        b->lb_withhold = withhold;
+    }
+    return NDT_OK;
+}
+
 int ndt_debug_trace(ndt_ctx* c, int enable) {
     if (!c) return NDT_ERR_INVALID_ARGUMENT;
     c->trace = enable != 0;

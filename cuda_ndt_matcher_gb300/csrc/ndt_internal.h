@@ -106,10 +106,15 @@ struct Map {
 };
 
 // Scratch used while building a map (kept for the next rebuild).
+constexpr unsigned long long LB_LIMIT_NS = 1000000000ull;  // look-back waits of a build: 1 s
 struct BuildScratch {
     DevBuf keys_a, keys_b, vals_a, vals_b, tmp;
     DevBuf seg_ids, seg_starts, seg_valid, seg_rank, seg_rec, small;
     PinBuf host;  // sizes read back between stages
+    // test hook: the waits' limit, and the look-back launch whose first tile withholds its word
+    // (1 the key sort's scans, 2 segment starts, 3 the size sort's scan, 4 ranks; 0 none)
+    unsigned long long lb_limit_ns = LB_LIMIT_NS;
+    int lb_withhold = 0;
 };
 
 // Temporary-storage sizing of the sort / scan primitives (two-phase convention).

@@ -89,7 +89,19 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* w
 // (top two bits: 0 not there yet, 1 the tile's sum, 2 the inclusive prefix) and value, so it
 // is read and written whole and needs no fence.
 // ---------------------------------------------------------------------------------------
-constexpr unsigned long long LB_LIMIT_NS = 1000000000ull;  // bounded waits: 1 s
+// Where a launch's words are (one ticket, then a word per tile, all zero at the start), how
+// long a wait may last, and (test hook) whether tile 0 withholds its word, so that the waits of
+// the others run out.
+struct LookBack {
+    unsigned long long* words;
+    unsigned long long limit_ns;
+    bool withhold;
+};
+// The look-back launch `stage` of a build (BuildScratch::lb_withhold)
+enum { LB_SORT = 1, LB_SEGMENTS = 2, LB_SIZES = 3, LB_RANKS = 4 };
+static LookBack look_back(const BuildScratch& sc, void* words, int stage) {
+    return {(unsigned long long*)words, sc.lb_limit_ns, sc.lb_withhold == stage};
+}
 
 __device__ __forceinline__ unsigned long long lb_now() {
     unsigned long long t;
@@ -97,14 +109,17 @@ __device__ __forceinline__ unsigned long long lb_now() {
     return t;
 }
 
-// Exclusive prefix of tile `tile` over 64-bit words w[0 .. tile), whose own sum is `sum`, by one
-// warp (32 earlier tiles at a time); publishes the tile's inclusive prefix. False when a word
-// did not arrive within the limit.
-__device__ __forceinline__ bool lookback_warp(unsigned long long* w, uint32_t tile,
+// Exclusive prefix of tile `tile`, whose own sum is `sum`, over the earlier tiles, by one warp (32
+// tiles at a time); publishes the tile's inclusive prefix. False (in every lane) when a word did
+// not arrive within the limit: the warp decides together, and on words read after the time was
+// taken, so a context that was paused for longer finds what has arrived meanwhile.
+__device__ __forceinline__ bool lookback_warp(const LookBack& lb, uint32_t tile,
                                               unsigned long long sum, int lane,
                                               unsigned long long& excl) {
     constexpr unsigned long long ONE = 1ull << 62, TWO = 2ull << 62, VAL = ONE - 1ull;
-    if (lane == 0) atomicExch(w + tile, (tile == 0 ? TWO : ONE) | sum);
+    unsigned long long* const w = lb.words + 1;
+    if (lane == 0 && !(tile == 0 && lb.withhold))
+        atomicExch(w + tile, (tile == 0 ? TWO : ONE) | sum);
     excl = 0ull;
     if (tile == 0) return true;
     const unsigned long long t0 = lb_now();
@@ -112,8 +127,9 @@ __device__ __forceinline__ bool lookback_warp(unsigned long long* w, uint32_t ti
     for (;;) {
         unsigned long long v = at >= 0 ? *(volatile unsigned long long*)(w + at) : TWO;
         while (__any_sync(0xffffffffu, (v >> 62) == 0ull)) {
-            if (lb_now() - t0 > LB_LIMIT_NS) return false;
+            const int late = __any_sync(0xffffffffu, lb_now() - t0 > lb.limit_ns);
             if ((v >> 62) == 0ull) v = *(volatile unsigned long long*)(w + at);
+            if (late && __any_sync(0xffffffffu, (v >> 62) == 0ull)) return false;
         }
         // the nearest inclusive prefix among these 32, and the sums after it
         const unsigned full = __ballot_sync(0xffffffffu, (v >> 62) == 2ull);
@@ -130,14 +146,14 @@ __device__ __forceinline__ bool lookback_warp(unsigned long long* w, uint32_t ti
 }
 
 // Exclusive scan in one launch, element order (thread t of a tile holds items t * ITEMS ..).
-// tmp: one ticket, then a word per tile, all zero at the start. In place allowed.
+// In place allowed.
 __global__ void __launch_bounds__(BT) k_scan(const uint32_t* __restrict__ in,
                                              uint32_t* __restrict__ out, size_t n,
-                                             unsigned long long* __restrict__ tmp) {
+                                             const LookBack lb) {
     __shared__ uint32_t ws[BT / 32];
     __shared__ uint32_t s_tile, s_excl;
     __shared__ bool s_ok;
-    if (threadIdx.x == 0) s_tile = atomicAdd((unsigned int*)tmp, 1u);
+    if (threadIdx.x == 0) s_tile = atomicAdd((unsigned int*)lb.words, 1u);
     __syncthreads();
     const uint32_t tile = s_tile;
     const size_t base = (size_t)tile * TILE + (size_t)threadIdx.x * ITEMS;
@@ -152,7 +168,7 @@ __global__ void __launch_bounds__(BT) k_scan(const uint32_t* __restrict__ in,
     const uint32_t pre = block_exclusive_scan(s, ws, &tot);
     if (threadIdx.x < 32) {
         unsigned long long e;
-        const bool ok = lookback_warp(tmp + 1, tile, tot, (int)threadIdx.x, e);
+        const bool ok = lookback_warp(lb, tile, tot, (int)threadIdx.x, e);
         if (threadIdx.x == 0) {
             s_excl = (uint32_t)e;
             s_ok = ok;
@@ -170,18 +186,18 @@ __global__ void __launch_bounds__(BT) k_scan(const uint32_t* __restrict__ in,
 
 size_t scan_temp_bytes(size_t n) { return align_up((size_t)ntiles(n) * 8 + 8, 256); }
 
-// exclusive scan in -> out (may alias); temp >= scan_temp_bytes(n), 8-byte aligned, all zero
-static int exclusive_scan_zeroed(const uint32_t* in, uint32_t* out, size_t n, void* temp,
+// exclusive scan in -> out (may alias); lb.words: scan_temp_bytes(n), 8-byte aligned, all zero
+static int exclusive_scan_zeroed(const uint32_t* in, uint32_t* out, size_t n, const LookBack& lb,
                                  cudaStream_t s) {
     if (n == 0) return 0;
-    k_scan<<<ntiles(n), BT, 0, s>>>(in, out, n, (unsigned long long*)temp);
+    k_scan<<<ntiles(n), BT, 0, s>>>(in, out, n, lb);
     return cuda_fail(cudaGetLastError(), "scan launch");
 }
 static int exclusive_scan(const uint32_t* in, uint32_t* out, size_t n, void* temp,
                           cudaStream_t s) {
     if (n == 0) return 0;
     cudaMemsetAsync(temp, 0, (size_t)ntiles(n) * 8 + 8, s);
-    return exclusive_scan_zeroed(in, out, n, temp, s);
+    return exclusive_scan_zeroed(in, out, n, {(unsigned long long*)temp, LB_LIMIT_NS, false}, s);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -556,11 +572,11 @@ __global__ void __launch_bounds__(BT, 4) k_sort_pass(
 }
 
 // Sorts n pairs (keys k0, values: the positions) with the workspace `work` and zeroed look-back
-// words `words`; counted: the first pass's tile counts are in the workspace already; alternate
+// words lb.words; counted: the first pass's tile counts are in the workspace already; alternate
 // buffers k1 and v1, values through v0 and v1. On return *kout and *vout
 // are the buffers that hold the result: v0 after an even number of passes, else v1.
 static int sort_positions(uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* v1, size_t n,
-                          SortPlan o, bool counted, void* work, void* words,
+                          SortPlan o, bool counted, void* work, const LookBack& lb,
                           uint32_t** kout, uint32_t** vout, cudaStream_t s) {
     uint32_t* hist = (uint32_t*)work;
     const size_t wb = scan_temp_bytes(sort_counts(n, o));
@@ -570,8 +586,9 @@ static int sort_positions(uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* v1
     for (int p = 0; p < o.passes; ++p) {
         if (p > 0 || !counted)
             k_tile_digits<<<nb, BT, 0, s>>>(ki, (uint32_t)n, p * o.width, o.width, hist);
-        if ((rc = exclusive_scan_zeroed(hist, hist, sort_counts(n, o), (char*)words + p * wb, s)))
-            return rc;
+        LookBack pass = lb;
+        pass.words += p * (wb / 8);
+        if ((rc = exclusive_scan_zeroed(hist, hist, sort_counts(n, o), pass, s))) return rc;
         k_sort_pass<<<nb, BT, 0, s>>>(ki, p == 0 ? nullptr : vi, ko, vo, (uint32_t)n,
                                       p * o.width, o.width, hist);
         std::swap(ki, ko);
@@ -716,10 +733,10 @@ size_t detect_segments_temp_bytes(size_t n) {
 
 // Segment starts without per-key flags (the map build's form, no segment ids), in one launch:
 // a block counts its tile's segment starts (key != previous key), finds the earlier tiles'
-// count by look-back and writes its starts there, in key order. tmp as for k_scan.
+// count by look-back and writes its starts there, in key order.
 template <typename K>
 __global__ void __launch_bounds__(BT) k_seg_starts(const K* __restrict__ keys, size_t n,
-                                                   unsigned long long* __restrict__ tmp,
+                                                   const LookBack lb,
                                                    uint32_t* __restrict__ starts,
                                                    uint32_t* __restrict__ num) {
     __shared__ uint32_t ws[BT / 32];
@@ -727,7 +744,7 @@ __global__ void __launch_bounds__(BT) k_seg_starts(const K* __restrict__ keys, s
     __shared__ bool s_ok;
     constexpr int ROUNDS = TILE / BT;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) s_tile = atomicAdd((unsigned int*)tmp, 1u);
+    if (threadIdx.x == 0) s_tile = atomicAdd((unsigned int*)lb.words, 1u);
     __syncthreads();
     const uint32_t tile = s_tile;
     // warp w holds the tile's keys [w * 512, (w + 1) * 512) as 16 rounds of 32
@@ -750,7 +767,7 @@ __global__ void __launch_bounds__(BT) k_seg_starts(const K* __restrict__ keys, s
     r0 = __shfl_sync(0xffffffffu, r0, 0);
     if (threadIdx.x < 32) {
         unsigned long long e;
-        const bool ok = lookback_warp(tmp + 1, tile, tot, (int)threadIdx.x, e);
+        const bool ok = lookback_warp(lb, tile, tot, (int)threadIdx.x, e);
         if (threadIdx.x == 0) {
             s_excl = (uint32_t)e;
             s_ok = ok;
@@ -770,13 +787,12 @@ __global__ void __launch_bounds__(BT) k_seg_starts(const K* __restrict__ keys, s
 }
 
 // starts of the runs of equal keys in sorted[0..n), their count in *num_segments (0 when a
-// wait ran out); *num_segments zero at the start, temp >= scan_temp_bytes(n), 8-byte aligned,
-// all zero; n > 0
+// wait ran out); *num_segments zero at the start, lb.words: scan_temp_bytes(n), 8-byte
+// aligned, all zero; n > 0
 template <typename K>
 static int segment_starts(const K* sorted, size_t n, uint32_t* seg_starts,
-                          uint32_t* num_segments, void* temp, cudaStream_t s) {
-    k_seg_starts<K><<<ntiles(n), BT, 0, s>>>(sorted, n, (unsigned long long*)temp, seg_starts,
-                                             num_segments);
+                          uint32_t* num_segments, const LookBack& lb, cudaStream_t s) {
+    k_seg_starts<K><<<ntiles(n), BT, 0, s>>>(sorted, n, lb, seg_starts, num_segments);
     return cuda_fail(cudaGetLastError(), "segments");
 }
 
@@ -2085,9 +2101,10 @@ int build_segments(BuildScratch& sc, const float* d_pts, size_t n, const ndt_con
         // the last pass writes the values to vals_a: an even number of passes starts there
         uint32_t *va = vals, *vb = v1;
         if (o.passes & 1) std::swap(va, vb);
-        if ((rc = sort_positions(k0, va, k1, vb, n, o, true, sc.tmp.p, words + w_sort, &ks, &vs,
-                                 s)) ||
-            (rc = segment_starts(ks, g.nf, (uint32_t*)sc.seg_starts.p, nseg, words + w_seg, s)))
+        if ((rc = sort_positions(k0, va, k1, vb, n, o, true, sc.tmp.p,
+                                 look_back(sc, words + w_sort, LB_SORT), &ks, &vs, s)) ||
+            (rc = segment_starts(ks, g.nf, (uint32_t*)sc.seg_starts.p, nseg,
+                                 look_back(sc, words + w_seg, LB_SEGMENTS), s)))
             return rc;
     } else {
         const uint32_t lv = std::max(bits[0], std::max(bits[1], bits[2]));
@@ -2096,7 +2113,8 @@ int build_segments(BuildScratch& sc, const float* d_pts, size_t n, const ndt_con
                                                                         mm, keys, vals);
         if ((rc = radix_sort_pairs(keys, vals, n, 0, std::min(64, (int)(3 * lv + 1)), sc.tmp.p,
                                    tmp, s)) ||
-            (rc = segment_starts(keys, g.nf, (uint32_t*)sc.seg_starts.p, nseg, words + w_seg, s)))
+            (rc = segment_starts(keys, g.nf, (uint32_t*)sc.seg_starts.p, nseg,
+                                 look_back(sc, words + w_seg, LB_SEGMENTS), s)))
             return rc;
     }
     cudaMemcpyAsync(hseg, nseg, 4, cudaMemcpyDeviceToHost, s);
@@ -2116,7 +2134,7 @@ int build_segments(BuildScratch& sc, const float* d_pts, size_t n, const ndt_con
     k_seg_size_keys<<<(g.S + 255) / 256, 256, 0, s>>>((const uint32_t*)sc.seg_starts.p, g.S,
                                                       (uint32_t)g.nf, skeys);
     if ((rc = sort_positions(skeys, nullptr, sorted, order, g.S, oz, false, sc.tmp.p,
-                             words + w_size, &kz, &vz, s)))
+                             look_back(sc, words + w_size, LB_SIZES), &kz, &vz, s)))
         return rc;
     // the large segments' sums behind the sort's workspace: at most nf / WARP_SEG_MIN segments
     // of SegSums, well inside its 8 bytes per point
@@ -2384,8 +2402,9 @@ int merge_tiles(Map& map, BuildScratch& sc, const std::vector<TileSegRef>& refs,
     uint32_t *ks, *vals;
     if ((rc = sort_positions(keys, (uint32_t*)sc.vals_a.p, keys + total,
                              (uint32_t*)((char*)sc.tmp.p + ob), total, o, false, sc.tmp.p,
-                             words + 256, &ks, &vals, s)) ||
-        (rc = segment_starts(ks, total, (uint32_t*)sc.seg_starts.p, ngroups, words + w_seg, s)))
+                             look_back(sc, words + 256, LB_SORT), &ks, &vals, s)) ||
+        (rc = segment_starts(ks, total, (uint32_t*)sc.seg_starts.p, ngroups,
+                             look_back(sc, words + w_seg, LB_SEGMENTS), s)))
         return rc;
     k_merge_groups<<<(unsigned)((total + 127) / 128), 128, 0, s>>>(
         dref, nt, vals, (const uint32_t*)sc.seg_starts.p, ngroups, (uint32_t)total,

@@ -458,6 +458,13 @@ int ndt_debug_read(ndt_ctx* ctx, uint64_t index, double* out, int32_t max_record
  * runs out: the error path can be tested without a fault. The context stays usable. */
 int ndt_debug_queue_stall(ndt_ctx* ctx, uint64_t limit_ns, int32_t withhold_next);
 
+/* Test hook for the waits of a map build (its scans run in one launch each; a tile waits for
+ * the sums of the tiles before it). A wait gives up after limit_ns (default 1 s; 0 restores it)
+ * and the build returns NDT_ERR_DEVICE. With withhold 1-4, until it is set to 0, the first tile
+ * of one kind of scan withholds its sum, so the others' waits run out: 1 the key sort's, 2 the
+ * segment starts', 3 the sort by segment size, 4 the ranks of the valid voxels. */
+int ndt_debug_lookback_stall(ndt_ctx* ctx, uint64_t limit_ns, int32_t withhold);
+
 const char* ndt_last_error_string(void);
 
 /* ---- build-stage primitives on caller device memory (the cuda_ffi roles) ------------ */
