@@ -83,6 +83,87 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* w
 }
 
 // ---------------------------------------------------------------------------------------
+// Exclusive scan in three launches, none of which waits for another block: the form of the
+// standalone entry points, which return before their kernels end and so could not report a wait
+// that ran out, and of the 64-bit sort.
+// ---------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(BT) k_tile_reduce(const uint32_t* __restrict__ in, size_t n,
+                                                    uint32_t* __restrict__ bsum) {
+    __shared__ uint32_t ws[BT / 32];
+    size_t base = (size_t)blockIdx.x * TILE;
+    uint32_t s = 0;
+#pragma unroll
+    for (int r = 0; r < ITEMS; ++r) {
+        size_t i = base + (size_t)r * BT + threadIdx.x;
+        if (i < n) s += in[i];
+    }
+    uint32_t tot;
+    block_exclusive_scan(s, ws, &tot);
+    if (threadIdx.x == 0) bsum[blockIdx.x] = tot;
+}
+
+__global__ void __launch_bounds__(BT) k_scan_bsums(uint32_t* __restrict__ bsum, uint32_t nb) {
+    __shared__ uint32_t ws[BT / 32];
+    uint32_t carry = 0;
+    for (uint32_t base = 0; base < nb; base += TILE) {
+        uint32_t v[ITEMS];
+        uint32_t s = 0;
+#pragma unroll
+        for (int k = 0; k < ITEMS; ++k) {
+            uint32_t i = base + threadIdx.x * ITEMS + k;
+            v[k] = i < nb ? bsum[i] : 0u;
+            s += v[k];
+        }
+        uint32_t tot;
+        uint32_t run = carry + block_exclusive_scan(s, ws, &tot);
+#pragma unroll
+        for (int k = 0; k < ITEMS; ++k) {
+            uint32_t i = base + threadIdx.x * ITEMS + k;
+            if (i < nb) bsum[i] = run;
+            run += v[k];
+        }
+        carry += tot;
+        __syncthreads();
+    }
+}
+
+// exclusive scan of a tile; element order: thread t holds items t*ITEMS .. t*ITEMS+15
+__global__ void __launch_bounds__(BT) k_tile_scan(const uint32_t* __restrict__ in,
+                                                  uint32_t* __restrict__ out, size_t n,
+                                                  const uint32_t* __restrict__ bsum) {
+    __shared__ uint32_t ws[BT / 32];
+    size_t base = (size_t)blockIdx.x * TILE + (size_t)threadIdx.x * ITEMS;
+    uint32_t v[ITEMS];
+    uint32_t s = 0;
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k) {
+        v[k] = (base + k < n) ? in[base + k] : 0u;
+        s += v[k];
+    }
+    uint32_t tot;
+    uint32_t run = bsum[blockIdx.x] + block_exclusive_scan(s, ws, &tot);
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k) {
+        if (base + k < n) out[base + k] = run;
+        run += v[k];
+    }
+}
+
+size_t scan_temp_bytes(size_t n) { return align_up((size_t)ntiles(n) * 4 + 4, 256); }
+
+// exclusive scan in -> out (may alias); temp >= scan_temp_bytes(n), 4-byte aligned
+static int exclusive_scan(const uint32_t* in, uint32_t* out, size_t n, void* temp,
+                          cudaStream_t s) {
+    if (n == 0) return 0;
+    uint32_t nb = ntiles(n);
+    uint32_t* bsum = (uint32_t*)temp;
+    k_tile_reduce<<<nb, BT, 0, s>>>(in, n, bsum);
+    k_scan_bsums<<<1, BT, 0, s>>>(bsum, nb);
+    k_tile_scan<<<nb, BT, 0, s>>>(in, out, n, bsum);
+    return cuda_fail(cudaGetLastError(), "scan launch");
+}
+
+// ---------------------------------------------------------------------------------------
 // Decoupled look-back (Merrill and Garland 2016): the tiles of a launch take their numbers from
 // a ticket, so every earlier tile is running or done; each publishes its own sum, then walks
 // back over the earlier tiles' words until it meets an inclusive prefix. A word holds state
@@ -184,20 +265,14 @@ __global__ void __launch_bounds__(BT) k_scan(const uint32_t* __restrict__ in,
     }
 }
 
-size_t scan_temp_bytes(size_t n) { return align_up((size_t)ntiles(n) * 8 + 8, 256); }
+static size_t lookback_bytes(size_t n) { return align_up((size_t)ntiles(n) * 8 + 8, 256); }
 
-// exclusive scan in -> out (may alias); lb.words: scan_temp_bytes(n), 8-byte aligned, all zero
+// exclusive scan in -> out (may alias); lb.words: lookback_bytes(n), 8-byte aligned, all zero
 static int exclusive_scan_zeroed(const uint32_t* in, uint32_t* out, size_t n, const LookBack& lb,
                                  cudaStream_t s) {
     if (n == 0) return 0;
     k_scan<<<ntiles(n), BT, 0, s>>>(in, out, n, lb);
     return cuda_fail(cudaGetLastError(), "scan launch");
-}
-static int exclusive_scan(const uint32_t* in, uint32_t* out, size_t n, void* temp,
-                          cudaStream_t s) {
-    if (n == 0) return 0;
-    cudaMemsetAsync(temp, 0, (size_t)ntiles(n) * 8 + 8, s);
-    return exclusive_scan_zeroed(in, out, n, {(unsigned long long*)temp, LB_LIMIT_NS, false}, s);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -420,7 +495,7 @@ static SortPlan sort_plan(int bits) {
 static size_t sort_counts(size_t n, SortPlan o) { return (size_t)ntiles(n) << o.width; }
 static size_t sort_bytes(size_t n, SortPlan o) { return align_up(sort_counts(n, o) * 4, 256); }
 static size_t sort_words_bytes(size_t n, SortPlan o) {
-    return (size_t)o.passes * scan_temp_bytes(sort_counts(n, o));
+    return (size_t)o.passes * lookback_bytes(sort_counts(n, o));
 }
 
 // Digit counts of a tile: shared-memory atomics into one counter set per warp, so keys of one
@@ -579,7 +654,7 @@ static int sort_positions(uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* v1
                           SortPlan o, bool counted, void* work, const LookBack& lb,
                           uint32_t** kout, uint32_t** vout, cudaStream_t s) {
     uint32_t* hist = (uint32_t*)work;
-    const size_t wb = scan_temp_bytes(sort_counts(n, o));
+    const size_t wb = lookback_bytes(sort_counts(n, o));
     const uint32_t nb = ntiles(n);
     uint32_t *ki = k0, *vi = v0, *ko = k1, *vo = v1;
     int rc;
@@ -787,7 +862,7 @@ __global__ void __launch_bounds__(BT) k_seg_starts(const K* __restrict__ keys, s
 }
 
 // starts of the runs of equal keys in sorted[0..n), their count in *num_segments (0 when a
-// wait ran out); *num_segments zero at the start, lb.words: scan_temp_bytes(n), 8-byte
+// wait ran out); *num_segments zero at the start, lb.words: lookback_bytes(n), 8-byte
 // aligned, all zero; n > 0
 template <typename K>
 static int segment_starts(const K* sorted, size_t n, uint32_t* seg_starts,
@@ -2061,7 +2136,7 @@ int build_segments(BuildScratch& sc, const float* d_pts, size_t n, const ndt_con
     // sort's passes (at most four of 8 bits), the segment starts, the size sort
     const SortPlan oz = {1, 8};
     const size_t w_sort = 256, w_seg = w_sort + sort_words_bytes(n, SortPlan{4, 8}),
-                 w_size = w_seg + scan_temp_bytes(n), w_end = w_size + sort_words_bytes(n, oz);
+                 w_size = w_seg + lookback_bytes(n), w_end = w_size + sort_words_bytes(n, oz);
     tmp = align_up(tmp, 256);
     if ((rc = dev_reserve(sc.tmp, tmp + w_end))) return rc;
     char* const words = (char*)sc.tmp.p + tmp;
@@ -2381,7 +2456,7 @@ int merge_tiles(Map& map, BuildScratch& sc, const std::vector<TileSegRef>& refs,
     const SortPlan o = sort_plan((int)ck.total);
     const size_t ob = sort_bytes(total, o);
     const size_t w_at = std::max(ob + align_up(total * 4, 256), scan_temp_bytes(total)),
-                 w_seg = 256 + sort_words_bytes(total, o), w_end = w_seg + scan_temp_bytes(total);
+                 w_seg = 256 + sort_words_bytes(total, o), w_end = w_seg + lookback_bytes(total);
     if ((rc = dev_reserve(d_refs, used.size() * sizeof(TileSegRef))) ||
         (rc = dev_reserve(sc.keys_a, total * 8)) || (rc = dev_reserve(sc.vals_a, total * 4)) ||
         (rc = dev_reserve(sc.small, 256)) || (rc = dev_reserve(sc.seg_starts, total * 4 + 4)) ||
