@@ -626,6 +626,7 @@ static int tile_segments(ndt_ctx* c, ndt_ctx::Tile& t) {
     float ms = 0.f;
     const int rc = build_tile_segments(c->bs_tile, (const float*)t.pts.p, (size_t)t.n, c->cfg,
                                        c->bstream, t.segs, &ms);
+    if (rc == NDT_ERR_DEVICE) t.seg_res = 0.f;  // the next commit builds them again
     if (rc) return rc;
     t.seg_res = c->cfg.resolution;
     t.seg_min = c->cfg.min_points_per_voxel;

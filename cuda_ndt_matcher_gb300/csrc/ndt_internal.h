@@ -111,6 +111,7 @@ struct BuildScratch {
     DevBuf keys_a, keys_b, vals_a, vals_b, tmp;
     DevBuf seg_ids, seg_starts, seg_valid, seg_rank, seg_rec, small;
     PinBuf host;  // sizes read back between stages
+    uint32_t* failed = nullptr;  // in tmp: a look-back wait of this build ran out; then the voxels
     // test hook: the waits' limit, and the look-back launch whose first tile withholds its word
     // (1 the key sort's scans, 2 segment starts, 3 the size sort's scan, 4 ranks; 0 none)
     unsigned long long lb_limit_ns = LB_LIMIT_NS;

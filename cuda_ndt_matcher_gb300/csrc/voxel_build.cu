@@ -172,16 +172,23 @@ static int exclusive_scan(const uint32_t* in, uint32_t* out, size_t n, void* tem
 // ---------------------------------------------------------------------------------------
 // Where a launch's words are (one ticket, then a word per tile, all zero at the start), how
 // long a wait may last, and (test hook) whether tile 0 withholds its word, so that the waits of
-// the others run out.
+// the others run out. A wait that runs out sets *failed, a word of the whole build: the kernels
+// behind it that would index memory with what the scan was to write leave at once, and the host
+// reads it with the sizes, before it uses them.
 struct LookBack {
     unsigned long long* words;
+    uint32_t* failed;
     unsigned long long limit_ns;
     bool withhold;
 };
 // The look-back launch `stage` of a build (BuildScratch::lb_withhold)
 enum { LB_SORT = 1, LB_SEGMENTS = 2, LB_SIZES = 3, LB_RANKS = 4 };
-static LookBack look_back(const BuildScratch& sc, void* words, int stage) {
-    return {(unsigned long long*)words, sc.lb_limit_ns, sc.lb_withhold == stage};
+static LookBack look_back(const BuildScratch& sc, void* words, uint32_t* failed, int stage) {
+    return {(unsigned long long*)words, failed, sc.lb_limit_ns, sc.lb_withhold == stage};
+}
+static int look_back_failed() {
+    set_error("map build: a look-back wait ran out");
+    return NDT_ERR_DEVICE;
 }
 
 __device__ __forceinline__ unsigned long long lb_now() {
@@ -210,7 +217,10 @@ __device__ __forceinline__ bool lookback_warp(const LookBack& lb, uint32_t tile,
         while (__any_sync(0xffffffffu, (v >> 62) == 0ull)) {
             const int late = __any_sync(0xffffffffu, lb_now() - t0 > lb.limit_ns);
             if ((v >> 62) == 0ull) v = *(volatile unsigned long long*)(w + at);
-            if (late && __any_sync(0xffffffffu, (v >> 62) == 0ull)) return false;
+            if (late && __any_sync(0xffffffffu, (v >> 62) == 0ull)) {
+                if (lane == 0) atomicExch(lb.failed, 1u);
+                return false;
+            }
         }
         // the nearest inclusive prefix among these 32, and the sums after it
         const unsigned full = __ballot_sync(0xffffffffu, (v >> 62) == 2ull);
@@ -227,10 +237,10 @@ __device__ __forceinline__ bool lookback_warp(const LookBack& lb, uint32_t tile,
 }
 
 // Exclusive scan in one launch, element order (thread t of a tile holds items t * ITEMS ..).
-// In place allowed.
+// In place allowed. total (may be null): the sum of all items.
 __global__ void __launch_bounds__(BT) k_scan(const uint32_t* __restrict__ in,
                                              uint32_t* __restrict__ out, size_t n,
-                                             const LookBack lb) {
+                                             const LookBack lb, uint32_t* __restrict__ total) {
     __shared__ uint32_t ws[BT / 32];
     __shared__ uint32_t s_tile, s_excl;
     __shared__ bool s_ok;
@@ -263,15 +273,16 @@ __global__ void __launch_bounds__(BT) k_scan(const uint32_t* __restrict__ in,
         if (base + k < n) out[base + k] = run;
         run += v[k];
     }
+    if (total && tile == gridDim.x - 1 && threadIdx.x == 0) *total = s_excl + tot;
 }
 
 static size_t lookback_bytes(size_t n) { return align_up((size_t)ntiles(n) * 8 + 8, 256); }
 
 // exclusive scan in -> out (may alias); lb.words: lookback_bytes(n), 8-byte aligned, all zero
 static int exclusive_scan_zeroed(const uint32_t* in, uint32_t* out, size_t n, const LookBack& lb,
-                                 cudaStream_t s) {
+                                 cudaStream_t s, uint32_t* total = nullptr) {
     if (n == 0) return 0;
-    k_scan<<<ntiles(n), BT, 0, s>>>(in, out, n, lb);
+    k_scan<<<ntiles(n), BT, 0, s>>>(in, out, n, lb, total);
     return cuda_fail(cudaGetLastError(), "scan launch");
 }
 
@@ -548,11 +559,12 @@ __global__ void __launch_bounds__(BT) k_tile_digits(const uint32_t* __restrict__
 // rank from the warp's counter: tile order within a digit, so the sort is stable. The digits'
 // tile positions (scanned over the block) and global positions (the scanned tile counts, offs)
 // then give each key's place; the tile leaves through shared memory as one contiguous run per
-// digit. vin null: the values are the positions.
+// digit. vin null: the values are the positions. Nothing moves when the scan of offs failed.
 __global__ void __launch_bounds__(BT, 4) k_sort_pass(
     const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin,
     uint32_t* __restrict__ kout, uint32_t* __restrict__ vout, uint32_t n, int shift, int width,
-    const uint32_t* __restrict__ offs) {
+    const uint32_t* __restrict__ offs, const uint32_t* __restrict__ failed) {
+    if (*failed) return;
     constexpr int NWARP = BT / 32, ROUNDS = TILE / BT, PER = SP_BINS / BT;
     __shared__ TileCounts wc;          // per warp: digit counts, then first positions
     __shared__ uint32_t base[SP_BINS]; // global position minus tile position of a digit
@@ -665,7 +677,7 @@ static int sort_positions(uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* v1
         pass.words += p * (wb / 8);
         if ((rc = exclusive_scan_zeroed(hist, hist, sort_counts(n, o), pass, s))) return rc;
         k_sort_pass<<<nb, BT, 0, s>>>(ki, p == 0 ? nullptr : vi, ko, vo, (uint32_t)n,
-                                      p * o.width, o.width, hist);
+                                      p * o.width, o.width, hist, lb.failed);
         std::swap(ki, ko);
         std::swap(vi, vo);
     }
@@ -1770,8 +1782,9 @@ __device__ __forceinline__ uint32_t large_segments(const uint32_t* __restrict__ 
 __global__ void __launch_bounds__(128) k_segment_sums(
     const float* __restrict__ pts, const uint32_t* __restrict__ sidx,
     const uint32_t* __restrict__ starts, const uint32_t* __restrict__ order,
-    const uint32_t* __restrict__ skey, uint32_t S, uint32_t nf, float res, int min_points,
-    SegSums* __restrict__ sums) {
+    const uint32_t* __restrict__ skey, const uint32_t* __restrict__ failed, uint32_t S,
+    uint32_t nf, float res, int min_points, SegSums* __restrict__ sums) {
+    if (*failed) return;
     __shared__ uint32_t sW;
     if (threadIdx.x == 0) sW = large_segments(skey, S);
     __syncthreads();
@@ -1830,9 +1843,10 @@ __global__ void __launch_bounds__(128) k_segment_sums(
 __global__ void __launch_bounds__(128) k_voxel_stats(
     const float* __restrict__ pts, const uint32_t* __restrict__ sidx,
     const uint32_t* __restrict__ starts, const uint32_t* __restrict__ order,
-    const uint32_t* __restrict__ skey, const SegSums* __restrict__ sums, uint32_t S,
-    uint32_t nf, float res, int min_points, float ratio, SegRec* __restrict__ rec,
-    uint32_t* __restrict__ valid) {
+    const uint32_t* __restrict__ skey, const uint32_t* __restrict__ failed,
+    const SegSums* __restrict__ sums, uint32_t S, uint32_t nf, float res, int min_points,
+    float ratio, SegRec* __restrict__ rec, uint32_t* __restrict__ valid) {
+    if (*failed) return;
     __shared__ uint32_t sW;
     if (threadIdx.x == 0) sW = large_segments(skey, S);
     __syncthreads();
@@ -2121,7 +2135,8 @@ static int box_bits(const int32_t* mn, const int32_t* mx, uint32_t* bits) {
 
 // Stages 1-5 of a build: cells and bounds, Morton keys, sort, segments, per-segment
 // statistics. Leaves in sc: vals (point indices in key order), seg_starts, seg_rec,
-// seg_valid; returns the counts and the cell box in g.
+// seg_valid; returns the counts and the cell box in g. The last launches may still run, and a
+// wait of theirs may run out: the caller reads *sc.failed before it uses the records.
 int build_segments(BuildScratch& sc, const float* d_pts, size_t n, const ndt_config& cfg,
                    cudaStream_t s, SegGeometry& g) {
     int rc = 0;
@@ -2143,6 +2158,7 @@ int build_segments(BuildScratch& sc, const float* d_pts, size_t n, const ndt_con
     cudaMemsetAsync(words, 0, w_end, s);
     int32_t* mm = (int32_t*)sc.small.p;
     uint32_t* nseg = (uint32_t*)words;
+    sc.failed = nseg + 1;
     int32_t* hmm = (int32_t*)sc.host.p;
     uint32_t* hseg = (uint32_t*)sc.host.p + 16;
 
@@ -2177,9 +2193,9 @@ int build_segments(BuildScratch& sc, const float* d_pts, size_t n, const ndt_con
         uint32_t *va = vals, *vb = v1;
         if (o.passes & 1) std::swap(va, vb);
         if ((rc = sort_positions(k0, va, k1, vb, n, o, true, sc.tmp.p,
-                                 look_back(sc, words + w_sort, LB_SORT), &ks, &vs, s)) ||
+                                 look_back(sc, words + w_sort, sc.failed, LB_SORT), &ks, &vs, s)) ||
             (rc = segment_starts(ks, g.nf, (uint32_t*)sc.seg_starts.p, nseg,
-                                 look_back(sc, words + w_seg, LB_SEGMENTS), s)))
+                                 look_back(sc, words + w_seg, sc.failed, LB_SEGMENTS), s)))
             return rc;
     } else {
         const uint32_t lv = std::max(bits[0], std::max(bits[1], bits[2]));
@@ -2189,16 +2205,13 @@ int build_segments(BuildScratch& sc, const float* d_pts, size_t n, const ndt_con
         if ((rc = radix_sort_pairs(keys, vals, n, 0, std::min(64, (int)(3 * lv + 1)), sc.tmp.p,
                                    tmp, s)) ||
             (rc = segment_starts(keys, g.nf, (uint32_t*)sc.seg_starts.p, nseg,
-                                 look_back(sc, words + w_seg, LB_SEGMENTS), s)))
+                                 look_back(sc, words + w_seg, sc.failed, LB_SEGMENTS), s)))
             return rc;
     }
-    cudaMemcpyAsync(hseg, nseg, 4, cudaMemcpyDeviceToHost, s);
+    cudaMemcpyAsync(hseg, nseg, 8, cudaMemcpyDeviceToHost, s);
     if ((rc = cuda_fail(cudaStreamSynchronize(s), "segments"))) return rc;
+    if (hseg[1]) return look_back_failed();
     g.S = hseg[0];
-    if (g.S == 0) {
-        set_error("map build: a look-back wait ran out");
-        return NDT_ERR_DEVICE;
-    }
     // visit order of the segments, largest first (the keys' buffer is free again: the
     // segments are recorded by their starts)
     uint32_t* skeys = (uint32_t*)sc.keys_a.p;
@@ -2209,18 +2222,18 @@ int build_segments(BuildScratch& sc, const float* d_pts, size_t n, const ndt_con
     k_seg_size_keys<<<(g.S + 255) / 256, 256, 0, s>>>((const uint32_t*)sc.seg_starts.p, g.S,
                                                       (uint32_t)g.nf, skeys);
     if ((rc = sort_positions(skeys, nullptr, sorted, order, g.S, oz, false, sc.tmp.p,
-                             look_back(sc, words + w_size, LB_SIZES), &kz, &vz, s)))
+                             look_back(sc, words + w_size, sc.failed, LB_SIZES), &kz, &vz, s)))
         return rc;
     // the large segments' sums behind the sort's workspace: at most nf / WARP_SEG_MIN segments
     // of SegSums, well inside its 8 bytes per point
     SegSums* sums = (SegSums*)((char*)sc.tmp.p + oz_bytes);
     const uint32_t wmax = (uint32_t)std::min<size_t>(g.S, g.nf / WARP_SEG_MIN + 1);
     const unsigned gs = (unsigned)std::min<uint32_t>((wmax + 3) / 4, 152u * 64u);
-    k_segment_sums<<<gs, 128, 0, s>>>(d_pts, vals, (uint32_t*)sc.seg_starts.p, order, kz, g.S,
-                                      (uint32_t)g.nf, cfg.resolution, cfg.min_points_per_voxel,
-                                      sums);
+    k_segment_sums<<<gs, 128, 0, s>>>(d_pts, vals, (uint32_t*)sc.seg_starts.p, order, kz,
+                                      sc.failed, g.S, (uint32_t)g.nf, cfg.resolution,
+                                      cfg.min_points_per_voxel, sums);
     k_voxel_stats<<<(g.S + 127) / 128, 128, 0, s>>>(
-        d_pts, vals, (uint32_t*)sc.seg_starts.p, order, kz, sums, g.S, (uint32_t)g.nf,
+        d_pts, vals, (uint32_t*)sc.seg_starts.p, order, kz, sc.failed, sums, g.S, (uint32_t)g.nf,
         cfg.resolution, cfg.min_points_per_voxel, cfg.eigenvalue_ratio, (SegRec*)sc.seg_rec.p,
         (uint32_t*)sc.seg_valid.p);
     return cuda_fail(cudaGetLastError(), "voxel statistics");
@@ -2231,20 +2244,23 @@ int build_segments(BuildScratch& sc, const float* d_pts, size_t n, const ndt_con
 int finish_map(Map& map, BuildScratch& sc, const SegRec* rec, const uint32_t* valid, uint32_t S,
                const SegGeometry& g, const ndt_config& cfg, uint32_t* d_status, cudaStream_t s) {
     int rc;
-    if ((rc = dev_reserve(sc.seg_rank, (size_t)S * 4 + 4)) ||
-        (rc = dev_reserve(sc.tmp, std::max(sc.tmp.bytes, scan_temp_bytes(S)))) ||
-        (rc = dev_reserve(sc.small, 256)))
+    if ((rc = dev_reserve(sc.seg_rank, (size_t)S * 4 + 4)) || (rc = dev_reserve(sc.small, 256)))
         return rc;
     uint32_t* mprobe = (uint32_t*)((char*)sc.small.p + 128);
     uint32_t bits[3];
     if ((rc = box_bits(g.mn, g.mx, bits))) return rc;
-    if ((rc = exclusive_scan(valid, (uint32_t*)sc.seg_rank.p, S, sc.tmp.p, s))) return rc;
-    if ((rc = pin_reserve(sc.host, 256))) return rc;
+    // (the words in front of sc.tmp; *sc.failed and the sum behind it lie beyond)
+    cudaMemsetAsync(sc.tmp.p, 0, lookback_bytes(S), s);
+    if ((rc = exclusive_scan_zeroed(valid, (uint32_t*)sc.seg_rank.p, S,
+                                    look_back(sc, sc.tmp.p, sc.failed, LB_RANKS), s,
+                                    sc.failed + 1)) ||
+        (rc = pin_reserve(sc.host, 256)))
+        return rc;
     uint32_t* hs = (uint32_t*)sc.host.p + 24;
-    cudaMemcpyAsync(&hs[0], (uint32_t*)sc.seg_rank.p + (S - 1), 4, cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(&hs[1], valid + (S - 1), 4, cudaMemcpyDeviceToHost, s);
+    cudaMemcpyAsync(hs, sc.failed, 8, cudaMemcpyDeviceToHost, s);
     if ((rc = cuda_fail(cudaStreamSynchronize(s), "voxel compaction"))) return rc;
-    const uint32_t V = hs[0] + hs[1];
+    if (hs[0]) return look_back_failed();
+    const uint32_t V = hs[1];
     if (V == 0) {
         set_error("No voxels created from target points (too sparse?)");
         return NDT_ERR_NO_VOXELS;
@@ -2374,8 +2390,9 @@ __global__ void k_merge_keys(const TileSegRef* __restrict__ tiles, int nt, uint3
 __global__ void __launch_bounds__(128) k_merge_groups(
     const TileSegRef* __restrict__ tiles, int nt, const uint32_t* __restrict__ members,
     const uint32_t* __restrict__ gstart, const uint32_t* __restrict__ num_groups,
-    uint32_t n_members, int min_points, float ratio, float res, SegRec* __restrict__ grec,
-    uint32_t* __restrict__ gvalid) {
+    const uint32_t* __restrict__ failed, uint32_t n_members, int min_points, float ratio,
+    float res, SegRec* __restrict__ grec, uint32_t* __restrict__ gvalid) {
+    if (*failed) return;
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t G = *num_groups;
     if (g >= G) return;
@@ -2455,7 +2472,7 @@ int merge_tiles(Map& map, BuildScratch& sc, const std::vector<TileSegRef>& refs,
     const CompactKey ck = compact_key(bits);
     const SortPlan o = sort_plan((int)ck.total);
     const size_t ob = sort_bytes(total, o);
-    const size_t w_at = std::max(ob + align_up(total * 4, 256), scan_temp_bytes(total)),
+    const size_t w_at = std::max(ob + align_up(total * 4, 256), lookback_bytes(total)),
                  w_seg = 256 + sort_words_bytes(total, o), w_end = w_seg + lookback_bytes(total);
     if ((rc = dev_reserve(d_refs, used.size() * sizeof(TileSegRef))) ||
         (rc = dev_reserve(sc.keys_a, total * 8)) || (rc = dev_reserve(sc.vals_a, total * 4)) ||
@@ -2471,28 +2488,26 @@ int merge_tiles(Map& map, BuildScratch& sc, const std::vector<TileSegRef>& refs,
                     cudaMemcpyHostToDevice, s);
     uint32_t* keys = (uint32_t*)sc.keys_a.p;
     uint32_t* ngroups = (uint32_t*)words;
+    sc.failed = ngroups + 1;
     const TileSegRef* dref = (const TileSegRef*)d_refs.p;
     k_merge_keys<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(
         dref, nt, (uint32_t)total, g.mn[0], g.mn[1], g.mn[2], ck, keys);
     uint32_t *ks, *vals;
     if ((rc = sort_positions(keys, (uint32_t*)sc.vals_a.p, keys + total,
                              (uint32_t*)((char*)sc.tmp.p + ob), total, o, false, sc.tmp.p,
-                             look_back(sc, words + 256, LB_SORT), &ks, &vals, s)) ||
+                             look_back(sc, words + 256, sc.failed, LB_SORT), &ks, &vals, s)) ||
         (rc = segment_starts(ks, total, (uint32_t*)sc.seg_starts.p, ngroups,
-                             look_back(sc, words + w_seg, LB_SEGMENTS), s)))
+                             look_back(sc, words + w_seg, sc.failed, LB_SEGMENTS), s)))
         return rc;
     k_merge_groups<<<(unsigned)((total + 127) / 128), 128, 0, s>>>(
-        dref, nt, vals, (const uint32_t*)sc.seg_starts.p, ngroups, (uint32_t)total,
+        dref, nt, vals, (const uint32_t*)sc.seg_starts.p, ngroups, sc.failed, (uint32_t)total,
         cfg.min_points_per_voxel, cfg.eigenvalue_ratio, cfg.resolution, (SegRec*)sc.seg_rec.p,
         (uint32_t*)sc.seg_valid.p);
     uint32_t* hseg = (uint32_t*)sc.host.p + 16;
-    cudaMemcpyAsync(hseg, ngroups, 4, cudaMemcpyDeviceToHost, s);
+    cudaMemcpyAsync(hseg, ngroups, 8, cudaMemcpyDeviceToHost, s);
     if ((rc = cuda_fail(cudaStreamSynchronize(s), "tile merge"))) return rc;
+    if (hseg[1]) return look_back_failed();
     g.S = hseg[0];
-    if (g.S == 0) {
-        set_error("map merge: a look-back wait ran out");
-        return NDT_ERR_DEVICE;
-    }
     rc = finish_map(map, sc, (const SegRec*)sc.seg_rec.p, (const uint32_t*)sc.seg_valid.p, g.S,
                     g, cfg, d_status, s);
     cudaEventRecord(e1, s);
@@ -2531,9 +2546,14 @@ int build_tile_segments(BuildScratch& sc, const float* d_pts, size_t n, const nd
         cudaMemcpyAsync(out.rec.p, sc.seg_rec.p, (size_t)g.S * sizeof(SegRec),
                         cudaMemcpyDeviceToDevice, s);
         cudaMemcpyAsync(out.valid.p, sc.seg_valid.p, (size_t)g.S * 4, cudaMemcpyDeviceToDevice, s);
+        cudaMemcpyAsync((uint32_t*)sc.host.p + 17, sc.failed, 4, cudaMemcpyDeviceToHost, s);
     }
     cudaEventRecord(e1, s);
     if (!rc) rc = cuda_fail(cudaEventSynchronize(e1), "tile segments");
+    if (!rc && out.geo.S && ((const uint32_t*)sc.host.p)[17]) {
+        out.geo = SegGeometry{};  // the tile adds no cell: its old segments are overwritten
+        rc = look_back_failed();
+    }
     float ms = 0.f;
     cudaEventElapsedTime(&ms, e0, e1);
     cudaEventDestroy(e0);

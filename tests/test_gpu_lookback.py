@@ -32,3 +32,51 @@ def test_segment_starts_give_up(gpu):
     ctx.debug_lookback_stall(0, 0)
     ctx.set_target(p)
     assert describe(ctx) == want
+
+
+@pytest.mark.parametrize("kind", [1, 2, 3, 4])
+def test_target_build_reports(gpu, kind):
+    p = cloud(200_000, 2)
+    ctx = capi.Context(resolution=2.0, min_points_per_voxel=2)
+    ctx.set_target(p)
+    want = describe(ctx)
+    ctx.debug_lookback_stall(1_000_000, kind)
+    with pytest.raises(capi.NdtError, match="look-back"):
+        ctx.set_target(p)
+    ctx.debug_lookback_stall(0, 0)
+    ctx.set_target(p)
+    assert describe(ctx) == want
+
+
+@pytest.mark.parametrize("kind", [1, 2, 3])
+def test_tile_put_reports(gpu, kind):
+    p = cloud(200_000, 3)
+    ctx = capi.Context(resolution=2.0, min_points_per_voxel=2)
+    ctx.tile_put(1, p)
+    ctx.tiles_commit()
+    want = describe(ctx)
+    ctx.debug_lookback_stall(1_000_000, kind)
+    with pytest.raises(capi.NdtError, match="look-back"):
+        ctx.tile_put(1, p)
+    ctx.debug_lookback_stall(0, 0)
+    ctx.tile_put(1, p)
+    ctx.tiles_commit()
+    assert describe(ctx) == want
+
+
+@pytest.mark.parametrize("kind", [1, 2, 4])
+def test_merge_reports(gpu, kind):
+    p = cloud(200_000, 4)
+    ctx = capi.Context(resolution=2.0, min_points_per_voxel=2)
+    # whole cells a tile: y = 200 is a cell's edge
+    ctx.tile_put(1, np.ascontiguousarray(p[p[:, 1] < 200]))
+    ctx.tile_put(2, np.ascontiguousarray(p[p[:, 1] >= 200]))
+    ctx.tiles_commit()
+    want = describe(ctx)
+    ctx.debug_lookback_stall(1_000_000, kind)
+    with pytest.raises(capi.NdtError, match="look-back"):
+        ctx.tiles_commit()
+    assert describe(ctx) == want  # the map in use is still the old one
+    ctx.debug_lookback_stall(0, 0)
+    ctx.tiles_commit()
+    assert describe(ctx) == want
