@@ -1245,17 +1245,6 @@ __device__ __forceinline__ double scale2(double v, int e) {
     return __longlong_as_double(b == 0ll ? b : b + ((long long)e << 52));
 }
 
-// 1 / d for a normal d: the f32 reciprocal and two Newton steps (error 2^-52 or so)
-__device__ __forceinline__ double recip2(double d) {
-    // d scaled into f32's range by its exponent, the reciprocal scaled back
-    const int e = (int)((__double_as_longlong(d) >> 52) & 0x7FF) - 1023;
-    const double m = scale2(d, -e);
-    double r = (double)(1.f / (float)m);
-    r = fma(r, fma(-m, r, 1.0), r);
-    r = fma(r, fma(-m, r, 1.0), r);
-    return scale2(r, -e);
-}
-
 // FP64 Rayleigh quotient v^T A v / v^T v of an f32 unit vector v (|v|^2 = 1 +- 1e-7, so
 // 1 / v^T v = 2 - v^T v to FP64 rounding): FP64-accurate for an eigenvalue, since its error
 // is quadratic in v's direction error. *w receives 1 / v^T v.
@@ -1278,7 +1267,7 @@ __device__ __forceinline__ bool inverse_sym3(const double* C, float* icov6) {
     const double c22 = C[0] * C[4] - C[1] * C[1];
     const double det = C[0] * c00 + C[1] * c01 + C[2] * c02;
     if (!(det > 0.0)) return false;
-    const double id = recip2(det);
+    const double id = 1.0 / det;
     icov6[0] = (float)(c00 * id);
     icov6[1] = (float)(c01 * id);
     icov6[2] = (float)(c02 * id);
@@ -1543,6 +1532,11 @@ __device__ __forceinline__ void exact_add(ExactMoments& em, const float* p) {
     add_prod128(em.s2h[5], em.s2l[5], d[2], d[2]);
 }
 
+// 2^e as an FP64 (normal range)
+__device__ __forceinline__ double pow2d(int e) {
+    return __longlong_as_double((long long)(e + 1023) << 52);
+}
+
 // A signed 128-bit integer (hi, lo) rounded once to the nearest FP64 (ties to even)
 __device__ __forceinline__ double i128_to_double(long long hi, unsigned long long lo) {
     const bool neg = hi < 0;
@@ -1559,7 +1553,7 @@ __device__ __forceinline__ double i128_to_double(long long hi, unsigned long lon
     unsigned long long top = lz ? (uh << lz) | (ul >> (64 - lz)) : uh;
     const unsigned long long rest = lz ? ul << lz : ul;
     if (rest != 0ull) top |= 1ull;  // sticky: the discarded bits decide ties and halves
-    const double v = scale2(__ull2double_rn(top), 64 - lz);
+    const double v = __ull2double_rn(top) * pow2d(64 - lz);
     return neg ? -v : v;
 }
 
@@ -1568,7 +1562,6 @@ __device__ __forceinline__ double i128_to_double(long long hi, unsigned long lon
 __device__ __forceinline__ int exact_finish(const ExactMoments& em, uint32_t n, double* mean,
                                             double* A) {
     const double nn = (double)n;
-    const double rn = 1.0 / nn;  // correctly rounded
     int redo = 0;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
@@ -1576,17 +1569,12 @@ __device__ __forceinline__ int exact_finish(const ExactMoments& em, uint32_t n, 
         const unsigned long long mag = tot < 0 ? (unsigned long long)(-tot) : (unsigned long long)tot;
         const int sig = mag ? 64 - __clzll((long long)mag) - min(em.tz[a], 63) : 0;
         if (em.rep[a] && sig <= 53) {
-            // tot / n from the rounded reciprocal: q = tot rn is corrected by its exact
-            // remainder, which gives the correctly rounded quotient (Markstein 1990); the
-            // scaling by 2^e0 is exact
-            const double t = __ll2double_rn(tot);
-            const double q = t * rn;
-            mean[a] = scale2(fma(fma(-q, nn, t), rn, q), em.e0[a]);
+            mean[a] = (__ll2double_rn(tot) * pow2d(em.e0[a])) / nn;
         } else {
             redo |= 1 << a;
         }
     }
-    const double inv_den = recip2(nn * (double)(n - 1u));
+    const double inv_den = 1.0 / (nn * (double)(n - 1u));
     const int ia[6] = {0, 0, 0, 1, 1, 2}, ib[6] = {0, 1, 2, 1, 2, 2};
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
@@ -1600,7 +1588,7 @@ __device__ __forceinline__ int exact_finish(const ExactMoments& em, uint32_t n, 
         const unsigned long long rl = nl - ql;
         const long long rh = nh - qh - (nl < ql ? 1ll : 0ll);
         const double v =
-            scale2(i128_to_double(rh, rl) * inv_den, em.e0[ia[k]] + em.e0[ib[k]]);
+            i128_to_double(rh, rl) * pow2d(em.e0[ia[k]] + em.e0[ib[k]]) * inv_den;
         A[ia[k] * 3 + ib[k]] = A[ib[k] * 3 + ia[k]] = v;
     }
     return redo;
