@@ -1160,9 +1160,7 @@ int morton_codes(const float* pts, size_t n, float res, uint64_t* codes, uint32_
 
 // Cyclic Jacobi for a symmetric 3x3 in f32 (row-major a, eigenvectors in the columns of v).
 // It only has to find the eigenvector directions to f32 accuracy: the eigenvalues and the
-// regularised covariance and inverse are then formed in FP64 (k_voxel_stats), so the rotations
-// use the approximate reciprocals. The caller scales the matrix to a largest diagonal entry of
-// about 1.
+// regularised covariance and inverse are then formed in FP64 (k_voxel_stats).
 __device__ void jacobi3f(float* a, float* v) {
     for (int i = 0; i < 3; ++i)
         for (int j = 0; j < 3; ++j) v[i * 3 + j] = (i == j) ? 1.f : 0.f;
@@ -1176,16 +1174,10 @@ __device__ void jacobi3f(float* a, float* v) {
             const int p = pq == 2 ? 1 : 0, q = pq == 0 ? 1 : 2;
             const float apq = a[p * 3 + q];
             if (apq == 0.f) continue;
-            // t = tan of the angle, |d + sqrt(d^2 + (2 a_pq)^2)| scaled clear of under- and
-            // overflow by the larger of the two
-            const float d = a[q * 3 + q] - a[p * 3 + p], o2 = 2.f * apq;
-            const float sc = fmaxf(fabsf(d), fabsf(o2));
-            if (!(sc > 1e-30f)) continue;  // (the largest entry is about 1)
-            const float dn = __fdividef(d, sc), on = __fdividef(o2, sc);
-            const float h = dn * dn + on * on;
-            float t = __fdividef(fabsf(on), fabsf(dn) + h * rsqrtf(h));
-            if ((d < 0.f) != (apq < 0.f)) t = -t;
-            const float c = rsqrtf(t * t + 1.f);
+            const float theta = (a[q * 3 + q] - a[p * 3 + p]) / (2.f * apq);
+            float t = 1.f / (fabsf(theta) + sqrtf(theta * theta + 1.f));
+            if (theta < 0.f) t = -t;
+            const float c = 1.f / sqrtf(t * t + 1.f);
             const float sn = t * c;
             a[p * 3 + p] -= t * apq;
             a[q * 3 + q] += t * apq;
@@ -1236,13 +1228,6 @@ __device__ void jacobi3_refine(double* B, double* V, int max_sweeps) {
             }
         }
     }
-}
-
-// v 2^e, v and the result zero or normal: an addition to the exponent field. (A warp's FP64
-// instruction occupies the SM's FP64 unit for 16 cycles; integer ones are free beside it.)
-__device__ __forceinline__ double scale2(double v, int e) {
-    const long long b = __double_as_longlong(v);
-    return __longlong_as_double(b == 0ll ? b : b + ((long long)e << 52));
 }
 
 // FP64 Rayleigh quotient v^T A v / v^T v of an f32 unit vector v (|v|^2 = 1 +- 1e-7, so
@@ -1316,9 +1301,8 @@ __device__ __forceinline__ void refine_vector(const double* A, double* v, double
 // (Gram-Schmidt), Jacobi sweeps on V^T A V to the reference's stopping rule, and the
 // reconstruction from the eigen-decomposition. Every route is FP64-accurate, so the f32
 // outputs agree with an FP64 eigen-decomposition to f32 rounding.
-// a32 carries the scale 2^-e32x of voxel_finish.
-__device__ bool regularize(const double* A, const float* a32, const float* V32, int e32x,
-                           float ratio, SegRec& r) {
+__device__ bool regularize(const double* A, const float* a32, const float* V32, float ratio,
+                           SegRec& r) {
     const float e32[3] = {a32[0], a32[4], a32[8]};
     const float mx32 = fmaxf(e32[0], fmaxf(e32[1], e32[2]));
     bool fast = mx32 > 0.f;
@@ -1342,33 +1326,21 @@ __device__ bool regularize(const double* A, const float* a32, const float* V32, 
             for (int q = 0; q < 9; ++q) r.cov[q] = (float)A[q];
             return inverse_sym3(A, r.icov);
         }
-        // FP64 eigenvalues of the largest eigenvector (the threshold) and of the one to refine
-        // (t); the others only enter as f32 gaps of the first-order correction
         double v[3][3], w[3], lam[3];
-        const int one = __popc(clamp) == 1;
-        const int t = one ? __ffs(clamp) - 1 : __ffs(7 & ~clamp) - 1;
-        const int top = e32[0] >= e32[1] ? (e32[0] >= e32[2] ? 0 : 2) : (e32[1] >= e32[2] ? 1 : 2);
-#pragma unroll
         for (int i = 0; i < 3; ++i) {
             for (int k = 0; k < 3; ++k) v[i][k] = (double)V32[k * 3 + i];
-            lam[i] = scale2((double)e32[i], e32x);
-            w[i] = 1.0;
-        }
-        double mx = 0.0, lt = 0.0;
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            if (i != top && i != t) continue;
             lam[i] = rayleigh(A, v[i], &w[i]);
-            if (i == top) mx = lam[i];
-            if (i == t) lt = lam[i];
         }
+        const double mx = fmax(lam[0], fmax(lam[1], lam[2]));
         if (!(mx > 0.0)) return false;
         const double thr = mx * (double)ratio;
+        const int one = __popc(clamp) == 1;
+        const int t = one ? __ffs(clamp) - 1 : __ffs(7 & ~clamp) - 1;  // the vector to refine
         double u[3] = {v[t][0], v[t][1], v[t][2]};
-        refine_vector(A, u, lt, v, lam, w, 7 & ~(1 << t));
+        refine_vector(A, u, lam[t], v, lam, w, 7 & ~(1 << t));
         const double wu = 2.0 - (u[0] * u[0] + u[1] * u[1] + u[2] * u[2]);
         double C[9];
-        const double c = one ? (thr - lt) * wu : (lt - thr) * wu;
+        const double c = one ? (thr - lam[t]) * wu : (lam[t] - thr) * wu;
         for (int rr = 0; rr < 3; ++rr)
             for (int cc = rr; cc < 3; ++cc) {  // upper triangle, mirrored: C stays symmetric
                 const double base = one ? A[rr * 3 + cc] : (rr == cc ? thr : 0.0);
@@ -1648,15 +1620,9 @@ __device__ __noinline__ void moments_two_pass(Each each, uint32_t cnt, double* m
 __device__ __forceinline__ bool voxel_finish(const double* mean, const double* A, float ratio,
                                              SegRec& r) {
     float a32[9], V32[9];
-    // scaled by the power of two of the largest diagonal entry (0 for a zero matrix)
-    int e = 0;
-    for (int q = 0; q < 9; q += 4)
-        e = max(e, (int)((__double_as_longlong(A[q]) >> 52) & 0x7FF));
-    e = e ? e - 1023 : 0;
-    const double dn = __longlong_as_double((long long)(1023 - min(e, 1000)) << 52);
-    for (int q = 0; q < 9; ++q) a32[q] = (float)(A[q] * dn);
+    for (int q = 0; q < 9; ++q) a32[q] = (float)A[q];
     jacobi3f(a32, V32);
-    if (!regularize(A, a32, V32, min(e, 1000), ratio, r)) return false;
+    if (!regularize(A, a32, V32, ratio, r)) return false;
     for (int q = 0; q < 3; ++q) r.mean[q] = (float)mean[q];
     return true;
 }
