@@ -249,8 +249,11 @@ constexpr int EMPTY_ORD = (int)0x80808080;  // the memset byte 0x80: below every
 // are bits in shared memory (a byte per column of eight z cells), so that every row is written
 // once, in order, 16 bytes a thread; features beyond the two grids are 0. Bound by the 74 KB
 // write of a row. (Zeroing X and its transpose and scattering ones into both took 76 us for 1,024
-// samples.)
-__global__ void __launch_bounds__(256)
+// samples.) T: 256 threads where samples fill the SMs, 1,024 where they do not and a long scan is one
+// block's walk (one scan of 1M points: network time 251 us, eight blocks of 256 that each scattered an
+// eighth 294; of 1,000 points 65 and 74).
+template <int T>
+__global__ void __launch_bounds__(T)
     k_features(const float* __restrict__ scan_pts, const PnScan* __restrict__ scans,
                const PnSample* __restrict__ smp, const PnMap* __restrict__ maps, int F,
                __nv_bfloat16* __restrict__ X) {
@@ -260,10 +263,10 @@ __global__ void __launch_bounds__(256)
     const PnScan sc = scans[s.scan];
     float sy, cy;
     sincosf(s.cyaw, &sy, &cy);
-    for (int i = tid; i < PN_SCAN_FEATS / 32; i += 256) bits[i] = 0u;
+    for (int i = tid; i < PN_SCAN_FEATS / 32; i += T) bits[i] = 0u;
     __syncthreads();
 #pragma unroll 4
-    for (uint32_t i = tid; i < sc.n; i += 256) {
+    for (uint32_t i = tid; i < sc.n; i += T) {
         const float* p = scan_pts + 3 * (sc.offset + i);
         const float px = p[0], py = p[1], pz = p[2];
         const float wx = cy * px - sy * py, wy = sy * px + cy * py;
@@ -277,7 +280,7 @@ __global__ void __launch_bounds__(256)
     const PnMap m = maps[s.map];
     uint4* const row = reinterpret_cast<uint4*>(X + (size_t)b * F);
     const uint32_t one = 0x3F80u;  // 1 in bf16
-    for (int q = tid; q < F / 8; q += 256) {
+    for (int q = tid; q < F / 8; q += T) {
         uint32_t h[4] = {0u, 0u, 0u, 0u};
         if (q < PN_SCAN_FEATS / 8) {
             const uint32_t c = bits[q >> 2] >> (8 * (q & 3));
@@ -395,7 +398,7 @@ struct PnLayer {
 
 struct ndt_pnet {
     ndt_pnet_config cfg{};
-    int device = 0;
+    int device = 0, num_sms = 0;
     cudaStream_t stream = nullptr;
     std::vector<PnLayer> L;
     // batch buffers (capacity cap_b samples)
@@ -435,13 +438,20 @@ static uint64_t host_sm64(uint64_t& s) {
     return z ^ (z >> 31);
 }
 
-// Host arrays go to and from the device through two pinned halves of PN_STAGE bytes: while the
-// copy engine works on one half, host threads copy the other. Copies from and to pageable memory
-// run on one host thread inside the driver: 256 scans of 3,200 points 829 us, 76 MB of parameters
-// into fresh pages 3.2 ms. 4 MB: a half's copy (about 40 us) still outlasts the hand-over of
-// the next half to the threads.
+// Short host arrays go to the device through two pinned halves of PN_STAGE bytes: while the copy
+// engine works on one half, host threads fill the other. A copy from pageable memory costs the
+// host 5 us and more (256 scans of 3,200 points 829 us). Long ones are faster as they lie: the
+// device reads pageable memory of this host at about 130 GB/s (four scans of 1M points 0.67 ms,
+// staged 1.21; eight of 100k points 304 us, staged 390; 160 of 20k 2.35 ms, staged 0.84). Parameters
+// come out through the halves, too: 76 MB into fresh pages took the driver 3.2 ms. 4 MB: a half's
+// copy (about 40 us) still outlasts the hand-over of the next half to the threads.
 constexpr size_t PN_STAGE = 4u << 20;
 constexpr size_t PN_PIECE = 128u << 10;  // bytes a host thread copies at a time
+// A part of a half of at most this size is filled by the calling thread alone: 2 scans of 1,000
+// points 106 us, with the threads 136; 48 (576 KB) 202 and 222; 24 of 3,200 points (922 KB) 194
+// and 191.
+constexpr size_t PN_ALONE = 768u << 10;
+constexpr uint64_t PN_LONG = 768u << 10;  // host arrays from this size on are copied as they lie
 
 // a list of host ranges that lie one after the other on the device
 struct PnRange {
@@ -449,35 +459,44 @@ struct PnRange {
     uint64_t at, bytes;  // place in the concatenation
 };
 
-// Copies the ranges (in order of `at`, no gaps, `total` bytes) to `dev` on the network's stream;
-// the caller synchronises before its arrays may change.
-static int pn_stage_in(ndt_pnet* p, const std::vector<PnRange>& r, uint64_t total, char* dev) {
+// Copies the ranges (in order of `at`, no gaps) to `dev` on the network's stream; the caller
+// synchronises before its arrays may change.
+static int pn_stage_in(ndt_pnet* p, const std::vector<PnRange>& r, char* dev) {
     int rc = pin_reserve(p->h_stage, 2 * PN_STAGE);
     if (rc) return rc;
-    size_t first = 0;  // first range that reaches into the half
-    for (uint64_t o = 0, k = 0; o < total; o += PN_STAGE, ++k) {
-        const uint64_t end = std::min<uint64_t>(o + PN_STAGE, total);
-        char* const half = (char*)p->h_stage.p + (k & 1) * PN_STAGE;
-        if (k >= 2 && (rc = cuda_fail(cudaEventSynchronize(p->ev_half[k & 1]), "staging")))
-            return rc;
-        while (r[first].at + r[first].bytes <= o) ++first;
-        size_t last = first;
-        while (last < r.size() && r[last].at < end) ++last;
-        if (last - first == 1) {  // one long range: by pieces
-            const char* const src = r[first].host + (o - r[first].at);
-            p->pool.run((end - o + PN_PIECE - 1) / PN_PIECE, [&](uint64_t i) {
-                const uint64_t b = i * PN_PIECE, n = std::min<uint64_t>(PN_PIECE, end - o - b);
-                std::memcpy(half + b, src + b, n);
-            });
-        } else {
-            p->pool.run(last - first, [&](uint64_t i) {
+    uint64_t k = 0;  // halves filled
+    for (size_t first = 0, stop; first < r.size(); first = stop) {
+        stop = first + 1;
+        if (r[first].bytes >= PN_LONG) {
+            rc = cuda_fail(cudaMemcpyAsync(dev + r[first].at, r[first].host, r[first].bytes,
+                                           cudaMemcpyHostToDevice, p->stream), "upload");
+            if (rc) return rc;
+            continue;
+        }
+        while (stop < r.size() && r[stop].bytes < PN_LONG) ++stop;
+        const uint64_t total = r[stop - 1].at + r[stop - 1].bytes;
+        for (uint64_t o = r[first].at; o < total; o += PN_STAGE, ++k) {
+            const uint64_t end = std::min<uint64_t>(o + PN_STAGE, total);
+            char* const half = (char*)p->h_stage.p + (k & 1) * PN_STAGE;
+            if (k >= 2 && (rc = cuda_fail(cudaEventSynchronize(p->ev_half[k & 1]), "staging")))
+                return rc;
+            while (r[first].at + r[first].bytes <= o) ++first;  // the first that reaches into it
+            size_t last = first;
+            while (last < stop && r[last].at < end) ++last;
+            auto fill = [&](uint64_t i) {
                 const PnRange& q = r[first + i];
                 const uint64_t a = std::max(q.at, o), b = std::min(q.at + q.bytes, end);
                 if (b > a) std::memcpy(half + (a - o), q.host + (a - q.at), b - a);
-            });
+            };
+            if (end - o <= PN_ALONE) {
+                for (uint64_t i = 0; i < last - first; ++i) fill(i);
+            } else {
+                p->pool.run(last - first, fill);
+            }
+            cudaMemcpyAsync(dev + o, half, end - o, cudaMemcpyHostToDevice, p->stream);
+            if ((rc = cuda_fail(cudaEventRecord(p->ev_half[k & 1], p->stream), "staging")))
+                return rc;
         }
-        cudaMemcpyAsync(dev + o, half, end - o, cudaMemcpyHostToDevice, p->stream);
-        if ((rc = cuda_fail(cudaEventRecord(p->ev_half[k & 1], p->stream), "staging"))) return rc;
     }
     return 0;
 }
@@ -516,6 +535,22 @@ static int pn_stage_out(ndt_pnet* p, const std::vector<std::pair<const void*, ui
         });
     }
     return 0;
+}
+
+// A query call's pinned block: one batch's coarse poses, results and samples; every query's range
+struct PnQuery {
+    size_t coarse, poses, logits, smp, sc, bytes;
+};
+static PnQuery pn_query(const ndt_pnet_config& c, uint64_t nq) {
+    const size_t cap = (size_t)std::min<uint64_t>(nq, (uint64_t)c.batch), P = (size_t)c.proposals;
+    PnQuery q;
+    q.coarse = 0;
+    q.poses = q.coarse + cap * 48;
+    q.logits = q.poses + cap * P * 48;
+    q.smp = q.logits + cap * P * 8;
+    q.sc = q.smp + cap * sizeof(PnSample);
+    q.bytes = q.sc + nq * sizeof(PnScan);
+    return q;
 }
 
 static int pn_check(ndt_pnet* p, const char* what) {
@@ -714,9 +749,14 @@ static int pn_loss(ndt_pnet* p, int B) {
 
 // input features of B samples into X[0]
 static int pn_features(ndt_pnet* p, int B, const void* pts, const void* scans) {
-    k_features<<<B, 256, 0, p->stream>>>((const float*)pts, (const PnScan*)scans,
-                                         (const PnSample*)p->smp.p, (const PnMap*)p->maps_d.p,
-                                         p->L[0].in, (__nv_bfloat16*)p->X[0].p);
+    if (B < p->num_sms)
+        k_features<1024><<<B, 1024, 0, p->stream>>>(
+            (const float*)pts, (const PnScan*)scans, (const PnSample*)p->smp.p,
+            (const PnMap*)p->maps_d.p, p->L[0].in, (__nv_bfloat16*)p->X[0].p);
+    else
+        k_features<256><<<B, 256, 0, p->stream>>>(
+            (const float*)pts, (const PnScan*)scans, (const PnSample*)p->smp.p,
+            (const PnMap*)p->maps_d.p, p->L[0].in, (__nv_bfloat16*)p->X[0].p);
     return cuda_fail(cudaGetLastError(), "proposal features");
 }
 
@@ -781,6 +821,7 @@ int ndt_pnet_create(const ndt_pnet_config* cfg, int32_t device, ndt_pnet** out) 
     ndt_pnet* p = new ndt_pnet();
     p->cfg = c;
     p->device = device;
+    cudaDeviceGetAttribute(&p->num_sms, cudaDevAttrMultiProcessorCount, device);
     cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking);
     cudaStreamCreateWithFlags(&p->side, cudaStreamNonBlocking);
     cudaEventCreateWithFlags(&p->ev_fork, cudaEventDisableTiming);
@@ -828,7 +869,10 @@ int ndt_pnet_create(const ndt_pnet_config* cfg, int32_t device, ndt_pnet** out) 
         rc = cuda_fail(cudaStreamSynchronize(p->stream), "proposal network init");
     }
     if (!rc) rc = pn_reserve_batch(p, std::max(c.batch, c.train_batch));
+    // a query call's block and threads: pinning and starting them in the first call took it 160 us
     if (!rc) rc = pin_reserve(p->h_stage, 2 * PN_STAGE);
+    if (!rc) rc = pin_reserve(p->h_query, pn_query(c, std::min<uint64_t>(c.batch, 256)).bytes);
+    if (!rc) p->pool.start();
     if (rc) {
         ndt_pnet_destroy(p);
         return rc;
@@ -1006,14 +1050,11 @@ int ndt_pnet_propose(ndt_pnet* p, int32_t map_id, const ndt_scan* q, uint64_t nq
     cudaSetDevice(p->device);
     const int P = p->cfg.proposals;
     cudaStream_t s = p->stream;
-    // the call's pinned block: one batch's samples, coarse poses, results; every query's range
-    const size_t cap = (size_t)std::min<uint64_t>(nq, (uint64_t)p->cfg.batch);
-    const size_t o_coarse = 0, o_poses = o_coarse + cap * 48, o_logits = o_poses + cap * P * 48,
-                 o_smp = o_logits + cap * P * 8, o_sc = o_smp + cap * sizeof(PnSample);
-    int rc = pin_reserve(p->h_query, o_sc + nq * sizeof(PnScan));
+    const PnQuery at = pn_query(p->cfg, nq);
+    int rc = pin_reserve(p->h_query, at.bytes);
     if (rc) return rc;
     char* const hq = (char*)p->h_query.p;
-    PnScan* const sc = (PnScan*)(hq + o_sc);
+    PnScan* const sc = (PnScan*)(hq + at.sc);
     std::vector<PnRange> ranges(nq);
     uint64_t total = 0;
     for (uint64_t i = 0; i < nq; ++i) {
@@ -1030,15 +1071,15 @@ int ndt_pnet_propose(ndt_pnet* p, int32_t map_id, const ndt_scan* q, uint64_t nq
     if ((rc = pn_upload_data(p)) || (rc = dev_reserve(p->q_pts, total * 12)) ||
         (rc = dev_reserve(p->q_scans, nq * sizeof(PnScan))))
         return rc;
-    if ((rc = pn_stage_in(p, ranges, total * 12, (char*)p->q_pts.p))) {
+    if ((rc = pn_stage_in(p, ranges, (char*)p->q_pts.p))) {
         cudaStreamSynchronize(s);  // what was issued still reads the pinned halves
         return rc;
     }
     cudaMemcpyAsync(p->q_scans.p, sc, nq * sizeof(PnScan), cudaMemcpyHostToDevice, s);
     for (uint64_t b0 = 0; b0 < nq && !rc; b0 += (uint64_t)p->cfg.batch) {
         const int B = (int)std::min<uint64_t>(nq - b0, (uint64_t)p->cfg.batch);
-        PnSample* const smp = (PnSample*)(hq + o_smp);
-        double* const coarse = (double*)(hq + o_coarse);
+        PnSample* const smp = (PnSample*)(hq + at.smp);
+        double* const coarse = (double*)(hq + at.coarse);
         for (int i = 0; i < B; ++i) {
             const double* const ip = q[b0 + i].initial_pose;
             smp[i] = {(uint32_t)(b0 + i), (uint32_t)map_id, (float)ip[0], (float)ip[1],
@@ -1054,13 +1095,13 @@ int ndt_pnet_propose(ndt_pnet* p, int32_t map_id, const ndt_scan* q, uint64_t nq
             (const float*)p->Z[p->L.size() - 1].p, (const PnSample*)p->smp.p,
             (const double*)p->coarse.p, B, P, (double*)p->poses.p, (double*)p->logits.p);
         cudaEventRecord(p->ev1, s);
-        cudaMemcpyAsync(hq + o_poses, p->poses.p, (size_t)B * P * 48, cudaMemcpyDeviceToHost, s);
+        cudaMemcpyAsync(hq + at.poses, p->poses.p, (size_t)B * P * 48, cudaMemcpyDeviceToHost, s);
         if (logits)
-            cudaMemcpyAsync(hq + o_logits, p->logits.p, (size_t)B * P * 8,
+            cudaMemcpyAsync(hq + at.logits, p->logits.p, (size_t)B * P * 8,
                             cudaMemcpyDeviceToHost, s);
         if ((rc = pn_check(p, "proposal inference"))) break;
-        std::memcpy(poses + 6 * P * b0, hq + o_poses, (size_t)B * P * 48);
-        if (logits) std::memcpy(logits + P * b0, hq + o_logits, (size_t)B * P * 8);
+        std::memcpy(poses + 6 * P * b0, hq + at.poses, (size_t)B * P * 48);
+        if (logits) std::memcpy(logits + P * b0, hq + at.logits, (size_t)B * P * 8);
         float ms = 0.f;
         if (cudaEventElapsedTime(&ms, p->ev0, p->ev1) == cudaSuccess)
             p->stats.inference_kernel_ms += ms;
