@@ -857,7 +857,8 @@ constexpr uint32_t FEW_JOBS = 8;
 constexpr uint64_t FEW_POINTS = 1ull << 26;
 constexpr uint64_t FEW_INLINE_POINTS = 32768;
 
-static LaunchShape choose_shape(ndt_ctx* c, uint32_t jobs, uint32_t max_n, uint64_t total) {
+static LaunchShape choose_shape(ndt_ctx* c, uint32_t jobs, uint32_t max_n, uint64_t total,
+                                bool tuned = true) {
     LaunchShape sh{0, 0, 128, 0};
     if (c->forced.cluster > 0) return c->forced;
     const bool ls = c->cfg.use_line_search != 0;
@@ -868,12 +869,11 @@ static LaunchShape choose_shape(ndt_ctx* c, uint32_t jobs, uint32_t max_n, uint6
         if (c->cfg.lanes_per_point > 1 && c->cfg.max_registers <= 0) sh.regcap = 64;
         sh.queue = c->cfg.work_queue;
         sh.npw = c->cfg.lanes_per_point > 1 ? c->cfg.lanes_per_point : 1;
-        sh.stage = c->cfg.stage_points > 0 ? 1 : 0;
         sh.units = queue_units(sh.threads);
         return sh;
     }
     auto it = c->tuned.find({log2_bucket(jobs), log2_bucket(max_n)});
-    if (it != c->tuned.end() && c->cfg.cluster_size <= 0 && c->cfg.threads_per_cta <= 0 &&
+    if (tuned && it != c->tuned.end() && c->cfg.cluster_size <= 0 && c->cfg.threads_per_cta <= 0 &&
         !(it->second.queue > 0 && (ls || c->cfg.work_queue < 0)))
         return it->second;
     sh.threads = c->cfg.threads_per_cta > 0
@@ -1938,34 +1938,41 @@ int ndt_autotune(ndt_ctx* c, const float* d_xyz, const uint64_t* offsets, const 
     int rc = need_target(c);
     if (rc) return rc;
     if (repeats < 1) repeats = 1;
-    uint64_t max_n = 0;
-    for (uint64_t i = 0; i < m; ++i) max_n = std::max(max_n, offsets[i + 1] - offsets[i]);
+    uint64_t max_n = 0, total = 0;
+    for (uint64_t i = 0; i < m; ++i) {
+        max_n = std::max(max_n, offsets[i + 1] - offsets[i]);
+        total += offsets[i + 1] - offsets[i];
+    }
     std::vector<ndt_result> tmp(m);
     ndt_stats saved = c->stats;
     const int Ks[4] = {1, 2, 4, 8};
     const int TC[8][2] = {{128, 128}, {128, 80}, {128, 64}, {256, 128},
                           {256, 80},  {256, 64}, {256, 48}, {512, 128}};
     // work-queue candidates: (threads, registers, points per thread per chunk, lanes sharing
-    // each point's neighbour search, stage_points: no effect)
-    const int QC[14][5] = {{256, 64, 2, 1, 0}, {256, 64, 4, 1, 0}, {256, 64, 8, 1, 0},
-                           {256, 80, 4, 1, 0}, {128, 64, 4, 1, 0}, {512, 128, 2, 1, 0},
-                           {256, 64, 4, 2, 0}, {256, 64, 4, 4, 0}, {256, 64, 8, 4, 0},
-                           {256, 64, 2, 1, 1}, {256, 64, 4, 1, 1}, {256, 64, 8, 1, 1},
-                           {256, 64, 4, 2, 1}, {256, 64, 4, 4, 1}};
+    // each point's neighbour search)
+    const int QC[14][4] = {{256, 64, 2, 1},  {256, 64, 4, 1},  {256, 64, 8, 1}, {256, 80, 4, 1},
+                           {128, 64, 4, 1},  {512, 128, 2, 1}, {256, 64, 4, 2}, {256, 64, 4, 4},
+                           {256, 64, 8, 4},  {256, 80, 1, 1},  {256, 80, 2, 1}, {256, 80, 8, 1},
+                           {256, 80, 16, 1}, {256, 64, 16, 1}};
     const bool graph_sem = c->cfg.semantics != NDT_SEMANTICS_CPU;
     const bool ls = c->cfg.use_line_search != 0;
     std::vector<LaunchShape> cands;
+    // the form that an untuned call takes, first (a tie keeps it): all SMs on a few alignments, or
+    // the work queue with a cluster's partition
+    const bool by_rule = c->cfg.work_queue == 0 && !ls;
+    if (by_rule)
+        cands.push_back(choose_shape(c, (uint32_t)m, (uint32_t)max_n, total, false));
     if (c->cfg.work_queue <= 0 || ls)
         for (int K : Ks)
             for (const auto& tc : TC) cands.push_back(LaunchShape{K, tc[0], tc[1], 0});
     if (c->cfg.work_queue >= 0 && !ls)
-        for (const auto& qc : QC)
-            if (qc[3] == 1 || graph_sem)
-                cands.push_back(LaunchShape{1, qc[0], qc[1], qc[2], qc[3], qc[4], 0,
-                                            queue_units(qc[0])});
+        for (int i = 0; i < (by_rule ? 13 : 14); ++i)
+            if (QC[i][3] == 1 || graph_sem)
+                cands.push_back(LaunchShape{1, QC[i][0], QC[i][1], QC[i][2], QC[i][3], 0,
+                                            queue_units(QC[i][0])});
     LaunchShape best{0, 0, 128, 0};
     double best_ms = 1e300;
-    int tried = 0;
+    int tried = 0, winner = 0;
     for (const LaunchShape& cand : cands) {
         c->forced = cand;
         rc = ndt_align_batch_device(c, d_xyz, offsets, poses, m, tmp.data());  // warm
@@ -1975,22 +1982,28 @@ int ndt_autotune(ndt_ctx* c, const float* d_xyz, const uint64_t* offsets, const 
             rc = ndt_align_batch_device(c, d_xyz, offsets, poses, m, tmp.data());
         if (rc) break;
         double ms = (c->stats.align_kernel_ms - before) / repeats;
-        tried++;
         if (ms < best_ms) {
             best_ms = ms;
             best = c->forced;
+            winner = tried;
         }
+        tried++;
     }
     c->forced = LaunchShape{0, 0, 0, 0};
     c->stats = saved;
     if (rc) return rc;
-    c->tuned[{log2_bucket(m), log2_bucket(max_n)}] = best;
-    out->cluster_size = best.cluster;
+    // where the untuned form wins, the rule stays: it fits every batch of the class
+    if (by_rule && winner == 0)
+        c->tuned.erase({log2_bucket(m), log2_bucket(max_n)});
+    else
+        c->tuned[{log2_bucket(m), log2_bucket(max_n)}] = best;
+    const bool own = best.queue > 0 && best.ranks == 0;  // the work queue's own partition
+    out->cluster_size = best.ranks > 0 ? best.ranks : best.cluster;
     out->threads_per_cta = best.threads;
     out->registers = best.regcap;
-    out->work_queue = best.queue;
-    out->lanes_per_point = best.queue > 0 ? std::max(1, best.npw) : 0;
-    out->stage_points = best.queue > 0 ? best.stage : 0;
+    out->work_queue = own ? best.queue : 0;
+    out->lanes_per_point = own ? std::max(1, best.npw) : 0;
+    out->stage_points = 0;
     out->reserved = 0;
     out->kernel_ms = best_ms;
     out->aligns_per_s = best_ms > 0 ? 1000.0 * (double)m / best_ms : 0.0;

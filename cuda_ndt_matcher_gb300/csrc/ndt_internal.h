@@ -347,7 +347,6 @@ struct LaunchShape {
     int regcap;  // 128 (default); 80, 64, 48: denser residency for 128/256-thread CTAs
     int queue;   // > 0: work-queue kernel, runs of `queue` points per thread (cluster 1)
     int npw;     // work-queue kernel: lanes sharing each point's neighbour search (0, 1: one)
-    int stage;   // the stage_points option (no effect)
     int ranks;   // work-queue and few-alignments kernels: > 0, a cluster's partition (its CTAs)
     int units;   // work-queue kernel: units per chunk
     int few;     // 1: few-alignments kernel (partition: ranks, threads)

@@ -257,8 +257,9 @@ int ndt_align_batch_device(ndt_ctx* ctx, const float* d_xyz, const uint64_t* off
 /* Autotuner for the Newton kernel's launch shape: times the cluster kernel at every
  * (cluster size 1, 2, 4, 8) x (threads per CTA, register cap) candidate and the work-queue
  * kernel at its (threads, registers, points per thread per chunk, lanes per point's neighbour
- * search) candidates (unless the
- * configuration fixes the form, or line search is on) on the given device-resident batch
+ * search) candidates, and the
+ * form that an untuned call takes (unless the configuration fixes the form, or line search is
+ * on), on the given device-resident batch
  * (as ndt_align_batch_device takes it), `repeats` timed runs each, and records the fastest
  * for batches of this size class (log2 of the scan count and of the largest scan). Later
  * calls in that class use it unless the configuration fixes cluster_size /
@@ -269,12 +270,13 @@ typedef struct ndt_tune_result {
     double kernel_ms;              /* Newton kernel time of the winner, per batch */
     double aligns_per_s;           /* batch size / kernel_ms */
     int32_t candidates;
-    int32_t registers;             /* register cap of the winning kernel instance */
+    int32_t registers;             /* register cap of the winner, as max_registers takes it */
     int32_t work_queue;            /* points per thread per chunk of the winner if it is the
-                                      work-queue kernel, else 0 */
+                                      work-queue kernel with its own partition, else 0: then
+                                      cluster_size and threads_per_cta are its partition */
     int32_t lanes_per_point;       /* lanes sharing each point's neighbour search in the
                                       winning work-queue kernel (1, 2, 4), else 0 */
-    int32_t stage_points;          /* stage_points of the winning candidate (no effect) */
+    int32_t stage_points;          /* 0 */
     int32_t reserved;
 } ndt_tune_result;
 int ndt_autotune(ndt_ctx* ctx, const float* d_xyz, const uint64_t* offsets,
