@@ -1101,6 +1101,26 @@ __device__ int cpu_direction(const AlignParams& P, CtlShared& sh, const AlignJob
     return 0;
 }
 
+// The per-iteration record of a traced call, up to the solver's outcome (lane 0, before the step)
+__device__ __noinline__ double* trace_record(const AlignParams& P, const CtlShared& sh,
+                                             uint32_t job, int it) {
+    double* const t = P.trace + ((size_t)job * P.max_iter + it) * TRACE_REC;
+    t[0] = it;
+    t[1] = sh.tot[A_SC];
+    t[2] = sh.tot[NACC];
+    for (int i = 0; i < 6; ++i) {
+        t[3 + i] = sh.pose[i];
+        t[9 + i] = sh.g[i];
+        t[36 + i] = sh.solve.x[i];
+    }
+    int u = 0;
+    for (int i = 0; i < 6; ++i)
+        for (int j = i; j < 6; ++j) t[15 + u++] = sh.H[i * 6 + j];
+    t[42] = sh.solve.path;
+    t[43] = sh.solve.ok;
+    return t;
+}
+
 // CPU path, second half: pose += step x (apply_pose_delta, types.rs:183-200), the oscillation
 // history, the max-iteration exit (best pose). Returns 1 when the alignment is finished.
 __device__ int cpu_step(const AlignParams& P, CtlShared& sh, AlignOut& o, int it,
@@ -1583,20 +1603,7 @@ __global__ void __launch_bounds__(THREADS, 65536 / (THREADS * REGCAP))
                 if (lane == 0) {
                     sh.n_eigen += sh.solve.path;
                     if (P.trace && it < P.max_iter) {  // per-iteration record (opt-in)
-                        t = P.trace + ((size_t)jid * P.max_iter + it) * TRACE_REC;
-                        t[0] = it;
-                        t[1] = sh.tot[A_SC];
-                        t[2] = sh.tot[NACC];
-                        for (int i = 0; i < 6; ++i) {
-                            t[3 + i] = sh.pose[i];
-                            t[9 + i] = sh.g[i];
-                            t[36 + i] = sh.solve.x[i];
-                        }
-                        int u = 0;
-                        for (int i = 0; i < 6; ++i)
-                            for (int j = i; j < 6; ++j) t[15 + u++] = sh.H[i * 6 + j];
-                        t[42] = sh.solve.path;
-                        t[43] = sh.solve.ok;
+                        t = trace_record(P, sh, (uint32_t)jid, it);
                     }
                     int ncorr = (int)sh.tot[NACC];
                     point_iters += n;
@@ -2078,20 +2085,7 @@ __device__ __noinline__ int queue_control(const AlignParams& P, CtlShared& sh, i
     if (lane == 0) {
         sh.n_eigen += sh.solve.path;
         if (P.trace && (int)it < P.max_iter) {
-            t = P.trace + ((size_t)job * P.max_iter + it) * TRACE_REC;
-            t[0] = it;
-            t[1] = sh.tot[A_SC];
-            t[2] = sh.tot[NACC];
-            for (int i = 0; i < 6; ++i) {
-                t[3 + i] = sh.pose[i];
-                t[9 + i] = sh.g[i];
-                t[36 + i] = sh.solve.x[i];
-            }
-            int u = 0;
-            for (int i = 0; i < 6; ++i)
-                for (int j = i; j < 6; ++j) t[15 + u++] = sh.H[i * 6 + j];
-            t[42] = sh.solve.path;
-            t[43] = sh.solve.ok;
+            t = trace_record(P, sh, (uint32_t)job, (int)it);
             t[44] = (double)(c1 - c0);  // state load
             t[45] = (double)(c2 - c1);  // assembly + solve
             t[47] = sh.solve.sweeps;
@@ -2816,10 +2810,22 @@ __device__ __forceinline__ void few_publish(FewJob* fj, const float* fr, uint32_
 template <bool CPU_SEM>
 __device__ __noinline__ int few_control(const AlignParams& P, CtlShared& ctl, FewJob* fj, int job,
                                         int it, uint32_t tag, int lane) {
+    const unsigned long long c0 = clock64();
     finalize_gH(ctl.tot, ctl.Ad, ctl.Bd, ctl.g, ctl.H, lane);
     __syncwarp();
+    const unsigned long long c1 = clock64();
     solve_warp<CPU_SEM>(ctl.H, ctl.g, ctl.solve, lane);
-    if (lane == 0) ctl.n_eigen += ctl.solve.path;
+    double* t = nullptr;
+    if (lane == 0) {
+        ctl.n_eigen += ctl.solve.path;
+        if (P.trace && it < P.max_iter) {
+            t = trace_record(P, ctl, (uint32_t)job, it);
+            t[44] = (double)(c1 - c0);
+            t[45] = (double)(clock64() - c1);
+            t[47] = ctl.solve.sweeps;
+        }
+    }
+    const unsigned long long c2 = clock64();
     const int ncorr = (int)ctl.tot[NACC];
     AlignOut& o = P.out[job];
     int done = 0;
@@ -2838,6 +2844,7 @@ __device__ __noinline__ int few_control(const AlignParams& P, CtlShared& ctl, Fe
     }
     if (!done) frame_first(ctl.pose, CPU_SEM, ctl.fr, ctl.trig, ctl.Ad, lane);
     few_publish(fj, ctl.fr, tag + (uint32_t)(it + 1), done != 0, lane);
+    if (t) t[46] = (double)(clock64() - c2);
     return done;
 }
 

@@ -892,7 +892,7 @@ static LaunchShape choose_shape(ndt_ctx* c, uint32_t jobs, uint32_t max_n, uint6
         c->cfg.max_registers <= 0) {
         // this cluster's partition of the points on another kernel: every lane's f32 sums are
         // the cluster kernel's
-        if (!c->trace && jobs <= (uint32_t)c->num_sms &&
+        if (jobs <= (uint32_t)c->num_sms &&
             total <= (jobs <= FEW_JOBS ? FEW_POINTS : FEW_POINTS_PER_SM * (uint64_t)c->num_sms)) {
             sh.cluster = 1;
             sh.ranks = K;
