@@ -36,7 +36,7 @@ EXPORTS = [
     "ndt_gemm_bf16",
     "ndt_neighbors_query", "ndt_stats_get", "ndt_stats_reset",
     "ndt_profile_enable", "ndt_debug_trace", "ndt_debug_read", "ndt_debug_queue_stall",
-    "ndt_debug_lookback_stall",
+    "ndt_debug_lookback_stall", "ndt_debug_sm_count",
     "ndt_last_error_string",
     "ndt_radix_sort_pairs_u64_u32", "ndt_radix_sort_pairs_u64_u32_static",
     "ndt_detect_segments", "ndt_morton_codes",
@@ -205,6 +205,7 @@ def load(build_if_missing=True):
         "ndt_stats_get": (C.c_int, [P, C.POINTER(Stats)]),
         "ndt_debug_queue_stall": (C.c_int, [P, C.c_uint64, C.c_int32]),
         "ndt_debug_lookback_stall": (C.c_int, [P, C.c_uint64, C.c_int32]),
+        "ndt_debug_sm_count": (C.c_int, [P, C.c_int32]),
         "ndt_stats_reset": (C.c_int, [P]),
         "ndt_profile_enable": (C.c_int, [P, C.c_int]),
         "ndt_debug_trace": (C.c_int, [P, C.c_int]),
@@ -513,6 +514,10 @@ class Context:
         """Test hook: the limit of a map build's waits, and the kind of scan whose first tile
         withholds its sum until this is called with 0."""
         check(self.lib.ndt_debug_lookback_stall(self.h, int(limit_ns), int(withhold)))
+
+    def debug_sm_count(self, sms):
+        """Test hook: the SM count that the rules for launch shapes go by (0: the device's)."""
+        check(self.lib.ndt_debug_sm_count(self.h, int(sms)))
 
     def trace(self, enable=True):
         check(self.lib.ndt_debug_trace(self.h, 1 if enable else 0))

@@ -147,6 +147,7 @@ struct ndt_ctx {
     DevBuf d_qjobs, d_qctl, d_qframe, d_qpart;          // work-queue kernel
     DevBuf d_few;                                       // few-alignments kernel's exchange words,
     uint32_t few_tag = 0;                               // and the last launch's last tag
+    bool no_few = false;  // its CTAs do not fit together here (a part of the SMs): clusters serve
     std::vector<double> h_trace;       // last call's records, by job order
     std::vector<uint32_t> trace_slot;  // job index -> caller's result index
     int trace_iters = 0;
@@ -527,6 +528,20 @@ int ndt_debug_queue_stall(ndt_ctx* c, uint64_t limit_ns, int32_t withhold_next) 
     return NDT_OK;
 }
 
+int ndt_debug_sm_count(ndt_ctx* c, int32_t sms) {
+    if (!c || sms < 0) return NDT_ERR_INVALID_ARGUMENT;
+    int n = sms;
+    if (sms == 0) {
+        const cudaError_t e =
+            cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, c->device);
+        if (e != cudaSuccess) return cuda_fail(e, "device");
+    }
+    c->num_sms = n;
+    c->no_few = false;
+    c->cfg_gen++;  // captured batches bake their shapes in
+    return NDT_OK;
+}
+
 int ndt_debug_lookback_stall(ndt_ctx* c, uint64_t limit_ns, int32_t withhold) {
     if (!c || withhold < 0 || withhold > 4) return NDT_ERR_INVALID_ARGUMENT;
     tiles_settle(c, true);  // a rebuild in the background reads the scratch
@@ -892,7 +907,7 @@ static LaunchShape choose_shape(ndt_ctx* c, uint32_t jobs, uint32_t max_n, uint6
         c->cfg.max_registers <= 0) {
         // this cluster's partition of the points on another kernel: every lane's f32 sums are
         // the cluster kernel's
-        if (jobs <= (uint32_t)c->num_sms &&
+        if (!c->no_few && jobs <= (uint32_t)c->num_sms &&
             total <= (jobs <= FEW_JOBS ? FEW_POINTS : FEW_POINTS_PER_SM * (uint64_t)c->num_sms)) {
             sh.cluster = 1;
             sh.ranks = K;
@@ -926,9 +941,8 @@ static LaunchShape choose_shape(ndt_ctx* c, uint32_t jobs, uint32_t max_n, uint6
 // run_align_finish needs in c->pend. With the work-queue kernel, a planned batch of more than
 // one copy chunk is copied in on c->cstream while the kernel already runs (see k_ndt_queue);
 // otherwise its copies precede the launch on the stream.
-static int run_align_enqueue(ndt_ctx* c, const float* d_pts, std::vector<AlignJob>& jobs,
-                             const std::vector<uint64_t>& n_by_slot,
-                             const StagePlan* plan = nullptr) {
+static int enqueue_batch(ndt_ctx* c, const float* d_pts, std::vector<AlignJob>& jobs,
+                         const std::vector<uint64_t>& n_by_slot, const StagePlan* plan) {
     uint32_t nj = (uint32_t)jobs.size();
     c->pend.active = false;
     if (nj == 0) return NDT_OK;
@@ -1203,6 +1217,19 @@ static int run_align_enqueue(ndt_ctx* c, const float* d_pts, std::vector<AlignJo
     return NDT_OK;
 }
 
+// Where the few-alignments kernel's CTAs cannot all be resident (a context limited to part of the
+// SMs), its launch is refused: the batch, and every later one of this context, takes clusters.
+static int run_align_enqueue(ndt_ctx* c, const float* d_pts, std::vector<AlignJob>& jobs,
+                             const std::vector<uint64_t>& n_by_slot,
+                             const StagePlan* plan = nullptr) {
+    const int rc = enqueue_batch(c, d_pts, jobs, n_by_slot, plan);
+    if (rc != (int)cudaErrorCooperativeLaunchTooLarge || c->no_few) return rc;
+    c->no_few = true;
+    cudaGetLastError();  // (not sticky)
+    const int e = cuda_fail(cudaStreamSynchronize(c->stream), "align");  // copies from the block
+    return e ? e : enqueue_batch(c, d_pts, jobs, n_by_slot, plan);
+}
+
 // Waits for the batch run_align_enqueue put on the stream and writes its results (caller's
 // order) to out.
 static int run_align_finish(ndt_ctx* c, ndt_result* out) {
@@ -1419,6 +1446,8 @@ int ndt_batch_submit(ndt_ctx* c, const ndt_scan* scans, uint64_t m, uint64_t* ti
     x->d1 = c->d1;
     x->d2 = c->d2;
     x->tuned = c->tuned;
+    x->num_sms = c->num_sms;
+    x->no_few = c->no_few;
     x->map.view = c->map.view;
     x->map.info = c->map.info;
     x->map.valid = true;

@@ -467,6 +467,11 @@ int ndt_debug_queue_stall(ndt_ctx* ctx, uint64_t limit_ns, int32_t withhold_next
  * segment starts', 3 the sort by segment size, 4 the ranks of the valid voxels. */
 int ndt_debug_lookback_stall(ndt_ctx* ctx, uint64_t limit_ns, int32_t withhold);
 
+/* Test hook: the SM count that the rules for launch shapes take for the device's (0: the device's
+ * own). With more than it has, the launch that needs all its CTAs resident together is refused,
+ * as on a context limited to part of the SMs, and the call takes the cluster kernel. */
+int ndt_debug_sm_count(ndt_ctx* ctx, int32_t sms);
+
 const char* ndt_last_error_string(void);
 
 /* ---- build-stage primitives on caller device memory (the cuda_ffi roles) ------------ */
