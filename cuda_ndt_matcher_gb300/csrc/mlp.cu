@@ -821,7 +821,7 @@ int ndt_pnet_create(const ndt_pnet_config* cfg, int32_t device, ndt_pnet** out) 
     ndt_pnet* p = new ndt_pnet();
     p->cfg = c;
     p->device = device;
-    cudaDeviceGetAttribute(&p->num_sms, cudaDevAttrMultiProcessorCount, device);
+    p->num_sms = device_sms();
     cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking);
     cudaStreamCreateWithFlags(&p->side, cudaStreamNonBlocking);
     cudaEventCreateWithFlags(&p->ev_fork, cudaEventDisableTiming);

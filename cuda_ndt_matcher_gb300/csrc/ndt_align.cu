@@ -2180,7 +2180,6 @@ constexpr int QCTLS = 2;         // Newton steps a CTA runs at a time
 // 1,300. Four chunks in hand instead of two: 3,104.
 constexpr uint32_t QLATE = 5;
 constexpr int QREADY = 16;        // more than the alignments a CTA can have in hand
-constexpr uint32_t QSTAY = 152;  // CTAs that stay to the end of a batch: one per SM
 
 // A chunk in a CTA's hands
 struct QSlot {
@@ -2362,11 +2361,11 @@ __device__ __forceinline__ bool queue_idle(const AlignParams& P, QShared& q) {
     } else if (now - q.idle_since > P.stall_ns) {
         atomicOr(P.status, ST_QUEUE_STALL);
         return true;
-    } else if (fed && !keeps && !P.qstay && blockIdx.x >= QSTAY &&
+    } else if (fed && !keeps && !P.qstay && blockIdx.x >= P.qkeep &&
                now - q.idle_since > 20000ull) {
-        // near the end of a batch: all but the first QSTAY CTAs leave after 20 us without
-        // work, so a kernel queued on another stream (the next asynchronous batch) can take
-        // their SMs; those that stay serve the remaining iterations
+        // near the end of a batch: all but the first P.qkeep CTAs (one an SM) leave after 20 us
+        // without work, so a kernel queued on another stream (the next asynchronous batch) can
+        // take their SMs; those that stay serve the remaining iterations
         return true;
     }
     return false;

@@ -35,6 +35,14 @@ int cuda_fail(cudaError_t e, const char* what) {
     return (int)e;
 }
 
+int device_sms() {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return 1;
+    return sms;
+}
+
 int dev_reserve(DevBuf& b, size_t bytes) {
     if (bytes <= b.bytes && b.p) return 0;
     if (b.p) cudaFree(b.p);
@@ -199,7 +207,7 @@ static void async_drain(ndt_ctx* c) {
 // Scoring workspace of nj jobs of at most max_n points: partials, and one finished-block
 // counter per job, zero at allocation and left at zero by every launch.
 static int score_reserve(ndt_ctx* c, uint32_t nj, uint32_t max_n) {
-    int rc = dev_reserve(c->d_part, score_part_bytes(nj, max_n));
+    int rc = dev_reserve(c->d_part, score_part_bytes(nj, max_n, c->num_sms));
     if (rc || (size_t)nj * 4 <= c->d_sdone.bytes) return rc;
     if ((rc = dev_reserve(c->d_sdone, (size_t)nj * 4))) return rc;
     return cuda_fail(cudaMemsetAsync(c->d_sdone.p, 0, c->d_sdone.bytes, c->stream),
@@ -982,6 +990,7 @@ static int enqueue_batch(ndt_ctx* c, const float* d_pts, std::vector<AlignJob>& 
     p.jobs = (const AlignJob*)c->d_jobs.p;
     p.out = (AlignOut*)c->d_aout.p;
     p.num_jobs = nj;
+    p.qkeep = (uint32_t)c->num_sms;
     p.max_iter = c->cfg.max_iterations;
     bool cpu = c->cfg.semantics == NDT_SEMANTICS_CPU;
     p.semantics = c->cfg.semantics;
@@ -1152,7 +1161,7 @@ static int enqueue_batch(ndt_ctx* c, const float* d_pts, std::vector<AlignJob>& 
         r = launch_score(c->map.view, d_pts, (const ScoreJob*)((char*)c->d_jobs.p + jb), nj,
                          max_n, (const AlignOut*)c->d_aout.p, c->d_part.p,
                          (uint32_t*)c->d_sdone.p, (ScoreOut*)((char*)c->d_aout.p + ob),
-                         (float)c->d1, (float)c->d2, st);
+                         (float)c->d1, (float)c->d2, c->num_sms, st);
         if (r) return r;
         cudaEventRecordWithFlags(c->ev2, st, evf);
         cudaMemcpyAsync(ho, c->d_aout.p, ob + sob, cudaMemcpyDeviceToHost, st);
@@ -2075,7 +2084,7 @@ int ndt_eval_batch(ndt_ctx* c, const float* xyz, uint64_t n, const double* T34, 
     if ((rc = launch_score(c->map.view, (const float*)c->d_in.p, (const ScoreJob*)c->d_sjobs.p,
                            (uint32_t)m, (uint32_t)n, nullptr, c->d_part.p,
                            (uint32_t*)c->d_sdone.p, (ScoreOut*)c->d_sout.p, (float)c->d1,
-                           (float)c->d2, st)))
+                           (float)c->d2, c->num_sms, st)))
         return rc;
     cudaEventRecord(c->ev1, st);
     cudaMemcpyAsync(c->h_sout.p, c->d_sout.p, sob, cudaMemcpyDeviceToHost, st);

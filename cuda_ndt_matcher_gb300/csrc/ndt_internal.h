@@ -94,6 +94,7 @@ void pin_free(PinBuf& b);
 
 void set_error(const std::string& msg);
 int cuda_fail(cudaError_t e, const char* what);
+int device_sms();  // SMs of the current device
 
 // Device-resident voxel map.
 struct Map {
@@ -252,6 +253,7 @@ struct AlignParams {
     const struct FewCta* few_ctas;  // qgrid CTAs
     uint64_t qunits_total;  // units of one iteration of every alignment (early iterations)
     int32_t qstay;          // idle CTAs stay to the end of the batch
+    uint32_t qkeep;         // CTAs that stay in any case: one per SM
     int32_t qsolo;          // every iteration of every alignment is one chunk, and all points
                             // are resident: CTAs keep their alignments
     uint32_t qgrid;         // CTAs of the launch
@@ -369,11 +371,12 @@ struct ScoreOut {
     uint64_t nvtl_count;
     uint64_t ncorr;
 };
-size_t score_part_bytes(uint32_t num_jobs, uint32_t max_n);
+// sms: the SM count that the launch's shape goes by
+size_t score_part_bytes(uint32_t num_jobs, uint32_t max_n, int sms);
 // part: score_part_bytes; done: one word per job, zero before the launch and after it
 int launch_score(const MapView& map, const float* pts, const ScoreJob* jobs, uint32_t num_jobs,
                  uint32_t max_n, const AlignOut* align_out, void* part, uint32_t* done,
-                 ScoreOut* out, float d1, float d2, cudaStream_t s);
+                 ScoreOut* out, float d1, float d2, int sms, cudaStream_t s);
 int launch_query(const MapView& map, const float* q, size_t n, int max_nb, int32_t* idx,
                  int32_t* cnt, cudaStream_t s);
 

@@ -32,20 +32,20 @@ struct ScorePartial {
 // Points per thread of a launch over `jobs` jobs of at most max_n points: one while the grid
 // is small, so a single scan's points spread over every SM (a 20k-point scan: 157 blocks
 // instead of 10; scoring it is one dependent chain of loads per point, 54 -> 16 us), then
-// doubled, up to 8, while about four blocks per resident slot (152 SMs x 8) remain: the
+// doubled, up to 8, while about four blocks per resident slot (8 an SM) remain: the
 // block's set-up and reduction are then paid once per 8 points (filling the slots once, four
 // and sixteen times measured 70, 64 and 72 us on 64 scans of 2k-40k points).
-static uint32_t score_ppt(uint32_t jobs, uint32_t max_n) {
+static uint32_t score_ppt(uint32_t jobs, uint32_t max_n, int sms) {
     uint32_t ppt = 1;
     while (ppt < SCORE_MAX_PPT &&
            (uint64_t)jobs * (((uint64_t)max_n + ST * 2 * ppt - 1) / (ST * 2 * ppt)) >=
-               4ull * 152 * 8)
+               4ull * 8 * (uint32_t)sms)
         ppt *= 2;
     return ppt;
 }
 
-static uint32_t score_blocks(uint32_t jobs, uint32_t max_n) {
-    const uint32_t per = ST * score_ppt(jobs, max_n);
+static uint32_t score_blocks(uint32_t jobs, uint32_t max_n, int sms) {
+    const uint32_t per = ST * score_ppt(jobs, max_n, sms);
     return std::max<uint32_t>(1u, (uint32_t)(((uint64_t)max_n + per - 1) / per));
 }
 
@@ -263,22 +263,22 @@ __global__ void __launch_bounds__(ST, 8) k_score(MapView m, const float* __restr
     }
 }
 
-size_t score_part_bytes(uint32_t num_jobs, uint32_t max_n) {
-    return (size_t)score_blocks(num_jobs, max_n) * num_jobs * sizeof(ScorePartial);
+size_t score_part_bytes(uint32_t num_jobs, uint32_t max_n, int sms) {
+    return (size_t)score_blocks(num_jobs, max_n, sms) * num_jobs * sizeof(ScorePartial);
 }
 
 int launch_score(const MapView& map, const float* pts, const ScoreJob* jobs, uint32_t num_jobs,
                  uint32_t max_n, const AlignOut* align_out, void* part, uint32_t* done,
-                 ScoreOut* out, float d1, float d2, cudaStream_t s) {
+                 ScoreOut* out, float d1, float d2, int sms, cudaStream_t s) {
     if (num_jobs == 0) return 0;
-    const uint32_t bx = score_blocks(num_jobs, max_n);
+    const uint32_t bx = score_blocks(num_jobs, max_n, sms);
     const uint64_t grid = (uint64_t)bx * num_jobs;
     if (grid > 0x7FFFFFFFull) {
         set_error("score launch: too many points times poses");
         return NDT_ERR_CAPACITY;
     }
     k_score<<<(unsigned)grid, ST, 0, s>>>(map, pts, jobs, align_out, d1, d2, bx,
-                                          ST * score_ppt(num_jobs, max_n), (ScorePartial*)part,
+                                          ST * score_ppt(num_jobs, max_n, sms), (ScorePartial*)part,
                                           done, out);
     return cuda_fail(cudaGetLastError(), "score launch");
 }

@@ -59,12 +59,12 @@ __host__ __device__ constexpr int gb_smem(int bn, int mt, int st) {  // with ali
 //   256 x 256 for a plain store from GB_SQUARE_TILES on: half the operand traffic of 128 x 128.
 //     1024, 512, 36864: 39 and 46; 640, 512, 36864 (96 tiles): 36 and 43; 512, 512, 36864 (64):
 //     35 and 28; 4096^3: 93 (1.47 PFLOP/s) and 119. One CTA to an SM.
-//   128 x 128, two CTAs to an SM, from GB_WIDE_TILES (one per SM) on. 640, 512, 36864: 43, as 128
+//   128 x 128, two CTAs to an SM, from a tile per SM on. 640, 512, 36864: 43, as 128
 //     x 64 50; 512, 36864, 1024: 61 and 77.
 //   128 x 128 with a deep ring for few tiles and a K beyond GB_DEEP_K. 256, 512, 36864: 19.1,
 //     as 128 x 64 21.6.
 //   128 x 64 else: twice the CTAs, half the epilogue. 1024, 512, 512: 6.0, deep 6.7.
-constexpr int GB_SQUARE_TILES = 96, GB_WIDE_TILES = 152, GB_DEEP_K = 2048;
+constexpr int GB_SQUARE_TILES = 96, GB_DEEP_K = 2048;
 constexpr uint64_t GB_WAIT_NS = 1000000000ull;  // bounded waits: 1 s
 constexpr uint32_t GB_NAP_NS = 20000;           // a waiting thread sleeps up to this long a try
 
@@ -654,7 +654,7 @@ int gemm_bf16(GemmOperand A, GemmOperand B, float* D, int M, int N, int K, int l
     auto tiles = [&](int m, int n) {
         return (long long)((M + m - 1) / m) * ((N + n - 1) / n) * splits;
     };
-    const bool wide = tiles(128, 128) >= GB_WIDE_TILES, deep = K / splits > GB_DEEP_K;
+    const bool wide = tiles(128, 128) >= device_sms(), deep = K / splits > GB_DEEP_K;
     if (e.mode == GEMM_EPI_STORE) {
         if (tiles(256, 256) >= GB_SQUARE_TILES)
             return launch_gemm<256, 2, 3, GB_STORE>(A, B, D, M, N, K, ldd, d_err, s, splits, e);
@@ -699,13 +699,10 @@ int gemm_adam(const GemmAdam* w, int count, int k, uint32_t* d_err, cudaStream_t
         }
         p.tiles += (int)t;
     }
-    int dev = 0, sms = 0;
     cudaError_t e = cudaFuncSetAttribute(k_gemm_adam, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          GA_SMEM);
-    if (e == cudaSuccess) e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return cuda_fail(e, "gemm launch");
-    k_gemm_adam<<<std::min(p.tiles, sms), GA_THREADS, GA_SMEM, s>>>(p, d_err);
+    k_gemm_adam<<<std::min(p.tiles, device_sms()), GA_THREADS, GA_SMEM, s>>>(p, d_err);
     return cuda_fail(cudaGetLastError(), "gemm launch");
 }
 

@@ -1141,7 +1141,8 @@ __global__ void __launch_bounds__(BT) k_compact_keys(const float* __restrict__ p
 static void cell_bounds(const float* pts, size_t n, float res, int32_t* mm, cudaStream_t s) {
     k_minmax_init<<<1, 32, 0, s>>>(mm);
     if (n) {
-        unsigned g = (unsigned)std::min<size_t>((n + 4 * BT - 1) / (4 * BT), 152 * 8);
+        unsigned g = (unsigned)std::min<size_t>((n + 4 * BT - 1) / (4 * BT),
+                                                  8 * (size_t)device_sms());
         k_cells_minmax<<<g, BT, 0, s>>>(pts, n, res, exact_inverse(res),
                                         ((uintptr_t)pts & 15u) == 0, mm);
     }
@@ -2182,7 +2183,7 @@ int build_segments(BuildScratch& sc, const float* d_pts, size_t n, const ndt_con
     // of SegSums, well inside its 8 bytes per point
     SegSums* sums = (SegSums*)((char*)sc.tmp.p + oz_bytes);
     const uint32_t wmax = (uint32_t)std::min<size_t>(g.S, g.nf / WARP_SEG_MIN + 1);
-    const unsigned gs = (unsigned)std::min<uint32_t>((wmax + 3) / 4, 152u * 64u);
+    const unsigned gs = (unsigned)std::min<uint32_t>((wmax + 3) / 4, 64u * (uint32_t)device_sms());
     k_segment_sums<<<gs, 128, 0, s>>>(d_pts, vals, (uint32_t*)sc.seg_starts.p, order, kz,
                                       sc.failed, g.S, (uint32_t)g.nf, cfg.resolution,
                                       cfg.min_points_per_voxel, sums);
