@@ -206,8 +206,8 @@ static void async_drain(ndt_ctx* c) {
 
 // Scoring workspace of nj jobs of at most max_n points: partials, and one finished-block
 // counter per job, zero at allocation and left at zero by every launch.
-static int score_reserve(ndt_ctx* c, uint32_t nj, uint32_t max_n) {
-    int rc = dev_reserve(c->d_part, score_part_bytes(nj, max_n, c->num_sms));
+static int score_reserve(ndt_ctx* c, uint32_t nj, uint32_t max_n, uint64_t points) {
+    int rc = dev_reserve(c->d_part, score_part_bytes(nj, max_n, points, c->num_sms));
     if (rc || (size_t)nj * 4 <= c->d_sdone.bytes) return rc;
     if ((rc = dev_reserve(c->d_sdone, (size_t)nj * 4))) return rc;
     return cuda_fail(cudaMemsetAsync(c->d_sdone.p, 0, c->d_sdone.bytes, c->stream),
@@ -957,13 +957,15 @@ static int enqueue_batch(ndt_ctx* c, const float* d_pts, std::vector<AlignJob>& 
     std::stable_sort(jobs.begin(), jobs.end(),
                      [](const AlignJob& a, const AlignJob& b) { return a.n > b.n; });
     uint32_t max_n = jobs.front().n;
+    uint64_t points = 0;
+    for (uint32_t j = 0; j < nj; ++j) points += jobs[j].n;
     int rc;
     size_t jb = nj * sizeof(AlignJob), ob = nj * sizeof(AlignOut), sjb = nj * sizeof(ScoreJob),
            sob = nj * sizeof(ScoreOut);
     // tables in one block each way (a copy costs a small call about 3 us): alignment jobs,
     // scoring jobs and partial-sum offsets in; alignment and scoring results out
     if ((rc = dev_reserve(c->d_jobs, jb + sjb)) || (rc = dev_reserve(c->d_aout, ob + sob)) ||
-        (rc = score_reserve(c, nj, max_n)) || (rc = pin_reserve(c->h_jobs, jb + sjb)) ||
+        (rc = score_reserve(c, nj, max_n, points)) || (rc = pin_reserve(c->h_jobs, jb + sjb)) ||
         (rc = pin_reserve(c->h_aout, ob + sob + 16)))
         return rc;
     AlignJob* hj = nullptr;
@@ -1022,8 +1024,6 @@ static int enqueue_batch(ndt_ctx* c, const float* d_pts, std::vector<AlignJob>& 
         cudaMemsetAsync(c->d_trace.p, 0xFF, tb, st);  // NaN marks iterations not run
         p.trace = (double*)c->d_trace.p;
     }
-    uint64_t points = 0;
-    for (uint32_t j = 0; j < nj; ++j) points += jobs[j].n;
     LaunchShape shape = choose_shape(c, nj, max_n, points);
     // work-queue kernel: chunk counts and partial-sum offsets per alignment (host, in the
     // pinned job block), per-alignment state and the partials (device)
@@ -1159,7 +1159,7 @@ static int enqueue_batch(ndt_ctx* c, const float* d_pts, std::vector<AlignJob>& 
             cudaEventRecordWithFlags(c->ev1, st, evf);
         }
         r = launch_score(c->map.view, d_pts, (const ScoreJob*)((char*)c->d_jobs.p + jb), nj,
-                         max_n, (const AlignOut*)c->d_aout.p, c->d_part.p,
+                         max_n, points, (const AlignOut*)c->d_aout.p, c->d_part.p,
                          (uint32_t*)c->d_sdone.p, (ScoreOut*)((char*)c->d_aout.p + ob),
                          (float)c->d1, (float)c->d2, c->num_sms, st);
         if (r) return r;
@@ -1179,6 +1179,7 @@ static int enqueue_batch(ndt_ctx* c, const float* d_pts, std::vector<AlignJob>& 
             c->map_gen, c->cfg_gen, (uint64_t)(uintptr_t)d_pts, (uint64_t)(uintptr_t)c->d_jobs.p,
             (uint64_t)(uintptr_t)c->d_aout.p, (uint64_t)(uintptr_t)c->d_part.p,
             (uint64_t)(uintptr_t)c->d_sdone.p,
+            score_part_bytes(nj, max_n, points, c->num_sms),
             (uint64_t)(uintptr_t)c->h_jobs.p, (uint64_t)(uintptr_t)c->h_aout.p};
         size_t gi = c->graphs.size();
         for (size_t i = 0; i < c->graphs.size(); ++i)
@@ -2063,7 +2064,7 @@ int ndt_eval_batch(ndt_ctx* c, const float* xyz, uint64_t n, const double* T34, 
     size_t sjb = m * sizeof(ScoreJob), sob = m * sizeof(ScoreOut);
     if ((rc = pin_reserve(c->h_pts, n * 12 + 16)) || (rc = dev_reserve(c->d_in, n * 12 + 16)) ||
         (rc = dev_reserve(c->d_sjobs, sjb)) || (rc = dev_reserve(c->d_sout, sob)) ||
-        (rc = score_reserve(c, (uint32_t)m, (uint32_t)n)) ||
+        (rc = score_reserve(c, (uint32_t)m, (uint32_t)n, m * n)) ||
         (rc = pin_reserve(c->h_sjobs, sjb)) || (rc = pin_reserve(c->h_sout, sob)))
         return rc;
     if (n) std::memcpy(c->h_pts.p, xyz, n * 12);
@@ -2082,7 +2083,7 @@ int ndt_eval_batch(ndt_ctx* c, const float* xyz, uint64_t n, const double* T34, 
     cudaMemcpyAsync(c->d_sjobs.p, hs, sjb, cudaMemcpyHostToDevice, st);
     cudaEventRecord(c->ev0, st);
     if ((rc = launch_score(c->map.view, (const float*)c->d_in.p, (const ScoreJob*)c->d_sjobs.p,
-                           (uint32_t)m, (uint32_t)n, nullptr, c->d_part.p,
+                           (uint32_t)m, (uint32_t)n, m * n, nullptr, c->d_part.p,
                            (uint32_t*)c->d_sdone.p, (ScoreOut*)c->d_sout.p, (float)c->d1,
                            (float)c->d2, c->num_sms, st)))
         return rc;

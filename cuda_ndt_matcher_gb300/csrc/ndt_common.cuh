@@ -245,106 +245,6 @@ __device__ __forceinline__ uint32_t cell_oct_of_sum(const MapView& m, const floa
     return oct;
 }
 
-// Neighbour search of the point q = qh + ql, in rounds. A round tests the cells' voxels in the
-// reference's order (dx outer, dy, dz inner) from where the last round stopped, and lists those
-// within one resolution, at most `room` (and LIST_CAP), in the thread's column of shared
-// memory: list[k * stride] = {q - centroid, record as int bits}. The list carries the
-// difference, so scoring a listed voxel takes one 256-bit load of its inverse covariance
-// instead of three loads on two cache lines: the kernels that search are bound by the lines
-// their loads touch in L1. `state` is what remains to be tested: with the dense index the
-// neighbourhood mask's bits (search_begin), with the hash the next of the 27 cells. Returns the
-// number listed; another round can only find more while search_more(state).
-constexpr int LIST_CAP = 8;
-
-__device__ __forceinline__ uint32_t search_begin(const MapView& m, const int32_t* gc,
-                                                 uint32_t oct, uint32_t& corner) {
-    corner = 0u;
-    return m.grid ? nbhd_mask(m, gc, oct, corner) : 0u;
-}
-
-__device__ __forceinline__ bool search_more(const MapView& m, uint32_t state) {
-    return m.grid ? state != 0u : state < 27u;
-}
-
-__device__ __forceinline__ int search_round(const MapView& m, const uint32_t* off27,
-                                            const int32_t* gc, const float* qh, const float* ql,
-                                            uint32_t& state, uint32_t corner, int room,
-                                            float4* list, int stride) {
-    int cnt = 0;
-    const int cap = min(room, LIST_CAP);
-    auto test = [&](float mx, float my, float mz, int32_t r) {
-        const float e0 = (qh[0] - mx) + ql[0];
-        const float e1 = (qh[1] - my) + ql[1];
-        const float e2 = (qh[2] - mz) + ql[2];
-        if (fmaf(e0, e0, fmaf(e1, e1, e2 * e2)) > m.r2) return;
-        list[cnt * stride] = make_float4(e0, e1, e2, __int_as_float(r));
-        cnt++;
-    };
-    if (m.grid) {
-        // {centroid, record} entries of the mask's cells, NB_BATCH independent loads at a time
-        constexpr int NB_BATCH = 4;
-#pragma unroll 1
-        while (state != 0u && cnt < cap) {
-            float4 e[NB_BATCH];
-            uint32_t rem = state;
-#pragma unroll
-            for (int k = 0; k < NB_BATCH; ++k) {
-                const uint32_t b = (uint32_t)(__ffs(rem) - 1) & 31u;  // 31 when empty
-                e[k] = rem != 0u ? __ldg(m.grid + (corner + off27[b]))
-                                 : make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
-                rem &= rem - 1u;
-            }
-#pragma unroll
-            for (int k = 0; k < NB_BATCH; ++k) {
-                const int32_t r = __float_as_int(e[k].w);
-                if (r < 0 || cnt >= cap) break;
-                state &= state - 1u;
-                test(e[k].x, e[k].y, e[k].z, r);
-            }
-        }
-        return cnt;
-    }
-    const uint32_t bxy = m.bits[0] + m.bits[1];
-    const uint32_t lz0 = (uint32_t)(gc[2] - m.min_cell[2]);
-#pragma unroll 1
-    for (int c9 = (int)state / 3; c9 < 9 && cnt < cap; ++c9) {
-        const int k0 = (int)state - 3 * c9;  // first cell of the column still to test
-        const int dx = c9 / 3 - 1, dy = c9 % 3 - 1;
-        const uint32_t lx = (uint32_t)(gc[0] + dx - m.min_cell[0]);
-        const uint32_t ly = (uint32_t)(gc[1] + dy - m.min_cell[1]);
-        if (!((lx >> m.bits[0]) | (ly >> m.bits[1]))) {
-            const uint32_t kxy = lx | (ly << m.bits[0]);
-            uint4 sv[3];
-            uint32_t key[3], home[3];
-            bool inb[3];
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {  // the column's three home slots, loaded together
-                const uint32_t lz = lz0 + (uint32_t)(k - 1);
-                inb[k] = k >= k0 && (lz >> m.bits[2]) == 0u;
-                key[k] = kxy | (lz << bxy);
-                home[k] = mix32(key[k]) & m.mask;
-                sv[k] = inb[k] ? __ldg(m.slots + home[k]) : make_uint4(0u, 0u, 0u, EMPTY_KEY);
-            }
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                if (cnt >= cap) return cnt;  // state names this cell
-                state = 3u * c9 + k + 1u;
-                if (!inb[k]) continue;
-                uint4 v = sv[k];
-                int32_t r = (int32_t)home[k];
-                if (v.w != key[k]) {
-                    if (v.w == EMPTY_KEY) continue;
-                    r = probe_next(m, key[k], home[k], &v);
-                    if (r < 0) continue;
-                }
-                test(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), r);
-            }
-        }
-        state = 3u * c9 + 3u;
-    }
-    return cnt;
-}
-
 // Offsets in the reference's fixed order (ndt_graph_kernels.cu:29-39): dx outer, dz inner.
 __host__ __device__ __forceinline__ void offset27(int n, int& dx, int& dy, int& dz) {
     dx = n / 9 - 1;

@@ -371,12 +371,12 @@ struct ScoreOut {
     uint64_t nvtl_count;
     uint64_t ncorr;
 };
-// sms: the SM count that the launch's shape goes by
-size_t score_part_bytes(uint32_t num_jobs, uint32_t max_n, int sms);
+// points: of all jobs; sms: the SM count that the launch's shape goes by
+size_t score_part_bytes(uint32_t num_jobs, uint32_t max_n, uint64_t points, int sms);
 // part: score_part_bytes; done: one word per job, zero before the launch and after it
 int launch_score(const MapView& map, const float* pts, const ScoreJob* jobs, uint32_t num_jobs,
-                 uint32_t max_n, const AlignOut* align_out, void* part, uint32_t* done,
-                 ScoreOut* out, float d1, float d2, int sms, cudaStream_t s);
+                 uint32_t max_n, uint64_t points, const AlignOut* align_out, void* part,
+                 uint32_t* done, ScoreOut* out, float d1, float d2, int sms, cudaStream_t s);
 int launch_query(const MapView& map, const float* q, size_t n, int max_nb, int32_t* idx,
                  int32_t* cnt, cudaStream_t s);
 

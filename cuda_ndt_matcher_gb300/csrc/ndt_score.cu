@@ -2,8 +2,8 @@
 //
 // k_score: for each (scan, pose) job, every point is transformed (compensated f32: the
 // transform as hi/lo pairs, so x = q - mean keeps f32 precision), the voxels whose
-// centroid lies within one resolution are found through the 27-cell hash probe (all of
-// them: kiddo's `within` set, src/ndt_cuda/src/voxel_grid/search.rs:90-99), and the block
+// centroid lies within one resolution are found through the neighbourhood masks of the dense
+// index, or the 27-cell hash probe (all of them: kiddo's `within` set, src/ndt_cuda/src/voxel_grid/search.rs:90-99), and the block
 // accumulates
 //   NVTL terms : max over those voxels of -d1 exp(-d2/2 x^T C x), for points with >= 1
 //                voxel (compute_nvtl_simple, src/ndt_cuda/src/scoring/nvtl.rs:211-260);
@@ -19,8 +19,7 @@
 
 namespace ndtgb {
 
-constexpr int ST = 128;  // threads per block
-constexpr uint32_t SCORE_MAX_PPT = 8;
+constexpr int ST = 256;  // threads per block
 
 struct ScorePartial {
     double nvtl_sum;
@@ -29,24 +28,26 @@ struct ScorePartial {
     uint64_t ncorr;
 };
 
-// Points per thread of a launch over `jobs` jobs of at most max_n points: one while the grid
-// is small, so a single scan's points spread over every SM (a 20k-point scan: 157 blocks
-// instead of 10; scoring it is one dependent chain of loads per point, 54 -> 16 us), then
-// doubled, up to 8, while about four blocks per resident slot (8 an SM) remain: the
-// block's set-up and reduction are then paid once per 8 points (filling the slots once, four
-// and sixteen times measured 70, 64 and 72 us on 64 scans of 2k-40k points).
-static uint32_t score_ppt(uint32_t jobs, uint32_t max_n, int sms) {
-    uint32_t ppt = 1;
-    while (ppt < SCORE_MAX_PPT &&
-           (uint64_t)jobs * (((uint64_t)max_n + ST * 2 * ppt - 1) / (ST * 2 * ppt)) >=
-               4ull * 8 * (uint32_t)sms)
-        ppt *= 2;
+// Points per thread of a launch over `jobs` jobs of `points` points in all, at most max_n each. One
+// while they do not fill the GPU, so that a single scan spreads over every SM (scoring a point is
+// one dependent chain of loads); more as they do, which pays the block's set-up and reduction
+// once for several points. By points in all, us at 1, 2, 4, 8 points per thread (a 400 m map with
+// octant masks; calls that evaluate 5,000 or 18,000 points at many poses):
+//     75k 48/49/52/72, 270k 65/55/66/77, 500k 74/63/61/73, 1.1M 103/91/91/91, 1.8M
+//     140/116/116/115, 3.6M 231/192/178/177, 18M 972/744/659/621.
+// Scans of uneven size leave the blocks past their end empty: no more than four in five.
+static uint32_t score_ppt(uint32_t jobs, uint32_t max_n, uint64_t points, int sms) {
+    const uint64_t per_sm = points / (uint64_t)std::max(1, sms);
+    uint32_t ppt = per_sm < 1000 ? 1 : (per_sm < 3000 ? 2 : (per_sm < 26000 ? 4 : 8));
+    auto blocks = [&](uint64_t n) { return (n + ST * (uint64_t)ppt - 1) / (ST * (uint64_t)ppt); };
+    while (ppt < 8 && jobs * blocks(max_n) > 4 * (blocks(points) + jobs)) ppt *= 2;
+    while (jobs * blocks(max_n) > 0x7FFFFFFFull) ppt *= 2;  // (blocks of a launch)
     return ppt;
 }
 
-static uint32_t score_blocks(uint32_t jobs, uint32_t max_n, int sms) {
-    const uint32_t per = ST * score_ppt(jobs, max_n, sms);
-    return std::max<uint32_t>(1u, (uint32_t)(((uint64_t)max_n + per - 1) / per));
+static uint32_t score_blocks(uint32_t max_n, uint32_t ppt) {
+    const uint64_t per = (uint64_t)ST * ppt;
+    return std::max<uint32_t>(1u, (uint32_t)((max_n + per - 1) / per));
 }
 
 // Transform of one job (row-major 3x4, FP64) by the lanes of one warp, as hi/lo f32 pairs: the
@@ -112,31 +113,16 @@ __device__ __forceinline__ void transform_comp(const float* Th, const float* Tl,
     }
 }
 
-// s + e == a + b exactly
-__device__ __forceinline__ void two_sum_f(float a, float b, float& s, float& e) {
-    s = a + b;
-    const float bp = s - a;
-    e = (a - (s - bp)) + (b - bp);
-}
-
-// hi + lo += (oh + ol), both unevaluated f32 pairs
-__device__ __forceinline__ void pair_add(float& hi, float& lo, float oh, float ol) {
-    float e;
-    two_sum_f(hi, oh, hi, e);
-    lo += ol + e;
-}
-
 // One block per `chunk` points of a job (bx blocks per job in the grid; those past the job's
-// end leave at once). A point's voxels are first listed (the radius test, candidates loaded
-// four at a time), then scored: the lanes of a warp stay on one instruction stream. The FP64
-// unit takes 16 cycles per SM for a warp instruction, so a thread's and a block's sums are
-// kept as f32 pairs (TwoSum: 48 bits, against the terms' own 24) and become FP64 once per
-// block. The block that finishes a job last adds its partials in a fixed order: no second
-// launch. `done` counts a job's finished blocks and is back at zero when the launch ends.
-// Bound: dependent loads (mask, candidates, records) and instruction issue. One 20k-point scan
-// 54 -> 16 us, 20k points at 100 poses 132 -> 112 us, 64 scans of 2k-40k 92 -> 62 us, 256 x
-// 20k points 266 -> 261 us.
-__global__ void __launch_bounds__(ST, 8) k_score(MapView m, const float* __restrict__ pts,
+// end leave at once). A voxel is scored as it passes the radius test; sums are FP64. The block
+// that finishes a job last adds its partials in a fixed order: no second launch. `done` counts
+// a job's finished blocks and is back at zero when the launch ends.
+// Bound: dependent loads (mask, candidates, records) hidden by 48 warps an SM at 40 registers, and
+// instruction issue. Listing a point's voxels first and scoring them in a second loop was
+// slower wherever the GPU is full (128 threads, 64 registers: 18M point-poses 775 us for 621; 200
+// scans of 5k points 94 for 64) and no faster elsewhere. Kernel: one 20k-point scan 52 -> 16 us,
+// 18k points at 100 poses 101 -> 81, 64 scans of 2k-18k 68 -> 49, 256 x 18k 203 -> 186.
+__global__ void __launch_bounds__(ST, 6) k_score(MapView m, const float* __restrict__ pts,
                                                  const ScoreJob* __restrict__ jobs,
                                                  const AlignOut* __restrict__ aout, float d1,
                                                  float d2, uint32_t bx, uint32_t chunk,
@@ -145,10 +131,9 @@ __global__ void __launch_bounds__(ST, 8) k_score(MapView m, const float* __restr
                                                  ScoreOut* __restrict__ out) {
     __shared__ float Th[12], Tl[12];
     __shared__ double trig[6];
-    __shared__ float red[ST / 32][4];
+    __shared__ double red[ST / 32][2];
     __shared__ uint32_t redc[ST / 32][2];
-    __shared__ uint32_t s_off[32];            // neighbour offsets of the dense index
-    __shared__ float4 s_list[LIST_CAP][ST];   // listed voxels per thread
+    __shared__ uint32_t s_off[32];  // neighbour offsets of the dense index
     __shared__ bool s_last;
     const uint32_t j = blockIdx.x / bx, blk = blockIdx.x % bx;
     const ScoreJob& job = jobs[j];
@@ -158,11 +143,10 @@ __global__ void __launch_bounds__(ST, 8) k_score(MapView m, const float* __restr
     nbhd_offsets(m, s_off);
     if (warp == 0) job_transform(job, aout, trig, Th, Tl, lane);
     __syncthreads();
-    float nvh = 0.f, nvl = 0.f, sch = 0.f, scl = 0.f;
-    uint32_t nvc = 0, nc = 0;
+    double nv = 0.0, sc = 0.0;
+    uint32_t nvc = 0, nc = 0;  // (at most 27 pairs a point, and fewer than 2^27 points a block)
     const float* P = pts + 3 * job.offset;
     const uint32_t first = blk * chunk, last = min(n, first + chunk);
-    float4* const list = &s_list[0][threadIdx.x];
     for (uint32_t i = first + threadIdx.x; i < last; i += ST) {
         float px = __ldg(P + 3 * (size_t)i), py = __ldg(P + 3 * (size_t)i + 1),
               pz = __ldg(P + 3 * (size_t)i + 2);
@@ -171,64 +155,75 @@ __global__ void __launch_bounds__(ST, 8) k_score(MapView m, const float* __restr
         transform_comp(Th, Tl, px, py, pz, qh, ql);
         int32_t gc[3];
         const uint32_t oct = cell_oct_of_sum(m, qh, ql, gc);
-        uint32_t corner;
-        uint32_t state = search_begin(m, gc, oct, corner);
         int total = 0;
         float best = -INFINITY, sum = 0.f;
-        do {
-            const int cnt = search_round(m, s_off, gc, qh, ql, state, corner, MAX_NB_ALL, list, ST);
-            total += cnt;
+        // one voxel with centroid (mx, my, mz) in record r: radius test, then its score term
+        auto visit = [&](float mx, float my, float mz, int32_t r) {
+            const float x0 = (qh[0] - mx) + ql[0], x1 = (qh[1] - my) + ql[1],
+                        x2 = (qh[2] - mz) + ql[2];
+            if (fmaf(x0, x0, fmaf(x1, x1, x2 * x2)) > m.r2) return;
+            float C[6];
+            load_icov(m, (uint32_t)r, C);
+            const float c0 = fmaf(C[0], x0, fmaf(C[1], x1, C[2] * x2));
+            const float c1 = fmaf(C[1], x0, fmaf(C[3], x1, C[4] * x2));
+            const float c2 = fmaf(C[2], x0, fmaf(C[4], x1, C[5] * x2));
+            const float md = fmaf(x0, c0, fmaf(x1, c1, x2 * c2));
+            const float s0 = -d1 * expf(-d2 * md * 0.5f);
+            best = fmaxf(best, s0);
+            sum += s0;
+            total++;
+        };
+        if (m.grid) {  // occupied neighbours only, in the same order, from the mask
+            uint32_t corner;
+            uint32_t bits = nbhd_mask(m, gc, oct, corner);
 #pragma unroll 1
-            for (int k = 0; k < cnt; ++k) {
-                const float4 x = list[k * ST];
-                float C[6];
-                load_icov(m, __float_as_uint(x.w), C);
-                const float c0 = fmaf(C[0], x.x, fmaf(C[1], x.y, C[2] * x.z));
-                const float c1 = fmaf(C[1], x.x, fmaf(C[3], x.y, C[4] * x.z));
-                const float c2 = fmaf(C[2], x.x, fmaf(C[4], x.y, C[5] * x.z));
-                const float md = fmaf(x.x, c0, fmaf(x.y, c1, x.z * c2));
-                const float s0 = -d1 * expf(-d2 * md * 0.5f);
-                best = fmaxf(best, s0);
-                sum += s0;
+            while (bits != 0u) {
+                const uint32_t b = (uint32_t)(__ffs(bits) - 1);
+                bits &= bits - 1u;
+                const float4 e = __ldg(m.grid + (corner + s_off[b]));
+                visit(e.x, e.y, e.z, __float_as_int(e.w));
             }
-        } while (search_more(m, state));
+        } else {
+#pragma unroll 1
+            for (int c = 0; c < 27; ++c) {
+                int dx, dy, dz;
+                offset27(c, dx, dy, dz);
+                float mx, my, mz;
+                const int32_t r = find_cell(m, (int32_t)((uint32_t)gc[0] + (uint32_t)dx),
+                                            (int32_t)((uint32_t)gc[1] + (uint32_t)dy),
+                                            (int32_t)((uint32_t)gc[2] + (uint32_t)dz), &mx, &my,
+                                            &mz);
+                if (r >= 0) visit(mx, my, mz, r);
+            }
+        }
         if (total == 0) continue;
-        float e;
-        two_sum_f(nvh, best, nvh, e);
-        nvl += e;
-        two_sum_f(sch, sum, sch, e);
-        scl += e;
+        nv += (double)best;
+        sc += (double)sum;
         nvc++;
         nc += (uint32_t)total;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-        pair_add(nvh, nvl, __shfl_xor_sync(0xffffffffu, nvh, o),
-                 __shfl_xor_sync(0xffffffffu, nvl, o));
-        pair_add(sch, scl, __shfl_xor_sync(0xffffffffu, sch, o),
-                 __shfl_xor_sync(0xffffffffu, scl, o));
+        nv += __shfl_xor_sync(0xffffffffu, nv, o);
+        sc += __shfl_xor_sync(0xffffffffu, sc, o);
     }
     nvc = __reduce_add_sync(0xffffffffu, nvc);
     nc = __reduce_add_sync(0xffffffffu, nc);
     if (lane == 0) {
-        red[warp][0] = nvh;
-        red[warp][1] = nvl;
-        red[warp][2] = sch;
-        red[warp][3] = scl;
+        red[warp][0] = nv;
+        red[warp][1] = sc;
         redc[warp][0] = nvc;
         redc[warp][1] = nc;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
         for (int w = 1; w < ST / 32; ++w) {
-            pair_add(nvh, nvl, red[w][0], red[w][1]);
-            pair_add(sch, scl, red[w][2], red[w][3]);
+            nv += red[w][0];
+            sc += red[w][1];
             nvc += redc[w][0];
             nc += redc[w][1];
         }
-        // an infinite sum has no low part
-        const ScorePartial p{(double)nvh + (isfinite(nvh) ? (double)nvl : 0.0),
-                             (double)sch + (isfinite(sch) ? (double)scl : 0.0), nvc, nc};
+        const ScorePartial p{nv, sc, nvc, nc};
         if (nblk == 1u) {
             out[j] = ScoreOut{p.nvtl_sum, p.score_sum, p.nvtl_count, p.ncorr};
             s_last = false;
@@ -263,23 +258,18 @@ __global__ void __launch_bounds__(ST, 8) k_score(MapView m, const float* __restr
     }
 }
 
-size_t score_part_bytes(uint32_t num_jobs, uint32_t max_n, int sms) {
-    return (size_t)score_blocks(num_jobs, max_n, sms) * num_jobs * sizeof(ScorePartial);
+size_t score_part_bytes(uint32_t num_jobs, uint32_t max_n, uint64_t points, int sms) {
+    return (size_t)score_blocks(max_n, score_ppt(num_jobs, max_n, points, sms)) * num_jobs *
+           sizeof(ScorePartial);
 }
 
 int launch_score(const MapView& map, const float* pts, const ScoreJob* jobs, uint32_t num_jobs,
-                 uint32_t max_n, const AlignOut* align_out, void* part, uint32_t* done,
-                 ScoreOut* out, float d1, float d2, int sms, cudaStream_t s) {
+                 uint32_t max_n, uint64_t points, const AlignOut* align_out, void* part,
+                 uint32_t* done, ScoreOut* out, float d1, float d2, int sms, cudaStream_t s) {
     if (num_jobs == 0) return 0;
-    const uint32_t bx = score_blocks(num_jobs, max_n, sms);
-    const uint64_t grid = (uint64_t)bx * num_jobs;
-    if (grid > 0x7FFFFFFFull) {
-        set_error("score launch: too many points times poses");
-        return NDT_ERR_CAPACITY;
-    }
-    k_score<<<(unsigned)grid, ST, 0, s>>>(map, pts, jobs, align_out, d1, d2, bx,
-                                          ST * score_ppt(num_jobs, max_n, sms), (ScorePartial*)part,
-                                          done, out);
+    const uint32_t ppt = score_ppt(num_jobs, max_n, points, sms), bx = score_blocks(max_n, ppt);
+    k_score<<<bx * num_jobs, ST, 0, s>>>(map, pts, jobs, align_out, d1, d2, bx, ST * ppt,
+                                         (ScorePartial*)part, done, out);
     return cuda_fail(cudaGetLastError(), "score launch");
 }
 
