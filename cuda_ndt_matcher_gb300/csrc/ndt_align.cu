@@ -2173,12 +2173,6 @@ __device__ __noinline__ int queue_control(const AlignParams& P, CtlShared& sh, i
 constexpr int QT = 256;          // threads per CTA
 constexpr int QSLOTS = 2;        // chunks a CTA has in hand
 constexpr int QCTLS = 2;         // Newton steps a CTA runs at a time
-// From the iteration QLATE on (the lowest to claim) a CTA with a chunk in hand or a step to run
-// claims nothing: late in a batch there are free CTAs, and a chunk claimed by a busy one waits for
-// warps. 256 scans of 20k points, up to 30 iterations: 3,396 us without the rule, 3,051 with it
-// (from 3 on 3,108, from 6 on 3,066; only CTAs with a step 3,227); up to 5 iterations 1,312 and
-// 1,300. Four chunks in hand instead of two: 3,104.
-constexpr uint32_t QLATE = 5;
 constexpr int QREADY = 16;        // more than the alignments a CTA can have in hand
 
 // A chunk in a CTA's hands
@@ -2268,29 +2262,37 @@ __device__ __forceinline__ int queue_claim(const AlignParams& P, QShared& q, int
         if (arrived >= P.qarrive_total) arrived = 0xFFFFFFFFu;
     }
     // whether alignment j has a chunk to claim; open: not finished; g: its iteration
-    // (saturated at 255)
-    auto claimable = [&](uint32_t j, bool& open, uint32_t& g) -> bool {
+    // (saturated at 255); left: its chunks to claim
+    auto claimable = [&](uint32_t j, bool& open, uint32_t& g, uint32_t& left) -> bool {
         const unsigned long long w = ld_volatile(&P.qjobs[j].gen_claim);
         open = qw_gen(w) != QDONE;
         g = min(qw_gen(w), 255u);
         bool ok = open && (uint32_t)w < qw_nch(w);
+        left = ok ? qw_nch(w) - (uint32_t)w : 0u;
         if (ok && arrived != 0xFFFFFFFFu && qw_gen(w) == 0u)
             ok = P.jobs[j].offset + P.jobs[j].n <= (uint64_t)arrived;
         return ok;
     };
     uint32_t best = 0xFFFFFFFFu;  // min over claimable j of min(iteration, 255) << 24 | j
+    uint32_t unclaimed = 0u;
 #pragma unroll 4
     for (uint32_t base = (uint32_t)q.lw; base < B; base += 32) {
         const uint32_t j = base + lane;
         bool open = false;
-        uint32_t g = 0;
-        if (j < B && claimable(j, open, g)) best = min(best, (g << 24) | j);
+        uint32_t g = 0, left = 0;
+        if (j < B && claimable(j, open, g, left)) best = min(best, (g << 24) | j);
+        unclaimed += left;
         const unsigned om = __ballot_sync(0xffffffffu, open);
         if (first_open < 0 && om) first_open = (int)base + __ffs(om) - 1;
     }
     best = __reduce_min_sync(0xffffffffu, best);
-    // late in a batch a CTA with a chunk in hand or a step leaves the chunks to the others
-    if (best != 0xFFFFFFFFu && (best >> 24) >= QLATE) {
+    unclaimed = __reduce_add_sync(0xffffffffu, unclaimed);
+    // With fewer chunks to claim than CTAs, one that has a chunk in hand or a step to run leaves them
+    // to the others: at a busy CTA a chunk waits for warps. Without the rule / with it, us: 64 scans
+    // of 18k points 324 and 289, 152 of 18k 588 and 551, 200 of 5k on work_queue = 8 464 and 378;
+    // 256 scans of 20k, up to 30 iterations, 3517 and 3405 (from the fifth iteration on instead:
+    // 3486; on work_queue = 4 4752 and 4226). Busy CTAs never claiming costs full batches 1 to 2%.
+    if (best != 0xFFFFFFFFu && unclaimed < P.qgrid) {
         bool busy = false;
         if (lane == 0) {
             busy = ld_shared_volatile(&q.ctl_busy) != 0u;
@@ -2306,8 +2308,8 @@ __device__ __forceinline__ int queue_claim(const AlignParams& P, QShared& q, int
         for (uint32_t base = start; base < B && job < 0; base += 32) {
             const uint32_t j = base + lane;
             bool ok = false, open = false;
-            uint32_t g = 0;
-            if (j < B) ok = claimable(j, open, g) && (pass == 2 || g == gsel);
+            uint32_t g = 0, left = 0;
+            if (j < B) ok = claimable(j, open, g, left) && (pass == 2 || g == gsel);
             unsigned okm = __ballot_sync(0xffffffffu, ok);
             while (okm != 0u && job < 0) {
                 const int src = __ffs(okm) - 1;
