@@ -1850,7 +1850,6 @@ __device__ __forceinline__ uint32_t qw_nch(unsigned long long w) {
 // each of their iterations over more SMs. The rule depends on the iteration alone, so every
 // run sums an alignment's points over the same tree (results are identical run to run).
 // Chunks hold P.qunits units; at most QMAXCH chunks.
-constexpr uint32_t QSPLIT_ITER = 10, QSPLIT_ITER2 = 20;
 struct QPart {
     uint32_t units, chunks;
     uint32_t runs, size;  // qranks = 0
@@ -2205,6 +2204,8 @@ struct QShared {
     // read by the claiming warp
     unsigned long long ready[QREADY];
     unsigned int ready_put, ready_get;
+    int cur_job;                 // P.qsolo: the alignment being handed out, its iteration, the next
+    uint32_t cur_gen, cur_next, cur_nch;  // chunk and the iteration's chunks (written under claiming)
     // P.qsolo: alignments that this CTA has taken and not finished. Only the claiming warp adds,
     // so while it holds the claim the count can only fall: at zero the CTA has nothing left.
     unsigned int kept;
@@ -2222,8 +2223,8 @@ __device__ __forceinline__ unsigned int ld_shared_volatile(const unsigned int* p
 // first one not known to be finished; pass 1 tries the claimable ones at that iteration in
 // order (from the oldest); if other CTAs took all of their chunks meanwhile, pass 2 takes any
 // claimable chunk, oldest alignment first. Returns the alignment or -1.
-// With P.qsolo (every iteration of every alignment is one chunk, and all points are resident) a
-// CTA keeps an alignment for all its iterations: it claims the ones whose step it has run, else
+// With P.qsolo (many small alignments, all points resident) a CTA keeps an alignment for all its
+// iterations and does all of its chunks: it claims the ones whose step it has run, else
 // the next untouched one from a counter. The scan above reads every open alignment's word for
 // each claim: 9 us a claim with 3,200 alignments (16 x 200 particles of 3,200 points: 8.2 ms, 4.2 ms
 // this way).
@@ -2232,8 +2233,8 @@ __device__ __forceinline__ int queue_claim(const AlignParams& P, QShared& q, int
     const uint32_t B = P.num_jobs;
     int job = -1, first_open = -1;
     if (P.qsolo) {
-        unsigned long long w = 0ull;
-        if (lane == 0) {
+        if (lane == 0 && q.cur_next == q.cur_nch) {  // every chunk of the last one handed out
+            unsigned long long w = 0ull;
             volatile unsigned long long* const e = &q.ready[q.ready_get % QREADY];
             if ((w = *e) != 0ull) {
                 *e = 0ull;
@@ -2247,13 +2248,22 @@ __device__ __forceinline__ int queue_claim(const AlignParams& P, QShared& q, int
                     q.lw = (int)B;
                 }
             }
+            q.cur_job = (int)(uint32_t)w - 1;
+            q.cur_gen = (uint32_t)(w >> 32);
+            q.cur_next = 0;
+            q.cur_nch =
+                q.cur_job < 0 ? 0u : queue_part(P, P.jobs[q.cur_job].n, q.cur_gen).chunks;
         }
-        w = __shfl_sync(0xffffffffu, w, 0);
         __threadfence();
-        chunk = 0;
-        nch = 1;
-        gen = (uint32_t)(w >> 32);
-        return (int)(uint32_t)w - 1;
+        __syncwarp();
+        job = q.cur_nch ? q.cur_job : -1;
+        gen = q.cur_gen;
+        nch = q.cur_nch;
+        chunk = q.cur_next;
+        __syncwarp();
+        if (lane == 0 && job >= 0) q.cur_next = chunk + 1u;
+        __syncwarp();
+        return job;
     }
     // points resident while the batch is still being copied in (all: ~0)
     uint32_t arrived = 0xFFFFFFFFu;
@@ -2448,6 +2458,7 @@ __global__ void __launch_bounds__(QT, 65536 / (QT * REGCAP)) k_ndt_queue(const A
         q.head = 0;
         q.claiming = q.exit_ = q.ctl_busy = 0;
         q.ready_put = q.ready_get = q.kept = 0;
+        q.cur_next = q.cur_nch = 0;
         for (int i = 0; i < QREADY; ++i) q.ready[i] = 0ull;
         q.lw = 0;
         q.idle_since = 0;

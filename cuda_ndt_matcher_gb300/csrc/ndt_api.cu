@@ -879,6 +879,14 @@ constexpr uint64_t FEW_POINTS_PER_SM = 500;
 constexpr uint32_t FEW_JOBS = 8;
 constexpr uint64_t FEW_POINTS = 1ull << 26;
 constexpr uint64_t FEW_INLINE_POINTS = 32768;
+// Work queue: a CTA keeps an alignment to its end where every iteration is one chunk, and for
+// alignments of at most QSOLO_POINTS points (eight a lane of a CTA) from two an SM on: a claim reads
+// every open alignment's word, which cost more than the points (us, as claimed / kept, 5
+// iterations: 700 x 1,100 on work_queue = 8 1062 and 707, on 4 1074 and 720, 3,000 x 1,100 on 2 5116
+// and 2207, 310 x 2,048 on 2 573 and 609). Beyond ten iterations the longest alignments end on one
+// CTA each, hence only from eight an SM on: 450 x 1,500 over 20 1139 and 1748, 1,300 x 2,048 over 30
+// 1864 and 1273.
+constexpr uint32_t QSOLO_POINTS = 2048;
 
 static LaunchShape choose_shape(ndt_ctx* c, uint32_t jobs, uint32_t max_n, uint64_t total,
                                 bool tuned = true) {
@@ -1039,7 +1047,11 @@ static int enqueue_batch(ndt_ctx* c, const float* d_pts, std::vector<AlignJob>& 
         hq = (uint32_t*)((char*)c->h_jobs.p + jb + sjb);
         // partial-sum slots per alignment: its chunk count, at the smallest (last iterations')
         // run size the most an iteration uses, capped at the claim word's 16-bit count
-        const uint32_t small = std::max(1u, chunk / (2 * QSPLIT_DIV));
+        const uint32_t small =
+            p.max_iter <= (int)QSPLIT_ITER
+                ? chunk
+                : std::max(1u, chunk / (p.max_iter <= (int)QSPLIT_ITER2 ? QSPLIT_DIV
+                                                                       : 2 * QSPLIT_DIV));
         uint64_t total = 0, full = 0;
         for (uint32_t j = 0; j < nj; ++j) {
             hq[j] = (uint32_t)total;
@@ -1070,7 +1082,13 @@ static int enqueue_batch(ndt_ctx* c, const float* d_pts, std::vector<AlignJob>& 
         p.qpart_off = (const uint32_t*)((char*)c->d_jobs.p + jb + sjb);
         p.qcount = (uint32_t*)c->d_status.p + 2;  // word 2 of the status block
         p.qunits_total = full;
-        p.qsolo = total == nj && !p.withhold ? 1 : 0;
+        const uint32_t most_jobs =
+            (p.max_iter <= (int)QSPLIT_ITER ? 2u : 8u) * (uint32_t)c->num_sms;
+        p.qsolo = !p.withhold && (total == nj || (nj >= most_jobs && max_n <= QSOLO_POINTS)) ? 1 : 0;
+        // 64 registers there (four CTAs an SM), as in choose_shape
+        if (p.qsolo && c->cfg.work_queue > 0 && c->cfg.max_registers <= 0 && shape.npw <= 1 &&
+            c->forced.cluster <= 0)
+            shape.regcap = 64;
         c->stats.h2d_bytes += qob;
     }
     if (shape.few > 0) {
@@ -1117,9 +1135,9 @@ static int enqueue_batch(ndt_ctx* c, const float* d_pts, std::vector<AlignJob>& 
     uint32_t* hst = (uint32_t*)((char*)c->h_aout.p + ob + sob);
     // host batch copied in during the launch: the kernel reads the resident-point count from
     // word 3 of the status block (32-bit: the batch holds fewer than 2^32 points)
-    // (not where CTAs keep their alignments, which are taken in order: 600 x 1.5k points 1015 us
-    // on clusters, 1335 streamed in)
-    const bool stream_in = plan && shape.queue > 0 && !c->trace && !(shape.ranks && p.qsolo) &&
+    // (not where CTAs keep their alignments: 600 x 1.5k points 1015 us on clusters, 1335 streamed
+    // in)
+    const bool stream_in = plan && shape.queue > 0 && !c->trace && !p.qsolo &&
                            plan->chunk_job.size() > 2 && plan->total < 0xFFFFFFFFull;
     if (plan && !stream_in) stage_plan(c, *plan, jobs, st, nullptr);
     uint32_t* d_arrive = nullptr;
@@ -1132,7 +1150,6 @@ static int enqueue_batch(ndt_ctx* c, const float* d_pts, std::vector<AlignJob>& 
         // leaves SMs to the next one: 256 x 20k points 65.6k against 68.0k aligns/s waiting, two
         // asynchronous batches in flight 83k against 75k
         p.qstay = c->borrowed_map ? 0 : 1;
-        p.qsolo = 0;
     }
     // the batch on the stream: job tables in, Newton kernel, NVTL scoring, results out (the
     // events are graph nodes when captured)

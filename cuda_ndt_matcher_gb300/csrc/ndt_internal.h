@@ -254,8 +254,7 @@ struct AlignParams {
     uint64_t qunits_total;  // units of one iteration of every alignment (early iterations)
     int32_t qstay;          // idle CTAs stay to the end of the batch
     uint32_t qkeep;         // CTAs that stay in any case: one per SM
-    int32_t qsolo;          // every iteration of every alignment is one chunk, and all points
-                            // are resident: CTAs keep their alignments
+    int32_t qsolo;          // many small alignments, all points resident: CTAs keep theirs
     uint32_t qgrid;         // CTAs of the launch
     // points copied in while the work-queue kernel runs: the device word counts the points of
     // the batch resident so far (a prefix of pts, written by the copy stream after each
@@ -298,6 +297,7 @@ constexpr uint32_t QUNITS = 8;        // units (warps' shares) per chunk at most
 // 1/(2 QSPLIT_DIV) in its last ones (the partial-sum slots are sized for those). At the
 // 20k-point bench batch, 2 and 8 were slower as the first split.
 constexpr uint32_t QSPLIT_DIV = 4;
+constexpr uint32_t QSPLIT_ITER = 10, QSPLIT_ITER2 = 20;  // iterations from which runs are shorter
 // Few-alignments kernel, one per alignment (global memory, zero at the start of a launch): the
 // frame of the next iteration and the end mark, as words {value, iteration}; behind all of them
 // the CTAs' sums, the same way.

@@ -43,3 +43,28 @@ def test_no_alignment_is_left_behind(gpu, scans, points):
         C.memset(res, 0xFF, C.sizeof(res))
         shared.align_batch_raw(batches[turn % 2][0], res)
         assert bytes(res) == want[turn % 2], turn
+
+
+@pytest.mark.parametrize("graph", [0, 1])
+@pytest.mark.parametrize("queue,iterations,scans", [(1, 5, 330), (2, 5, 500), (4, 10, 310),
+                                                    (2, 30, 1300)])
+def test_kept_alignments_of_several_chunks(gpu, queue, iterations, scans, graph):
+    """Who sums a chunk does not matter: a batch large enough for its CTAs to keep their alignments
+    gives each scan the result that it gets in a small batch, whose chunks any CTA claims."""
+    w = synth.queue_scans(seed=61, n_scans=8, lo=4000, hi=5000)
+    size = [1 + (371 * i) % 2048 for i in range(scans)]
+    size[0] = 2048
+    cut = [np.ascontiguousarray(w.scans[i % 8][i % 40:i % 40 + n]) for i, n in enumerate(size)]
+    poses = w.true_poses[np.arange(scans) % 8].copy()
+    poses[:, 0] += 0.1
+    ctx = capi.Context(max_iterations=iterations, work_queue=queue, cuda_graph=graph)
+    ctx.set_target(w.map_points)
+    both = []
+    for parts in ([slice(0, scans)], [slice(i, i + 100) for i in range(0, scans, 100)]):
+        got = []
+        for s in parts:
+            got += ctx.align_batch(cut[s], poses[s])
+        both.append(got)
+    for i, (a, b) in enumerate(zip(*both)):
+        for k in ("pose", "score", "hessian", "iterations", "status", "num_correspondences"):
+            assert np.array_equal(a[k], b[k]), (i, size[i], k)
