@@ -1185,8 +1185,13 @@ static int enqueue_batch(ndt_ctx* c, const float* d_pts, std::vector<AlignJob>& 
         cudaMemcpyAsync(hst, c->d_status.p, 4, cudaMemcpyDeviceToHost, st);
         return cuda_fail(cudaGetLastError(), "align enqueue");
     };
-    if (c->cfg.cuda_graph && !c->trace && !stream_in) {
+    // (a withheld launch, the test hook's, is not captured: a replay would withhold again)
+    if (c->cfg.cuda_graph && !c->trace && !stream_in && !p.withhold) {
+        // the work queue's grid goes by the units of all scans up to the resident CTAs (at most
+        // eight an SM)
+        const uint64_t chunks = shape.queue > 0 ? p.qunits_total / (uint64_t)shape.units + 1 : 0;
         const std::vector<uint64_t> key = {
+            std::min<uint64_t>(chunks, 8ull * (uint64_t)c->num_sms), (uint64_t)p.qsolo,
             nj, max_n, (uint64_t)shape.cluster, (uint64_t)shape.threads, (uint64_t)shape.regcap,
             (uint64_t)shape.queue, (uint64_t)shape.npw, (uint64_t)shape.ranks, (uint64_t)shape.units,
             (uint64_t)shape.few, (uint64_t)p.qgrid, (uint64_t)(uintptr_t)c->d_few.p,
