@@ -260,7 +260,7 @@ def scan_array(scans, poses):
     m = len(scans)
     try:
         p = np.asarray(poses)
-    except ValueError:  # rows of different lengths
+    except Exception:  # rows of different lengths; tensors that NumPy does not read as an array
         p = None
     if m and p is not None and p.dtype.kind in "fiu" and p.ndim == 2 and p.shape[1] >= 6 \
             and len(p) >= m:
