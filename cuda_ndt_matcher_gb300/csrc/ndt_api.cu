@@ -933,7 +933,8 @@ static LaunchShape choose_shape(ndt_ctx* c, uint32_t jobs, uint32_t max_n, uint6
         const uint64_t resident = (uint64_t)c->num_sms * (512 / sh.threads);  // CTAs of a wave
         const uint64_t quarters = 4 * (uint64_t)jobs * K / resident;         // of waves
         if ((sh.threads == 512 || (sh.threads == 256 && K == 1)) &&
-            quarters >= (uint64_t)std::max(7, c->cfg.max_iterations + 1)) {
+            quarters >= std::max<uint64_t>(7, (uint64_t)c->cfg.max_iterations + 1) &&
+            (uint64_t)c->cfg.max_iterations < QDONE) {
             sh.cluster = 1;
             sh.ranks = K;
             sh.queue = 1;
