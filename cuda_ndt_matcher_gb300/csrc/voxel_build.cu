@@ -2409,7 +2409,9 @@ int merge_tiles(Map& map, BuildScratch& sc, const std::vector<TileSegRef>& refs,
         set_error("Target point cloud is empty");
         return NDT_ERR_EMPTY_INPUT;
     }
-    if (total >= SP_MAX_PAIRS) {
+    // (the sort indexes with 32 bits, a tile past the end included; the 64-bit keys of builds from
+    // SP_MAX_PAIRS points on are a matter of speed)
+    if (total >= 0xFFFFFFFFull - TILE) {
         set_error("too many occupied cells in the tiles");
         return NDT_ERR_CAPACITY;
     }
