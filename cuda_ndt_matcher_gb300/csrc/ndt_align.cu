@@ -2787,11 +2787,12 @@ __device__ __forceinline__ bool few_wait2(const ulonglong2* p, uint32_t it, ulon
                                           unsigned long long limit_ns) {
     if (few_there(v, it)) return true;
     const unsigned long long t0 = global_ns();
-    do {
+    for (;;) {  // (the time before the words: a context that was paused finds what has arrived)
+        const bool late = global_ns() - t0 >= limit_ns;
         v = few_get2(p);
         if (few_there(v, it)) return true;
-    } while (global_ns() - t0 < limit_ns);
-    return false;
+        if (late) return false;
+    }
 }
 
 // The frame of iteration `it` (or, with the last word set, the end) to the alignment's CTAs:
