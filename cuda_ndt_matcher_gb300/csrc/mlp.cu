@@ -51,12 +51,6 @@ __device__ __forceinline__ float gelu(float z) {  // tanh approximation
     const float u = k * (z + 0.044715f * z * z * z);
     return 0.5f * z * (1.f + tanhf(u));
 }
-__device__ __forceinline__ float gelu_grad(float z) {
-    const float k = 0.7978845608f;
-    const float u = k * (z + 0.044715f * z * z * z);
-    const float t = tanhf(u);
-    return 0.5f * (1.f + t) + 0.5f * z * (1.f - t * t) * k * (1.f + 3.f * 0.044715f * z * z);
-}
 __device__ __forceinline__ float wrap_pi(float a) {
     return a - 2.f * PN_PI * floorf((a + PN_PI) / (2.f * PN_PI));
 }

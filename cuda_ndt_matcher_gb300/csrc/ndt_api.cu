@@ -465,17 +465,15 @@ int ndt_ctx_destroy(ndt_ctx* c) {
     if (c->builder.joinable()) c->builder.join();
     for (auto& t : c->tiles) tile_free(t);
     tile_free(c->spare);
-    for (DevBuf* b : {&c->bs_tile.keys_a, &c->bs_tile.keys_b, &c->bs_tile.vals_a,
-                      &c->bs_tile.vals_b, &c->bs_tile.tmp, &c->bs_tile.seg_ids,
+    for (DevBuf* b : {&c->bs_tile.keys_a, &c->bs_tile.vals_a, &c->bs_tile.tmp,
                       &c->bs_tile.seg_starts, &c->bs_tile.seg_valid, &c->bs_tile.seg_rank,
                       &c->bs_tile.seg_rec, &c->bs_tile.small, &c->d_tile_refs})
         dev_free(*b);
     for (DevBuf* b : {&c->map_b.slots, &c->map_b.icov8, &c->map_b.slot_vidx, &c->map_b.grid,
                       &c->map_b.nmask,
                       &c->map_b.vox_coord, &c->map_b.vox_mean, &c->map_b.vox_cov,
-                      &c->map_b.vox_icov, &c->map_b.vox_count, &c->bs_b.keys_a, &c->bs_b.keys_b,
-                      &c->bs_b.vals_a, &c->bs_b.vals_b, &c->bs_b.tmp, &c->bs_b.seg_ids,
-                      &c->bs_b.seg_starts, &c->bs_b.seg_valid, &c->bs_b.seg_rank,
+                      &c->map_b.vox_icov, &c->map_b.vox_count, &c->bs_b.keys_a, &c->bs_b.vals_a,
+                      &c->bs_b.tmp, &c->bs_b.seg_starts, &c->bs_b.seg_valid, &c->bs_b.seg_rank,
                       &c->bs_b.seg_rec, &c->bs_b.small, &c->d_gather, &c->d_status_b})
         dev_free(*b);
     if (c->bstream) cudaStreamDestroy(c->bstream);
@@ -484,15 +482,15 @@ int ndt_ctx_destroy(ndt_ctx* c) {
                       &c->map.nmask,
                       &c->map.vox_coord,
                       &c->map.vox_mean, &c->map.vox_cov, &c->map.vox_icov, &c->map.vox_count,
-                      &c->bs.keys_a, &c->bs.keys_b, &c->bs.vals_a, &c->bs.vals_b, &c->bs.tmp,
-                      &c->bs.seg_ids, &c->bs.seg_starts, &c->bs.seg_valid, &c->bs.seg_rank,
+                      &c->bs.keys_a, &c->bs.vals_a, &c->bs.tmp,
+                      &c->bs.seg_starts, &c->bs.seg_valid, &c->bs.seg_rank,
                       &c->bs.seg_rec, &c->bs.small, &c->d_in, &c->d_jobs, &c->d_aout,
                       &c->d_sjobs, &c->d_sout, &c->d_part, &c->d_sdone, &c->d_status, &c->d_q, &c->d_qidx,
                       &c->d_qcnt, &c->d_trace, &c->d_qjobs, &c->d_qctl, &c->d_qframe,
                       &c->d_qpart, &c->d_few})
         dev_free(*b);
-    for (PinBuf* b : {&c->bs.host, &c->bs_b.host, &c->bs_tile.host, &c->h_pts, &c->h_jobs, &c->h_aout, &c->h_sjobs, &c->h_sout, &c->h_misc,
-                      &c->h_arrive})
+    for (PinBuf* b : {&c->bs.host, &c->bs_b.host, &c->bs_tile.host, &c->h_pts, &c->h_jobs,
+                      &c->h_aout, &c->h_sjobs, &c->h_sout, &c->h_misc, &c->h_arrive})
         pin_free(*b);
     for (cudaEvent_t ev : {c->ev0, c->ev1, c->ev2, c->ev3, c->ev_in0, c->ev_in1})
         if (ev) cudaEventDestroy(ev);

@@ -109,8 +109,8 @@ struct Map {
 // Scratch used while building a map (kept for the next rebuild).
 constexpr unsigned long long LB_LIMIT_NS = 1000000000ull;  // look-back waits of a build: 1 s
 struct BuildScratch {
-    DevBuf keys_a, keys_b, vals_a, vals_b, tmp;
-    DevBuf seg_ids, seg_starts, seg_valid, seg_rank, seg_rec, small;
+    DevBuf keys_a, vals_a, tmp;
+    DevBuf seg_starts, seg_valid, seg_rank, seg_rec, small;
     PinBuf host;  // sizes read back between stages
     uint32_t* failed = nullptr;  // in tmp: a look-back wait of this build ran out; then the voxels
     // test hook: the waits' limit, and the look-back launch whose first tile withholds its word
@@ -121,7 +121,6 @@ struct BuildScratch {
 
 // Temporary-storage sizing of the sort / scan primitives (two-phase convention).
 size_t radix_sort_temp_bytes(size_t n);
-size_t scan_temp_bytes(size_t n);
 int radix_sort_pairs(uint64_t* keys, uint32_t* vals, size_t n, int begin_bit, int end_bit,
                      void* temp, size_t temp_bytes, cudaStream_t s);
 int detect_segments(const uint64_t* sorted, size_t n, uint32_t* seg_ids, uint32_t* seg_starts,

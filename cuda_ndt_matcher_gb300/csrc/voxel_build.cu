@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(BT) k_tile_scan(const uint32_t* __restrict__ i
     }
 }
 
-size_t scan_temp_bytes(size_t n) { return align_up((size_t)ntiles(n) * 4 + 4, 256); }
+static size_t scan_temp_bytes(size_t n) { return align_up((size_t)ntiles(n) * 4 + 4, 256); }
 
 // exclusive scan in -> out (may alias); temp >= scan_temp_bytes(n), 4-byte aligned
 static int exclusive_scan(const uint32_t* in, uint32_t* out, size_t n, void* temp,
@@ -287,13 +287,12 @@ static int exclusive_scan_zeroed(const uint32_t* in, uint32_t* out, size_t n, co
 }
 
 // ---------------------------------------------------------------------------------------
-// Stable LSD radix sort of (key, u32 value) pairs, 8-bit digits; keys u64 or, when the
-// significant bits fit, u32 (half the key traffic per pass).
+// Stable LSD radix sort of (u64 key, u32 value) pairs, 8-bit digits: the standalone form, and the
+// build's from 2^30 points on.
 // ---------------------------------------------------------------------------------------
 // Digit counts of each TILE-key tile: shared-memory atomics into one counter set per warp
 // (keys of one digit then queue only within their warp), summed per digit at the end.
-template <typename K>
-__global__ void __launch_bounds__(BT) k_radix_hist(const K* __restrict__ keys, size_t n,
+__global__ void __launch_bounds__(BT) k_radix_hist(const uint64_t* __restrict__ keys, size_t n,
                                                    int shift, uint32_t dmask,
                                                    uint32_t* __restrict__ hist, uint32_t nb) {
     __shared__ uint32_t h[BT / 32][256];
@@ -302,11 +301,11 @@ __global__ void __launch_bounds__(BT) k_radix_hist(const K* __restrict__ keys, s
     __syncthreads();
     uint32_t* const hw = h[threadIdx.x >> 5];
     const size_t base = (size_t)blockIdx.x * TILE;
-    K kv[ITEMS];
+    uint64_t kv[ITEMS];
 #pragma unroll
     for (int r = 0; r < ITEMS; ++r) {
         const size_t i = base + (size_t)r * BT + threadIdx.x;
-        kv[r] = i < n ? keys[i] : K(0);
+        kv[r] = i < n ? keys[i] : 0ull;
     }
 #pragma unroll
     for (int r = 0; r < ITEMS; ++r)
@@ -340,16 +339,15 @@ __device__ __forceinline__ uint32_t digit_peers(uint32_t d) {
 // the round's same-digit lanes: tile order within each digit, so the sort is stable. Last, the
 // keys leave in that order: the keys of one digit as one contiguous run at base[digit] (the
 // scanned histogram), so the stores coalesce.
-template <typename K>
-__global__ void __launch_bounds__(BT, sizeof(K) == 4 ? 4 : 3) k_radix_scatter(
-    const K* __restrict__ kin, const uint32_t* __restrict__ vin, K* __restrict__ kout,
-    uint32_t* __restrict__ vout, size_t n, int shift, uint32_t dmask,
+__global__ void __launch_bounds__(BT, 3) k_radix_scatter(
+    const uint64_t* __restrict__ kin, const uint32_t* __restrict__ vin,
+    uint64_t* __restrict__ kout, uint32_t* __restrict__ vout, size_t n, int shift, uint32_t dmask,
     const uint32_t* __restrict__ offs, uint32_t nb) {
     constexpr int NWARP = BT / 32;
     constexpr int WROUNDS = TILE / BT;  // rounds of 32 keys per warp
     extern __shared__ __align__(16) unsigned char sc_smem[];
-    K* skey = reinterpret_cast<K*>(sc_smem);
-    uint32_t* sval = reinterpret_cast<uint32_t*>(sc_smem + TILE * sizeof(K));
+    uint64_t* skey = reinterpret_cast<uint64_t*>(sc_smem);
+    uint32_t* sval = reinterpret_cast<uint32_t*>(sc_smem + TILE * sizeof(uint64_t));
     __shared__ uint32_t wpos[NWARP][256];  // per warp: digit counts, then running positions
     __shared__ uint32_t base[256];         // global position of the tile's first key of each digit
     __shared__ uint32_t loff[256];         // tile-local position of the first key of each digit
@@ -361,11 +359,11 @@ __global__ void __launch_bounds__(BT, sizeof(K) == 4 ? 4 : 3) k_radix_scatter(
 #pragma unroll
     for (int w = 0; w < NWARP; ++w) wpos[w][threadIdx.x] = 0;
     __syncthreads();
-    K key[WROUNDS];
+    uint64_t key[WROUNDS];
 #pragma unroll
     for (int r = 0; r < WROUNDS; ++r) {
         const uint32_t li = wbase + (uint32_t)r * 32 + lane;
-        key[r] = li < tn ? kin[tbase + li] : K(0);
+        key[r] = li < tn ? kin[tbase + li] : 0ull;
     }
 #pragma unroll
     for (int r = 0; r < WROUNDS; ++r) {
@@ -411,7 +409,7 @@ __global__ void __launch_bounds__(BT, sizeof(K) == 4 ? 4 : 3) k_radix_scatter(
     }
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < tn; i += BT) {
-        const K k = skey[i];
+        const uint64_t k = skey[i];
         const uint32_t d = (uint32_t)(k >> shift) & dmask;
         const uint32_t pos = base[d] + (i - loff[d]);
         kout[pos] = k;
@@ -419,63 +417,54 @@ __global__ void __launch_bounds__(BT, sizeof(K) == 4 ? 4 : 3) k_radix_scatter(
     }
 }
 
-template <typename K>
-static size_t radix_temp_bytes(size_t n) {
+size_t radix_sort_temp_bytes(size_t n) {
     size_t nb = ntiles(n);
-    return align_up(n * sizeof(K), 256) + align_up(n * 4, 256) + align_up(256 * nb * 4, 256) +
+    return align_up(n * 8, 256) + align_up(n * 4, 256) + align_up(256 * nb * 4, 256) +
            scan_temp_bytes(256 * nb);
 }
 
-size_t radix_sort_temp_bytes(size_t n) { return radix_temp_bytes<uint64_t>(n); }
-
-template <typename K>
-static int radix_sort_t(K* keys, uint32_t* vals, size_t n, int begin_bit, int end_bit,
-                        void* temp, size_t temp_bytes, cudaStream_t s) {
+int radix_sort_pairs(uint64_t* keys, uint32_t* vals, size_t n, int begin_bit, int end_bit,
+                     void* temp, size_t temp_bytes, cudaStream_t s) {
     if (n <= 1 || end_bit <= begin_bit) return 0;
-    if (temp_bytes < radix_temp_bytes<K>(n)) {
+    if (temp_bytes < radix_sort_temp_bytes(n)) {
         set_error("radix sort: temporary storage too small");
         return NDT_ERR_INVALID_ARGUMENT;
     }
     uint32_t nb = ntiles(n);
     char* t = (char*)temp;
-    K* kalt = (K*)t;
-    t += align_up(n * sizeof(K), 256);
+    uint64_t* kalt = (uint64_t*)t;
+    t += align_up(n * sizeof(uint64_t), 256);
     uint32_t* valt = (uint32_t*)t;
     t += align_up(n * 4, 256);
     uint32_t* hist = (uint32_t*)t;
     t += align_up(256 * (size_t)nb * 4, 256);
     void* stemp = t;
-    K* kin = keys;
+    uint64_t* kin = keys;
     uint32_t* vin = vals;
-    K* kout = kalt;
+    uint64_t* kout = kalt;
     uint32_t* vout = valt;
     int passes = 0;
     // the scatter's tile staging may exceed the default dynamic shared-memory limit (set on
     // the current device at every call: a host-side attribute, no allocation)
-    constexpr int smem = TILE * (int)(sizeof(K) + 4);
-    cudaFuncSetAttribute(k_radix_scatter<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    constexpr int smem = TILE * (int)(sizeof(uint64_t) + 4);
+    cudaFuncSetAttribute(k_radix_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     for (int shift = begin_bit; shift < end_bit; shift += 8, ++passes) {
         int width = std::min(8, end_bit - shift);
         uint32_t dmask = (1u << width) - 1u;
-        k_radix_hist<K><<<nb, BT, 0, s>>>(kin, n, shift, dmask, hist, nb);
+        k_radix_hist<<<nb, BT, 0, s>>>(kin, n, shift, dmask, hist, nb);
         int rc = exclusive_scan(hist, hist, 256 * (size_t)nb, stemp, s);
         if (rc) return rc;
-        k_radix_scatter<K><<<nb, BT, smem, s>>>(kin, vin, kout, vout, n, shift, dmask, hist, nb);
+        k_radix_scatter<<<nb, BT, smem, s>>>(kin, vin, kout, vout, n, shift, dmask, hist, nb);
         int e = cuda_fail(cudaGetLastError(), "radix scatter launch");
         if (e) return e;
         std::swap(kin, kout);
         std::swap(vin, vout);
     }
     if (passes & 1) {
-        cudaMemcpyAsync(keys, kin, n * sizeof(K), cudaMemcpyDeviceToDevice, s);
+        cudaMemcpyAsync(keys, kin, n * sizeof(uint64_t), cudaMemcpyDeviceToDevice, s);
         cudaMemcpyAsync(vals, vin, n * 4, cudaMemcpyDeviceToDevice, s);
     }
     return cuda_fail(cudaGetLastError(), "radix sort");
-}
-
-int radix_sort_pairs(uint64_t* keys, uint32_t* vals, size_t n, int begin_bit, int end_bit,
-                     void* temp, size_t temp_bytes, cudaStream_t s) {
-    return radix_sort_t(keys, vals, n, begin_bit, end_bit, temp, temp_bytes, s);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -796,8 +785,8 @@ namespace ndtgb {
 // ---------------------------------------------------------------------------------------
 // Segments of sorted keys.
 // ---------------------------------------------------------------------------------------
-template <typename K>
-__global__ void k_seg_flags(const K* __restrict__ keys, size_t n, uint32_t* __restrict__ flags) {
+__global__ void k_seg_flags(const uint64_t* __restrict__ keys, size_t n,
+                            uint32_t* __restrict__ flags) {
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) flags[i] = (i > 0 && keys[i] != keys[i - 1]) ? 1u : 0u;
 }
@@ -883,10 +872,8 @@ static int segment_starts(const K* sorted, size_t n, uint32_t* seg_starts,
     return cuda_fail(cudaGetLastError(), "segments");
 }
 
-template <typename K>
-static int detect_segments_t(const K* sorted, size_t n, uint32_t* seg_ids, uint32_t* seg_starts,
-                             uint32_t* num_segments, void* temp, size_t temp_bytes,
-                             cudaStream_t s) {
+int detect_segments(const uint64_t* sorted, size_t n, uint32_t* seg_ids, uint32_t* seg_starts,
+                    uint32_t* num_segments, void* temp, size_t temp_bytes, cudaStream_t s) {
     cudaMemsetAsync(num_segments, 0, 4, s);
     if (n == 0) return cuda_fail(cudaGetLastError(), "segments");
     if (temp_bytes < detect_segments_temp_bytes(n)) {
@@ -904,11 +891,6 @@ static int detect_segments_t(const K* sorted, size_t n, uint32_t* seg_ids, uint3
     if (rc) return rc;
     k_seg_finish<<<g, BT, 0, s>>>(flags, ex, n, seg_ids, seg_starts, num_segments);
     return cuda_fail(cudaGetLastError(), "segments");
-}
-
-int detect_segments(const uint64_t* sorted, size_t n, uint32_t* seg_ids, uint32_t* seg_starts,
-                    uint32_t* num_segments, void* temp, size_t temp_bytes, cudaStream_t s) {
-    return detect_segments_t(sorted, n, seg_ids, seg_starts, num_segments, temp, temp_bytes, s);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1022,16 +1004,15 @@ __global__ void k_minmax_init(int32_t* mm) {
 }
 
 // Morton key of each point's cell relative to the minimum cell, all ones for a non-finite
-// point (it sorts last). K = uint32_t when the key's significant bits fit.
-template <typename K>
+// point (it sorts last).
 __global__ void __launch_bounds__(BT) k_morton(const float* __restrict__ pts, size_t n, float res,
                                                const int32_t* __restrict__ mm,
-                                               K* __restrict__ codes,
+                                               uint64_t* __restrict__ codes,
                                                uint32_t* __restrict__ idx) {
     size_t i = (size_t)blockIdx.x * BT + threadIdx.x;
     if (i >= n) return;
     float p[3] = {pts[3 * i], pts[3 * i + 1], pts[3 * i + 2]};
-    K code = ~K(0);
+    uint64_t code = ~0ull;
     if (finite3(p[0], p[1], p[2])) {
         int32_t c[3];
         cell_of(p, res, c);
@@ -1041,7 +1022,7 @@ __global__ void __launch_bounds__(BT) k_morton(const float* __restrict__ pts, si
             int64_t d = (int64_t)c[a] - (int64_t)mm[a];
             q[a] = d > 0x1FFFFF ? 0x1FFFFFu : (uint32_t)d;
         }
-        code = (K)morton3(q[0], q[1], q[2]);
+        code = (uint64_t)morton3(q[0], q[1], q[2]);
     }
     codes[i] = code;
     idx[i] = (uint32_t)i;
@@ -1151,7 +1132,7 @@ static void cell_bounds(const float* pts, size_t n, float res, int32_t* mm, cuda
 int morton_codes(const float* pts, size_t n, float res, uint64_t* codes, uint32_t* idx,
                  int32_t* mm, cudaStream_t s) {
     cell_bounds(pts, n, res, mm, s);
-    if (n) k_morton<uint64_t><<<(unsigned)((n + BT - 1) / BT), BT, 0, s>>>(pts, n, res, mm, codes, idx);
+    if (n) k_morton<<<(unsigned)((n + BT - 1) / BT), BT, 0, s>>>(pts, n, res, mm, codes, idx);
     return cuda_fail(cudaGetLastError(), "morton codes");
 }
 
@@ -2155,8 +2136,8 @@ int build_segments(BuildScratch& sc, const float* d_pts, size_t n, const ndt_con
     } else {
         const uint32_t lv = std::max(bits[0], std::max(bits[1], bits[2]));
         uint64_t* keys = (uint64_t*)sc.keys_a.p;
-        k_morton<uint64_t><<<(unsigned)((n + BT - 1) / BT), BT, 0, s>>>(d_pts, n, cfg.resolution,
-                                                                        mm, keys, vals);
+        k_morton<<<(unsigned)((n + BT - 1) / BT), BT, 0, s>>>(d_pts, n, cfg.resolution, mm, keys,
+                                                              vals);
         if ((rc = radix_sort_pairs(keys, vals, n, 0, std::min(64, (int)(3 * lv + 1)), sc.tmp.p,
                                    tmp, s)) ||
             (rc = segment_starts(keys, g.nf, (uint32_t*)sc.seg_starts.p, nseg,

@@ -98,7 +98,10 @@ typedef struct ndt_config {
                                       of any alignment's iteration); -1 one thread-block
                                       cluster per alignment; 0 autotuned (until tuned, by
                                       the batch's size). Line search always uses the cluster
-                                      kernel. */
+                                      kernel. A large batch holds every SM until it ends: a
+                                      live scan aligned on another context meanwhile waits
+                                      longer than beside a batch on clusters (-1), which takes
+                                      about a quarter longer itself. */
     int32_t lanes_per_point;       /* work-queue kernel, graph semantics, 256 threads at 64
                                       registers: 2 or 4 lanes share each point's neighbour
                                       search (the occupied cells among its 27); 0 or 1: each
