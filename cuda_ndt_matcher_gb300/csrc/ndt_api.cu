@@ -886,8 +886,29 @@ constexpr uint64_t FEW_INLINE_POINTS = 32768;
 // 1864 and 1273.
 constexpr uint32_t QSOLO_POINTS = 2048;
 
+// The same for a cluster's partition of larger alignments (two chunks an iteration): the words that
+// a claim reads grow with the alignments, the points that it hands out with their size. Kernel us
+// on clusters / claimed / kept, a particle search over 5 m and the circle, up to 30 iterations:
+// 40,000 x 5,000 points 295,869 / 1,401,115 / 207,280, 3,200 x 6,500 30,328 / 34,701 / 24,343,
+// 3,200 x 12,000 47,065 / 41,613 / 41,268, 2,400 x 12,000 35,051 / 29,527 / 31,255; scans that are
+// copied in meanwhile (calls): 3,200 x 5,000 15,131 / 13,332 / 12,778, 3,200 x 9,000 21,926 / 16,849
+// / 20,825. Below sixteen an SM the longest alignments end on one CTA each: 1,200 x 5,000 over 30
+// iterations 5,313 / 4,987 / 6,907. And no alignment may be larger than a third of an SM's share.
+static bool queue_keeps(int sms, uint64_t jobs, uint64_t max_n, uint64_t points, bool copied_in) {
+    const uint64_t least = 16ull * (uint64_t)sms;
+    return jobs >= least && points / jobs <= (copied_in ? 2 : 3) * jobs &&
+           max_n <= points / (3ull * (uint64_t)sms);
+}
+
+// Fewer alignments than that, all resident: below this size the claims of one-CTA partitions cost
+// more than the points they hand out (search, calls, clusters / claimed: 1,200 x 4,200 9,819 and
+// 12,175, 1,700 x 6,500 17,100 and 18,243, 1,700 x 9,000 20,942 and 18,884; 5 iterations: 1,000 x
+// 5,000 2,157 and 2,481, 700 x 9,000 2,049 and 1,807). Scans that are copied in while the kernel
+// runs gain from claims at any size (1,000 x 4,200 3,027 and 2,539).
+constexpr uint32_t QCLAIM_POINTS = 8192;
+
 static LaunchShape choose_shape(ndt_ctx* c, uint32_t jobs, uint32_t max_n, uint64_t total,
-                                bool tuned = true) {
+                                bool copied_in, bool tuned = true) {
     LaunchShape sh{0, 0, 128, 0};
     if (c->forced.cluster > 0) return c->forced;
     const bool ls = c->cfg.use_line_search != 0;
@@ -930,7 +951,10 @@ static LaunchShape choose_shape(ndt_ctx* c, uint32_t jobs, uint32_t max_n, uint6
         }
         const uint64_t resident = (uint64_t)c->num_sms * (512 / sh.threads);  // CTAs of a wave
         const uint64_t quarters = 4 * (uint64_t)jobs * K / resident;         // of waves
-        if ((sh.threads == 512 || (sh.threads == 256 && K == 1)) &&
+        const bool claimed = sh.threads == 512 && (K > 1 || copied_in || max_n >= QCLAIM_POINTS ||
+                                                   queue_keeps(c->num_sms, jobs, max_n, total,
+                                                               copied_in));
+        if ((claimed || (sh.threads == 256 && K == 1)) &&
             quarters >= std::max<uint64_t>(7, (uint64_t)c->cfg.max_iterations + 1) &&
             (uint64_t)c->cfg.max_iterations < QDONE) {
             sh.cluster = 1;
@@ -1031,7 +1055,10 @@ static int enqueue_batch(ndt_ctx* c, const float* d_pts, std::vector<AlignJob>& 
         cudaMemsetAsync(c->d_trace.p, 0xFF, tb, st);  // NaN marks iterations not run
         p.trace = (double*)c->d_trace.p;
     }
-    LaunchShape shape = choose_shape(c, nj, max_n, points);
+    // a batch of several copy chunks can be copied in while the work-queue kernel runs (which reads
+    // a 32-bit count of resident points)
+    const bool copied_in = plan && plan->chunk_job.size() > 2 && plan->total < 0xFFFFFFFFull;
+    LaunchShape shape = choose_shape(c, nj, max_n, points, copied_in);
     // work-queue kernel: chunk counts and partial-sum offsets per alignment (host, in the
     // pinned job block), per-alignment state and the partials (device)
     size_t qob = 0;  // bytes behind the two job tables: partial-sum offsets, or the CTA table
@@ -1083,7 +1110,11 @@ static int enqueue_batch(ndt_ctx* c, const float* d_pts, std::vector<AlignJob>& 
         p.qunits_total = full;
         const uint32_t most_jobs =
             (p.max_iter <= (int)QSPLIT_ITER ? 2u : 8u) * (uint32_t)c->num_sms;
-        p.qsolo = !p.withhold && (total == nj || (nj >= most_jobs && max_n <= QSOLO_POINTS)) ? 1 : 0;
+        p.qsolo = !p.withhold && (total == nj || (nj >= most_jobs && max_n <= QSOLO_POINTS) ||
+                                  (shape.ranks > 0 &&
+                                   queue_keeps(c->num_sms, nj, max_n, points, copied_in)))
+                      ? 1
+                      : 0;
         // 64 registers there (four CTAs an SM), as in choose_shape
         if (p.qsolo && c->cfg.work_queue > 0 && c->cfg.max_registers <= 0 && shape.npw <= 1 &&
             c->forced.cluster <= 0)
@@ -1133,11 +1164,10 @@ static int enqueue_batch(ndt_ctx* c, const float* d_pts, std::vector<AlignJob>& 
     AlignOut* ho = (AlignOut*)c->h_aout.p;
     uint32_t* hst = (uint32_t*)((char*)c->h_aout.p + ob + sob);
     // host batch copied in during the launch: the kernel reads the resident-point count from
-    // word 3 of the status block (32-bit: the batch holds fewer than 2^32 points)
+    // word 3 of the status block
     // (not where CTAs keep their alignments: 600 x 1.5k points 1015 us on clusters, 1335 streamed
     // in)
-    const bool stream_in = plan && shape.queue > 0 && !c->trace && !p.qsolo &&
-                           plan->chunk_job.size() > 2 && plan->total < 0xFFFFFFFFull;
+    const bool stream_in = copied_in && shape.queue > 0 && !c->trace && !p.qsolo;
     if (plan && !stream_in) stage_plan(c, *plan, jobs, st, nullptr);
     uint32_t* d_arrive = nullptr;
     if (stream_in) {
@@ -2021,7 +2051,7 @@ int ndt_autotune(ndt_ctx* c, const float* d_xyz, const uint64_t* offsets, const 
     // the work queue with a cluster's partition
     const bool by_rule = c->cfg.work_queue == 0 && !ls;
     if (by_rule)
-        cands.push_back(choose_shape(c, (uint32_t)m, (uint32_t)max_n, total, false));
+        cands.push_back(choose_shape(c, (uint32_t)m, (uint32_t)max_n, total, false, false));
     if (c->cfg.work_queue <= 0 || ls)
         for (int K : Ks)
             for (const auto& tc : TC) cands.push_back(LaunchShape{K, tc[0], tc[1], 0});
