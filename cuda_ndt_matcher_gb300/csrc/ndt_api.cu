@@ -886,14 +886,16 @@ constexpr uint64_t FEW_INLINE_POINTS = 32768;
 // 1864 and 1273.
 constexpr uint32_t QSOLO_POINTS = 2048;
 
-// The same for a cluster's partition of larger alignments (two chunks an iteration): the words that
-// a claim reads grow with the alignments, the points that it hands out with their size. Kernel us
-// on clusters / claimed / kept, a particle search over 5 m and the circle, up to 30 iterations:
-// 40,000 x 5,000 points 295,869 / 1,401,115 / 207,280, 3,200 x 6,500 30,328 / 34,701 / 24,343,
-// 3,200 x 12,000 47,065 / 41,613 / 41,268, 2,400 x 12,000 35,051 / 29,527 / 31,255; scans that are
-// copied in meanwhile (calls): 3,200 x 5,000 15,131 / 13,332 / 12,778, 3,200 x 9,000 21,926 / 16,849
-// / 20,825. Below sixteen an SM the longest alignments end on one CTA each: 1,200 x 5,000 over 30
-// iterations 5,313 / 4,987 / 6,907. And no alignment may be larger than a third of an SM's share.
+// The same for larger alignments: the words that a claim reads grow with the alignments, the
+// points that it hands out with their size. Kernel us on clusters / claimed / kept, a particle
+// search over 5 m and the circle, up to 30 iterations: 40,000 x 5,000 points 295,869 / 1,401,115
+// / 207,280, 3,200 x 6,500 30,328 / 34,701 / 24,343, 3,200 x 12,000 47,065 / 41,613 / 41,268,
+// 2,400 x 12,000 35,051 / 29,527 / 31,255; scans that are copied in meanwhile (calls): 3,200 x
+// 5,000 15,131 / 13,332 / 12,778, 3,200 x 9,000 21,926 / 16,849 / 20,825; in the kernel's own
+// partition (batches' calls, claimed / kept): work_queue = 4 10,000 x 5,000 162,900 / 42,599, 8
+// 3,200 x 3,000 14,668 / 10,541. Below sixteen an SM the longest alignments end on one CTA each:
+// 1,200 x 5,000 over 30 iterations 5,313 / 4,987 / 6,907. And no alignment may be larger than a
+// third of an SM's share.
 static bool queue_keeps(int sms, uint64_t jobs, uint64_t max_n, uint64_t points, bool copied_in) {
     const uint64_t least = 16ull * (uint64_t)sms;
     return jobs >= least && points / jobs <= (copied_in ? 2 : 3) * jobs &&
@@ -1111,13 +1113,16 @@ static int enqueue_batch(ndt_ctx* c, const float* d_pts, std::vector<AlignJob>& 
         const uint32_t most_jobs =
             (p.max_iter <= (int)QSPLIT_ITER ? 2u : 8u) * (uint32_t)c->num_sms;
         p.qsolo = !p.withhold && (total == nj || (nj >= most_jobs && max_n <= QSOLO_POINTS) ||
-                                  (shape.ranks > 0 &&
-                                   queue_keeps(c->num_sms, nj, max_n, points, copied_in)))
+                                  queue_keeps(c->num_sms, nj, max_n, points, copied_in))
                       ? 1
                       : 0;
-        // 64 registers there (four CTAs an SM), as in choose_shape
-        if (p.qsolo && c->cfg.work_queue > 0 && c->cfg.max_registers <= 0 && shape.npw <= 1 &&
-            c->forced.cluster <= 0)
+        // 64 registers there (four CTAs an SM), as in choose_shape, and where claims weigh more than
+        // the spills: six alignments an SM of more points than that (search calls, us, 80 and 64:
+        // 1,200 x 9,000 over 30 iterations on work_queue = 8 25,635 and 22,612, on 4 38,769 and
+        // 32,840; 700 x 3,000 on 8 7,593 and 7,737)
+        const bool many = !cpu && nj >= 6u * (uint32_t)c->num_sms && max_n > QSOLO_POINTS;
+        if ((p.qsolo || many) && c->cfg.work_queue > 0 && c->cfg.max_registers <= 0 &&
+            shape.npw <= 1 && c->forced.cluster <= 0)
             shape.regcap = 64;
         c->stats.h2d_bytes += qob;
     }
